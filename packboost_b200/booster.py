@@ -45,8 +45,8 @@ from . import backends as B
 from .config import PackBoostConfig
 from .forest import validate_forest
 from .sharding import agree_all, block_size, choose_replicated, dealt_part, feature_map, local_part, owned_range
-from .data import (BinningResult, PackedMatrix, PackedRows, code_bits_for, detect_prebinned, pack_feature_major,
-                   pack_feature_major_distributed, pack_row_major, quantile_edges_device)
+from .data import (BinningResult, PackedMatrix, PackedRows, code_bits_for, detect_prebinned, detect_prebinned_tensor,
+                   pack_feature_major, pack_feature_major_distributed, pack_row_major, quantile_edges_device, sort_eras)
 
 # ------------------------------ tree containers ------------------------------
 
@@ -206,7 +206,7 @@ _RING = 4  # staging slots: at most three rounds are in flight (previous, a disc
 class _DeviceTrainer:
     """Owns the device buffers of one fit and launches the round phases."""
 
-    def __init__(self, cfg: PackBoostConfig, matrix: PackedMatrix, y_sorted: np.ndarray, era_offsets: np.ndarray,
+    def __init__(self, cfg: PackBoostConfig, matrix: PackedMatrix, y_sorted: np.ndarray | torch.Tensor, era_offsets: np.ndarray,
                  n_features_total: int, feat_local: np.ndarray, rank: int, world: int,
                  workspace_bytes: int | None = None, replicated: bool = False):
         self.cfg = cfg
@@ -236,7 +236,10 @@ class _DeviceTrainer:
         self.thr_ids = torch.from_numpy(thr).to(self.dev)
         self.era_offsets = torch.from_numpy(np.ascontiguousarray(era_offsets, dtype=np.int32)).to(self.dev)
         self.feat_local = torch.from_numpy(np.ascontiguousarray(feat_local, dtype=np.int32)).to(self.dev)
-        self.y = torch.from_numpy(np.ascontiguousarray(y_sorted, dtype=np.float32)).to(self.dev)
+        if isinstance(y_sorted, torch.Tensor):   # (a copy: the caller may go on writing to its tensor)
+            self.y = torch.empty(n, dtype=torch.float32, device=self.dev).copy_(y_sorted)
+        else:
+            self.y = torch.from_numpy(np.ascontiguousarray(y_sorted, dtype=np.float32)).to(self.dev)
         self.preds = torch.zeros(n, dtype=torch.float32, device=self.dev)
         self.gq = torch.zeros(npad, dtype=torch.int32, device=self.dev)
         self.slot = torch.full((npad,), -1, dtype=torch.int16, device=self.dev)  # 0xFFFF: no slot
@@ -287,8 +290,11 @@ class _DeviceTrainer:
         want = 24 * self.F * stride + per_feat * min(local_sampled, max(matrix.n_features_local, 1)) + (1 << 20)
         min_bytes = int(self.lib.pb_workspace_min_bytes(C.byref(st)))
         if workspace_bytes is None:
-            free, _total = torch.cuda.mem_get_info(self.dev)
-            cap = int(os.getenv("PACKBOOST_WORKSPACE_BYTES", str(min(8 << 30, int(free * 0.6)))))
+            # (the query takes a driver lock, milliseconds at times, and a small workspace needs no cap)
+            cap = os.getenv("PACKBOOST_WORKSPACE_BYTES")
+            if cap is None:
+                cap = min(8 << 30, int(torch.cuda.mem_get_info(self.dev)[0] * 0.6)) if want > 1 << 30 else want
+            cap = int(cap)
             workspace_bytes = max(min_bytes, min(want, cap))
         self.workspace = torch.empty(int(workspace_bytes), dtype=torch.uint8, device=self.dev)
         st.workspace = self.workspace.data_ptr()
@@ -685,7 +691,11 @@ class PackBoost:
         # torch tensors (device-resident, or pinned host memory) are consumed without conversion
         on_device = isinstance(X, torch.Tensor)
         X_np = X.detach() if on_device else np.asarray(X)
-        y_np = np.asarray(y.detach().cpu().numpy() if isinstance(y, torch.Tensor) else y, dtype=np.float32)
+        # (targets that are on the GPU stay there: they are gathered and copied on the device)
+        if isinstance(y, torch.Tensor) and y.is_cuda:
+            y_np = y.detach().to(device=self._device, dtype=torch.float32)
+        else:
+            y_np = np.asarray(y.detach().numpy() if isinstance(y, torch.Tensor) else y, dtype=np.float32)
         if y_np.ndim != 1:
             raise ValueError("y must be 1-D")
         N, F = X_np.shape
@@ -696,35 +706,13 @@ class PackBoost:
             raise ValueError("max_bins must be ≤ 128 when using int8 bin storage")
         if cfg.max_bins > 256:
             raise ValueError("max_bins must be ≤ 256")
-        if era is None:
-            era_encoded = np.zeros(N, dtype=np.int16)
-            uniq = np.array([0], dtype=np.int16)
-        else:
-            era_np = np.asarray(era, dtype=np.int16)
-            if era_np.shape[0] != N:
+        if era is not None:
+            era = np.asarray(era, dtype=np.int16)
+            if era.shape[0] != N:
                 raise ValueError("era must align with X rows")
-            if N > 1 and np.all(era_np[1:] >= era_np[:-1]):
-                # eras already contiguous and ascending: their runs give the unique values directly
-                starts = np.concatenate([[0], np.flatnonzero(era_np[1:] != era_np[:-1]) + 1])
-                uniq = era_np[starts]
-                era_encoded = np.repeat(np.arange(starts.shape[0], dtype=np.int16),
-                                        np.diff(np.concatenate([starts, [N]])))
-            else:
-                uniq, inv = np.unique(era_np, return_inverse=True)
-                era_encoded = inv.astype(np.int16)
+        uniq, era_offsets, order = sort_eras(era, N)
         self._era_unique = uniq
-        E = int(uniq.shape[0])
         self._feature_names = list(feature_names) if feature_names is not None else [f"f{i}" for i in range(F)]
-
-        # rows ordered by (era, row); identity when eras are already contiguous and ascending
-        if N <= 1 or np.all(era_encoded[1:] >= era_encoded[:-1]):
-            order = None
-            era_sorted = era_encoded
-        else:
-            order = np.argsort(era_encoded, kind="stable")
-            era_sorted = era_encoded[order]
-        counts = np.bincount(era_sorted.astype(np.int64), minlength=E)
-        era_offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
 
         # binning (packboost/data.py:61-93)
         small_int = X_np.dtype in (torch.uint8, torch.int8, np.dtype(np.uint8), np.dtype(np.int8))
@@ -732,8 +720,7 @@ class PackBoost:
         if validate_on_device:
             is_binned = True   # declared by the caller; the range is checked on the device while packing
         elif on_device:
-            host_view = X_np.cpu().numpy() if X_np.is_cuda else X_np.numpy()
-            is_binned = detect_prebinned(host_view, cfg.max_bins)
+            is_binned = detect_prebinned_tensor(X_np, cfg.max_bins)
         else:
             is_binned = detect_prebinned(X_np, cfg.max_bins)
         if bool(cfg.prebinned) and not is_binned:
@@ -793,11 +780,14 @@ class PackBoost:
                                         defer_validation=True)
         if validate_on_device and not agree_all(matrix.max_code < min(cfg.max_bins, 128), self._device):
             raise ValueError("prebinned=True requires X to contain integer bins within [0, max_bins).")
-        y_sorted = y_np if order is None else y_np[order]
+        if order is None:
+            y_sorted = y_np
+        else:
+            y_sorted = y_np[torch.from_numpy(order).to(self._device) if isinstance(y_np, torch.Tensor) else order]
         self._trainer = _DeviceTrainer(cfg, matrix, y_sorted, era_offsets, F, feat_local, rank, world,
                                        replicated=replicate)
         self._row_order = order
-        self._fit_ctx = {"era_sorted": era_sorted, "y_sorted": y_sorted, "F": F}
+        self._fit_ctx = {"F": F}
 
         self._depth_logs = []
         self._round_depths = []

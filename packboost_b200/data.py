@@ -50,6 +50,35 @@ def detect_prebinned(X: np.ndarray, max_bins: int) -> bool:
     return top <= 127
 
 
+def detect_prebinned_tensor(X: torch.Tensor, max_bins: int) -> bool:
+    """:func:`detect_prebinned` of a tensor where it is: only an integer table is looked at, and only
+    its smallest and largest value leave the device."""
+    if X.is_floating_point() or X.is_complex() or X.dtype == torch.bool:
+        return False
+    if X.numel() == 0:
+        return max_bins > 0
+    low, top = (int(v) for v in torch.stack(torch.aminmax(X)).tolist())
+    return low >= 0 and top < max_bins and top <= 127
+
+
+def sort_eras(era: np.ndarray | None, n_rows: int) -> tuple[np.ndarray, np.ndarray, np.ndarray | None]:
+    """``(era ids ascending, offsets of their row ranges, row order)`` of the rows grouped by era;
+    the order is ``None`` when the rows are grouped already.  The runs of equal ids give the ids and
+    the offsets, so rows that come in ascending order cost one comparison pass."""
+    if era is None:
+        return np.array([0], dtype=np.int16), np.array([0, n_rows], dtype=np.int32), None
+    order = None
+    for attempt in range(2):
+        starts = np.flatnonzero(era[1:] != era[:-1]) + 1
+        starts = np.concatenate([[0], starts]) if n_rows else starts
+        uniq = era[starts]
+        if np.all(uniq[1:] > uniq[:-1]):
+            break
+        order = np.argsort(era, kind="stable")
+        era = era[order]
+    return uniq, np.concatenate([starts, [n_rows]]).astype(np.int32), order
+
+
 def quantile_edges(X: np.ndarray, max_bins: int) -> np.ndarray:
     """``[max_bins-1, F]`` float32 edges at the interior quantiles (``packboost/data.py:49-50``)."""
     q = np.linspace(0.0, 1.0, max_bins + 1, dtype=np.float64)[1:-1]
