@@ -102,12 +102,33 @@ int pb_pack_codes_u8(const uint8_t* x, int64_t n_chunk, int64_t n_features, int6
                      const int32_t* feature_map, uint8_t* codes, int64_t pitch,
                      int64_t code_bits, void* stream);
 
+/* Both of the above in one entry: `x_is_f32` with edges, else bin ids (uint8).  `src_rows[i]` is the
+ * source row of destination row `row_offset + i` (NULL: rows in order), for rows that are brought
+ * into era order while they are packed.  `top` (NULL: not wanted) takes the maximum of itself and
+ * the largest byte of a bin-id table, the range check of packboost/data.py:32-42. */
+int pb_pack_table(const void* x, int64_t x_is_f32, const int32_t* src_rows, int64_t n_chunk, int64_t n_features,
+                  int64_t row_offset, const float* edges, int64_t n_edges, int64_t max_bins,
+                  const int32_t* feature_map, uint8_t* codes, int64_t pitch, int64_t code_bits,
+                  uint32_t* top, void* stream);
+
 /* Row-major packing for the predictor: `out[row][pitch_row]`, 4-bit (two features per byte,
  * even feature in the low nibble) or 8-bit.  Float input is binned with `edges` first
  * (`edges == NULL`: input is uint8 bin ids). */
 int pb_pack_rows(const void* x, int64_t x_is_f32, int64_t n_rows, int64_t n_features,
                  const float* edges, int64_t n_edges, int64_t max_bins,
                  uint8_t* out, int64_t pitch_row, int64_t code_bits, void* stream);
+
+/* The same with the range check of pb_pack_table. */
+int pb_pack_rows_top(const void* x, int64_t x_is_f32, int64_t n_rows, int64_t n_features,
+                     const float* edges, int64_t n_edges, int64_t max_bins,
+                     uint8_t* out, int64_t pitch_row, int64_t code_bits, uint32_t* top, void* stream);
+
+/* Pageable host memory to the device through the caller's page-locked ring of at least
+ * pb_upload_ring_bytes(bytes) bytes: a few host threads copy into the ring while finished pieces
+ * are handed to the copy engine.  Returns when everything is in the ring or on its way; the ring
+ * must stay until `stream` has passed the call. */
+int64_t pb_upload_ring_bytes(int64_t bytes);
+int pb_upload(void* dst, const void* src, int64_t bytes, void* ring, int64_t ring_bytes, void* stream);
 
 /* ---- training state ------------------------------------------------------------------ */
 

@@ -78,6 +78,10 @@ _PROTOS: dict[str, tuple[Any, list[Any]]] = {
     "pb_bin_pack_f32": (C.c_int, [vp, i64, i64, i64, vp, i64, i64, vp, vp, i64, i64, vp]),
     "pb_pack_codes_u8": (C.c_int, [vp, i64, i64, i64, vp, vp, i64, i64, vp]),
     "pb_pack_rows": (C.c_int, [vp, i64, i64, i64, vp, i64, i64, vp, i64, i64, vp]),
+    "pb_pack_table": (C.c_int, [vp, i64, vp, i64, i64, i64, vp, i64, i64, vp, vp, i64, i64, vp, vp]),
+    "pb_pack_rows_top": (C.c_int, [vp, i64, i64, i64, vp, i64, i64, vp, i64, i64, vp, vp]),
+    "pb_upload_ring_bytes": (i64, [i64]),
+    "pb_upload": (C.c_int, [vp, vp, i64, vp, i64, vp]),
     "pb_train_state_bytes": (i64, []),
     "pb_ctl_bytes": (i64, []),
     "pb_workspace_min_bytes": (i64, [C.POINTER(TrainState)]),

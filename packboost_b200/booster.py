@@ -45,8 +45,9 @@ from . import backends as B
 from .config import PackBoostConfig
 from .forest import validate_forest
 from .sharding import agree_all, block_size, choose_replicated, dealt_part, feature_map, local_part, owned_range
-from .data import (BinningResult, PackedMatrix, PackedRows, code_bits_for, detect_prebinned, detect_prebinned_tensor,
-                   pack_feature_major, pack_feature_major_distributed, pack_row_major, quantile_edges_device, sort_eras)
+from .data import (BinningResult, PackedMatrix, PackedRows, Uploads, code_bits_for, detect_prebinned,
+                   detect_prebinned_tensor, fits_on_device, pack_feature_major, pack_feature_major_distributed,
+                   pack_row_major, quantile_edges_device, sort_eras)
 
 # ------------------------------ tree containers ------------------------------
 
@@ -200,6 +201,7 @@ def _era_correlation_np(era_ids: np.ndarray, target: np.ndarray, preds: np.ndarr
 # ------------------------------ device training state ------------------------------
 
 
+_NOT_BINNED = "Input must already be prebinned when no edges are provided"
 _RING = 4  # staging slots: at most three rounds are in flight (previous, a discarded one, its redo)
 
 
@@ -640,6 +642,7 @@ class PackBoost:
         self._use_native_cuda = True
         self._cuda_backend = B
         self._forest_cache: dict | None = None
+        self._edges_cache: tuple | None = None
         self._train_preds: np.ndarray | None = None
         self._trainer: _DeviceTrainer | None = None
         self._row_order: np.ndarray | None = None
@@ -733,6 +736,7 @@ class PackBoost:
         # ceil(F / world) features).
         c0, c1 = owned_range(F, rank, world)
         blk = block_size(F, world)
+        uploads = Uploads()
         if is_binned:
             edges = None
             self._binner = BinningResult(bins=None, bin_edges=None, prebinned=True)
@@ -743,6 +747,8 @@ class PackBoost:
                 X_src = X_src.view(np.uint8)
         else:
             X_src = X_np.to(torch.float32) if on_device else X_np.astype(np.float32, copy=False)
+            if world == 1 and not (on_device and X_src.is_cuda) and fits_on_device(N * F * 4):
+                X_src = uploads(X_src, torch.float32)   # once: the edges and the codes are both taken from this copy
             if world > 1:
                 # each rank sorts its own columns; the edge tables are exchanged
                 own = np.zeros((cfg.max_bins - 1, blk), dtype=np.float32)
@@ -1075,7 +1081,8 @@ class PackBoost:
             if y_eval is None:
                 raise ValueError(f"eval set '{name}' requires y values for correlation logging")
             Xe = np.asarray(X_eval)
-            rows = self._pack_rows(Xe)
+            rows, top = self._pack_rows(Xe)
+            self._check_top(top)
             era_e = np.zeros(Xe.shape[0], dtype=np.int16) if era_eval is None else np.asarray(era_eval, dtype=np.int16)
             if era_e.shape[0] != Xe.shape[0]:
                 raise ValueError(f"eval set '{name}' era ids must align with X rows")
@@ -1095,27 +1102,47 @@ class PackBoost:
             stt["done"] = len(self._distinct)
 
     # -- prediction -------------------------------------------------------------
-    def _pack_rows(self, X: np.ndarray) -> PackedRows:
+    def _device_edges(self) -> torch.Tensor | None:
+        """The bin edges on the device, brought there once per edge table."""
+        edges = self._binner.bin_edges
+        if edges is None:
+            return None
+        if self._edges_cache is None or self._edges_cache[0] is not edges:
+            own = np.ascontiguousarray(edges, dtype=np.float32)
+            self._edges_cache = (edges, torch.from_numpy(own).to(self._device))
+        return self._edges_cache[1]
+
+    def _pack_rows(self, X, uploads: Uploads | None = None) -> tuple[PackedRows, torch.Tensor | None]:
+        """Packed rows and, for codes whose range is checked on the device, the tensor that holds the
+        largest of them (see :meth:`_check_top`)."""
         if self._binner is None:
             raise RuntimeError("Model must be fitted before predict()")
-        if isinstance(X, torch.Tensor) and X.is_cuda:
-            # device input is consumed where it is (codes: range-checked on the device)
-            Xd = X.detach()
-            if self._binner.bin_edges is None:
-                if Xd.dtype not in (torch.uint8, torch.int8):
-                    raise ValueError("Input must already be prebinned when no edges are provided")
-                Xd = Xd.view(torch.uint8)
-                if Xd.numel() and int(Xd.max()) >= int(self.config.max_bins):
-                    raise ValueError("Input must already be prebinned when no edges are provided")
-                return pack_row_major(Xd, None, self.config.max_bins)
-            return pack_row_major(Xd.to(torch.float32), self._binner.bin_edges, self.config.max_bins)
-        X_np = X.detach().cpu().numpy() if isinstance(X, torch.Tensor) else np.asarray(X)
-        if self._binner.bin_edges is None:
-            if not detect_prebinned(X_np, self.config.max_bins):
-                raise ValueError("Input must already be prebinned when no edges are provided")
-            src = X_np if X_np.dtype in (np.uint8, np.int8) else X_np.astype(np.uint8)
-            return pack_row_major(src.view(np.uint8), None, self.config.max_bins)
-        return pack_row_major(X_np.astype(np.float32, copy=False), self._binner.bin_edges, self.config.max_bins)
+        max_bins, edges = self.config.max_bins, self._device_edges()
+        if isinstance(X, torch.Tensor):
+            X = X.detach()
+        else:
+            X = np.asarray(X)
+        if edges is not None:
+            if isinstance(X, torch.Tensor) and X.is_cuda:
+                X = X.to(torch.float32)
+            return pack_row_major(X, edges, max_bins, uploads=uploads), None
+        top = None
+        if X.dtype in (torch.uint8, torch.int8, np.dtype(np.uint8), np.dtype(np.int8)):
+            # (negative int8 values are bytes of 128 and more)
+            X = X.view(torch.uint8 if isinstance(X, torch.Tensor) else np.uint8)
+            top = torch.zeros(1, dtype=torch.int32, device=self._device)
+        elif isinstance(X, torch.Tensor) and X.is_cuda:
+            raise ValueError(_NOT_BINNED)
+        else:
+            X = X.numpy() if isinstance(X, torch.Tensor) else X
+            if not detect_prebinned(X, max_bins):
+                raise ValueError(_NOT_BINNED)
+            X = X.astype(np.uint8)
+        return pack_row_major(X, None, max_bins, top=top, uploads=uploads), top
+
+    def _check_top(self, top: torch.Tensor | None) -> None:
+        if top is not None and int(top.item()) >= min(int(self.config.max_bins), 128):
+            raise ValueError(_NOT_BINNED)
 
     def _pack_forest(self, distinct: Sequence[tuple[Tree, int]]) -> dict[str, torch.Tensor]:
         arrs = [t.arrays() for t, _ in distinct]
@@ -1172,8 +1199,11 @@ class PackBoost:
             raise RuntimeError("Model must be fitted before predict()")
         self._drain()
         self._flush_pending_tree()
-        rows = self._pack_rows(X)
+        uploads = Uploads()
+        rows, top = self._pack_rows(X, uploads)
         if not self._trees:
+            self._check_top(top)
+            torch.cuda.current_stream().synchronize()
             return np.zeros(rows.n_rows, dtype=np.float32)
         if self._tree_weight is None:
             raise RuntimeError("Missing _tree_weight; call fit() first.")
@@ -1182,7 +1212,9 @@ class PackBoost:
         if self._forest_cache is None or self._forest_cache["n_distinct"] != len(self._distinct):
             self._forest_cache = self._pack_forest(self._distinct)
             self._forest_cache["n_distinct"] = len(self._distinct)
-        return self._predict_packed(rows, self._forest_cache).cpu().numpy()
+        out = self._predict_packed(rows, self._forest_cache).cpu().numpy()
+        self._check_top(top)
+        return out
 
     def predict_packwise(self, X: np.ndarray, block_size_trees: int = 8) -> np.ndarray:
         if block_size_trees <= 0:

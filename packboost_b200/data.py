@@ -122,6 +122,7 @@ def quantile_edges_device(X: np.ndarray | torch.Tensor, max_bins: int) -> np.nda
     of a zero.  ``X``: float32 ``[N, F]``, host array or tensor on either side."""
     dev = _device()
     n, f = X.shape
+    uploads = Uploads()
     cols = max(1, min(f, (256 << 20) // max(4 * n, 1)))   # about 256 MB of floats per sort
     out = np.empty((max_bins - 1, f), dtype=np.float64)
     for c0 in range(0, f, cols):
@@ -129,7 +130,7 @@ def quantile_edges_device(X: np.ndarray | torch.Tensor, max_bins: int) -> np.nda
         if isinstance(X, torch.Tensor):
             block = X[:, c0:c1].to(device=dev, dtype=torch.float32)
         else:
-            block = torch.from_numpy(np.ascontiguousarray(X[:, c0:c1], dtype=np.float32)).to(dev)
+            block = uploads(X[:, c0:c1], torch.float32)
         out[:, c0:c1] = edges_from_sorted(torch.sort(block, dim=0).values, max_bins)
     return out.astype(np.float32)
 
@@ -157,7 +158,7 @@ class PackedMatrix:
     """Feature-major packed bin codes on the device (layout of ``pb_train_state.codes``)."""
 
     def __init__(self, n_rows: int, n_features_local: int, code_bits: int, device: torch.device,
-                 pitch: int | None = None):
+                 pitch: int | None = None, zero: bool = True):
         self.n_rows = int(n_rows)
         self.rows_padded = (self.n_rows + 255) // 256 * 256
         self.code_bits = int(code_bits)
@@ -168,7 +169,8 @@ class PackedMatrix:
             self.pitch = int(pitch)
         self.n_features_local = int(n_features_local)
         self.max_code = 0   # largest pre-binned code seen while packing (when validation was asked for)
-        self.codes = torch.zeros((max(self.n_features_local, 1), self.pitch), dtype=torch.uint8, device=device)
+        make = torch.zeros if zero else torch.empty
+        self.codes = make((max(self.n_features_local, 1), self.pitch), dtype=torch.uint8, device=device)
 
     def unpack(self) -> torch.Tensor:
         """``uint8 [F_local, n_rows]`` (tests and the legacy feature-major predictors)."""
@@ -180,36 +182,48 @@ class PackedMatrix:
         return full[: self.n_features_local, : self.n_rows].contiguous()
 
 
-_STAGE: dict = {}
+class Uploads:
+    """Host arrays on their way to the device.  Page-locked tensors go to the copy engine as they are,
+    everything else through a page-locked ring filled by the library's copy threads.  The rings stay
+    with this object, which has to live until the current stream has passed the copies."""
+
+    def __init__(self) -> None:
+        self._rings: list[torch.Tensor] = []
+
+    def __call__(self, host, dtype: torch.dtype, out: torch.Tensor | None = None) -> torch.Tensor:
+        """Device copy of a host array or tensor, converted to ``dtype`` on the host where it differs."""
+        if isinstance(host, torch.Tensor):
+            src = host if host.dtype == dtype else host.to(dtype)
+            if src.is_pinned() and src.is_contiguous():
+                dev = torch.empty(src.shape, dtype=dtype, device=_device()) if out is None else out
+                return dev.copy_(src, non_blocking=True)
+            src = src.contiguous()
+        else:
+            src = torch.from_numpy(np.ascontiguousarray(host, dtype=_NUMPY_OF[dtype]))
+        dev = torch.empty(src.shape, dtype=dtype, device=_device()) if out is None else out
+        nbytes = src.numel() * src.element_size()
+        need = int(B.lib().pb_upload_ring_bytes(nbytes))
+        ring = next((r for r in self._rings if r.numel() >= need), None)
+        if ring is not None:
+            torch.cuda.current_stream().synchronize()   # (the ring's last user)
+        else:
+            ring = torch.empty(max(need, 1), dtype=torch.uint8, pin_memory=True)
+            self._rings.append(ring)
+        B.check(B.lib().pb_upload(dev.data_ptr(), src.data_ptr(), nbytes, ring.data_ptr(), ring.numel(),
+                                  torch.cuda.current_stream().cuda_stream))
+        return dev
 
 
-def _parallel_copy(dst: np.ndarray, src: np.ndarray) -> None:
-    """``dst[...] = src`` for 2-D arrays with the rows dealt over a few threads (numpy releases the
-    GIL while it copies): one thread moves ~10 GB/s, the host link takes five times that."""
-    import os
-    from concurrent.futures import ThreadPoolExecutor
-    n = src.shape[0]
-    workers = max(1, min(8, (os.cpu_count() or 2) // 2, n // 4096))
-    if workers == 1:
-        np.copyto(dst, src, casting="unsafe")
-        return
-    pool = _STAGE.get("pool")
-    if pool is None:
-        pool = _STAGE["pool"] = ThreadPoolExecutor(max_workers=8)
-    step = (n + workers - 1) // workers
-    futs = [pool.submit(np.copyto, dst[a:a + step], src[a:a + step], "unsafe") for a in range(0, n, step)]
-    for f in futs:
-        f.result()
+_NUMPY_OF = {torch.float32: np.float32, torch.uint8: np.uint8, torch.int32: np.int32}
 
 
-def _staging(nbytes: int) -> list[tuple[torch.Tensor, torch.cuda.Event]]:
-    """Two reusable page-locked buffers (and the events that guard their reuse) for bringing
-    pageable host arrays to the device chunk by chunk."""
-    have = _STAGE.get("bufs")
-    if have is None or have[0][0].numel() < nbytes:
-        have = [(torch.empty(nbytes, dtype=torch.uint8).pin_memory(), torch.cuda.Event()) for _ in range(2)]
-        _STAGE["bufs"] = have
-    return have
+def fits_on_device(nbytes: int) -> bool:
+    """Whether a whole table may be brought to the device for a while: always when it is small next to
+    the device, else a third of what is free."""
+    dev = _device()
+    if nbytes <= torch.cuda.get_device_properties(dev).total_memory // 64:
+        return True
+    return nbytes <= torch.cuda.mem_get_info(dev)[0] // 3
 
 
 def pack_feature_major(
@@ -236,9 +250,9 @@ def pack_feature_major(
     ``defer_validation`` the largest code seen is only recorded in ``PackedMatrix.max_code`` (several
     ranks must agree before any of them raises).
 
-    Host input reaches the device asynchronously: a page-locked tensor is read in place, a pageable
-    array goes through two reusable page-locked staging buffers so that the host copy of chunk
-    ``i + 1`` overlaps the transfer and the packing of chunk ``i``.
+    A device table of the right type is packed in one launch, rows in any order.  Host input reaches
+    the device in pieces (see :class:`Uploads`): the copy of piece ``i + 1`` overlaps the packing of
+    piece ``i``.
     """
     dev = _device()
     lib = B.lib()
@@ -246,67 +260,64 @@ def pack_feature_major(
     bits = code_bits_for(max_bins)
     r0, r1 = (0, n_rows) if rows is None else (int(rows[0]), int(rows[1]))
     n_local = n_feat if n_features_local is None else n_features_local
-    pm = out if out is not None else PackedMatrix(r1 - r0, n_local, bits, dev)
+    # (the pack kernels write the padding of every row they write: only rows nobody writes need zeros)
+    pm = out if out is not None else PackedMatrix(r1 - r0, n_local, bits, dev,
+                                                  zero=feature_map is not None or n_local != n_feat or r1 <= r0)
     if r1 <= r0:
         return pm
     fmap_t = None
     if feature_map is not None:
         fmap_t = torch.from_numpy(np.ascontiguousarray(feature_map, dtype=np.int32)).to(dev)
     is_f32 = edges is not None
-    edges_t = torch.from_numpy(np.ascontiguousarray(edges, dtype=np.float32)).to(dev) if is_f32 else None
+    edges_t = None
+    if is_f32:
+        edges_t = edges if isinstance(edges, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(edges, dtype=np.float32))
+        edges_t = edges_t.to(dev)
     stream = torch.cuda.current_stream().cuda_stream
-    is_tensor = isinstance(X, torch.Tensor)
     want = torch.float32 if is_f32 else torch.uint8
-    item = 4 if is_f32 else 1
-    np_want = np.float32 if is_f32 else np.uint8
-    # a tensor that torch can hand to the copy engine as it is: on the device, or page-locked
-    direct = is_tensor and (X.is_cuda or X.is_pinned())
-    order_t = None
-    if row_order is not None and is_tensor:
-        order_t = torch.from_numpy(np.ascontiguousarray(row_order, dtype=np.int64)).to(X.device)
-    top = torch.zeros((), dtype=torch.uint8, device=dev)
-    # (smaller pieces for a pageable source: its two page-locked staging buffers are allocated on first
-    # use, at about half a second per GB)
-    chunks = [(r0 + a, r0 + b) for a, b in _row_chunks(r1 - r0, n_feat * item, _CHUNK_BYTES if direct else 64 << 20)]
-    stage = None
-    for i, (a, b) in enumerate(chunks):
-        n = b - a
-        if direct:
-            src = X[a:b] if order_t is None else X.index_select(0, order_t[a:b])
-            if src.dtype == torch.int8 and not is_f32:
-                src = src.view(torch.uint8)
-            chunk = src.to(device=dev, dtype=want, non_blocking=True).contiguous()
-        else:
-            # pageable source: through a page-locked staging buffer
-            if stage is None:
-                stage = _staging((chunks[0][1] - chunks[0][0]) * n_feat * item)
-            buf, ev = stage[i % 2]
-            ev.synchronize()                       # the transfer that last used this buffer is done
-            dst = buf[: n * n_feat * item].view(want).view(n, n_feat)
-            if is_tensor:
-                src = X[a:b] if order_t is None else X.index_select(0, order_t[a:b])
-                if src.dtype == torch.int8 and not is_f32:
-                    src = src.view(torch.uint8)
-                dst.copy_(src)
-            else:
-                src = X[a:b] if row_order is None else X[row_order[a:b]]
-                if src.dtype == np.int8 and not is_f32:
-                    src = src.view(np.uint8)
-                _parallel_copy(dst.numpy(), src)
-            chunk = dst.to(dev, non_blocking=True)
-            ev.record()
-        if validate_codes and not is_f32:
-            top = torch.maximum(top, chunk.max())
+    top = torch.zeros(1, dtype=torch.int32, device=dev) if validate_codes and not is_f32 else None
+
+    def pack(chunk, n, at, order=None):
+        B.check(lib.pb_pack_table(chunk.data_ptr(), 1 if is_f32 else 0, B._ptr(order), n, n_feat, at, B._ptr(edges_t),
+                                  edges_t.shape[0] if is_f32 else 0, max_bins if is_f32 else (16 if bits == 4 else 256),
+                                  B._ptr(fmap_t), pm.codes.data_ptr(), pm.pitch, bits, B._ptr(top), stream))
+
+    def as_codes(src):
+        """int8 is read as the bytes it is: negative values fail the range check."""
         if is_f32:
-            B.check(lib.pb_bin_pack_f32(chunk.data_ptr(), n, n_feat, a - r0, edges_t.data_ptr(), edges_t.shape[0],
-                                        max_bins, B._ptr(fmap_t), pm.codes.data_ptr(), pm.pitch, bits, stream))
+            return src
+        if isinstance(src, torch.Tensor):
+            return src.view(torch.uint8) if src.dtype == torch.int8 else src
+        return src.view(np.uint8) if src.dtype == np.int8 else src
+
+    uploads = Uploads()
+    if isinstance(X, torch.Tensor) and X.device == dev and as_codes(X).dtype == want and X.is_contiguous():
+        if row_order is None:
+            pack(as_codes(X[r0:r1]), r1 - r0, 0)
         else:
-            B.check(lib.pb_pack_codes_u8(chunk.data_ptr(), n, n_feat, a - r0, B._ptr(fmap_t), pm.codes.data_ptr(),
-                                         pm.pitch, bits, stream))
-        # no synchronisation per chunk: the copy, the pack kernel and the release of `chunk` are
-        # ordered on the current stream
-    torch.cuda.current_stream().synchronize()
-    pm.max_code = max(pm.max_code, int(top.item())) if validate_codes else pm.max_code
+            order = np.ascontiguousarray(row_order[r0:r1], dtype=np.int32)
+            pack(as_codes(X), r1 - r0, 0, torch.from_numpy(order).to(dev))
+    else:
+        order_t = None
+        if row_order is not None and isinstance(X, torch.Tensor):
+            order_t = torch.from_numpy(np.ascontiguousarray(row_order, dtype=np.int64)).to(X.device)
+        for a, b in _row_chunks(r1 - r0, n_feat * (4 if is_f32 else 1)):
+            if order_t is not None:
+                src = X.index_select(0, order_t[r0 + a:r0 + b])
+            else:
+                src = X[r0 + a:r0 + b] if row_order is None else X[row_order[r0 + a:r0 + b]]
+            src = as_codes(src)
+            if isinstance(src, torch.Tensor) and src.is_cuda:
+                chunk = src.to(device=dev, dtype=want).contiguous()
+            else:
+                chunk = uploads(src, want)
+            pack(chunk, b - a, a)
+            # no synchronisation per chunk: the copy, the pack kernel and the release of `chunk` are
+            # ordered on the current stream
+    if top is not None:
+        pm.max_code = max(pm.max_code, int(top.item()))
+    else:
+        torch.cuda.current_stream().synchronize()
     if validate_codes and not defer_validation and pm.max_code >= min(max_bins, 128):
         raise ValueError("prebinned=True requires X to contain integer bins within [0, max_bins).")
     return pm
@@ -372,27 +383,35 @@ class PackedRows:
         self.codes = torch.empty((max(self.n_rows, 1), self.pitch_row), dtype=torch.uint8, device=device)
 
 
-def pack_row_major(X: np.ndarray | torch.Tensor, edges: np.ndarray | None, max_bins: int) -> PackedRows:
+def pack_row_major(X: np.ndarray | torch.Tensor, edges: np.ndarray | torch.Tensor | None, max_bins: int, *,
+                   top: torch.Tensor | None = None, uploads: Uploads | None = None) -> PackedRows:
     """Bin (when ``edges`` is given) and pack rows for prediction.  ``X`` may already be a
-    device tensor (float32 or uint8)."""
+    device tensor (float32 or uint8); edges too.  ``top`` (``int32 [1]`` on the device) takes the largest
+    byte of pre-binned input.  With ``uploads`` the call only enqueues and the caller synchronises
+    before it lets that object go."""
     dev = _device()
     lib = B.lib()
     bits = code_bits_for(max_bins)
     is_f32 = edges is not None
     n_rows, n_feat = X.shape
     pr = PackedRows(n_rows, n_feat, bits, dev)
-    edges_t = torch.from_numpy(np.ascontiguousarray(edges, dtype=np.float32)).to(dev) if is_f32 else None
+    edges_t = None
+    if is_f32:
+        edges_t = edges if isinstance(edges, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(edges, dtype=np.float32))
+        edges_t = edges_t.to(dev)
     stream = torch.cuda.current_stream().cuda_stream
     want = torch.float32 if is_f32 else torch.uint8
-    for a, b in _row_chunks(n_rows, n_feat * (4 if is_f32 else 1)):
-        if isinstance(X, torch.Tensor):
-            chunk = X[a:b].to(device=dev, dtype=want).contiguous()
-        else:
-            chunk = torch.from_numpy(np.ascontiguousarray(X[a:b], dtype=np.float32 if is_f32 else np.uint8)).to(dev)
-        out = pr.codes[a:b]
-        B.check(lib.pb_pack_rows(chunk.data_ptr(), 1 if is_f32 else 0, b - a, n_feat, B._ptr(edges_t),
-                                 edges_t.shape[0] if is_f32 else 0, max_bins, out.data_ptr(), pr.pitch_row, bits,
-                                 stream))
+    up = Uploads() if uploads is None else uploads
+    whole = isinstance(X, torch.Tensor) and X.device == dev and X.dtype == want and X.is_contiguous()
+    for a, b in ([(0, n_rows)] if whole else _row_chunks(n_rows, n_feat * (4 if is_f32 else 1))):
+        chunk = X[a:b]
+        if not whole:
+            on_gpu = isinstance(chunk, torch.Tensor) and chunk.is_cuda
+            chunk = chunk.to(device=dev, dtype=want).contiguous() if on_gpu else up(chunk, want)
+        B.check(lib.pb_pack_rows_top(chunk.data_ptr(), 1 if is_f32 else 0, b - a, n_feat, B._ptr(edges_t),
+                                     edges_t.shape[0] if is_f32 else 0, max_bins, pr.codes[a:b].data_ptr(), pr.pitch_row,
+                                     bits, B._ptr(top), stream))
+    if uploads is None:
         torch.cuda.current_stream().synchronize()
     return pr
 

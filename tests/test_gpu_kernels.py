@@ -282,3 +282,44 @@ def test_histogram_exact_in_every_launch_shape(shape):
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-4000:]
     assert res.stdout.strip().endswith("ok")
     assert "hist_lane_kernel<%s>" % shape.replace(" ", ",") in res.stderr, res.stderr[-2000:]
+
+
+@pytest.mark.parametrize("n,f,max_bins", [(1, 1, 5), (255, 127, 5), (256, 128, 5), (257, 129, 16), (1030, 301, 5),
+                                          (513, 131, 64), (300, 33, 2), (259, 97, 128)])
+def test_pack_kernels_at_tile_edges(n, f, max_bins):
+    """Byte and float packers (both layouts, rows in order and gathered) where rows start on odd bytes
+    and tiles are partly filled; padding rows are code 0 and the range check sees the largest byte."""
+    from packboost_b200.data import pack_feature_major, pack_row_major
+    rng = np.random.default_rng(n * f)
+    codes = rng.integers(0, max_bins, size=(n, f), dtype=np.uint8)
+    order = rng.permutation(n)
+    X = rng.normal(size=(n, f)).astype(np.float32)
+    edges = np.sort(rng.normal(size=(max_bins - 1, f)).astype(np.float32), axis=0)
+    binned = po.bin_codes(X, edges, max_bins).astype(np.uint8)
+
+    def rows_of(pr):
+        raw = pr.codes.cpu().numpy()
+        return (np.stack([raw & 0xF, raw >> 4], axis=2).reshape(raw.shape[0], -1) if pr.code_bits == 4 else raw)[:, :f]
+
+    for src, e, want in ((codes, None, codes), (X, edges, binned)):
+        for device in (False, True):
+            table = torch.from_numpy(src).to(_dev()) if device else src
+            for row_order in (None, order):
+                pm = pack_feature_major(table, e, max_bins, row_order=row_order, validate_codes=e is None)
+                np.testing.assert_array_equal(pm.unpack().cpu().numpy(), (want if row_order is None else want[order]).T)
+                if pm.code_bits == 8:
+                    assert not pm.codes[:, n:].any()
+                if e is None:
+                    assert pm.max_code == int(codes.max())
+            np.testing.assert_array_equal(rows_of(pack_row_major(table, e, max_bins)), want)
+
+
+@pytest.mark.parametrize("nbytes", [1, (384 << 10) + 1, (1 << 20) - 3, (16 << 20) + 5, (37 << 20) + 1])
+def test_upload_moves_every_byte(nbytes):
+    """The page-locked ring below, at and beyond its size."""
+    from packboost_b200.data import Uploads
+    src = np.random.default_rng(nbytes).integers(0, 256, nbytes, dtype=np.uint8)
+    uploads = Uploads()
+    for _ in range(2):
+        got = uploads(src, torch.uint8)
+        np.testing.assert_array_equal(got.cpu().numpy(), src)
