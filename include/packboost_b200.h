@@ -410,6 +410,54 @@ int pb_predict_rows(const uint8_t* codes, int64_t n_rows, int64_t pitch_row, int
                     const int32_t* tree_offsets, const int32_t* repeat, int64_t n_trees,
                     float weight, float* out, const float* init, void* stream);
 
+/* The same sum for trees of at most 256 nodes: `trees` holds `copies` times the forest (about eight
+ * spread the reads of all SMs over the L2), per tree `slot_nodes` words (a multiple of 4).  A split is `feature << 16 | left child << 8 | 255 - threshold` (the right child is the next
+ * node); every path has exactly `depth` splits (early leaves are led on by splits with threshold 255)
+ * and ends at a word that is the float leaf value.  `repeat` may be NULL when every tree is added
+ * total_repeat / n_trees times.  pb_predict_forest_fits tells whether rows of `n_features` codes fit
+ * this form. */
+int pb_predict_forest(const uint8_t* codes, int64_t n_rows, int64_t pitch_row, int64_t code_bits,
+                      int64_t n_features, const void* trees, int64_t copies, int64_t slot_nodes, int64_t depth,
+                      const int32_t* repeat, int64_t total_repeat, int64_t n_trees, float weight,
+                      float* out, const float* init, void* stream);
+/* Host side of that form: trees as concatenated node arrays (children relative to their tree, as in
+ * packboost/booster.py:172-190).  pb_forest_shape validates them (an error: malformed) and gives the
+ * words per tree and the depth, 0 words when the form does not hold them; pb_forest_words fills
+ * `out[n_trees][slot_nodes]`. */
+int pb_forest_shape(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                    const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                    int64_t* slot_nodes, int64_t* depth);
+int pb_forest_words(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                    const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                    int64_t slot_nodes, int64_t depth, uint32_t* out);
+int64_t pb_predict_forest_fits(int64_t n_features, int64_t code_bits, int64_t slot_nodes);
+
+/* A whole prediction - upload, binning or range check, packing, the trees, the predictions back in
+ * host memory - for models in the form of pb_predict_forest (packboost/booster.py:658-712).  `edges`
+ * is [n_edges][n_features] on the device, or NULL for tables of bin ids (uint8); `x` is row-major,
+ * pageable host memory or device memory.  `dev` and `pinned` are scratch of the sizes that
+ * pb_predict_table_bytes gives, device memory and page-locked host memory; the call returns when the
+ * predictions are in `out` and the scratch is free again.  `top`: largest bin id of the table. */
+typedef struct pb_model {
+    const float* edges;
+    int64_t n_edges;
+    int64_t max_bins;
+    int64_t code_bits;
+    const void* trees;
+    int64_t copies;
+    int64_t slot_nodes;
+    int64_t depth;
+    const int32_t* repeat;
+    int64_t total_repeat;
+    int64_t n_trees;
+    double weight;
+} pb_model;
+int pb_predict_table_bytes(const pb_model* m, int64_t x_on_device, int64_t n_rows, int64_t n_features,
+                           int64_t* dev_bytes, int64_t* pinned_bytes);
+int pb_predict_table(const pb_model* m, const void* x, int64_t x_on_device, int64_t n_rows, int64_t n_features,
+                     void* dev, int64_t dev_bytes, void* pinned, int64_t pinned_bytes, float* out,
+                     int64_t* top, void* stream);
+
 /* Same ensemble sum with the trees in the packed form the training loop can produce directly:
  * one 8-byte record per node, word 0 = feature (bits 0-15) | threshold (bits 16-23) | leaf flag
  * (bit 31), word 1 = tree-relative index of the left child (the right child is the next node,

@@ -64,6 +64,16 @@ class TrainState(C.Structure):
     ]
 
 
+class Model(C.Structure):
+    """Mirror of ``pb_model``."""
+
+    _fields_ = [
+        ("edges", vp), ("n_edges", i64), ("max_bins", i64), ("code_bits", i64), ("trees", vp), ("copies", i64),
+        ("slot_nodes", i64), ("depth", i64), ("repeat", vp), ("total_repeat", i64), ("n_trees", i64),
+        ("weight", C.c_double),
+    ]
+
+
 _PROTOS: dict[str, tuple[Any, list[Any]]] = {
     "pb_last_error": (C.c_char_p, []),
     "pb_abi_version": (C.c_int, []),
@@ -111,6 +121,12 @@ _PROTOS: dict[str, tuple[Any, list[Any]]] = {
                                         C.c_float, C.c_float, i64, i64, i64, i64, vp, vp]),
     "pb_predict_rows": (C.c_int, [vp, i64, i64, i64, vp, vp, vp, vp, vp, vp, vp, vp, i64, C.c_float, vp, vp, vp]),
     "pb_predict_rows_packed": (C.c_int, [vp, i64, i64, i64, vp, vp, vp, i64, i64, C.c_float, vp, vp, vp]),
+    "pb_predict_forest": (C.c_int, [vp, i64, i64, i64, i64, vp, i64, i64, i64, vp, i64, i64, C.c_float, vp, vp, vp]),
+    "pb_predict_forest_fits": (i64, [i64, i64, i64]),
+    "pb_predict_table_bytes": (C.c_int, [vp, i64, i64, i64, vp, vp]),
+    "pb_predict_table": (C.c_int, [vp, vp, i64, i64, i64, vp, i64, vp, i64, vp, vp, vp]),
+    "pb_forest_shape": (C.c_int, [vp, vp, vp, vp, vp, vp, vp, i64, vp, vp]),
+    "pb_forest_words": (C.c_int, [vp, vp, vp, vp, vp, vp, vp, i64, i64, i64, vp]),
     "pb_predict_bins_fm": (C.c_int, [vp, i64, i64, vp, vp, vp, vp, vp, vp, i64, vp, vp]),
     "pb_predict_pack_fm": (C.c_int, [vp, i64, i64, vp, vp, vp, vp, vp, vp, vp, i64, C.c_float, vp, vp]),
 }

@@ -34,6 +34,7 @@ import json
 import math
 import os
 import sys
+import threading
 from dataclasses import dataclass, field
 from time import perf_counter
 from typing import Callable, Iterable, List, Sequence, Tuple
@@ -43,7 +44,7 @@ import torch
 
 from . import backends as B
 from .config import PackBoostConfig
-from .forest import validate_forest
+from .forest import forest_slots, validate_forest
 from .sharding import agree_all, block_size, choose_replicated, dealt_part, feature_map, local_part, owned_range
 from .data import (BinningResult, PackedMatrix, PackedRows, Uploads, code_bits_for, detect_prebinned,
                    detect_prebinned_tensor, fits_on_device, pack_feature_major, pack_feature_major_distributed,
@@ -202,6 +203,8 @@ def _era_correlation_np(era_ids: np.ndarray, target: np.ndarray, preds: np.ndarr
 
 
 _NOT_BINNED = "Input must already be prebinned when no edges are provided"
+_SMALL_SCRATCH = 512 << 10
+_FOREST_COPIES = 8  # of a forest on the device: see predict_forest_kernel
 _RING = 4  # staging slots: at most three rounds are in flight (previous, a discarded one, its redo)
 
 
@@ -643,6 +646,7 @@ class PackBoost:
         self._cuda_backend = B
         self._forest_cache: dict | None = None
         self._edges_cache: tuple | None = None
+        self._small_lock, self._small_scratch = threading.Lock(), None   # see _predict_table
         self._train_preds: np.ndarray | None = None
         self._trainer: _DeviceTrainer | None = None
         self._row_order: np.ndarray | None = None
@@ -1149,13 +1153,27 @@ class PackBoost:
         offs = np.zeros(len(arrs) + 1, dtype=np.int32)
         np.cumsum([a["feature"].shape[0] for a in arrs], out=offs[1:])
         cat = {k: np.concatenate([a[k] for a in arrs]) for k in ("feature", "threshold", "left", "right", "value", "is_leaf")}
+        reps = np.asarray([r for _, r in distinct], dtype=np.int32)
+        out: dict = {"n_trees": len(arrs), "total_repeat": int(reps.sum()),
+                     "max_feature": int(cat["feature"][cat["is_leaf"] == 0].max(initial=-1))}
+        out["repeat"] = torch.from_numpy(reps).to(self._device)
+        out["even"] = bool(np.all(reps == reps[0]))
         # nothing malformed reaches the device: children inside their tree and after their parent
-        validate_forest(cat["feature"], cat["threshold"], cat["left"], cat["right"], cat["is_leaf"], offs)
-        out = {k: torch.from_numpy(v).to(self._device) for k, v in cat.items()}
-        out["offsets"] = torch.from_numpy(offs).to(self._device)
-        out["repeat"] = torch.tensor([r for _, r in distinct], dtype=torch.int32, device=self._device)
-        out["n_trees"] = len(arrs)
-        out["max_feature"] = int(cat["feature"][cat["is_leaf"] == 0].max(initial=-1))
+        slots = forest_slots(**cat, offsets=offs)
+        if slots is not None:
+            copies = _FOREST_COPIES if len(arrs) > 8 else 1
+            out["slots"] = torch.from_numpy(slots[0].view(np.int32)).to(self._device).repeat(copies, 1)
+            out["copies"], out["slot"], out["depth"] = copies, slots[0].shape[1], slots[1]
+        out["host"] = (cat, offs)   # for the forms below, built when a table asks for them
+        return out
+
+    def _large_forest(self, forest: dict) -> None:
+        """The node arrays of the predictors for large trees or very wide rows."""
+        if "offsets" in forest:
+            return
+        cat, offs = forest["host"]
+        forest.update({k: torch.from_numpy(v).to(self._device) for k, v in cat.items()})
+        forest["offsets"] = torch.from_numpy(offs).to(self._device)
         # packed 8-byte nodes when the trees allow it (right child == left child + 1, small ids)
         internal = cat["is_leaf"] == 0
         ok = (bool(np.all(cat["right"][internal] == cat["left"][internal] + 1))
@@ -1166,8 +1184,76 @@ class PackBoost:
                           1 << 31).astype(np.uint32)
             w1 = np.where(internal, cat["left"].astype(np.int64) & 0xFFFFFFFF,
                           cat["value"].astype(np.float32).view(np.uint32).astype(np.int64)).astype(np.uint32)
-            out["packed"] = torch.from_numpy(np.stack([w0, w1], axis=1).view(np.int32).copy()).to(self._device)
-            out["max_tree_nodes"] = int(np.diff(offs).max()) if len(arrs) else 1
+            forest["packed"] = torch.from_numpy(np.stack([w0, w1], axis=1).view(np.int32).copy()).to(self._device)
+            forest["max_tree_nodes"] = int(np.diff(offs).max()) if forest["n_trees"] else 1
+
+    def _current_forest(self) -> dict:
+        if self._forest_cache is None or self._forest_cache["n_distinct"] != len(self._distinct):
+            self._forest_cache = self._pack_forest(self._distinct)
+            self._forest_cache["n_distinct"] = len(self._distinct)
+        return self._forest_cache
+
+    def _predict_table(self, X) -> np.ndarray | None:
+        """The whole prediction in one library call, for small trees and a table that needs no conversion;
+        ``None`` when it is another case (or one to complain about), which the general way takes."""
+        codes = self._binner.bin_edges is None
+        n_dim = getattr(X, "ndim", 0)
+        if n_dim != 2 or not self._distinct or self._tree_weight is None:
+            return None
+        if self._trained_pack_size is not None and int(self.config.pack_size) != self._trained_pack_size:
+            return None
+        if isinstance(X, np.ndarray):
+            if not (X.flags.c_contiguous and (X.dtype == np.uint8 or X.dtype == np.int8 if codes else X.dtype == np.float32)):
+                return None
+            ptr, on_device = X.ctypes.data, 0
+        elif isinstance(X, torch.Tensor) and X.device == self._device:
+            if not (X.is_contiguous() and (X.dtype in (torch.uint8, torch.int8) if codes else X.dtype == torch.float32)):
+                return None
+            ptr, on_device = X.data_ptr(), 1
+        else:
+            return None
+        n, f = X.shape
+        forest, lib = self._current_forest(), B.lib()
+        edges = self._device_edges()
+        if n == 0 or "slots" not in forest or forest["max_feature"] >= f or n * f > (1 << 32) \
+                or (edges is not None and edges.shape[1] != f):
+            return None
+        model = forest.get("model")
+        if model is None:
+            model = B.Model()
+            model.max_bins, model.code_bits = int(self.config.max_bins), code_bits_for(self.config.max_bins)
+            model.trees, model.copies, model.slot_nodes = forest["slots"].data_ptr(), forest["copies"], forest["slot"]
+            model.depth, model.n_trees = forest["depth"], forest["n_trees"]
+            model.repeat, model.total_repeat = None if forest["even"] else forest["repeat"].data_ptr(), forest["total_repeat"]
+            model.weight = float(self._tree_weight)
+            if edges is not None:
+                model.edges, model.n_edges = edges.data_ptr(), edges.shape[0]
+            forest["model"], forest["edges"] = model, edges
+        if not lib.pb_predict_forest_fits(f, model.code_bits, model.slot_nodes):
+            return None
+        ref = C.byref(model)
+        dev_bytes, pin_bytes, top = C.c_int64(), C.c_int64(), C.c_int64()
+        B.check(lib.pb_predict_table_bytes(ref, on_device, n, f, C.byref(dev_bytes), C.byref(pin_bytes)))
+        # requests of a few rows share buffers kept with the model, one call at a time
+        small = max(dev_bytes.value, pin_bytes.value) <= _SMALL_SCRATCH and self._small_lock.acquire(blocking=False)
+        try:
+            if small:
+                if self._small_scratch is None:
+                    self._small_scratch = (torch.empty(_SMALL_SCRATCH, dtype=torch.uint8, device=self._device),
+                                           torch.empty(_SMALL_SCRATCH, dtype=torch.uint8, pin_memory=True))
+                dev, pinned = self._small_scratch
+            else:
+                dev = torch.empty(dev_bytes.value, dtype=torch.uint8, device=self._device)
+                pinned = torch.empty(pin_bytes.value, dtype=torch.uint8, pin_memory=True)
+            out = np.empty(n, dtype=np.float32)
+            B.check(lib.pb_predict_table(ref, ptr, on_device, n, f, dev.data_ptr(), dev.numel(), pinned.data_ptr(),
+                                         pinned.numel(), out.ctypes.data, C.byref(top),
+                                         torch.cuda.current_stream().cuda_stream))
+        finally:
+            if small:
+                self._small_lock.release()
+        if codes and top.value >= min(int(self.config.max_bins), 128):
+            raise ValueError(_NOT_BINNED)
         return out
 
     def _predict_packed(self, rows: PackedRows, forest: dict, init: torch.Tensor | None = None) -> torch.Tensor:
@@ -1177,6 +1263,16 @@ class PackBoost:
         f = forest
         if f["max_feature"] >= rows.n_features:
             raise ValueError(f"the ensemble splits on feature {f['max_feature']} but the input has {rows.n_features} columns")
+        # one-word nodes while the trees are small and 32 rows fit in shared memory (measured faster
+        # there at every size, 1.5 to 7 times)
+        if "slots" in f and B.lib().pb_predict_forest_fits(rows.n_features, rows.code_bits, f["slot"]):
+            B.check(B.lib().pb_predict_forest(
+                rows.codes.data_ptr(), rows.n_rows, rows.pitch_row, rows.code_bits, rows.n_features, f["slots"].data_ptr(),
+                f["copies"], f["slot"], f["depth"], 0 if f["even"] else f["repeat"].data_ptr(), f["total_repeat"], f["n_trees"],
+                float(self._tree_weight), out.data_ptr(), B._ptr(init) if init is not None else 0,
+                torch.cuda.current_stream().cuda_stream))
+            return out
+        self._large_forest(f)
         if "packed" in f:
             B.check(B.lib().pb_predict_rows_packed(
                 rows.codes.data_ptr(), rows.n_rows, rows.pitch_row, rows.code_bits, f["packed"].data_ptr(),
@@ -1199,6 +1295,9 @@ class PackBoost:
             raise RuntimeError("Model must be fitted before predict()")
         self._drain()
         self._flush_pending_tree()
+        fast = self._predict_table(X)
+        if fast is not None:
+            return fast
         uploads = Uploads()
         rows, top = self._pack_rows(X, uploads)
         if not self._trees:
@@ -1209,10 +1308,7 @@ class PackBoost:
             raise RuntimeError("Missing _tree_weight; call fit() first.")
         if self._trained_pack_size is not None and int(self.config.pack_size) != self._trained_pack_size:
             raise RuntimeError("pack_size differs from training; keep it constant.")
-        if self._forest_cache is None or self._forest_cache["n_distinct"] != len(self._distinct):
-            self._forest_cache = self._pack_forest(self._distinct)
-            self._forest_cache["n_distinct"] = len(self._distinct)
-        out = self._predict_packed(rows, self._forest_cache).cpu().numpy()
+        out = self._predict_packed(rows, self._current_forest()).cpu().numpy()
         self._check_top(top)
         return out
 

@@ -5,6 +5,10 @@
 // rules contributes 0 for that row (the guards of packboost/backends/cuda/frontier_cuda.cu:214-231
 // and 953-966).  A malformed ensemble therefore cannot hang the device or read outside its buffers.
 
+#include <stdlib.h>
+
+#include <vector>
+
 #include "common.cuh"
 
 namespace pb {
@@ -380,6 +384,241 @@ __global__ void __launch_bounds__(512) predict_rows_packed_smem_kernel(PredictPa
 }
 
 
+// ---- small trees: every lane a row, every step the same ------------------------------------------------
+//
+// Trees of at most 256 nodes as slots of `slot` words.  A split is one word, feature << 16 | left
+// child << 8 | 255 - threshold (the right child is the next node).  Adding the code of the row to the
+// word carries into the child when the code is above the threshold, so a step is two shared-memory
+// loads, an add and a byte extraction, without a branch or a comparison.  Every path is exactly
+// `depth` splits long - early leaves are led on by splits with threshold 255, which no code exceeds -
+// and the word it ends at is the leaf value.  So a walk ends by itself whatever the words hold (child
+// indices have eight bits, features are clamped to the row).
+//
+// The bound of the form above was shared memory: lanes of a warp sat in four trees and eight rows, so
+// node loads hit many banks twice and codes of different rows lay a row apart.  Here a warp holds 32
+// rows and one tree at a time.  Codes are staged feature-major (the nibbles of 32 rows are 16
+// consecutive bytes), so lanes at the same node read one or two wavefronts, and the nodes of a level
+// are consecutive words.  The other bound was the ordered sum: a model of 2 000 rounds with packs of
+// 32 adds 64 000 numbers one after the other to each prediction, four cycles each, and the walking
+// threads did it four times over.  Here `adders` (one warp per 64 rows, two rows per lane and
+// instruction; the CTA's first warps, which the scheduler prefers) add the terms of the batch before
+// while `walkers` (walk_warps warps per 32 rows) produce those of the next and one warp fetches the
+// trees after that; the sum stays the sequential one.
+// 500 000 rows x 2 376 features, 2 000 trees of depth 6 added 32 times: 22.2 -> 5.5 ms, of which the
+// additions alone take 3.5; 5 417 rows, 1 000 trees: 417 -> 119 us.
+struct PredictForestArgs {
+    const uint8_t* codes;
+    int64_t n_rows;
+    int64_t pitch_row;
+    int n_features;
+    const uint32_t* trees;   // [copies][n_trees][slot]
+    int copies;
+    int slot;
+    int depth;
+    const int32_t* repeat;   // per tree, or null: every tree `rep` times
+    int rep;
+    int n_trees;
+    float weight;
+    float* out;
+    const float* init;
+    int groups;              // groups of 32 rows per CTA
+    int walk_warps;          // walkers per group
+};
+
+constexpr int kTreesPerWalker = 4;  // walked at a time by a lane: independent chains
+constexpr int kAddGroup = 8;        // trees whose terms an adder holds; a batch is a multiple of it
+// Batches of trees in shared memory: the one being walked and those on their way.
+constexpr int kTreeBuffers = 2;
+
+// Words per feature.  The words of 32 rows are `bits` neighbouring banks; an odd number of groups puts
+// those of different features at every multiple of that, an even one needs a word of padding.
+__host__ __device__ constexpr int forest_words(int bits, int groups) { return groups * bits + (groups % 2 == 0 ? 1 : 0); }
+
+__host__ __device__ constexpr int forest_adders(int groups) { return (groups + 1) / 2; }
+__host__ __device__ constexpr int forest_threads(int groups, int walk_warps) {
+    return 32 * (forest_adders(groups) + groups * walk_warps + 1);
+}
+
+// acc += v for two rows at once, each sum rounded like a scalar one
+__device__ __forceinline__ void add2(unsigned long long& acc, unsigned long long v) {
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v));
+}
+
+// (an index of a malformed tree may reach 256 words past its slot: the terms and the pad lie there)
+inline int64_t forest_smem(int64_t n_features, int bits, int groups, int walk_warps, int64_t slot) {
+    const int64_t tb = kTreesPerWalker * walk_warps;
+    return ((n_features + 7) / 8 * 8 * forest_words(bits, groups) + 3) / 4 * 16 + kTreeBuffers * tb * slot * 4 + 2 * tb * 32 * groups * 4 + 128 + 1040;
+}
+
+template <int REP>
+__device__ __forceinline__ void add_times(unsigned long long& acc, const unsigned long long (&v)[kAddGroup]) {
+#pragma unroll
+    for (int u = 0; u < kAddGroup; ++u)
+#pragma unroll
+        for (int i = 0; i < REP; ++i) add2(acc, v[u]);
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(1024) predict_forest_kernel(PredictForestArgs a) {
+    extern __shared__ __align__(16) uint32_t s_mem[];
+    constexpr int PER = 32 / BITS;                       // codes per word
+    const int G = a.groups, R = 32 * G;
+    const int W = forest_words(BITS, G);
+    const int f_pad = (a.n_features + 7) / 8 * 8;
+    const int TB = kTreesPerWalker * a.walk_warps;       // trees per batch
+    const int batch_words = TB * a.slot;
+    uint32_t* s_codes = s_mem;                           // [f_pad][W]
+    uint32_t* s_trees = s_mem + (size_t)(f_pad * W + 3) / 4 * 4;       // [kTreeBuffers][TB][slot]
+    const int TR = R;                                    // (the last adder of an odd G reads 32 rows past its terms)
+    float* s_term = reinterpret_cast<float*>(s_trees + kTreeBuffers * batch_words);  // [2][TB][TR]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    const int64_t row0 = (int64_t)blockIdx.x * R;
+    const int nr = (int)min((int64_t)R, a.n_rows - row0);
+    const int n_batches = (a.n_trees + TB - 1) / TB;
+
+    // All CTAs ask for the same few lines at the same time, and a line is served by one slice of the L2:
+    // 0.9 us per batch of eight trees, more than walking it takes.  The copies spread them.
+    const uint32_t* forest = a.trees + (size_t)(blockIdx.x % a.copies) * a.n_trees * a.slot;
+    auto fetch = [&](int b) {                            // (one warp) batch b into its buffer
+        const int n16 = max(min(TB, a.n_trees - b * TB), 0) * a.slot / 4;
+        const uint4* src = reinterpret_cast<const uint4*>(forest + (size_t)b * batch_words);
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_trees + (b % kTreeBuffers) * batch_words);
+#pragma unroll 4
+        for (int i = lane; i < n16; i += 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * i), "l"(src + i) : "memory");
+        cp_async_commit();
+    };
+    const int A = forest_adders(G);
+    const bool adder = warp < A, loader = warp == n_warps - 1;
+    if (loader) {
+        for (int b = 0; b < kTreeBuffers - 1; ++b) fetch(b);
+    }
+
+    // ---- rows: PER x PER blocks of codes turned over (rows of a word's features -> features of rows) ----
+    {
+        const int row_groups = R / PER;                  // words of a feature
+        const int src_words = (a.n_features + PER - 1) / PER;
+        const int g_blocks = (row_groups + 7) / 8, w_blocks = (src_words + 3) / 4;
+        for (int task = warp; task < g_blocks * w_blocks; task += n_warps) {
+            const int g = (task % g_blocks) * 8 + (lane >> 2);
+            const int fw = (task / g_blocks) * 4 + (lane & 3);
+            if (g >= row_groups || fw >= src_words) continue;
+            uint32_t w[PER];
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int r = g * PER + i;
+                w[i] = r < nr ? __ldg(reinterpret_cast<const uint32_t*>(a.codes + (row0 + r) * a.pitch_row) + fw) : 0u;
+            }
+            // swap off-diagonal blocks of 1, 2, 4 codes between words 1, 2, 4 apart
+#pragma unroll
+            for (int d = 1; d < PER; d <<= 1) {
+                const int sh = d * BITS;
+                const uint32_t m = sh == 4 ? 0x0F0F0F0Fu : (sh == 8 ? 0x00FF00FFu : 0x0000FFFFu);
+#pragma unroll
+                for (int i = 0; i < PER; ++i)
+                    if (!(i & d)) {
+                        const uint32_t t = ((w[i] >> sh) ^ w[i + d]) & m;
+                        w[i + d] ^= t;
+                        w[i] ^= t << sh;
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < PER; ++j) s_codes[(fw * PER + j) * W + g] = w[j];
+        }
+    }
+
+    if (loader) {
+        for (int b = 0; b <= n_batches; ++b) {
+            cp_async_wait<kTreeBuffers - 2>();
+            __syncthreads();   // batch b is here, the walk of b - 1 and the sums of b - 2 are done
+            fetch(b + kTreeBuffers - 1);                 // its buffer held batch b - 1
+        }
+    } else if (!adder) {
+        const int group = (warp - A) % G;
+        const int q = (warp - A) / G;                    // trees q * kTreesPerWalker .. of a batch
+        const int my_row = group * 32 + lane;
+        const uint32_t lane_at = (uint32_t)__cvta_generic_to_shared(s_codes) +
+                                 (BITS == 4 ? (uint32_t)(group * 16 + (lane >> 1)) : (uint32_t)my_row);
+        const uint32_t nibble = (uint32_t)(lane & 1) * 4u;
+        const uint32_t fmax = (uint32_t)a.n_features - 1u, pitch = (uint32_t)W * 4u;
+        const uint32_t slot_bytes = (uint32_t)a.slot * 4u;
+        const uint32_t first = (uint32_t)__cvta_generic_to_shared(s_trees) + (uint32_t)(q * kTreesPerWalker) * slot_bytes;
+        float* term = s_term + (q * kTreesPerWalker) * TR + my_row;
+        for (int b = 0; b <= n_batches; ++b) {
+            __syncthreads();
+            if (b == n_batches) break;
+            // (trees past the last one are walked too: what the buffer holds there is never added)
+            const uint32_t base = first + (uint32_t)((b % kTreeBuffers) * batch_words) * 4u;
+            uint32_t idx[kTreesPerWalker];
+#pragma unroll
+            for (int u = 0; u < kTreesPerWalker; ++u) idx[u] = 0u;
+            for (int s = 0; s < a.depth; ++s) {
+                uint32_t w[kTreesPerWalker], c[kTreesPerWalker];
+#pragma unroll
+                for (int u = 0; u < kTreesPerWalker; ++u) w[u] = lds_u32(base + u * slot_bytes + idx[u] * 4u);
+#pragma unroll
+                for (int u = 0; u < kTreesPerWalker; ++u) c[u] = lds_u8(min(w[u] >> 16, fmax) * pitch + lane_at);
+#pragma unroll
+                for (int u = 0; u < kTreesPerWalker; ++u) {
+                    const uint32_t code = BITS == 4 ? (c[u] >> nibble) & 0xFu : c[u];
+                    idx[u] = __byte_perm(w[u] + code, 0u, 0x4441u);  // (a code above the threshold carries into the child)
+                }
+            }
+            float* out = term + (b & 1) * TB * TR;
+#pragma unroll
+            for (int u = 0; u < kTreesPerWalker; ++u)
+                out[u * TR] = __fmul_rn(a.weight, __uint_as_float(lds_u32(base + u * slot_bytes + idx[u] * 4u)));
+        }
+    } else {
+        const int my_row = warp * 64 + 2 * lane;         // and the next one
+        float2 start = make_float2(0.f, 0.f);
+        if (a.init) {
+            if (my_row < nr) start.x = a.init[row0 + my_row];
+            if (my_row + 1 < nr) start.y = a.init[row0 + my_row + 1];
+        }
+        unsigned long long acc = (unsigned long long)__float_as_uint(start.y) << 32 | __float_as_uint(start.x);
+        const unsigned long long* term = reinterpret_cast<const unsigned long long*>(s_term + my_row);
+        for (int b = 0; b <= n_batches; ++b) {
+            __syncthreads();
+            if (b == 0) continue;
+            const int t0 = (b - 1) * TB, nt = min(TB, a.n_trees - t0);
+            const unsigned long long* in = term + ((b - 1) & 1) * TB * TR / 2;
+            for (int k0 = 0; k0 < nt; k0 += kAddGroup) {
+                unsigned long long v[kAddGroup];
+#pragma unroll
+                for (int u = 0; u < kAddGroup; ++u) v[u] = in[(k0 + u) * TR / 2];
+                // A lone warp pays some 20 cycles for a branch, five additions' worth: the usual pack sizes
+                // run straight through eight trees.
+                switch (k0 + kAddGroup <= nt ? a.rep : 0) {
+                    case 1: add_times<1>(acc, v); break;
+                    case 2: add_times<2>(acc, v); break;
+                    case 4: add_times<4>(acc, v); break;
+                    case 8: add_times<8>(acc, v); break;
+                    case 16: add_times<16>(acc, v); break;
+                    case 32: add_times<32>(acc, v); break;
+                    case 64: add_times<64>(acc, v); break;
+                    default:
+                        for (int u = 0; u < kAddGroup && k0 + u < nt; ++u) {
+                            int n = a.repeat ? __ldg(a.repeat + t0 + k0 + u) : a.rep;
+                            const unsigned long long vu = in[(k0 + u) * TR / 2];
+                            for (; n >= 16; n -= 16) {
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) add2(acc, vu);
+                            }
+                            for (; n >= 4; n -= 4) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) add2(acc, vu);
+                            }
+                            for (; n > 0; --n) add2(acc, vu);
+                        }
+                }
+            }
+        }
+        if (my_row < nr) a.out[row0 + my_row] = __uint_as_float((uint32_t)acc);
+        if (my_row + 1 < nr) a.out[row0 + my_row + 1] = __uint_as_float((uint32_t)(acc >> 32));
+    }
+}
+
 __global__ void __launch_bounds__(256) predict_bins_fm_kernel(
     const uint8_t* __restrict__ bins, int n_features, int64_t n_rows, const int32_t* __restrict__ feature,
     const int32_t* __restrict__ threshold, const int32_t* __restrict__ left, const int32_t* __restrict__ right,
@@ -573,5 +812,286 @@ extern "C" int pb_predict_rows_packed(const uint8_t* codes, int64_t n_rows, int6
     }
     count_launch(1);
     PB_LAUNCH_CHECK("predict_rows_packed_kernel");
+    return PB_OK;
+}
+
+extern "C" int pb_predict_forest(const uint8_t* codes, int64_t n_rows, int64_t pitch_row, int64_t code_bits,
+                                 int64_t n_features, const void* trees, int64_t copies, int64_t slot_nodes, int64_t depth,
+                                 const int32_t* repeat, int64_t total_repeat, int64_t n_trees, float weight, float* out,
+                                 const float* init, void* stream_) {
+    PB_REQUIRE(codes && trees && out, "null buffer");
+    PB_REQUIRE(code_bits == 4 || code_bits == 8, "code_bits must be 4 or 8");
+    PB_REQUIRE(pitch_row >= 16 && pitch_row % 16 == 0, "pitch_row must be a positive multiple of 16");
+    PB_REQUIRE(n_features >= 1 && n_features <= pitch_row * (code_bits == 4 ? 2 : 1) && n_features < (1ll << 24),
+               "n_features out of range");
+    PB_REQUIRE(((uintptr_t)codes % 16) == 0 && ((uintptr_t)trees % 16) == 0, "codes / trees must be 16-byte aligned");
+    PB_REQUIRE(slot_nodes >= 4 && slot_nodes <= 256 && slot_nodes % 4 == 0, "slot_nodes must be a multiple of 4 up to 256");
+    PB_REQUIRE(depth >= 0 && depth <= 255, "depth out of range");
+    PB_REQUIRE(copies >= 1 && copies <= 1024, "copies out of range");
+    PB_REQUIRE(n_trees >= 0 && n_trees < (1ll << 31), "n_trees out of range");
+    PB_REQUIRE(total_repeat >= 0, "total_repeat out of range");
+    cudaStream_t stream = (cudaStream_t)stream_;
+    if (n_rows <= 0) return PB_OK;
+    if (n_trees == 0) {
+        if (init) PB_CUDA_TRY(cudaMemcpyAsync(out, init, (size_t)n_rows * 4, cudaMemcpyDeviceToDevice, stream));
+        else PB_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)n_rows * 4, stream));
+        return PB_OK;
+    }
+    PB_REQUIRE(repeat || (total_repeat % n_trees == 0 && total_repeat / n_trees < (1ll << 31)),
+               "without per-tree counts every tree is added total_repeat / n_trees times");
+    PredictForestArgs a{codes, n_rows, pitch_row, (int)n_features, static_cast<const uint32_t*>(trees), (int)copies, (int)slot_nodes,
+                        (int)depth, repeat, repeat ? 0 : (int)(total_repeat / n_trees), (int)n_trees, weight, out, init, 0, 0};
+    // Launch shape: groups of 32 rows per CTA and walkers per group.  Per tree a resident row costs its
+    // walkers `depth` steps of about 170 cycles, four trees and walk_warps walkers at a time, and its
+    // adder `adds` dependent additions of 4.2 cycles (the two overlap); an SM issues about 10
+    // instructions per step and warp and 0.6 per addition, four per cycle, and a batch costs a barrier.
+    // The slower of the two sets the time of a wave of CTAs.
+    const double adds = (double)total_repeat / (double)n_trees;
+    double best = 1e300;
+    size_t best_smem = 0;
+    for (int g = 1; g <= 8; ++g) {
+        for (int ww = kAddGroup / kTreesPerWalker; ww <= 8; ww *= 2) {
+            const int threads = forest_threads(g, ww);
+            if (threads > 1024) continue;
+            const double tb = kTreesPerWalker * ww;
+            const int64_t smem = forest_smem(n_features, (int)code_bits, g, ww, slot_nodes);
+            if (smem > 227 * 1024) continue;
+            int per_sm = (int)(228 * 1024 / (smem + 1024));
+            if (per_sm > 2048 / threads) per_sm = 2048 / threads;
+            const double ctas = (double)((n_rows + 32 * g - 1) / (32 * g));
+            const double waves = ctas <= 148.0 * per_sm ? 1.0 : ctas / (148.0 * per_sm);
+            double here = ctas / 148.0;                 // CTAs an SM holds at a time
+            here = here < 1.0 ? 1.0 : (here > per_sm ? per_sm : here);
+            const double walk = ((double)depth * 170.0 + 100.0) / tb, sum = adds * 4.2 + 10.0;
+            const double issue = here * g * ((10.5 * (double)depth + 12.0) + 0.6 * adds + 8.0) / 4.0;
+            const double latency = (walk > sum ? walk : sum) + 80.0 / tb;
+            // (every CTA brings the trees in: about 24 bytes a cycle, half of it beside the rest)
+            const double cost = waves * ((latency > issue ? latency : issue) + here * (double)slot_nodes * 4.0 / 48.0);
+            if (cost < best) {
+                best = cost;
+                a.groups = g;
+                a.walk_warps = ww;
+                best_smem = (size_t)smem;
+            }
+        }
+    }
+    PB_REQUIRE(a.groups > 0, "a row of %lld features does not fit in shared memory: use pb_predict_rows_packed",
+               (long long)n_features);
+    static const int* const forced = [] {  // PACKBOOST_FOREST_SHAPE="groups walkers" (tuning)
+        static int v[2];
+        const char* e = getenv("PACKBOOST_FOREST_SHAPE");
+        return (e && sscanf(e, "%d %d", &v[0], &v[1]) == 2) ? v : (const int*)nullptr;
+    }();
+    if (forced && forced[0] >= 1 && forced[1] >= 1 && forced[1] * kTreesPerWalker % kAddGroup == 0 && forest_threads(forced[0], forced[1]) <= 1024 &&
+        forest_smem(n_features, (int)code_bits, forced[0], forced[1], slot_nodes) <= 227 * 1024) {
+        a.groups = forced[0];
+        a.walk_warps = forced[1];
+        best_smem = (size_t)forest_smem(n_features, (int)code_bits, forced[0], forced[1], slot_nodes);
+    }
+    const int R = 32 * a.groups;
+    const unsigned grid = (unsigned)((n_rows + R - 1) / R);
+    const int threads = forest_threads(a.groups, a.walk_warps);
+    if (code_bits == 4) {
+        PB_CUDA_TRY(cudaFuncSetAttribute(predict_forest_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best_smem));
+        predict_forest_kernel<4><<<grid, threads, best_smem, stream>>>(a);
+    } else {
+        PB_CUDA_TRY(cudaFuncSetAttribute(predict_forest_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best_smem));
+        predict_forest_kernel<8><<<grid, threads, best_smem, stream>>>(a);
+    }
+    count_launch(1);
+    PB_LAUNCH_CHECK("predict_forest_kernel");
+    return PB_OK;
+}
+
+extern "C" int64_t pb_predict_forest_fits(int64_t n_features, int64_t code_bits, int64_t slot_nodes) {
+    return forest_smem(n_features, (int)code_bits, 1, kAddGroup / kTreesPerWalker, slot_nodes) <= 227 * 1024 ? 1 : 0;
+}
+
+// ---- a whole prediction in one call ----------------------------------------------------------------------
+
+static int64_t up256(int64_t v) { return (v + 255) / 256 * 256; }
+
+// Tables this small are read by the packing kernel from page-locked host memory, and the predictions
+// are written there, which saves two copies on the stream (about 10 us of a 64-row call); their codes
+// are range-checked on the host.
+static const int64_t kTableInPlace = 128 << 10;
+
+struct TablePlan {
+    int64_t raw, pitch, in_place, dev_bytes, pinned_bytes, off_codes, off_raw, off_in;
+};
+
+static TablePlan table_plan(const pb_model* m, int64_t on_device, int64_t n_rows, int64_t n_features) {
+    TablePlan p;
+    p.raw = n_rows * n_features * (m->edges ? 4 : 1);
+    p.pitch = ((m->code_bits == 4 ? (n_features + 1) / 2 : n_features) + 15) / 16 * 16;
+    p.in_place = (!on_device && p.raw <= kTableInPlace) ? 1 : 0;
+    p.off_codes = up256(16 + n_rows * 4);   // after the range word and the predictions
+    p.off_raw = p.off_codes + up256(n_rows * p.pitch);
+    p.dev_bytes = p.off_raw + (on_device || p.in_place ? 0 : up256(p.raw));
+    p.off_in = up256(16 + n_rows * 4);
+    p.pinned_bytes = p.off_in + (on_device ? 0 : p.in_place ? up256(p.raw) : pb_upload_ring_bytes(p.raw));
+    return p;
+}
+
+static int check_model(const pb_model* m, int64_t n_rows, int64_t n_features) {
+    PB_REQUIRE(m && m->trees && m->n_trees >= 1, "the model has no trees");
+    PB_REQUIRE(n_rows >= 1 && n_features >= 1 && n_features < (1ll << 24) && n_rows < (1ll << 40), "bad shape");
+    PB_REQUIRE(m->code_bits == 4 || m->code_bits == 8, "code_bits must be 4 or 8");
+    return PB_OK;
+}
+
+extern "C" int pb_predict_table_bytes(const pb_model* m, int64_t x_on_device, int64_t n_rows, int64_t n_features,
+                                      int64_t* dev_bytes, int64_t* pinned_bytes) {
+    int rc = check_model(m, n_rows, n_features);
+    if (rc) return rc;
+    PB_REQUIRE(dev_bytes && pinned_bytes, "null argument");
+    const TablePlan p = table_plan(m, x_on_device, n_rows, n_features);
+    *dev_bytes = p.dev_bytes;
+    *pinned_bytes = p.pinned_bytes;
+    return PB_OK;
+}
+
+extern "C" int pb_predict_table(const pb_model* m, const void* x, int64_t x_on_device, int64_t n_rows, int64_t n_features,
+                                void* dev, int64_t dev_bytes, void* pinned, int64_t pinned_bytes, float* out,
+                                int64_t* top, void* stream_) {
+    int rc = check_model(m, n_rows, n_features);
+    if (rc) return rc;
+    PB_REQUIRE(x && dev && pinned && out && top, "null buffer");
+    const TablePlan p = table_plan(m, x_on_device, n_rows, n_features);
+    PB_REQUIRE(dev_bytes >= p.dev_bytes && pinned_bytes >= p.pinned_bytes, "scratch too small");
+    PB_REQUIRE((uintptr_t)dev % 256 == 0 && (uintptr_t)pinned % 16 == 0, "scratch is misaligned");
+    cudaStream_t stream = (cudaStream_t)stream_;
+    char* d = static_cast<char*>(dev);
+    char* h = static_cast<char*>(pinned);
+    *top = 0;
+    uint32_t* d_top = nullptr;
+    const void* src = x;
+    float* pred = reinterpret_cast<float*>((p.in_place ? h : d) + 16);
+    if (p.in_place) {
+        memcpy(h + p.off_in, x, (size_t)p.raw);
+        src = h + p.off_in;
+        if (!m->edges) {
+            const uint8_t* b = static_cast<const uint8_t*>(x);
+            uint8_t t = 0;
+            for (int64_t i = 0; i < p.raw; ++i) t = b[i] > t ? b[i] : t;
+            *top = t;
+        }
+    } else {
+        if (!m->edges) {
+            d_top = reinterpret_cast<uint32_t*>(d);
+            PB_CUDA_TRY(cudaMemsetAsync(d_top, 0, 16, stream));
+        }
+        if (!x_on_device) {
+            rc = pb_upload(d + p.off_raw, x, p.raw, h + p.off_in, pinned_bytes - p.off_in, stream_);
+            if (rc) return rc;
+            src = d + p.off_raw;
+        }
+    }
+    uint8_t* codes = reinterpret_cast<uint8_t*>(d + p.off_codes);
+    rc = pb_pack_rows_top(src, m->edges ? 1 : 0, n_rows, n_features, m->edges, m->n_edges, m->max_bins, codes, p.pitch,
+                          m->code_bits, d_top, stream_);
+    if (rc == PB_OK)
+        rc = pb_predict_forest(codes, n_rows, p.pitch, m->code_bits, n_features, m->trees, m->copies, m->slot_nodes, m->depth,
+                               m->repeat, m->total_repeat, m->n_trees, (float)m->weight, pred, nullptr, stream_);
+    if (rc == PB_OK && !p.in_place) {
+        cudaError_t e = cudaMemcpyAsync(h, d, (size_t)(16 + n_rows * 4), cudaMemcpyDeviceToHost, stream);
+        if (e != cudaSuccess) rc = fail_cuda(e, "pb_predict_table");
+    }
+    // (the scratch is the caller's again after this, also when something failed)
+    cudaError_t e = cudaStreamSynchronize(stream);
+    if (rc) return rc;
+    if (e != cudaSuccess) return fail_cuda(e, "pb_predict_table");
+    if (d_top) *top = (int64_t)*reinterpret_cast<uint32_t*>(h);
+    memcpy(out, h + 16, (size_t)n_rows * 4);
+    return PB_OK;
+}
+
+// ---- forests in the one-word form (host) ---------------------------------------------------------------------
+
+// Depths of the nodes of one tree and the words it takes once every path is `depth` splits long; false
+// when the tree is not a proper one (children inside the tree and after their parent, ids in range).
+static bool tree_depths(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                        const uint8_t* is_leaf, int64_t n, std::vector<int32_t>& depth, int32_t* deepest, bool* adjacent) {
+    if (n < 1) return false;
+    depth.assign((size_t)n, 0);
+    for (int64_t i = 0; i < n; ++i) {
+        if (is_leaf[i]) continue;
+        const int64_t l = left[i], r = right[i];
+        if (l <= i || r <= i || l >= n || r >= n || feature[i] < 0 || threshold[i] < 0 || threshold[i] >= 256) return false;
+        if (r != l + 1 || feature[i] >= (1 << 16)) *adjacent = false;
+        depth[l] = depth[r] = depth[i] + 1;
+    }
+    // (only nodes that are reached count)
+    std::vector<uint8_t> seen((size_t)n, 0);
+    seen[0] = 1;
+    for (int64_t i = 0; i < n; ++i) {
+        if (!seen[i]) {
+            depth[i] = -1;
+            continue;
+        }
+        if (is_leaf[i]) *deepest = depth[i] > *deepest ? depth[i] : *deepest;
+        else seen[left[i]] = seen[right[i]] = 1;
+    }
+    return true;
+}
+
+extern "C" int pb_forest_shape(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                               const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                               int64_t* slot_nodes, int64_t* depth_out) {
+    PB_REQUIRE(feature && threshold && left && right && value && is_leaf && offsets && slot_nodes && depth_out, "null buffer");
+    *slot_nodes = 0;
+    int32_t deepest = 0;
+    bool adjacent = true;
+    std::vector<std::vector<int32_t>> depths((size_t)n_trees);
+    for (int64_t t = 0; t < n_trees; ++t) {
+        const int64_t o = offsets[t], n = (int64_t)offsets[t + 1] - o;
+        PB_REQUIRE(n >= 1 && tree_depths(feature + o, threshold + o, left + o, right + o, is_leaf + o, n, depths[t], &deepest, &adjacent),
+                   "tree %lld is malformed", (long long)t);
+    }
+    if (!adjacent || deepest > 16) return PB_OK;
+    int64_t most = 0;
+    for (int64_t t = 0; t < n_trees; ++t) {
+        const int64_t o = offsets[t], n = (int64_t)offsets[t + 1] - o;
+        int64_t words = n;
+        for (int64_t i = 0; i < n; ++i)
+            if (is_leaf[o + i] && depths[t][i] >= 0) words += deepest - depths[t][i];
+        most = words > most ? words : most;
+        if (most > 256) return PB_OK;
+    }
+    *slot_nodes = (most + 3) / 4 * 4;
+    *depth_out = deepest;
+    return PB_OK;
+}
+
+extern "C" int pb_forest_words(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                               const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                               int64_t slot_nodes, int64_t depth, uint32_t* out) {
+    PB_REQUIRE(feature && threshold && left && right && value && is_leaf && offsets && out, "null buffer");
+    std::vector<int32_t> at;
+    memset(out, 0, (size_t)(n_trees * slot_nodes) * 4);
+    for (int64_t t = 0; t < n_trees; ++t) {
+        const int64_t o = offsets[t], n = (int64_t)offsets[t + 1] - o;
+        uint32_t* w = out + t * slot_nodes;
+        int32_t deepest = 0;
+        bool adjacent = true;
+        PB_REQUIRE(n >= 1 && tree_depths(feature + o, threshold + o, left + o, right + o, is_leaf + o, n, at, &deepest, &adjacent) &&
+                       adjacent && deepest <= depth,
+                   "tree %lld does not have the shape pb_forest_shape found", (long long)t);
+        int64_t next = n;   // words of led-on leaves are appended
+        for (int64_t i = 0; i < n; ++i) {
+            if (at[i] < 0) continue;
+            if (!is_leaf[o + i]) {
+                w[i] = (uint32_t)feature[o + i] << 16 | (uint32_t)left[o + i] << 8 | (uint32_t)(255 - threshold[o + i]);
+                continue;
+            }
+            int64_t here = i;
+            for (int64_t d = at[i]; d < depth; ++d) {
+                PB_REQUIRE(next < slot_nodes, "tree %lld needs more than %lld words", (long long)t, (long long)slot_nodes);
+                w[here] = (uint32_t)next << 8;
+                here = next++;
+            }
+            memcpy(w + here, value + o + i, 4);
+        }
+    }
     return PB_OK;
 }

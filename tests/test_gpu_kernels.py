@@ -323,3 +323,35 @@ def test_upload_moves_every_byte(nbytes):
     for _ in range(2):
         got = uploads(src, torch.uint8)
         np.testing.assert_array_equal(got.cpu().numpy(), src)
+
+
+@pytest.mark.parametrize("rows,features,bins,depth,trees", [
+    (1, 1, 2, 0, 1), (31, 7, 5, 1, 3), (33, 8, 16, 3, 9), (257, 300, 5, 6, 40), (500, 2376, 5, 6, 17),
+    (64, 33, 64, 5, 8), (999, 257, 128, 7, 33), (4099, 20, 5, 7, 5), (20_000, 64, 5, 4, 12)])
+def test_small_tree_predictor_equals_the_general_one(rows, features, bins, depth, trees):
+    """Bit for bit, with partial row groups and batches, uneven repeats, early leaves and a start value."""
+    from packboost_b200 import PackBoost, PackBoostConfig
+    from packboost_b200.booster import TreeBuilder
+    rng = np.random.default_rng(rows + features)
+    X = torch.from_numpy(rng.integers(0, bins, size=(rows, features), dtype=np.uint8)).to(_dev())
+    forest = []
+    for t in range(trees):
+        tb = TreeBuilder()
+        level = [0]
+        for d in range(depth):
+            keep = [n for n in level if d == 0 or rng.random() > 0.1]
+            level = [c for n in keep for c in tb.split(n, int(rng.integers(features)), int(rng.integers(bins - 1)))]
+        for node in tb.nodes:
+            node.value = float(np.float32(rng.normal()))
+        forest.append(tb.build())
+    model = PackBoost(PackBoostConfig(max_bins=bins, prebinned=True))
+    model.set_forest(forest, 0.3, repeats=[int(v) for v in rng.integers(0, 20, trees)])
+    packed, _ = model._pack_rows(X)
+    small = model._pack_forest(model._distinct)
+    assert "slots" in small
+    large = {k: v for k, v in small.items() if k != "slots"}
+    init = torch.from_numpy(rng.normal(size=rows).astype(np.float32)).to(_dev())
+    for start in (None, init):
+        got = model._predict_packed(packed, small, init=start)
+        want = model._predict_packed(packed, dict(large), init=start)
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
