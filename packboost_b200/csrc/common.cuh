@@ -226,6 +226,41 @@ int launch_score(const ScoreLaunch& s, cudaStream_t stream);
 // stored histogram: thr_out[f][n_thr].
 int launch_mass_thresholds(const uint32_t* cnt, int n_feat, const int32_t* n_nodes_ptr, int n_nodes_max, int node_stride,
                            int n_eras, int max_bins, int n_thr, int32_t* thr_out, cudaStream_t stream);
+// ---- histogram and score in one kernel (walk.cu) --------------------------------------------
+
+struct WalkLaunch {
+    const uint8_t* codes;        // 8-bit codes
+    int64_t pitch;
+    const int32_t* feat_rows;
+    const int32_t* feat_pos;
+    int n_feat;
+    int n_rows;
+    const int32_t* gq;
+    const uint16_t* slot;
+    const int32_t* era_offsets;
+    int n_eras;
+    int max_bins;
+    int tile_rows;               // most rows the count field of a cell holds
+    int max_era_rows;
+    const int32_t* n_nodes_ptr;
+    int n_nodes;                 // upper bound
+    int node_stride;
+    int count_bits, lo_bits;
+    const int32_t* thr_ids;      // [n_thr] ascending bin ids; unused with `mass`
+    int n_thr;
+    uint32_t* mass;              // [n_feat][256] scratch of the mass cuts, or null
+    const float* inv_scale_ptr;
+    const FrontierNode* frontier;
+    const int32_t* any_dir_ptr;
+    float lambda_l2, lambda_dro, direction_weight, era_alpha;
+    int direction_form;
+    int min_samples_leaf;
+    Cand* cand;
+    void* prof;
+    uint32_t* debug_flags;
+    int cell_nodes, div_table;   // set by launch_walk
+};
+int launch_walk(WalkLaunch a, cudaStream_t stream);
 size_t score_scratch_bytes_per_feature(int node_stride, int n_eras, int n_thr);
 
 }  // namespace pb

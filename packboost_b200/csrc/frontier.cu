@@ -678,6 +678,58 @@ static bool use_fused_flush(const pb_train_state* st, int64_t depth) {
     return hist_can_fuse(hist_launch_of(st, depth, c));
 }
 
+// Tables of many bins are accumulated and scored by one kernel that walks the eras (walk.cu); a CTA
+// works through all rows of its feature, so few features of very many rows keep the two-step path,
+// which cuts the rows (PACKBOOST_WALK=0 keeps it everywhere, for comparisons).
+static bool use_walk(const pb_train_state* st, int64_t n_feat) {
+    static const bool enabled = [] {
+        const char* e = getenv("PACKBOOST_WALK");
+        return !(e && e[0] == '0' && e[1] == 0);
+    }();
+    return enabled && st->code_bits == 8 && n_feat <= 65535 && (n_feat >= 32 || st->n_rows <= (1 << 18));
+}
+
+static int walk_depth(const pb_train_state* st, int64_t depth, const int32_t* feat_rows, const int32_t* feat_pos, int64_t n_feat,
+                      void* mass, Cand* cand, cudaStream_t stream) {
+    Ctl c = ctl_view(st->ctl);
+    WalkLaunch w;
+    memset(&w, 0, sizeof(w));
+    w.codes = st->codes;
+    w.pitch = st->pitch;
+    w.feat_rows = feat_rows;
+    w.feat_pos = feat_pos;
+    w.n_feat = (int)n_feat;
+    w.n_rows = (int)st->n_rows;
+    w.gq = st->gq;
+    w.slot = st->slot;
+    w.era_offsets = st->era_offsets;
+    w.n_eras = (int)st->n_eras;
+    w.max_bins = (int)st->max_bins;
+    w.tile_rows = kTileRowsMax;
+    w.max_era_rows = (int)st->max_era_rows;
+    w.n_nodes_ptr = &c.head->n_ctx[depth];
+    w.n_nodes = node_stride_of(depth);
+    w.node_stride = node_stride_of(depth);
+    w.count_bits = (int)st->count_bits;
+    w.lo_bits = (int)st->lo_bits;
+    w.thr_ids = st->thr_ids;
+    w.n_thr = (int)st->n_thresholds;
+    w.mass = st->cut_mass ? static_cast<uint32_t*>(mass) : nullptr;
+    w.inv_scale_ptr = &c.head->inv_scale;
+    w.frontier = c.frontier[depth & 1];
+    w.any_dir_ptr = &c.head->any_dir[depth];
+    w.lambda_l2 = (float)st->lambda_l2;
+    w.lambda_dro = (float)st->lambda_dro;
+    w.direction_weight = (float)st->direction_weight;
+    w.era_alpha = (float)(st->era_alpha > 0.0 ? st->era_alpha : 0.0);
+    w.direction_form = st->direction_form ? 1 : 0;
+    w.min_samples_leaf = (int)st->min_samples_leaf;
+    w.cand = cand;
+    w.prof = st->profile;
+    w.debug_flags = &c.head->debug_flags;
+    return launch_walk(w, stream);
+}
+
 static int hist_score_blocks(const pb_train_state* st, int64_t depth, const int32_t* feat_rows, const int32_t* feat_pos,
                              int64_t n_feat, char* scratch, const BlockPlan& plan, Cand* cand, cudaStream_t stream) {
     Ctl c = ctl_view(st->ctl);
@@ -849,6 +901,9 @@ extern "C" int pb_depth_hist_score(const pb_train_state* st, int64_t depth, cons
     const size_t cand_bytes = align_up(sizeof(Cand) * (size_t)n_sampled * stride, 256);
     PB_REQUIRE((int64_t)cand_bytes < st->workspace_bytes, "workspace too small for the candidate table");
     char* ws = static_cast<char*>(st->workspace);
+    const int64_t mass_bytes = st->cut_mass ? n_feat * 256 * (int64_t)sizeof(uint32_t) : 0;
+    if (use_walk(st, n_feat) && (int64_t)cand_bytes + mass_bytes <= st->workspace_bytes)
+        return walk_depth(st, depth, feat_rows, feat_pos, n_feat, ws + cand_bytes, reinterpret_cast<Cand*>(ws), (cudaStream_t)stream_);
     BlockPlan plan;
     PB_REQUIRE(plan_block((size_t)st->workspace_bytes - cand_bytes, stride, st->n_eras, st->max_bins, st->n_thresholds,
                           n_feat, use_fused_flush(st, depth), &plan),

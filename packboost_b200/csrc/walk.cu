@@ -1,0 +1,601 @@
+// Histogram and scorer of one depth in one kernel, for tables of many bins (8-bit codes).
+//
+// With more than 16 bins a stored histogram is the largest thing a depth moves: 12 bytes per
+// (feature, era, node, bin) written and read back, then 8 bytes per threshold of (gain, weight) written
+// and read again - 13 GB for one round of 500 000 rows, 256 features, 100 eras, 128 bins and depth 6,
+// against 0.9 GB of codes and row state.  None of it outlives its era: the score of a threshold is a
+// Welford recursion over the eras in ascending order.  So a CTA owns one feature and up to sixteen
+// frontier nodes and walks the eras; the state of the recursion stays in registers to the end, and what
+// leaves the CTA is one candidate per node.
+//
+// Cells are the two words of the histogram kernel (sum of low gradient bits << CB | count, sum of high
+// bits).  The eras go by in batches of sixteen (era, node) pairs, sixteen eras at one node, one at
+// sixteen: (a) all warps add the rows of the batch to its cells; (b) a warp per pair scans the bins (a
+// lane per BPL consecutive ones), computes the gains and leaves them in shared memory; (c) a thread per
+// threshold advances the recursion through the eras of the batch.  So the latency of the scan, its
+// shuffles and divisions, is paid once a batch by sixteen warps side by side.  An era of more rows than
+// the count field holds is cut into tiles whose prefix sums are added up before (b) goes on.
+//
+// Divisions: every divisor of the gains is count + lambda, so an era's divisors and their correctly
+// rounded reciprocals come from a table in shared memory, and a quotient takes two corrected products
+// instead of a general division (see divide_by).
+//
+// Bound: the shared-memory atomics (two per row and feature, about four wavefronts each with 128 bins)
+// at the upper depths, the gains at the lower ones.
+// 500 000 rows x 256 features, 100 eras, 128 bins, by depth: 0.23, 0.27, 0.31, 0.40, 0.59, 1.13 ms, 2.9 ms a
+// round (histogram, gain and chain kernels: 4.6 ms); 200 000 x 100, depth 10: 3.2 ms a round (6.1).
+//
+// Float arithmetic as in the scorer: the same separately rounded operations in the same order
+// (this file is compiled with -fmad=false), so candidates are bit-identical to the other path's.
+
+#include "common.cuh"
+#include "des_math.cuh"
+
+namespace pb {
+
+namespace {
+
+constexpr int kWalkWarps = 16;
+constexpr int kWalkThreads = 32 * kWalkWarps;
+constexpr int kWalkNodes = kWalkWarps;   // (era, node) pairs of a batch, and most nodes of a CTA: one warp each
+constexpr int kWalkInv = 4096;           // longest table of era reciprocals
+
+struct RowGroup {                        // four consecutive rows
+    uint32_t codes;
+    uint2 slots;
+    int4 gq;
+};
+
+__device__ __forceinline__ float sign3(float v) { return v > 0.f ? 1.f : (v < 0.f ? -1.f : v); }
+
+// a / d, correctly rounded, from d and y = 1 / d correctly rounded.  Markstein (Computation of
+// elementary functions on the IBM RISC System/6000, 1990): when q is within one ulp of a / d and
+// r = a - d q is exact, q + r y rounds to the correctly rounded quotient.  The product a y is within two
+// ulps; the first correction brings it within one, the second is the theorem's.  Valid while no
+// intermediate leaves the normal range (division_in_range; zero numerators give zero).
+__device__ __forceinline__ float divide_by(float a, float2 dy) {
+    float q = f_mul(a, dy.y);
+    q = __fmaf_rn(__fmaf_rn(-dy.x, q, a), dy.y, q);
+    return __fmaf_rn(__fmaf_rn(-dy.x, q, a), dy.y, q);
+}
+
+// Gradient sums are multiples of inv_scale below 2^44 inv_scale, so the squares divided here are zero or
+// between inv_scale^2 / 2 and 2^88 inv_scale^2, the divisors between lambda and 2^13 + lambda.
+__device__ __forceinline__ bool division_in_range(float inv_scale, float lam) {
+    return inv_scale >= 3.5527137e-15f && inv_scale <= 32.f && lam >= 5.9604645e-8f && lam <= 16777216.f;  // 2^-48, 2^5; 2^-24, 2^24
+}
+
+// Thresholds of one feature at the count-mass quantiles of its bins over all frontier rows, as the
+// reference's compiled split finder takes them (packboost/backends/cpu/frontier_cpu.cpp:35-109): targets
+// i / (k - 1) of total * (1 - 1e-12) in float64, a threshold one below the first bin whose cumulative
+// mass reaches the target, evenly spaced ids when targets coincide, the k smallest.  Called by all
+// threads; s_m: bin masses (cumulated here), s_set: 0 / 1 per bin on return.
+__device__ void mass_cut_set(uint32_t* s_m, uint8_t* s_set, int nb, int K) {
+    const int max_thr = max(1, nb - 1), kk = max(1, min(K, max_thr));
+    const int lane = threadIdx.x & 31;
+    __shared__ int s_have;
+    if (threadIdx.x < 32) {              // inclusive prefix of up to 256 masses, eight per lane
+        uint32_t v[8], run = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            run += (lane * 8 + j < nb) ? s_m[lane * 8 + j] : 0u;
+            v[j] = run;
+        }
+        uint32_t incl = run;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += up;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (lane * 8 + j < nb) s_m[lane * 8 + j] = v[j] + incl - run;
+    }
+    for (int b = threadIdx.x; b < 256; b += blockDim.x) s_set[b] = 0;
+    if (threadIdx.x == 0) s_have = 0;
+    __syncthreads();
+    const uint32_t total = s_m[nb - 1];
+    if (total > 0) {
+        const double upper = (double)total * (1.0 - 1e-12);
+        for (int i = threadIdx.x; i < kk; i += blockDim.x) {
+            const double alpha = (kk == 1) ? 0.0 : (double)i / (double)(kk - 1);
+            const double target = upper * alpha;
+            int idx = nb - 1;
+            for (int b = 0; b < nb; ++b)
+                if (!((double)s_m[b] < target)) {
+                    idx = b;
+                    break;
+                }
+            s_set[max(0, min(idx - 1, max_thr - 1))] = 1;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int have = 0;
+        for (int b = lane; b < max_thr; b += 32) have += s_set[b];
+        have = __reduce_add_sync(0xFFFFFFFFu, have);
+        if (lane == 0) s_have = have;
+    }
+    __syncthreads();
+    if (s_have < kk) {
+        if (kk == 1) {
+            if (threadIdx.x == 0) s_set[0] = 1;
+        } else {
+            const double step = (double)(max_thr - 1) / (double)(kk - 1);
+            for (int i = threadIdx.x; i < kk; i += blockDim.x) {
+                const long long idx = llround(round((double)i * step));
+                s_set[(int)max(0ll, min(idx, (long long)max_thr - 1))] = 1;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {          // (more than k ids now: the k smallest stay)
+            int w = 0;
+            for (int b = 0; b < max_thr; ++b)
+                if (s_set[b] && ++w > kk) s_set[b] = 0;
+        }
+    }
+    __syncthreads();
+}
+
+// Bin masses of the frontier rows of each feature: counts[f][256] += .  grid (feature, row part).
+__global__ void __launch_bounds__(256) mass_count_kernel(WalkLaunch a) {
+    __shared__ uint32_t s_m[8][257];
+    for (int i = threadIdx.x; i < 8 * 257; i += 256) (&s_m[0][0])[i] = 0u;
+    __syncthreads();
+    const int n_nodes = min(*a.n_nodes_ptr, a.n_nodes);
+    const int warp = threadIdx.x >> 5;
+    const uint8_t* codes = a.codes + (int64_t)a.feat_rows[blockIdx.x] * a.pitch;
+    // (rows past the end have no slot; the row arrays are padded)
+    for (int64_t g = blockIdx.y * 256 + threadIdx.x; 4 * g < a.n_rows; g += gridDim.y * 256) {
+        const uint32_t c = *reinterpret_cast<const uint32_t*>(codes + 4 * g);
+        const uint2 s = *reinterpret_cast<const uint2*>(a.slot + 4 * g);
+        const uint32_t sl[4] = {s.x & 0xFFFFu, s.x >> 16, s.y & 0xFFFFu, s.y >> 16};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if ((int)sl[j] < n_nodes) atomicAdd(&s_m[warp][(c >> (8 * j)) & 0xFFu], 1u);
+    }
+    __syncthreads();
+    uint32_t t = 0;
+    for (int w = 0; w < 8; ++w) t += s_m[w][threadIdx.x];
+    if (t) atomicAdd(a.mass + (size_t)blockIdx.x * 256 + threadIdx.x, t);
+}
+
+// What the state of a threshold has to hold (its registers decide how many CTAs an SM takes).
+constexpr int kUnit = 0;       // era weights 0 / 1, an era is one tile
+constexpr int kUnitTiles = 1;  // era weights 0 / 1, eras of several tiles
+constexpr int kGeneral = 2;    // any weights, directional term, any eras
+
+// Interleaved copies of the cells, for the lanes of a warp that meet in a bin: columns of few values
+// (32 lanes on ten bins) took twice as long as the others and were what a launch waited for.
+__host__ __device__ constexpr int walk_copies(int bpl) { return bpl <= 4 ? 2 : 1; }
+
+// Shared memory: cells [pairs][NBP][copies] word A, then word B | gains [pairs][NBP] | agreement [pairs][NBP]
+// (kGeneral) or 1 / n [eras + 1] | (divisor, reciprocal) [largest era + 1] when an era is one tile.
+// A pair's gains lie at i * 32 + lane for bin lane * BPL + i.
+template <int BPL, int MODE>
+__global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ? 2 : 1) walk_kernel(WalkLaunch a) {
+    constexpr bool UNIT = MODE != kGeneral, TILES = MODE != kUnit;
+    constexpr int NBP = 32 * BPL;        // bins of a pair's cells
+    constexpr int SLOTS = kWalkNodes * NBP / kWalkThreads;   // thresholds a thread may own
+    constexpr int plane = kWalkNodes * NBP;
+    constexpr int COPIES = walk_copies(BPL);
+    constexpr int words = plane * COPIES;                    // of word A; word B follows
+    extern __shared__ __align__(16) uint32_t s_cells[];      // [pairs][NBP][COPIES]
+    float2* s_gain = reinterpret_cast<float2*>(s_cells + 2 * words);
+    float* s_agree = reinterpret_cast<float*>(s_gain + plane);
+    float* s_inv = s_agree;
+    float2* s_div = reinterpret_cast<float2*>(s_agree + (UNIT ? (a.n_eras + 2) / 2 * 2 : plane));
+    __shared__ uint32_t s_mass[256];
+    __shared__ uint8_t s_set[256];
+    __shared__ int s_off[kWalkNodes + 2];                    // row ranges of the batch's eras
+    const int n_nodes = min(*a.n_nodes_ptr, a.n_nodes);
+    const int node0 = blockIdx.x * kWalkNodes;
+    const int live = min(kWalkNodes, n_nodes - node0);       // nodes of this CTA
+    if (live <= 0) return;
+    const int f = blockIdx.y;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nb = a.max_bins, E = a.n_eras, K = a.n_thr;
+    const int CN = a.cell_nodes;                             // nodes the cells hold: a power of two
+    const int EB = TILES ? 1 : kWalkNodes / CN;              // eras of a batch
+    const int CB = a.count_bits, LB = a.lo_bits;
+    const uint32_t lo_mask = (1u << LB) - 1u, cmask = (1u << CB) - 1u;
+    const float inv_scale = *a.inv_scale_ptr, lam = a.lambda_l2;
+    const bool table = a.div_table && division_in_range(inv_scale, lam);
+
+    for (int i = threadIdx.x; i < 2 * words; i += kWalkThreads) s_cells[i] = 0u;
+    if (UNIT)
+        for (int n = threadIdx.x; n <= E; n += kWalkThreads) s_inv[n] = n > 0 ? f_div(1.f, (float)n) : 0.f;
+    if (table)
+        for (int n = threadIdx.x; n <= a.max_era_rows; n += kWalkThreads) {
+            const float d = f_add((float)n, lam);
+            s_div[n] = make_float2(d, f_div(1.f, d));
+        }
+
+    // ---- which bins are thresholds ----
+    if (a.mass) {
+        for (int b = threadIdx.x; b < 256; b += kWalkThreads) s_mass[b] = a.mass[(size_t)f * 256 + b];
+        __syncthreads();
+        mass_cut_set(s_mass, s_set, nb, K);
+    } else {
+        for (int b = threadIdx.x; b < 256; b += kWalkThreads) s_set[b] = 0;
+        __syncthreads();
+        for (int k = threadIdx.x; k < K; k += kWalkThreads) s_set[a.thr_ids[k]] = 1;
+        __syncthreads();
+    }
+
+    // ---- rows: groups of four; a row of another CTA's node is predicated off, so the usual group has
+    //      no branch per row ----
+    const uint8_t* codes = a.codes + (int64_t)a.feat_rows[f] * a.pitch;
+    const bool sparse = gridDim.x > 1;   // most rows belong to other CTAs: gradients are read when a row is ours
+    constexpr uint32_t PAIR = 4u * NBP * COPIES;             // bytes of a pair's cells
+    const uint32_t cells_at = (uint32_t)__cvta_generic_to_shared(s_cells) + 4u * (threadIdx.x & (COPIES - 1));
+    auto load_group = [&](uint32_t g, int r1, RowGroup& x) {
+        if ((int)(4 * g) < r1) {
+            x.codes = *reinterpret_cast<const uint32_t*>(codes + 4 * g);
+            x.slots = *reinterpret_cast<const uint2*>(a.slot + 4 * g);
+            if (!sparse) x.gq = *reinterpret_cast<const int4*>(a.gq + 4 * g);
+        }
+    };
+    auto add_row = [&](uint32_t base, uint32_t n, uint32_t code, int q) {
+#ifdef PB_DEBUG_BOUNDS
+        const uint32_t sl = n + (uint32_t)node0;
+        if ((sl & 0xFFFFu) != kSlotNone && (int)sl >= a.n_nodes && a.debug_flags) atomicOr(a.debug_flags, kDbgSlot);
+        if (n < (uint32_t)live && code >= (uint32_t)nb) {
+            if (a.debug_flags) atomicOr(a.debug_flags, kDbgCode);
+            return;
+        }
+#endif
+        // (a byte that is no bin falls into a neighbour's cells or, after the last, into the gains)
+        asm volatile(
+            "{ .reg .pred p; setp.lt.u32 p, %0, %1;\n"
+            "@p red.shared.add.u32 [%2], %3;\n"
+            "@p red.shared.add.u32 [%2 + %5], %4; }\n" ::"r"(n), "r"(live), "r"(base + n * PAIR + code * (4u * COPIES)),
+            "r"((((uint32_t)q & lo_mask) << CB) + 1u), "r"(q >> LB), "n"(4 * words)
+            : "memory");
+    };
+    // `e`, `lim`: era of the batch at the thread's last row and where that era ends (rows ascend)
+    auto add_group = [&](uint32_t g, int r0, int r1, RowGroup& x, int& e, int& lim) {
+        const int r = (int)(4 * g);
+        if (!TILES)
+            while (r >= lim) lim = s_off[++e + 1];
+        const uint32_t n0 = (x.slots.x & 0xFFFFu) - (uint32_t)node0, n1 = (x.slots.x >> 16) - (uint32_t)node0;
+        const uint32_t n2 = (x.slots.y & 0xFFFFu) - (uint32_t)node0, n3 = (x.slots.y >> 16) - (uint32_t)node0;
+        if (sparse) {
+            if (min(min(n0, n1), min(n2, n3)) >= (uint32_t)live) return;
+            x.gq = *reinterpret_cast<const int4*>(a.gq + 4 * g);
+        }
+        const uint32_t here = cells_at + (TILES ? 0u : (uint32_t)(e * CN) * PAIR);
+        if (r >= r0 && r + 4 <= (TILES ? r1 : lim)) {
+            add_row(here, n0, x.codes & 0xFFu, x.gq.x);
+            add_row(here, n1, __byte_perm(x.codes, 0u, 0x4441u), x.gq.y);
+            add_row(here, n2, __byte_perm(x.codes, 0u, 0x4442u), x.gq.z);
+            add_row(here, n3, x.codes >> 24, x.gq.w);
+        } else {                         // rows of a neighbouring batch, or of several eras
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j) {
+                if (r + j >= r0 && r + j < r1) {
+                    int ej = e;
+                    if (!TILES)
+                        while (r + j >= s_off[ej + 1]) ++ej;
+                    add_row(cells_at + (TILES ? 0u : (uint32_t)(ej * CN) * PAIR), (x.slots.x & 0xFFFFu) - (uint32_t)node0,
+                            x.codes & 0xFFu, x.gq.x);
+                }
+                x.codes >>= 8;
+                x.slots.x = x.slots.x >> 16 | x.slots.y << 16;
+                x.slots.y >>= 16;
+                x.gq = make_int4(x.gq.y, x.gq.z, x.gq.w, 0);
+            }
+        }
+    };
+
+    // ---- the warp's pair: node warp % CN, every EB-th era from warp / CN on ----
+    const int my_node = warp & (CN - 1), my_era = warp / CN;
+    const bool scans = my_node < live && my_era < EB;
+    uint32_t lc_sum[BPL], pc[BPL], tc = 0u;
+    long long lg_sum[BPL], pg[BPL], tg = 0ll;
+#pragma unroll
+    for (int i = 0; i < BPL; ++i) {
+        lc_sum[i] = pc[i] = 0u;
+        lg_sum[i] = pg[i] = 0ll;
+    }
+    const long long g_par = scans ? a.frontier[node0 + my_node].gq : 0ll;
+    const bool use_dir = !UNIT && a.direction_weight != 0.f && (a.direction_form == 1 || *a.any_dir_ptr != 0);
+    const float pa = g_par > 0 ? -1.f : (g_par < 0 ? 1.f : 0.f);  // sign(-G / (H + lambda))
+
+    // ---- state of this thread's thresholds: slots t, t + 512, ... of [node][i * 32 + lane] ----
+    float mean[SLOTS], m2[SLOTS], wsum[UNIT ? 1 : SLOTS], a_num[UNIT ? 1 : SLOTS], a_den[UNIT ? 1 : SLOTS];
+    int n_valid[UNIT ? SLOTS : 1];
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+        mean[q] = m2[q] = 0.f;
+        if (UNIT) n_valid[q] = 0;
+        else wsum[q] = a_num[q] = a_den[q] = 0.f;
+    }
+    const int n_slots = live * NBP;
+
+    int e0 = 0, r0 = a.era_offsets[0], r1 = 0, ne = 0;       // eras [e0, e0 + ne), rows [r0, r1) of the batch
+    auto batch_end = [&]() {
+        ne = min(EB, E - e0);
+        const int end = ne > 0 ? a.era_offsets[e0 + ne] : r0;
+        r1 = TILES ? min(end, r0 + a.tile_rows) : end;
+        return TILES ? r1 >= end : true;                     // the batch completes its eras
+    };
+    bool complete = batch_end();
+    RowGroup cur;                        // the thread's next group of rows
+    load_group(r0 / 4 + threadIdx.x, r1, cur);
+    if (threadIdx.x <= kWalkNodes) s_off[threadIdx.x] = a.era_offsets[min((int)threadIdx.x, E)];
+    __syncthreads();                     // cells are zero; offsets and tables are there
+    while (ne > 0) {
+        // ---- (a) ----
+        {
+            int e = 0, lim = s_off[1];
+            for (uint32_t g = r0 / 4 + threadIdx.x; (int)(4 * g) < r1; g += kWalkThreads) {
+                RowGroup x = cur;
+                load_group(g + kWalkThreads, r1, cur);
+                add_group(g, r0, r1, x, e, lim);
+            }
+        }
+        const int n_eras_now = complete ? ne : 0;            // eras that (b) finishes
+        if (complete) e0 += ne;
+        r0 = r1;
+        complete = batch_end();
+        load_group(r0 / 4 + threadIdx.x, r1, cur);           // (on its way during (b) and (c))
+        __syncthreads();                 // the cells are complete, (c) of the batch before is done
+        if (threadIdx.x <= kWalkNodes) s_off[threadIdx.x] = a.era_offsets[min(e0 + (int)threadIdx.x, E)];
+
+        // ---- (b) prefix over the bins; the packed words are added as they are (the rows behind them are
+        //      distinct rows of a tile, so no field overflows) ----
+        if (scans && (TILES || my_era < n_eras_now)) {
+            uint32_t A[BPL], B[BPL];
+            uint32_t* at = s_cells + (warp * NBP + lane * BPL) * COPIES;
+#pragma unroll
+            for (int i = 0; i < BPL; ++i) {
+                A[i] = at[i * COPIES];
+                B[i] = at[words + i * COPIES];
+#pragma unroll
+                for (int c = 1; c < COPIES; ++c) {
+                    A[i] += at[i * COPIES + c];
+                    B[i] += at[words + i * COPIES + c];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < BPL * COPIES; ++i) at[i] = at[words + i] = 0u;
+#pragma unroll
+            for (int i = 1; i < BPL; ++i) {
+                A[i] += A[i - 1];
+                B[i] += B[i - 1];
+            }
+            uint32_t sa = A[BPL - 1], sb = B[BPL - 1];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t ua = __shfl_up_sync(0xFFFFFFFFu, sa, d), ub = __shfl_up_sync(0xFFFFFFFFu, sb, d);
+                if (lane >= d) {
+                    sa += ua;
+                    sb += ub;
+                }
+            }
+            const uint32_t ta = __shfl_sync(0xFFFFFFFFu, sa, 31), tb = __shfl_sync(0xFFFFFFFFu, sb, 31);
+            sa -= A[BPL - 1];
+            sb -= B[BPL - 1];
+            tc = (TILES ? tc : 0u) + (ta & cmask);
+            tg = (TILES ? tg : 0ll) + (long long)(int32_t)tb * (1ll << LB) + (long long)(ta >> CB);
+#pragma unroll
+            for (int i = 0; i < BPL; ++i) {
+                const uint32_t av = A[i] + sa, bv = B[i] + sb;
+                pc[i] = (TILES ? pc[i] : 0u) + (av & cmask);
+                pg[i] = (TILES ? pg[i] : 0ll) + (long long)(int32_t)bv * (1ll << LB) + (long long)(av >> CB);
+            }
+            if (!TILES || n_eras_now > 0) {
+                float2* out = s_gain + warp * NBP + lane;
+                const float w_era = (tc == 0u) ? 0.f : (a.era_alpha > 0.f ? f_add((float)tc, a.era_alpha) : 1.f);
+                const float tgf = f_mul(__ll2float_rn(tg), inv_scale);
+#pragma unroll
+                for (int i = 0; i < BPL; ++i) {
+                    lc_sum[i] += pc[i];
+                    lg_sum[i] += pg[i];
+                }
+                if (table) {             // the operations of era_totals and gain_of, divisions by the table
+                    const float parent = divide_by(f_mul(0.5f, f_mul(tgf, tgf)), s_div[tc]);
+#pragma unroll
+                    for (int i = 0; i < BPL; ++i) {
+                        const float lg = f_mul(__ll2float_rn(pg[i]), inv_scale), rg = f_sub(tgf, lg);
+                        const uint32_t rc = tc - pc[i];
+                        const float g2 = f_mul(0.5f, f_add(divide_by(f_mul(lg, lg), s_div[pc[i]]), divide_by(f_mul(rg, rg), s_div[rc])));
+                        out[i * 32] = make_float2(f_sub(g2, parent), (pc[i] > 0u && rc > 0u) ? w_era : 0.f);
+                    }
+                } else {
+                    const EraTotals et = era_totals(tc, tg, inv_scale, lam, a.era_alpha);
+#pragma unroll
+                    for (int i = 0; i < BPL; ++i)
+                        out[i * 32] = gain_of(pc[i], pg[i], tc, et.tg, et.th, et.parent, inv_scale, lam, et.w_era);
+                }
+                if (use_dir) {
+#pragma unroll
+                    for (int i = 0; i < BPL; ++i) {
+                        const float lg = f_mul(__ll2float_rn(pg[i]), inv_scale), lh = (float)pc[i];
+                        const float vl = f_div(-lg, f_add(lh, lam));
+                        const float vr = f_div(-f_sub(tgf, lg), f_add(f_sub((float)tc, lh), lam));
+                        s_agree[warp * NBP + i * 32 + lane] = a.direction_form == 1
+                            ? (vl > vr ? 1.f : -1.f)
+                            : f_mul(0.5f, f_add(sign3(vl) == pa ? 1.f : 0.f, sign3(vr) == pa ? 1.f : 0.f));  // (an absent era has weight 0)
+                    }
+                }
+                if (TILES) {
+                    tc = 0u;
+                    tg = 0ll;
+#pragma unroll
+                    for (int i = 0; i < BPL; ++i) {
+                        pc[i] = 0u;
+                        pg[i] = 0ll;
+                    }
+                }
+            }
+        }
+        __syncthreads();                 // gains are there, cells are zero, offsets are the next batch's
+
+        // ---- (c) recursion ----
+#pragma unroll
+        for (int q = 0; q < SLOTS; ++q) {
+            const int s = threadIdx.x + q * kWalkThreads;
+            if (s >= n_slots) break;
+            for (int e = 0; e < n_eras_now; ++e) {
+                const float2 gw = s_gain[(e * CN) * NBP + s];
+                float fac, w;
+                if (UNIT) {
+                    w = gw.y > 0.f ? 1.f : 0.f;
+                    n_valid[q] += gw.y > 0.f ? 1 : 0;
+                    fac = gw.y > 0.f ? s_inv[n_valid[q]] : 0.f;
+                } else {
+                    w = gw.y;
+                    wsum[q] = f_add(wsum[q], w);
+                    fac = wsum[q] > 0.f ? f_div(w, wsum[q]) : 0.f;
+                }
+                const float delta = f_sub(gw.x, mean[q]);
+                mean[q] = f_add(mean[q], f_mul(fac, delta));
+                m2[q] = f_add(m2[q], f_mul(f_mul(w, delta), f_sub(gw.x, mean[q])));
+                if (use_dir) {
+                    a_num[q] = f_add(a_num[q], f_mul(w, s_agree[(e * CN) * NBP + s]));
+                    a_den[q] = f_add(a_den[q], w);
+                }
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- left counts and gradient sums over all eras, from the warps that scanned the node ----
+    // (the cells are free now: counts in [node][NBP] of word A, 64-bit sums in the gains' place)
+    unsigned long long* s_lg = reinterpret_cast<unsigned long long*>(s_gain);
+    for (int i = threadIdx.x; i < plane; i += kWalkThreads) {
+        s_cells[i] = 0u;
+        s_lg[i] = 0ull;
+    }
+    __syncthreads();
+    if (scans) {
+#pragma unroll
+        for (int i = 0; i < BPL; ++i) {
+            const int s = my_node * NBP + i * 32 + lane;
+            if (EB == 1) {
+                s_cells[s] = lc_sum[i];
+                s_lg[s] = (unsigned long long)lg_sum[i];
+            } else {
+                if (lc_sum[i]) atomicAdd(s_cells + s, lc_sum[i]);
+                if (lg_sum[i]) atomicAdd(s_lg + s, (unsigned long long)lg_sum[i]);
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- score of every threshold under the global min_samples_leaf mask ----
+    float* s_score = reinterpret_cast<float*>(s_cells + plane);
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+        const int s = threadIdx.x + q * kWalkThreads;
+        if (s >= n_slots) break;
+        const float ws0 = UNIT ? (float)n_valid[q] : wsum[q];
+        const float ws = ws0 < 1e-12f ? 1e-12f : ws0;
+        float var = f_div(m2[q], ws);
+        if (var < 0.f) var = 0.f;        // NaN stays NaN
+        float score = f_sub(mean[q], f_mul(a.lambda_dro, __fsqrt_rn(var)));
+        if (use_dir) score = f_add(score, f_mul(a.direction_weight, a_den[q] > 0.f ? f_div(a_num[q], a_den[q]) : 0.f));
+        const long long lc = s_cells[s], total = a.frontier[node0 + s / NBP].count;
+        s_score[s] = (lc >= a.min_samples_leaf && total - lc >= a.min_samples_leaf) ? score : -INFINITY;
+    }
+    __syncthreads();
+    if (warp >= live) return;
+
+    // ---- best threshold of a node: largest score, then largest left count, then the last ----
+    float bs = -INFINITY;
+    uint32_t bc = 0u, mine = 0u;         // bit i of `mine`: bin lane * BPL + i is a threshold
+    int bb = -1;                         // bin of the best threshold
+    bool nan = false;
+#pragma unroll
+    for (int i = 0; i < BPL; ++i) {
+        const int bin = lane * BPL + i, s = warp * NBP + i * 32 + lane;
+        if (bin >= nb - 1 || !s_set[bin]) continue;
+        mine |= 1u << i;
+        const float sc = s_score[s];
+        const uint32_t lc = s_cells[s];
+        if (sc != sc) {
+            nan = true;
+        } else if (bb < 0 || sc > bs || (sc == bs && lc >= bc)) {
+            bs = sc;
+            bc = lc;
+            bb = bin;
+        }
+    }
+    nan = __any_sync(0xFFFFFFFFu, nan);
+    for (int d = 16; d > 0; d >>= 1) {
+        const float os = __shfl_xor_sync(0xFFFFFFFFu, bs, d);
+        const uint32_t oc = __shfl_xor_sync(0xFFFFFFFFu, bc, d);
+        const int ob = __shfl_xor_sync(0xFFFFFFFFu, bb, d);
+        if (ob >= 0 && (bb < 0 || os > bs || (os == bs && (oc > bc || (oc == bc && ob > bb))))) {
+            bs = os;
+            bc = oc;
+            bb = ob;
+        }
+    }
+    const int upto = bb - lane * BPL;    // this lane's bins below the best
+    const uint32_t below = upto <= 0 ? 0u : (upto >= BPL ? mine : mine & ((1u << upto) - 1u));
+    const int k = __reduce_add_sync(0xFFFFFFFFu, __popc(below));
+    if (lane == 0) {
+        Cand out;
+        out.score = bs;
+        out.k = bb >= 0 ? k : -1;
+        out.left_count = bb >= 0 ? bc : 0u;
+        out.flags = (nan ? 1u : 0u) | ((uint32_t)(bb >= 0 ? bb : 0) << 8);
+        out.left_gq = bb >= 0 ? (int64_t)s_lg[warp * NBP + bb % BPL * 32 + bb / BPL] : 0ll;
+        a.cand[(size_t)a.feat_pos[f] * a.node_stride + node0 + warp] = out;
+    }
+}
+
+template <int BPL, int MODE>
+int launch_mode(const WalkLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    if (smem > 40 * 1024)   // (beside the static arrays)
+        PB_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<BPL, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    walk_kernel<BPL, MODE><<<grid, kWalkThreads, smem, stream>>>(a);
+    return PB_OK;
+}
+
+template <int BPL>
+int launch_bpl(const WalkLaunch& a, int mode, dim3 grid, size_t smem, cudaStream_t stream) {
+    return mode == kUnit ? launch_mode<BPL, kUnit>(a, grid, smem, stream)
+           : mode == kUnitTiles ? launch_mode<BPL, kUnitTiles>(a, grid, smem, stream)
+                                : launch_mode<BPL, kGeneral>(a, grid, smem, stream);
+}
+
+}  // namespace
+
+int launch_walk(WalkLaunch a, cudaStream_t stream) {
+    if (a.n_feat <= 0 || a.n_nodes <= 0) return PB_OK;
+    if (a.max_bins > 256) return fail_arg("max_bins=%d outside [2,256]", a.max_bins);
+    const int bpl = a.max_bins <= 32 ? 1 : a.max_bins <= 64 ? 2 : a.max_bins <= 128 ? 4 : 8;
+    a.cell_nodes = a.n_nodes < kWalkNodes ? a.n_nodes : kWalkNodes;
+    const bool unit = a.era_alpha <= 0.f && a.direction_weight == 0.f && a.n_eras < kWalkInv;
+    const int mode = !unit ? kGeneral : a.max_era_rows <= a.tile_rows ? kUnit : kUnitTiles;
+    const size_t plane = (size_t)kWalkNodes * 32 * bpl * 4;
+    size_t smem = (2 * walk_copies(bpl) + 2) * plane + (mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
+    // the table of divisors is 8 bytes per row of the largest era: while it leaves room for two CTAs per SM
+    a.div_table = a.max_era_rows <= a.tile_rows && smem + (size_t)(a.max_era_rows + 1) * 8 <= 110 * 1024;
+    if (a.div_table) smem += (size_t)(a.max_era_rows + 1) * 8;
+    dim3 grid((unsigned)((a.n_nodes + kWalkNodes - 1) / kWalkNodes), (unsigned)a.n_feat);
+    if (grid.y > 65535u) return fail_arg("too many features in one launch");
+    prof_begin(a.prof, kProfHist, stream);
+    if (a.mass) {
+        PB_CUDA_TRY(cudaMemsetAsync(a.mass, 0, (size_t)a.n_feat * 256 * sizeof(uint32_t), stream));
+        int parts = (148 * 8 + a.n_feat - 1) / a.n_feat;   // about eight CTAs per SM
+        const int most = (a.n_rows + 4095) / 4096;
+        if (parts > most) parts = most;
+        if (parts < 1) parts = 1;
+        mass_count_kernel<<<dim3((unsigned)a.n_feat, (unsigned)parts), 256, 0, stream>>>(a);
+        count_launch(1);
+    }
+    int rc = bpl == 1 ? launch_bpl<1>(a, mode, grid, smem, stream)
+             : bpl == 2 ? launch_bpl<2>(a, mode, grid, smem, stream)
+             : bpl == 4 ? launch_bpl<4>(a, mode, grid, smem, stream) : launch_bpl<8>(a, mode, grid, smem, stream);
+    prof_end(a.prof, kProfHist, stream);
+    if (rc) return rc;
+    count_launch(1);
+    PB_LAUNCH_CHECK("walk_kernel");
+    return PB_OK;
+}
+
+}  // namespace pb

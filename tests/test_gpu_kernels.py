@@ -355,3 +355,44 @@ def test_small_tree_predictor_equals_the_general_one(rows, features, bins, depth
         got = model._predict_packed(packed, small, init=start)
         want = model._predict_packed(packed, dict(large), init=start)
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("n,f,eras,bins,depth,extra", [
+    (700, 32, 1, 17, 3, {}), (5_003, 33, 7, 64, 6, {}), (9_000, 40, 40, 128, 5, dict(era_alpha=4.0)),
+    (20_001, 32, 2, 33, 4, {}), (6_000, 35, 9, 100, 5, dict(direction_weight=0.3)),
+    (4_000, 32, 5, 64, 4, dict(k_cuts=7, cut_selection="even")), (8_000, 36, 11, 64, 6, dict(k_cuts=9, cut_selection="mass")),
+    (3_000, 32, 6, 70, 4, dict(y_scale=1e-12)), (3_000, 32, 6, 70, 4, dict(lambda_l2=1e-9))])
+def test_era_walk_equals_the_stored_histogram_path(n, f, eras, bins, depth, extra, tmp_path):
+    """Trees, scores and predictions bit for bit between the kernel that walks the eras and the two-step
+    path (run in a child process, which the switch is read in): partly filled node groups, eras longer
+    than a tile, every form of the score, thresholds in lists, gradients too small for the division table."""
+    import json
+    import os
+    import subprocess
+    import sys
+    script = r"""
+import json, sys
+import numpy as np
+from packboost_b200 import PackBoost, PackBoostConfig
+n, f, eras, bins, depth, extra, out = json.loads(sys.argv[1])
+rng = np.random.default_rng(n + f)
+X = rng.normal(size=(n, f)).astype(np.float32)
+X[:, ::5] = rng.integers(0, 6, size=X[:, ::5].shape)
+y = ((X[:, 0] + X[:, 1] * X[:, 2] + 0.3 * rng.normal(size=n)) * extra.pop("y_scale", 1.0)).astype(np.float32)
+era = np.sort(rng.integers(0, eras, n)).astype(np.int16)
+cfg = dict(pack_size=2, max_depth=depth, learning_rate=0.2, lambda_l2=1.0, lambda_dro=0.4, min_samples_leaf=5, max_bins=bins, random_state=1)
+cfg.update(extra)
+b = PackBoost(PackBoostConfig(**cfg)).fit(X, y, era, num_rounds=3)
+np.savez(out, preds=b.train_predictions().view(np.int32), **{k: v.view(np.int32) if v.dtype == np.float32 else v for k, v in b.split_records().items()})
+"""
+    got = []
+    for walk in ("1", "0"):
+        path = str(tmp_path / f"{walk}.npz")
+        res = subprocess.run([sys.executable, "-c", script, json.dumps([n, f, eras, bins, depth, extra, path])],
+                             env=dict(os.environ, PACKBOOST_WALK=walk), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                             capture_output=True, text=True)
+        assert res.returncode == 0, res.stderr[-2000:]
+        got.append(np.load(path))
+    assert len(got[0]["node"]) > 3
+    for key in got[0].files:
+        np.testing.assert_array_equal(got[0][key], got[1][key], err_msg=key)
