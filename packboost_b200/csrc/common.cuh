@@ -171,6 +171,7 @@ struct HistLaunch {
     // into the per-threshold (gain, weight) rows and adds the left counts / gradient sums into the
     // era-summed tables, i.e. it does the work of the scorer's gain kernel.
     struct HistFuse* fuse;
+    int zeroed;                  // 1: the output arrays (histogram or totals) are zero already
     void* prof;                  // pb_train_state.profile
     uint32_t* debug_flags;       // &CtlHead::debug_flags, or nullptr
 };
@@ -183,6 +184,10 @@ struct HistFuse {
     int full_sweep;              // thr_ids[k] == k for all k and n_thr == max_bins - 1
     const float* inv_scale_ptr;
     float lambda_l2, era_alpha;
+    uint8_t* agree;              // [n_feat][n_eras][node_stride][n_thr] directional term of the era, or null: 0, 1, 2 for
+                                 // agreement 0, 0.5, 1 (form 0); 0, 1 for -1, +1 (form 1)
+    int direction_form;
+    const FrontierNode* frontier;
     int tot_fpl, tot_lanes;      // OUT: layout of the totals tables chosen by launch_hist
 };
 // True when launch_hist(h) would run the lane kernel with one tile per era, which is what the
@@ -215,9 +220,11 @@ struct ScoreLaunch {
     Cand* cand;                  // [n_sampled][node_stride]
     // scratch of the two-kernel scorer, for the n_feat features of this block
     float2* gw;                  // [n_feat][n_eras][node_stride][n_thr] (gain, validity weight)
+    uint8_t* agree;              // directional term like HistFuse::agree, or null; a fused flush has filled it
     uint32_t* lc_tot;            // [n_feat][node_stride][n_thr] left counts summed over eras
     int64_t* lg_tot;             // [n_feat][node_stride][n_thr] left gradient sums summed over eras
     void* prof;                  // pb_train_state.profile
+    int zeroed;                  // 1: the totals are zero already
     int fused;                   // 1: gw and the totals were written by the histogram kernel's fused flush
     int tot_fpl, tot_lanes;      // layout of lc_tot / lg_tot (tot_index(); 0, 0: the classic layout above)
 };

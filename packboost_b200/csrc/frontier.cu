@@ -602,7 +602,7 @@ static int need_workspace(const pb_train_state* st, const char* who) {
 struct BlockPlan {
     int64_t fb;  // features per block
     bool fused;  // the histogram is never stored (fused flush): no gsum / cnt arrays
-    size_t off_gsum, off_cnt, off_gw, off_lg, off_lc, off_thr;
+    size_t off_gsum, off_cnt, off_gw, off_ag, off_lg, off_lc, off_thr;  // gsum, cnt, lg, lc are neighbours: zeroed together
 };
 
 // The era-summed tables of the fused flush are laid out per lane of the histogram kernel and so
@@ -610,10 +610,11 @@ struct BlockPlan {
 constexpr int64_t kTotPad = 256;
 
 static bool plan_block(size_t avail, int stride, int64_t n_eras, int64_t max_bins, int64_t n_thr, int64_t n_feat,
-                       bool fused, BlockPlan* p) {
+                       bool fused, bool agree, BlockPlan* p) {
     const size_t cells = fused ? 0 : (size_t)stride * n_eras * max_bins;
-    const size_t per_feat = cells * 12 + score_scratch_bytes_per_feature(stride, (int)n_eras, (int)n_thr) + (size_t)n_thr * 4;
-    const size_t fixed = 6 * 256 + (fused ? (size_t)kTotPad * stride * n_thr * 12 : 0);
+    const size_t per_feat = cells * 12 + score_scratch_bytes_per_feature(stride, (int)n_eras, (int)n_thr) + (size_t)n_thr * 4 +
+                            (agree ? (size_t)stride * n_eras * n_thr : 0);
+    const size_t fixed = 7 * 256 + (fused ? (size_t)kTotPad * stride * n_thr * 12 : 0);
     if (avail < per_feat + fixed) return false;
     int64_t fb = (int64_t)((avail - fixed) / per_feat);
     if (fb > n_feat) fb = n_feat;
@@ -622,12 +623,14 @@ static bool plan_block(size_t avail, int stride, int64_t n_eras, int64_t max_bin
     p->fused = fused;
     const size_t tot_feats = (size_t)fb + (fused ? kTotPad : 0);
     size_t o = 0;
+    p->off_gw = o;
+    o += align_up((size_t)fb * stride * n_eras * n_thr * 8, 256);
+    p->off_ag = o;
+    o += align_up(agree ? (size_t)fb * stride * n_eras * n_thr : 0, 256);
     p->off_gsum = o;
     o += align_up((size_t)fb * cells * 8, 256);
     p->off_cnt = o;
     o += align_up((size_t)fb * cells * 4, 256);
-    p->off_gw = o;
-    o += align_up((size_t)fb * stride * n_eras * n_thr * 8, 256);
     p->off_lg = o;
     o += align_up(tot_feats * stride * n_thr * 8, 256);
     p->off_lc = o;
@@ -660,20 +663,21 @@ static HistLaunch hist_launch_of(const pb_train_state* st, int64_t depth, const 
     h.cnt = nullptr;
     h.gsum = nullptr;
     h.fuse = nullptr;
+    h.zeroed = 0;
     h.prof = st->profile;
     h.debug_flags = &c.head->debug_flags;
     return h;
 }
 
 // The flush of the histogram kernel does the per-era gain step itself when a CTA holds a whole era
-// of few-bin cells and no directional term needs the stored histogram (PACKBOOST_FUSED_FLUSH=0
+// of few-bin cells (PACKBOOST_FUSED_FLUSH=0
 // keeps the separate gain kernel, for comparisons).
 static bool use_fused_flush(const pb_train_state* st, int64_t depth) {
     static const bool enabled = [] {
         const char* e = getenv("PACKBOOST_FUSED_FLUSH");
         return !(e && e[0] == '0' && e[1] == 0);
     }();
-    if (!enabled || st->direction_weight != 0.0 || st->cut_mass) return false;  // (mass cuts need the stored histogram)
+    if (!enabled || st->cut_mass) return false;  // (mass cuts need the stored histogram)
     Ctl c = ctl_view(st->ctl);
     return hist_can_fuse(hist_launch_of(st, depth, c));
 }
@@ -756,10 +760,20 @@ static int hist_score_blocks(const pb_train_state* st, int64_t depth, const int3
             fz.inv_scale_ptr = &c.head->inv_scale;
             fz.lambda_l2 = (float)st->lambda_l2;
             fz.era_alpha = (float)(st->era_alpha > 0.0 ? st->era_alpha : 0.0);
+            if (st->direction_weight != 0.0) {
+                fz.agree = reinterpret_cast<uint8_t*>(scratch + plan.off_ag);
+                fz.direction_form = st->direction_form ? 1 : 0;
+                fz.frontier = c.frontier[depth & 1];
+            }
             h.fuse = &fz;
             h.cnt = nullptr;
             h.gsum = nullptr;
         }
+        // one fill for everything that is added to with atomics: the totals, and a histogram of several
+        // tiles per era (which lies right before them)
+        const size_t zero_from = (!plan.fused && st->max_era_rows > kTileRowsMax) ? plan.off_gsum : plan.off_lg;
+        PB_CUDA_TRY(cudaMemsetAsync(scratch + zero_from, 0, plan.off_thr - zero_from, stream));
+        h.zeroed = 1;
         int rc = launch_hist(h, stream);
         if (rc) return rc;
         const int32_t* thr_ids = st->thr_ids;
@@ -796,6 +810,8 @@ static int hist_score_blocks(const pb_train_state* st, int64_t depth, const int3
         s.gw = reinterpret_cast<float2*>(scratch + plan.off_gw);
         s.lg_tot = reinterpret_cast<int64_t*>(scratch + plan.off_lg);
         s.lc_tot = reinterpret_cast<uint32_t*>(scratch + plan.off_lc);
+        s.agree = st->direction_weight != 0.0 ? reinterpret_cast<uint8_t*>(scratch + plan.off_ag) : nullptr;
+        s.zeroed = 1;
         s.prof = st->profile;
         s.fused = plan.fused ? 1 : 0;
         s.tot_fpl = plan.fused ? fz.tot_fpl : 0;
@@ -906,7 +922,7 @@ extern "C" int pb_depth_hist_score(const pb_train_state* st, int64_t depth, cons
         return walk_depth(st, depth, feat_rows, feat_pos, n_feat, ws + cand_bytes, reinterpret_cast<Cand*>(ws), (cudaStream_t)stream_);
     BlockPlan plan;
     PB_REQUIRE(plan_block((size_t)st->workspace_bytes - cand_bytes, stride, st->n_eras, st->max_bins, st->n_thresholds,
-                          n_feat, use_fused_flush(st, depth), &plan),
+                          n_feat, use_fused_flush(st, depth), st->direction_weight != 0.0, &plan),
                "workspace too small for one feature of histogram at depth %lld", (long long)depth);
     return hist_score_blocks(st, depth, feat_rows, feat_pos, n_feat, ws + cand_bytes, plan, reinterpret_cast<Cand*>(ws),
                              (cudaStream_t)stream_);
@@ -1071,6 +1087,7 @@ extern "C" int pb_hist_build(const pb_train_state* st, const int32_t* feat_rows,
     h.cnt = cnt;
     h.gsum = gsum;
     h.fuse = nullptr;
+    h.zeroed = 0;
     h.prof = st->profile;
     h.debug_flags = &ctl_view(st->ctl).head->debug_flags;
     return launch_hist(h, (cudaStream_t)stream);
@@ -1123,7 +1140,7 @@ extern "C" int pb_depth_hist_score_static(const pb_train_state* st, int64_t dept
     const int stride = node_stride_of(depth);
     BlockPlan plan;
     PB_REQUIRE(plan_block(kStaticScratchBytes, stride, st->n_eras, st->max_bins, st->n_thresholds, n_feat,
-                          use_fused_flush(st, depth), &plan),
+                          use_fused_flush(st, depth), st->direction_weight != 0.0, &plan),
                "static scratch too small: one feature of histogram and scorer tables at depth %lld needs %llu bytes, "
                "the fixed array holds %llu; use pb_depth_hist_score with a workspace",
                (long long)depth,

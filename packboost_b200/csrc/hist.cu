@@ -519,22 +519,30 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
                 }
             }
             const EraTotals et = era_totals(tc, tgq, inv_scale, z.lambda_l2, z.era_alpha);
-            float2* out = z.gw + (((size_t)(feat0 + fl) * a.n_eras + era) * a.node_stride + n) * K;
+            const size_t row = (((size_t)(feat0 + fl) * a.n_eras + era) * a.node_stride + n) * K;
+            float2* out = z.gw + row;
+            const int pa = z.agree ? parent_direction(z.frontier[n].gq) : 0;
+            auto agree_of = [&](uint32_t lc, long long lgq) {
+                return agree_code(lc, lgq, et.tg, et.th, inv_scale, z.lambda_l2, z.direction_form, pa);
+            };
             const size_t tot0 = (((size_t)n * K) * FPL + fl) * lanes_total + lane_global;  // threshold 0
             const size_t tot_step = (size_t)FPL * lanes_total;
             uint32_t c = 0;
             long long g = 0;
             if (NBT == 5 && z.full_sweep) {
                 float2 gk[4];
+                uint32_t ak = 0u;
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
                     c += cb[b];
                     g += gb[b];
                     gk[b] = gain_of(c, g, tc, et.tg, et.th, et.parent, inv_scale, z.lambda_l2, et.w_era);
+                    if (z.agree) ak |= agree_of(c, g) << (8 * b);
                     if (c) atomicAdd(z.lc_tot + tot0 + b * tot_step, c);
                     if (g) atomicAdd(reinterpret_cast<unsigned long long*>(z.lg_tot + tot0 + b * tot_step), (unsigned long long)g);
                 }
-reinterpret_cast<float4*>(out)[0] = make_float4(gk[0].x, gk[0].y, gk[1].x, gk[1].y);
+                if (z.agree) *reinterpret_cast<uint32_t*>(z.agree + row) = ak;
+                reinterpret_cast<float4*>(out)[0] = make_float4(gk[0].x, gk[0].y, gk[1].x, gk[1].y);
                 reinterpret_cast<float4*>(out)[1] = make_float4(gk[2].x, gk[2].y, gk[3].x, gk[3].y);
             } else {
                 int kk = 0;
@@ -546,6 +554,7 @@ reinterpret_cast<float4*>(out)[0] = make_float4(gk[0].x, gk[0].y, gk[1].x, gk[1]
                         g += gb[b];
                         if (b == next) {
                             out[kk] = gain_of(c, g, tc, et.tg, et.th, et.parent, inv_scale, z.lambda_l2, et.w_era);
+                            if (z.agree) z.agree[row + kk] = (uint8_t)agree_of(c, g);
                             if (c) atomicAdd(z.lc_tot + tot0 + kk * tot_step, c);
                             if (g) atomicAdd(reinterpret_cast<unsigned long long*>(z.lg_tot + tot0 + kk * tot_step), (unsigned long long)g);
                             ++kk;
@@ -826,17 +835,17 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
         a.tiles_per_era = 1;
         a.use_atomics = 0;
     } else {
-        a.tiles_per_era = (h.max_era_rows + kTileRowsMax - 1) / kTileRowsMax;
+        a.tiles_per_era = (h.max_era_rows + a.tile_rows - 1) / a.tile_rows;
         a.use_atomics = 1;
     }
-    const int max_tile = (h.max_era_rows < kTileRowsMax) ? h.max_era_rows : kTileRowsMax;
+    const int max_tile = (h.max_era_rows < a.tile_rows) ? h.max_era_rows : a.tile_rows;
     int threads = (max_tile + rpi - 1) / rpi + 1;  // +1: a tile may straddle one extra chunk
     threads = (threads + 31) / 32 * 32;
     const int thread_cap = (h.code_bits == 4) ? 256 : 512;
     if (threads > thread_cap) return fail_arg("histogram tile of %d rows exceeds the thread block", max_tile);
 
     const size_t out_cells = (size_t)h.n_feat * h.node_stride * h.n_eras * h.max_bins;
-    if (a.use_atomics) {
+    if (a.use_atomics && !h.zeroed) {
         PB_CUDA_TRY(cudaMemsetAsync(h.cnt, 0, out_cells * sizeof(uint32_t), stream));
         PB_CUDA_TRY(cudaMemsetAsync(h.gsum, 0, out_cells * sizeof(int64_t), stream));
     }
@@ -866,9 +875,10 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
         }();
         int64_t cpn = h.max_bins;
         double best = 1e30;
+        int best_tile = a.tile_rows;
         {
-            constexpr double kPass = 15.0, kPassFeat = 2.2, kTuple = 33.0, kCell = 0.145;
-            const double tile_scale = (double)max_tile / 4700.0;
+            constexpr double kPass = 15.0, kPassFeat = 2.2, kTuple = 33.0, kCell = 0.145, kCellAtomic = 0.45;
+            const int tiles_min = a.tiles_per_era;
             int64_t c = h.max_bins;
             for (int a_try = 1; a_try <= cap; ++a_try, c *= h.max_bins) {
                 for (int t_try = 1; t_try * a_try <= 8; t_try *= 2) {
@@ -879,17 +889,46 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
                         const int blocks = (h.n_feat + per_cta - 1) / per_cta;
                         const size_t smem = bytes + lane_extra_bytes(r_try, a_try * t_try) + 1024;
                         const int per_sm = (2 * smem <= (size_t)228 * 1024) ? 2 : 1;
-                        const double ctas = (double)h.n_eras * a.tiles_per_era * blocks;
                         const double slots = 148.0 * per_sm;
-                        const double waves = ctas > slots ? ctas / slots : 1.0;
-                        // (a few per cent against more phases: equal estimates favour whole-warp tuples)
-                        double cost = (r_try == 1 ? 1.0 : r_try == 2 ? 1.04 : 1.08) * waves * per_sm * (per_sm == 1 ? 1.2 : 1.0) *
-                                      (tile_scale * (kPass + kPassFeat * a_try * t_try + kTuple * t_try / r_try) +
-                                       kCell * (double)bytes / 1024.0);
-                        if (forced) cost = (a_try == forced[0] && t_try == forced[1] && r_try == forced[2]) ? 0.0 : cost + 1e9;
-                        if (cost < best * (1.0 - 1e-9)) { best = cost; arity = a_try; tuples = t_try; phases = r_try; cpn = c; }
+                        // Eras that are cut into tiles anyway are cut so that the CTAs fill whole waves (1.3 M
+                        // rows without eras are 160 largest tiles, two blocks of features: 24 of 320 CTAs
+                        // ran alone: 70 us a launch, 51 with whole waves); every tile pays its flush of global atomics.
+                        for (int w = 1; w <= (a.use_atomics ? 6 : 1); ++w) {
+                            int tile = a.tile_rows, tiles = tiles_min;
+                            if (a.use_atomics) {
+                                tiles = (int)(w * slots / ((double)h.n_eras * blocks));
+                                if (tiles < tiles_min) {
+                                    if (w < 6) continue;
+                                    tiles = tiles_min;
+                                }
+                                tile = ((h.max_era_rows + tiles - 1) / tiles + 255) / 256 * 256;
+                                if (tile > kTileRowsMax) tile = kTileRowsMax;
+                                tiles = (h.max_era_rows + tile - 1) / tile;
+                            }
+                            const double tile_scale = (double)(a.use_atomics ? tile : max_tile) / 4700.0;
+                            const double ctas = (double)h.n_eras * tiles * blocks;
+                            double waves = ctas > slots ? ctas / slots : 1.0;
+                            if (a.use_atomics) waves = (double)(int64_t)(waves + 0.999);
+                            // (a few per cent against more phases: equal estimates favour whole-warp tuples)
+                            double cost = (r_try == 1 ? 1.0 : r_try == 2 ? 1.04 : 1.08) * waves * per_sm * (per_sm == 1 ? 1.2 : 1.0) *
+                                          (tile_scale * (kPass + kPassFeat * a_try * t_try + kTuple * t_try / r_try) +
+                                           (a.use_atomics ? kCellAtomic : kCell) * (double)bytes / 1024.0);
+                            if (forced) cost = (a_try == forced[0] && t_try == forced[1] && r_try == forced[2]) ? cost * 1e-6 : cost + 1e9;
+                            if (cost < best * (1.0 - 1e-9)) {
+                                best = cost;
+                                arity = a_try;
+                                tuples = t_try;
+                                phases = r_try;
+                                cpn = c;
+                                best_tile = tile;
+                            }
+                        }
                     }
                 }
+            }
+            if (a.use_atomics) {
+                a.tile_rows = best_tile;
+                a.tiles_per_era = (h.max_era_rows + best_tile - 1) / best_tile;
             }
         }
         if (forced)
@@ -906,8 +945,10 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
             h.fuse->tot_lanes = ((h.n_feat + a.feats_per_cta - 1) / a.feats_per_cta) * (32 / phases);
             a.fz = *h.fuse;
             const size_t tot = (size_t)h.node_stride * a.fz.n_thr * a.fz.tot_fpl * a.fz.tot_lanes;
-            PB_CUDA_TRY(cudaMemsetAsync(a.fz.lc_tot, 0, tot * sizeof(uint32_t), stream));
-            PB_CUDA_TRY(cudaMemsetAsync(a.fz.lg_tot, 0, tot * sizeof(int64_t), stream));
+            if (!h.zeroed) {
+                PB_CUDA_TRY(cudaMemsetAsync(a.fz.lc_tot, 0, tot * sizeof(uint32_t), stream));
+                PB_CUDA_TRY(cudaMemsetAsync(a.fz.lg_tot, 0, tot * sizeof(int64_t), stream));
+            }
         } else if (h.fuse) {
             return fail_arg("fused flush requested for a launch that cannot fuse (check hist_can_fuse first)");
         }

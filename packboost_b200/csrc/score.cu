@@ -29,7 +29,7 @@ constexpr int kGainThreads = 256;
 constexpr int kChainThreads = 256;
 constexpr int kSmallBins = 8;
 
-__device__ __forceinline__ float sign_of(float v) {
+__device__ __forceinline__ float sign_of(float v) {  // (general hessians)
     // torch.sign: -1, 0, +1, NaN stays NaN (compares false to everything)
     if (v > 0.f) return 1.f;
     if (v < 0.f) return -1.f;
@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(kGainThreads, (KT <= 4 && NBT <= 5) ? 3 : 2) g
         lg_sum[k] = 0ll;
     }
 
+    const int pa = (s.agree && node < n_nodes) ? parent_direction(s.frontier[node].gq) : 0;
     if (node < n_nodes) {
         // The histogram row of the next era is loaded while the current one is worked on: the rows
         // come from HBM and a thread has little else to overlap their latency with.
@@ -134,6 +135,12 @@ __global__ void __launch_bounds__(kGainThreads, (KT <= 4 && NBT <= 5) ? 3 : 2) g
             const float w_era = (tc == 0) ? 0.f : ((s.era_alpha > 0.f) ? f_add((float)tc, s.era_alpha) : 1.f);
             float2* out = s.gw + (((size_t)f * E + e) * s.node_stride + node) * K;
             float2 gk[KT];
+            if (s.agree) {
+                uint8_t* ag = s.agree + (((size_t)f * E + e) * s.node_stride + node) * K;
+#pragma unroll
+                for (int k = 0; k < KT; ++k)
+                    if (k < K) ag[k] = (uint8_t)agree_code(lcs[k], lgs[k], tg, th, inv_scale, lam, s.direction_form, pa);
+            }
 #pragma unroll
             for (int k = 0; k < KT; ++k) {
                 if (k < K) {
@@ -220,6 +227,7 @@ __global__ void __launch_bounds__(kGainThreads) gain_kernel_wide(GainArgs a) {
         lg_sum[i] = 0ll;
     }
 
+    const int pa = s.agree ? parent_direction(s.frontier[node].gq) : 0;
     // the histogram row of the next era is loaded while the current one is scanned and scored
     uint32_t rc[8], rc_next[8];
     long long rg[8], rg_next[8];
@@ -274,6 +282,9 @@ __global__ void __launch_bounds__(kGainThreads) gain_kernel_wide(GainArgs a) {
                 const int k = (b < NB) ? s_kof[b] : -1;
                 if (k >= 0) {
                     out[k] = gain_of(pc[it], pg[it], tc, tg, th, parent, inv_scale, lam, w_era);
+                    if (s.agree)
+                        s.agree[(((size_t)f * E + e) * s.node_stride + node) * K + k] =
+                            (uint8_t)agree_code(pc[it], pg[it], tg, th, inv_scale, lam, s.direction_form, pa);
                     lc_sum[it] += pc[it];
                     lg_sum[it] += pg[it];
                 }
@@ -422,7 +433,8 @@ __global__ void __launch_bounds__(kChainThreads) chain_kernel(ChainArgs a) {
     const float2* gw_cta = s.gw + ((size_t)f * E * s.node_stride + node0) * K;  // + e * e_stride + slot
     const size_t e_stride = (size_t)s.node_stride * K;
 
-    if (!use_dir) {
+    {
+        const uint8_t* agree = s.agree + ((size_t)f * E * s.node_stride + node0) * K + threadIdx.x;  // + e * e_stride
         // The (gain, weight) table of this CTA is streamed through shared memory in chunks of EC
         // eras with asynchronous copies, the next chunk in flight while the current one is walked;
         // only the mean / M2 updates form the long dependent chain.
@@ -460,6 +472,18 @@ __global__ void __launch_bounds__(kChainThreads) chain_kernel(ChainArgs a) {
                             ws = f_add(ws, v[q].y);
                             fac[q] = ws;
                         }
+                        if (use_dir) {   // (left by the gain kernel or the flush of the histogram kernel)
+                            uint32_t ag[kSub];
+#pragma unroll
+                            for (int q = 0; q < kSub; ++q)
+                                ag[q] = (e0 + q < ec) ? __ldg(agree + (size_t)(c * EC + e0 + q) * e_stride) : 0u;
+#pragma unroll
+                            for (int q = 0; q < kSub; ++q) {
+                                const float term = s.direction_form == 1 ? (ag[q] ? 1.f : -1.f) : f_mul(0.5f, (float)ag[q]);
+                                a_num = f_add(a_num, f_mul(v[q].y, term));
+                                a_den = f_add(a_den, v[q].y);
+                            }
+                        }
                         wsum = ws;
 #pragma unroll
                         for (int q = 0; q < kSub; ++q) fac[q] = (fac[q] > 0.f) ? f_div(v[q].y, fac[q]) : 0.f;
@@ -474,47 +498,6 @@ __global__ void __launch_bounds__(kChainThreads) chain_kernel(ChainArgs a) {
                 }
             }
             __syncthreads();
-        }
-    } else {
-        __syncthreads();
-        if (scorer) {
-            // directional agreement needs the per-era left / right leaf directions: recompute them
-            // from the histogram prefix of this threshold
-            const float2* gw = gw_cta + threadIdx.x;
-            const long long gpar = s.frontier[node].gq;
-            const float pa = (gpar > 0) ? -1.f : ((gpar < 0) ? 1.f : 0.f);  // sign(-G/(H+lambda)), H+lambda > 0
-            const float inv_scale = *s.inv_scale_ptr;
-            const int NB = s.max_bins;
-            const int t = s.thr_ids[(s.thr_per_feature ? (size_t)f * K : 0) + my_k];
-            for (int e = 0; e < E; ++e) {
-                const float2 v = gw[(size_t)e * e_stride];
-                const float w = v.y;
-                welford_step(v.x, w, wsum, mean, m2);
-                const size_t base = (((size_t)f * E + e) * s.node_stride + node) * NB;
-                uint32_t lc = 0, tc = 0;
-                long long lgq = 0, tgq = 0;
-                for (int b = 0; b < NB; ++b) {
-                    const uint32_t cc = s.cnt[base + b];
-                    const long long gg = s.gsum[base + b];
-                    tc += cc;
-                    tgq += gg;
-                    if (b <= t) {
-                        lc += cc;
-                        lgq += gg;
-                    }
-                }
-                if (tc == 0) continue;
-                const float lg = f_mul(__ll2float_rn(lgq), inv_scale);
-                const float tg = f_mul(__ll2float_rn(tgq), inv_scale);
-                const float lh = (float)lc, th = (float)tc;
-                const float vl = f_div(-lg, f_add(lh, lam));
-                const float vr = f_div(-f_sub(tg, lg), f_add(f_sub(th, lh), lam));
-                const float agree = (s.direction_form == 1)
-                    ? ((vl > vr) ? 1.f : -1.f)
-                    : f_mul(0.5f, f_add((sign_of(vl) == pa) ? 1.f : 0.f, (sign_of(vr) == pa) ? 1.f : 0.f));
-                a_num = f_add(a_num, f_mul(w, agree));
-                a_den = f_add(a_den, w);
-            }
         }
     }
 
@@ -926,8 +909,9 @@ int launch_score(const ScoreLaunch& s, cudaStream_t stream) {
     const int K = s.n_thr, NB = s.max_bins;
     if (K < 1 || K > kChainThreads) return fail_arg("n_thresholds=%d outside [1,%d]", K, kChainThreads);
     if (!s.gw || !s.lc_tot || !s.lg_tot) return fail_arg("scorer scratch is null");
+    if (s.direction_weight != 0.f && !s.agree) return fail_arg("the directional term needs its table");
     const size_t tot_cells = (size_t)s.n_feat * s.node_stride * K;
-    if (!s.fused) {
+    if (!s.fused && !s.zeroed) {
         PB_CUDA_TRY(cudaMemsetAsync(s.lc_tot, 0, tot_cells * sizeof(uint32_t), stream));
         PB_CUDA_TRY(cudaMemsetAsync(s.lg_tot, 0, tot_cells * sizeof(int64_t), stream));
     }
@@ -938,7 +922,6 @@ int launch_score(const ScoreLaunch& s, cudaStream_t stream) {
     if (s.fused) {
         // the histogram kernel's flush already wrote the (gain, weight) table and the era-summed
         // totals: only the era recursion is left
-        if (s.direction_weight != 0.f) return fail_arg("the fused flush cannot serve the directional term");
     } else if (NB <= kSmallBins) {
         int npc = 1;
         while (npc < 32 && npc < s.n_nodes_max) npc *= 2;

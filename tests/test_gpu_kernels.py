@@ -396,3 +396,32 @@ np.savez(out, preds=b.train_predictions().view(np.int32), **{k: v.view(np.int32)
     assert len(got[0]["node"]) > 3
     for key in got[0].files:
         np.testing.assert_array_equal(got[0][key], got[1][key], err_msg=key)
+
+
+@pytest.mark.parametrize("form", ["frontier", "helper"])
+@pytest.mark.parametrize("n,eras,bins", [(3_000, 7, 5), (20_000, 1, 5), (17_000, 2, 4), (6_000, 9, 14)])
+def test_directional_term_streamed_with_the_gains_matches_the_oracle(form, n, eras, bins, monkeypatch):
+    """Few-bin codes: agreement left by the fused flush (one tile per era), by the gain kernel behind
+    several tiles and by its many-bin form; era weights on."""
+    if form == "helper":
+        monkeypatch.setenv("PACKBOOST_DIRECTION_FORM", "helper")
+    from packboost_b200 import PackBoost, PackBoostConfig
+    rng = np.random.default_rng(n + bins)
+    X = rng.integers(0, bins, size=(n, 11), dtype=np.uint8)
+    y = (0.3 * X[:, 1] - 0.2 * X[:, 3] * (X[:, 5] > 1) + rng.normal(size=n)).astype(np.float32)
+    era = np.sort(rng.integers(0, eras, n)).astype(np.int16)
+    cfg = dict(pack_size=2, max_depth=4, learning_rate=0.2, lambda_l2=1.0, lambda_dro=0.3, direction_weight=0.2, era_alpha=3.0,
+               min_samples_leaf=10, max_bins=bins, prebinned=True, random_state=5)
+    b = PackBoost(PackBoostConfig(device="cuda", **cfg)).fit(X, y, era, num_rounds=2)
+    got = b.split_records()
+    assert len(got["node"]) > 8
+    # the same splits re-scored one node at a time by the general scorer, first round's root
+    root = b._find_best_split(_root_shard(era, eras), torch.from_numpy(-y), torch.ones(n), torch.from_numpy(X.astype(np.int64)),
+                              torch.arange(11))
+    assert (got["feature"][0], got["threshold"][0]) == (root.feature, root.threshold)
+    np.testing.assert_allclose(got["score"][0], root.score, rtol=2e-6)
+
+
+def _root_shard(era, eras):
+    from packboost_b200.booster import NodeShard
+    return NodeShard(tree_id=0, node_id=0, depth=0, era_rows=[torch.from_numpy(np.flatnonzero(era == e)) for e in range(eras)])
