@@ -333,6 +333,24 @@ int pb_era_correlation(const float* y, const float* preds, const int32_t* era_of
  * pb_round_end; layout: pb_round_log below). */
 int pb_round_log_buffer(const pb_train_state* st, void** ptr, int64_t* bytes);
 
+/* A whole round of one GPU in one call (the loop body of packboost/booster.py:494-599): the feature
+ * lists `lists_host` [max_depth][3][k] (global ids, local rows, positions; page-locked) go to
+ * `lists_dev`, the phases are enqueued - with `use_graph` and `apply_previous` replayed as a CUDA graph
+ * captured on first use and tied to the state's buffers - and the decision log comes to `log_host`
+ * (page-locked).  pb_loop_wait waits for the log of a slot (0 .. 7).  pb_loop_counts: kernels per replay
+ * and replays so far. */
+void* pb_loop_create(void);
+void pb_loop_destroy(void* loop);
+int pb_loop_submit(void* loop, const pb_train_state* st, int64_t slot, const int32_t* lists_host, int32_t* lists_dev,
+                   int64_t k, void* log_host, int64_t apply_previous, int64_t use_graph, void* stream);
+int pb_loop_wait(void* loop, int64_t slot);
+int pb_loop_counts(void* loop, int64_t* graph_launches, int64_t* replays);
+
+/* Node arrays (2^(max_depth + 1) - 1 entries at most) of the tree behind a decision log; an error when
+ * the log's child numbering is not the order in which splits append children. */
+int pb_tree_from_log(const void* log_head, const void* log_winners, int64_t max_depth, int32_t* feature,
+                     int32_t* threshold, int32_t* left, int32_t* right, double* value, uint8_t* is_leaf, int64_t* n_nodes);
+
 typedef struct pb_winner {
     int32_t feature;      /* global feature id, -1: node not split */
     int32_t threshold;    /* bin id: rows with code <= threshold go left */

@@ -116,6 +116,12 @@ _PROTOS: dict[str, tuple[Any, list[Any]]] = {
     "pb_apply_leaf_delta": (C.c_int, [C.POINTER(TrainState), vp]),
     "pb_era_correlation": (C.c_int, [vp, vp, vp, i64, vp, vp]),
     "pb_round_log_buffer": (C.c_int, [C.POINTER(TrainState), C.POINTER(vp), C.POINTER(i64)]),
+    "pb_loop_create": (vp, []),
+    "pb_loop_destroy": (None, [vp]),
+    "pb_loop_submit": (C.c_int, [vp, vp, i64, vp, vp, i64, vp, i64, i64, vp]),
+    "pb_loop_wait": (C.c_int, [vp, i64]),
+    "pb_loop_counts": (C.c_int, [vp, vp, vp]),
+    "pb_tree_from_log": (C.c_int, [vp, vp, i64, vp, vp, vp, vp, vp, vp, vp]),
     "pb_hist_build": (C.c_int, [C.POINTER(TrainState), vp, i64, i64, i64, vp, vp, vp]),
     "pb_score_node_general": (C.c_int, [vp, vp, vp, i64, i64, i64, vp, i64, C.c_float, C.c_float, C.c_float, C.c_float,
                                         C.c_float, C.c_float, i64, i64, i64, i64, vp, vp]),

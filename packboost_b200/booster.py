@@ -63,10 +63,34 @@ class TreeNode:
     is_leaf: bool = True
 
 
-@dataclass(slots=True)
 class Tree:
-    nodes: List[TreeNode]
-    _arrays: dict | None = field(init=False, repr=False, default=None)
+    """A tree as node arrays, a list of ``TreeNode`` or both: a fit leaves arrays, the list is built when
+    somebody asks for it (and from then on is what counts, since nodes can be written to)."""
+
+    __slots__ = ("_nodes", "_arrays", "_values")
+
+    def __init__(self, nodes: List[TreeNode] | None = None, *, arrays: dict | None = None, values: np.ndarray | None = None):
+        self._nodes = nodes
+        self._arrays = arrays
+        self._values = values          # leaf values in float64 (arrays hold them as float32)
+
+    @property
+    def nodes(self) -> List[TreeNode]:
+        if self._nodes is None:
+            a = self._arrays
+            self._nodes = [TreeNode(*row) for row in
+                           zip(a["feature"].tolist(), a["threshold"].tolist(), a["left"].tolist(), a["right"].tolist(),
+                               self._values.tolist(), (a["is_leaf"] != 0).tolist())]
+            self._arrays = self._values = None
+        return self._nodes
+
+    def __eq__(self, other) -> bool:
+        return isinstance(other, Tree) and self.nodes == other.nodes
+
+    __hash__ = None
+
+    def __repr__(self) -> str:
+        return f"Tree(nodes={self.nodes!r})"
 
     def arrays(self) -> dict[str, np.ndarray]:
         if self._arrays is None:
@@ -319,7 +343,12 @@ class _DeviceTrainer:
         # ring: a slot is reused only after the round that used it has delivered its log.
         self.log_host = [torch.empty(self.log_bytes, dtype=torch.uint8).pin_memory() for _ in range(_RING)]
         self.feat_host = [torch.empty((D, 3, max(k_sampled, 1)), dtype=torch.int32).pin_memory() for _ in range(_RING)]
-        self.log_event = [torch.cuda.Event() for _ in range(_RING)]
+        # (a round of one GPU is one library call; the lists' third row, the positions, never changes there)
+        self.loop = self.lib.pb_loop_create() if world == 1 else None
+        self.log_event = [] if self.loop else [torch.cuda.Event() for _ in range(_RING)]
+        self.feat_np = [t.numpy() for t in self.feat_host]
+        for f in self.feat_np:
+            f[:, 2, :] = np.arange(f.shape[2], dtype=np.int32)
         self.feat_dev = torch.empty((D, 3, max(k_sampled, 1)), dtype=torch.int32, device=self.dev)
         self.corr_dev = None
         self.enqueued = 0
@@ -329,8 +358,8 @@ class _DeviceTrainer:
         self.use_graph = os.getenv("PACKBOOST_CUDA_GRAPH") != "0" and (world == 1 or self.replicated)
         self.graph = None
         self.graph_signature = None
-        self.graph_launches = 0
-        self.graph_replays = 0
+        self._graph_launches = 0
+        self._graph_replays = 0
         self.pending_delta = False
         self.prof = None
         # PACKBOOST_COMM=native: the per-depth exchanges go through the library's own NCCL entry
@@ -373,6 +402,10 @@ class _DeviceTrainer:
             return
         try:
             self.disable_profile()
+            if getattr(self, "loop", None):
+                torch.cuda.synchronize(self.dev)
+                self.lib.pb_loop_destroy(self.loop)
+                self.loop = None
         except Exception:
             pass
 
@@ -439,6 +472,20 @@ class _DeviceTrainer:
         k = subsets[0].shape[0]
         ticket = self.enqueued
         slot = ticket % _RING
+        apply_previous = 1 if (self.pending_delta and not redo) else 0
+        if self.loop:
+            if ticket >= _RING:
+                B.check(lib.pb_loop_wait(self.loop, slot))   # the slot's previous round has long finished
+            lists = self.feat_np[slot]
+            lists[:, 0, :] = subsets
+            lists[:, 1, :] = lists[:, 0, :]                  # one GPU holds the features in order
+            B.check(lib.pb_loop_submit(self.loop, st, slot, lists.ctypes.data, self.feat_dev.data_ptr(), k,
+                                       self.log_host[slot].data_ptr(), apply_previous, 1 if self.use_graph else 0, stream))
+            self.pending_delta = True
+            self.enqueued += 1
+            if not redo:
+                self.rounds_done += 1
+            return ticket
         if ticket >= _RING:
             self.log_event[slot].synchronize()  # the slot's previous round has long finished
         fh = self.feat_host[slot]
@@ -454,7 +501,6 @@ class _DeviceTrainer:
             fh[d, 1, : pos.shape[0]] = torch.from_numpy(rows)
             fh[d, 2, : pos.shape[0]] = torch.from_numpy(pos)
         self.feat_dev.copy_(fh, non_blocking=True)
-        apply_previous = 1 if (self.pending_delta and not redo) else 0
         # The phases of a round are the same launches every round (the feature lists change only as
         # data in feat_dev), so from the second round on they are replayed as one CUDA graph.  The
         # graph is tied to the per-depth local feature counts; any other round runs eagerly.
@@ -468,7 +514,7 @@ class _DeviceTrainer:
                     self.use_graph = False
             if self.graph_signature == signature:
                 self.graph.replay()
-                self.graph_replays += 1
+                self._graph_replays += 1
                 return self._round_enqueued(slot, redo)
         self._enqueue_phases(k, n_local, apply_previous)
         return self._round_enqueued(slot, redo)
@@ -493,7 +539,23 @@ class _DeviceTrainer:
                 graph.capture_end()
         cur.wait_stream(side)
         self.graph, self.graph_signature = graph, signature
-        self.graph_launches = int(self.lib.pb_launch_count()) - before  # kernels per replay
+        self._graph_launches = int(self.lib.pb_launch_count()) - before  # kernels per replay
+
+    def _loop_counts(self) -> tuple[int, int]:
+        if not self.loop:
+            return self._graph_launches, self._graph_replays
+        launches, replays = C.c_int64(), C.c_int64()
+        B.check(self.lib.pb_loop_counts(self.loop, C.byref(launches), C.byref(replays)))
+        return launches.value, replays.value
+
+    @property
+    def graph_launches(self) -> int:
+        """Kernels per replay of the round graph."""
+        return self._loop_counts()[0]
+
+    @property
+    def graph_replays(self) -> int:
+        return self._loop_counts()[1]
 
     def close_comm(self) -> None:
         if self.comm is not None:
@@ -577,7 +639,10 @@ class _DeviceTrainer:
         if not 0 <= self.enqueued - 1 - ticket < _RING:
             raise RuntimeError("round log is no longer held")
         slot = ticket % _RING
-        self.log_event[slot].synchronize()
+        if self.loop:
+            B.check(self.lib.pb_loop_wait(self.loop, slot))
+        else:
+            self.log_event[slot].synchronize()
         raw = self.log_host[slot].numpy()
         head = raw[:88].view(_HEADER_DT)[0]
         winners = raw[88:].view(_WINNER_DT)
@@ -586,30 +651,23 @@ class _DeviceTrainer:
 
 def _tree_from_log(head, winners, max_depth: int) -> tuple[Tree, list[int]]:
     """Replay the device's decisions into a ``Tree`` (``packboost/booster.py:527-563``)."""
-    tb = TreeBuilder()
-    tb.set_leaf(0, float(head["root_value"]))
-    n_ctx = [int(v) for v in head["n_ctx"][: max_depth + 1]]
-    for d in range(max_depth):
-        if n_ctx[d] == 0:
-            break
-        base = (1 << d) - 1
-        sl = winners[base: base + n_ctx[d]]
-        # (field columns as plain lists: element access on structured records is what costs here)
-        for nid, feat, thr, lid, rid, lv, rv in zip(sl["tree_node"].tolist(), sl["feature"].tolist(),
-                                                    sl["threshold"].tolist(), sl["left_id"].tolist(),
-                                                    sl["right_id"].tolist(), sl["left_value"].tolist(),
-                                                    sl["right_value"].tolist()):
-            if feat < 0:
-                tb.set_leaf(nid, lv)
-                continue
-            l, r = tb.split(nid, feat, thr)
-            if l != lid or r != rid:
-                raise RuntimeError("device and host child numbering disagree")
-            tb.set_leaf(l, lv)
-            tb.set_leaf(r, rv)
-    if len(tb.nodes) != int(head["n_tree_nodes"]):
-        raise RuntimeError("device and host tree sizes disagree")
-    return tb.build(), n_ctx
+    cap = (2 << max_depth) - 1
+    if winners.shape[0] < (1 << max_depth) - 1:
+        raise ValueError("decision log is too short")
+    head_mem, winners = np.ascontiguousarray(head), np.ascontiguousarray(winners)
+    ints = np.empty((4, cap), dtype=np.int32)
+    values = np.empty(cap, dtype=np.float64)
+    leaf = np.empty(cap, dtype=np.uint8)
+    count = C.c_int64()
+    at, step = ints.ctypes.data, 4 * cap
+    rc = B.lib().pb_tree_from_log(head_mem.ctypes.data, winners.ctypes.data, max_depth, at, at + step, at + 2 * step,
+                                  at + 3 * step, values.ctypes.data, leaf.ctypes.data, C.byref(count))
+    if rc:
+        raise RuntimeError(B.lib().pb_last_error().decode("utf-8", "replace"))
+    n = count.value
+    arrays = {"feature": ints[0, :n], "threshold": ints[1, :n], "left": ints[2, :n], "right": ints[3, :n],
+              "value": values[:n].astype(np.float32), "is_leaf": leaf[:n]}
+    return Tree(arrays=arrays, values=values[:n]), head["n_ctx"][: max_depth + 1].tolist()
 
 
 # ------------------------------ the booster ------------------------------
@@ -634,6 +692,7 @@ class PackBoost:
         self._histogram_mode = mode
         self._logger = logging.getLogger(__name__)
         self._depth_logs: list[dict[str, object]] = []
+        self._depth_log_base: dict | None = None
         self._binner: BinningResult | None = None
         self._trees: list[Tree] = []
         self._distinct: list[tuple[Tree, int]] = []  # (tree, repeat) per round
@@ -654,7 +713,7 @@ class PackBoost:
         self._eval_states: list = []
         self._last_n_ctx: list[int] = []
         self._round_depths: list[int] = []   # depths with live nodes (= feature draws consumed) per round
-        self._split_log: list[np.ndarray] = []
+        self._split_log: list[tuple] = []    # (live nodes per depth, winners) per round
         self._pending_log = None
         self._predrawn = None
         self._inflight = None  # (log ticket, generator state at the round's start) of the enqueued round
@@ -869,7 +928,7 @@ class PackBoost:
         metrics["trees_per_second"] = (cfg.pack_size / dt) if dt > 0 else float("inf")
         metrics["round_seconds"] = dt
         for stt in eval_states:
-            metrics[f"{stt['name']}_corr"] = _era_correlation_np(stt["era"], stt["y"], stt["preds"].cpu().numpy())
+            metrics[f"{stt['name']}_corr"] = self._mean_era_correlation(stt)
         self._round_metrics.append(metrics)
         return metrics
 
@@ -891,7 +950,7 @@ class PackBoost:
         ticket, state0 = inflight
         D = int(self.config.max_depth)
         head, winners = self._trainer.read_log(ticket)
-        n_ctx = [int(v) for v in head["n_ctx"][: D + 1]]
+        n_ctx = head["n_ctx"][: D + 1].tolist()
         self._last_n_ctx = n_ctx
         used = next((d for d in range(D) if n_ctx[d] == 0), D)
         self._round_depths.append(used)
@@ -904,10 +963,10 @@ class PackBoost:
         phase_ms = self._trainer.profile_by_depth() if getattr(self._trainer, "prof", None) is not None else []
         for d in range(used):
             self._depth_logs.append(self._depth_log(d, n_ctx[d], k, phase_ms[d] if d < len(phase_ms) else None))
-            w = winners[(1 << d) - 1: (1 << d) - 1 + n_ctx[d]]
-            self._split_log.append(w[w["feature"] >= 0].copy())
         self._flush_pending_tree()
-        self._pending_log = (head.copy(), winners[: (1 << D) - 1].copy())
+        log = (head.copy(), winners[: (1 << D) - 1].copy())
+        self._pending_log = log
+        self._split_log.append((n_ctx[:used], log[1]))
         return used == D
 
     def _drain(self) -> None:
@@ -1049,7 +1108,12 @@ class PackBoost:
         position): tree node, feature, threshold, DES score (the ``SplitDecision.score`` of
         ``packboost/booster.py:206-217``), rows sent left and rows of the node."""
         self._drain()
-        rec = (np.concatenate(self._split_log) if self._split_log else np.zeros(0, dtype=_WINNER_DT))
+        # (records as raw bytes: concatenating structured arrays promotes their types field by field)
+        size = _WINNER_DT.itemsize
+        parts = [w.view(np.uint8)[((1 << d) - 1) * size: ((1 << d) - 1 + n) * size]
+                 for n_ctx, w in self._split_log for d, n in enumerate(n_ctx)]
+        rec = (np.concatenate(parts) if parts else np.zeros(0, dtype=np.uint8)).view(_WINNER_DT)
+        rec = rec[rec["feature"] >= 0]
         return {"node": rec["tree_node"].astype(np.int32), "feature": rec["feature"].astype(np.int32),
                 "threshold": rec["threshold"].astype(np.int32), "score": rec["score"].astype(np.float32),
                 "left_count": rec["left_count"].astype(np.int64),
@@ -1060,21 +1124,27 @@ class PackBoost:
         The millisecond fields are device times of the depth's kernels (CUDA events) when per-round
         metrics were asked for, else 0: timing needs eager launches, which the fast path avoids.
         ``scan_ms`` stays 0 (the prefix scan is part of the scorer kernels)."""
-        blk = int(self.config.feature_block_size)
-        blk = k if (blk <= 0 or blk > k) else blk
-        ms = ms or {}
-        return {
-            "nodes_processed": n_nodes, "nodes_skipped": 0, "rows_total": 0,
-            "feature_blocks": (k + blk - 1) // blk, "bincount_calls": 0,
-            "hist_ms": ms.get("hist_ms", 0.0), "scan_ms": 0.0,
-            "score_ms": ms.get("score_ms", 0.0) + ms.get("select_ms", 0.0), "partition_ms": ms.get("partition_ms", 0.0),
-            "nodes_subtract_ok": 0, "nodes_rebuild": n_nodes, "nodes_subtract_fallback": 0,
-            "nodes_collapsed": n_nodes * (int(self.config.pack_size) - 1), "feature_block_size": blk,
-            "depth": depth, "feature_subset_size": k, "pack_size": int(self.config.pack_size),
-            "layer_feature_fraction": float(self.config.layer_feature_fraction),
-            "histogram_mode": self._histogram_mode, "seed": self.config.random_state,
-            "torch_threads": torch.get_num_threads(),
-        }
+        base = self._depth_log_base
+        if base is None or base["feature_subset_size"] != k:
+            blk = int(self.config.feature_block_size)
+            blk = k if (blk <= 0 or blk > k) else blk
+            base = self._depth_log_base = {
+                "nodes_processed": 0, "nodes_skipped": 0, "rows_total": 0, "feature_blocks": (k + blk - 1) // blk,
+                "bincount_calls": 0, "hist_ms": 0.0, "scan_ms": 0.0, "score_ms": 0.0, "partition_ms": 0.0,
+                "nodes_subtract_ok": 0, "nodes_rebuild": 0, "nodes_subtract_fallback": 0, "nodes_collapsed": 0,
+                "feature_block_size": blk, "depth": 0, "feature_subset_size": k, "pack_size": int(self.config.pack_size),
+                "layer_feature_fraction": float(self.config.layer_feature_fraction),
+                "histogram_mode": self._histogram_mode, "seed": self.config.random_state,
+                "torch_threads": torch.get_num_threads(),
+            }
+        log = dict(base)
+        log["nodes_processed"] = log["nodes_rebuild"] = n_nodes
+        log["nodes_collapsed"] = n_nodes * (log["pack_size"] - 1)
+        log["depth"] = depth
+        if ms:
+            log["hist_ms"], log["partition_ms"] = ms.get("hist_ms", 0.0), ms.get("partition_ms", 0.0)
+            log["score_ms"] = ms.get("score_ms", 0.0) + ms.get("select_ms", 0.0)
+        return log
 
     # -- evaluation sets -----------------------------------------------------
     def _prepare_eval_sets(self, eval_sets):
@@ -1090,9 +1160,32 @@ class PackBoost:
             era_e = np.zeros(Xe.shape[0], dtype=np.int16) if era_eval is None else np.asarray(era_eval, dtype=np.int16)
             if era_e.shape[0] != Xe.shape[0]:
                 raise ValueError(f"eval set '{name}' era ids must align with X rows")
-            states.append({"name": name, "rows": rows, "y": np.asarray(y_eval, dtype=np.float32), "era": era_e,
+            y_e = np.asarray(y_eval, dtype=np.float32)
+            if y_e.shape[0] != Xe.shape[0]:
+                raise ValueError(f"eval set '{name}' targets must align with X rows")
+            # rows grouped by era, as the correlation kernel takes them
+            _, offsets, order = sort_eras(era_e, Xe.shape[0])
+            if order is not None:
+                y_e = y_e[order]
+                rows.codes = rows.codes.index_select(0, torch.from_numpy(order).to(self._device))
+            states.append({"name": name, "rows": rows, "y": torch.from_numpy(np.ascontiguousarray(y_e)).to(self._device),
+                           "offsets": torch.from_numpy(offsets).to(self._device),
+                           "corr": torch.empty(max(offsets.shape[0] - 1, 1), dtype=torch.float64, device=self._device),
                            "preds": torch.zeros(Xe.shape[0], dtype=torch.float32, device=self._device), "done": 0})
         return states
+
+    def _mean_era_correlation(self, stt) -> float:
+        """Mean per-era correlation of an evaluation set (``packboost/booster.py:909-929``), on the device."""
+        if stt["rows"].n_rows == 0:
+            return float("nan")
+        n_eras, most = stt["offsets"].shape[0] - 1, 32767    # (eras of one launch)
+        for e in range(0, n_eras, most):
+            B.check(B.lib().pb_era_correlation(stt["y"].data_ptr(), stt["preds"].data_ptr(), stt["offsets"][e:].data_ptr(),
+                                               min(most, n_eras - e), stt["corr"][e:].data_ptr(),
+                                               torch.cuda.current_stream().cuda_stream))
+        c = stt["corr"].cpu().numpy()
+        c = c[np.isfinite(c)]
+        return float(c.mean()) if c.size else float("nan")
 
     def _update_eval_sets(self, states) -> None:
         # predictions accumulate in tree order, so adding only the new rounds reproduces a

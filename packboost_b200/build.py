@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_NAME = "libpackboost_b200.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
 
-SOURCES = ["api.cu", "hist.cu", "score.cu", "walk.cu", "frontier.cu", "pack.cu", "predict.cu", "metrics.cu", "upload.cu", "comm.cu"]
+SOURCES = ["api.cu", "hist.cu", "score.cu", "walk.cu", "frontier.cu", "pack.cu", "predict.cu", "metrics.cu", "upload.cu", "loop.cu", "comm.cu"]
 # The scorer, and the histogram kernel whose flush computes the per-era gains, must round every
 # product and sum separately (no fused multiply-add) to keep the float32 operation order of the
 # algorithm they implement.
