@@ -22,8 +22,8 @@
 //
 // Bound: the shared-memory atomics (two per row and feature, about four wavefronts each with 128 bins)
 // at the upper depths, the gains at the lower ones.
-// 500 000 rows x 256 features, 100 eras, 128 bins, by depth: 0.23, 0.27, 0.31, 0.40, 0.59, 1.13 ms, 2.9 ms a
-// round (histogram, gain and chain kernels: 4.6 ms); 200 000 x 100, depth 10: 3.2 ms a round (6.1).
+// 500 000 rows x 256 features, 100 eras, 128 bins, by depth: 0.24, 0.27, 0.31, 0.40, 0.59, 0.96 ms, 2.8 ms a
+// round (histogram, gain and chain kernels: 4.6 ms); 200 000 x 100, depth 10: 2.7 ms a round (6.1).
 //
 // Float arithmetic as in the scorer: the same separately rounded operations in the same order
 // (this file is compiled with -fmad=false), so candidates are bit-identical to the other path's.
@@ -164,20 +164,36 @@ constexpr int kUnit = 0;       // era weights 0 / 1, an era is one tile
 constexpr int kUnitTiles = 1;  // era weights 0 / 1, eras of several tiles
 constexpr int kGeneral = 2;    // any weights, directional term, any eras
 
-// Interleaved copies of the cells, for the lanes of a warp that meet in a bin: columns of few values
-// (32 lanes on ten bins) took twice as long as the others and were what a launch waited for.
-__host__ __device__ constexpr int walk_copies(int bpl) { return bpl <= 4 ? 2 : 1; }
+// W neighbouring words of a lane, in as few accesses as they take.
+template <int W>
+__device__ __forceinline__ void take_words(uint32_t* at, uint32_t (&v)[W]) {  // reads, leaves zeros
+    if (W >= 4) {
+#pragma unroll
+        for (int i = 0; i < W; i += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(at + i);
+            v[i] = q.x; v[(i + 1) % W] = q.y; v[(i + 2) % W] = q.z; v[(i + 3) % W] = q.w;
+        }
+#pragma unroll
+        for (int i = 0; i < W; i += 4) *reinterpret_cast<uint4*>(at + i) = make_uint4(0u, 0u, 0u, 0u);
+    } else if (W == 2) {
+        const uint2 q = *reinterpret_cast<const uint2*>(at);
+        v[0] = q.x; v[1 % W] = q.y;
+        *reinterpret_cast<uint2*>(at) = make_uint2(0u, 0u);
+    } else {
+        v[0] = *at;
+        *at = 0u;
+    }
+}
 
 // Shared memory: cells [pairs][NBP][copies] word A, then word B | gains [pairs][NBP] | agreement [pairs][NBP]
 // (kGeneral) or 1 / n [eras + 1] | (divisor, reciprocal) [largest era + 1] when an era is one tile.
-// A pair's gains lie at i * 32 + lane for bin lane * BPL + i.
-template <int BPL, int MODE>
+// A pair's gains lie at i * 32 + lane for bin lane * BPL + i.  COPIES: interleaved copies of the cells.
+template <int BPL, int MODE, int COPIES>
 __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ? 2 : 1) walk_kernel(WalkLaunch a) {
     constexpr bool UNIT = MODE != kGeneral, TILES = MODE != kUnit;
     constexpr int NBP = 32 * BPL;        // bins of a pair's cells
     constexpr int SLOTS = kWalkNodes * NBP / kWalkThreads;   // thresholds a thread may own
     constexpr int plane = kWalkNodes * NBP;
-    constexpr int COPIES = walk_copies(BPL);
     constexpr int words = plane * COPIES;                    // of word A; word B follows
     extern __shared__ __align__(16) uint32_t s_cells[];      // [pairs][NBP][COPIES]
     float2* s_gain = reinterpret_cast<float2*>(s_cells + 2 * words);
@@ -188,13 +204,13 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
     __shared__ uint8_t s_set[256];
     __shared__ int s_off[kWalkNodes + 2];                    // row ranges of the batch's eras
     const int n_nodes = min(*a.n_nodes_ptr, a.n_nodes);
-    const int node0 = blockIdx.x * kWalkNodes;
-    const int live = min(kWalkNodes, n_nodes - node0);       // nodes of this CTA
+    const int CN = a.cell_nodes;                             // nodes of a CTA at most: a power of two
+    const int node0 = blockIdx.x * CN;
+    const int live = min(CN, n_nodes - node0);
     if (live <= 0) return;
     const int f = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = a.max_bins, E = a.n_eras, K = a.n_thr;
-    const int CN = a.cell_nodes;                             // nodes the cells hold: a power of two
     const int EB = TILES ? 1 : kWalkNodes / CN;              // eras of a batch
     const int CB = a.count_bits, LB = a.lo_bits;
     const uint32_t lo_mask = (1u << LB) - 1u, cmask = (1u << CB) - 1u;
@@ -225,7 +241,7 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
     // ---- rows: groups of four; a row of another CTA's node is predicated off, so the usual group has
     //      no branch per row ----
     const uint8_t* codes = a.codes + (int64_t)a.feat_rows[f] * a.pitch;
-    const bool sparse = gridDim.x > 1;   // most rows belong to other CTAs: gradients are read when a row is ours
+    const bool sparse = gridDim.x > 2;   // most rows belong to other CTAs: gradients are read when a row is ours
     constexpr uint32_t PAIR = 4u * NBP * COPIES;             // bytes of a pair's cells
     const uint32_t cells_at = (uint32_t)__cvta_generic_to_shared(s_cells) + 4u * (threadIdx.x & (COPIES - 1));
     auto load_group = [&](uint32_t g, int r1, RowGroup& x) {
@@ -347,18 +363,19 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
         if (scans && (TILES || my_era < n_eras_now)) {
             uint32_t A[BPL], B[BPL];
             uint32_t* at = s_cells + (warp * NBP + lane * BPL) * COPIES;
+            uint32_t wa[BPL * COPIES], wb[BPL * COPIES];
+            take_words(at, wa);
+            take_words(at + words, wb);
 #pragma unroll
             for (int i = 0; i < BPL; ++i) {
-                A[i] = at[i * COPIES];
-                B[i] = at[words + i * COPIES];
+                A[i] = wa[i * COPIES];
+                B[i] = wb[i * COPIES];
 #pragma unroll
                 for (int c = 1; c < COPIES; ++c) {
-                    A[i] += at[i * COPIES + c];
-                    B[i] += at[words + i * COPIES + c];
+                    A[i] += wa[i * COPIES + c];
+                    B[i] += wb[i * COPIES + c];
                 }
             }
-#pragma unroll
-            for (int i = 0; i < BPL * COPIES; ++i) at[i] = at[words + i] = 0u;
 #pragma unroll
             for (int i = 1; i < BPL; ++i) {
                 A[i] += A[i - 1];
@@ -547,19 +564,18 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
     }
 }
 
-template <int BPL, int MODE>
-int launch_mode(const WalkLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
+template <int BPL, int MODE, int COPIES>
+int launch_one(const WalkLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
     if (smem > 40 * 1024)   // (beside the static arrays)
-        PB_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<BPL, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    walk_kernel<BPL, MODE><<<grid, kWalkThreads, smem, stream>>>(a);
+        PB_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<BPL, MODE, COPIES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    walk_kernel<BPL, MODE, COPIES><<<grid, kWalkThreads, smem, stream>>>(a);
     return PB_OK;
 }
 
 template <int BPL>
-int launch_bpl(const WalkLaunch& a, int mode, dim3 grid, size_t smem, cudaStream_t stream) {
-    return mode == kUnit ? launch_mode<BPL, kUnit>(a, grid, smem, stream)
-           : mode == kUnitTiles ? launch_mode<BPL, kUnitTiles>(a, grid, smem, stream)
-                                : launch_mode<BPL, kGeneral>(a, grid, smem, stream);
+int launch_bpl(const WalkLaunch& a, int mode, int copies, dim3 grid, size_t smem, cudaStream_t stream) {
+    if (mode == kUnit) return copies == 2 ? launch_one<BPL, kUnit, 2>(a, grid, smem, stream) : launch_one<BPL, kUnit, 1>(a, grid, smem, stream);
+    return mode == kUnitTiles ? launch_one<BPL, kUnitTiles, 1>(a, grid, smem, stream) : launch_one<BPL, kGeneral, 1>(a, grid, smem, stream);
 }
 
 }  // namespace
@@ -568,15 +584,27 @@ int launch_walk(WalkLaunch a, cudaStream_t stream) {
     if (a.n_feat <= 0 || a.n_nodes <= 0) return PB_OK;
     if (a.max_bins > 256) return fail_arg("max_bins=%d outside [2,256]", a.max_bins);
     const int bpl = a.max_bins <= 32 ? 1 : a.max_bins <= 64 ? 2 : a.max_bins <= 128 ? 4 : 8;
+    // Nodes of a CTA: sixteen, fewer while the CTAs do not fill the GPU (two per SM): the scan and the
+    // recursion of an era are then spread over more SMs, each of which goes through the rows of the
+    // feature.  That pays up to about 320 rows per era and node of the CTA (20 000 rows, 64 features, 20
+    // eras, 16 nodes: 57 -> 28 us; 200 000 rows, 100 features, 40 eras: 16 nodes 152 -> 135, 8 nodes 97 -> 110).
     a.cell_nodes = a.n_nodes < kWalkNodes ? a.n_nodes : kWalkNodes;
+    while (a.cell_nodes > 1 && (int64_t)a.n_feat * (a.n_nodes / a.cell_nodes) * 2 <= 148 * 2 &&
+           a.n_rows <= (int64_t)320 * a.cell_nodes * a.n_eras)
+        a.cell_nodes /= 2;
     const bool unit = a.era_alpha <= 0.f && a.direction_weight == 0.f && a.n_eras < kWalkInv;
     const int mode = !unit ? kGeneral : a.max_era_rows <= a.tile_rows ? kUnit : kUnitTiles;
     const size_t plane = (size_t)kWalkNodes * 32 * bpl * 4;
-    size_t smem = (2 * walk_copies(bpl) + 2) * plane + (mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
+    // Two copies of the cells while few nodes share the rows of a warp: its lanes then meet in the bins of
+    // a column of few values, which took twice as long as the others.  With many nodes they meet less and
+    // the copies only lengthen the scan (500 000 rows, 256 features: 8 nodes 401 us with copies, 454
+    // without, 16 nodes 594 either way, 32 nodes 1 125 and 965).
+    const int copies = (mode == kUnit && bpl <= 4 && a.n_nodes <= 8) ? 2 : 1;
+    size_t smem = (2 * copies + 2) * plane + (mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
     // the table of divisors is 8 bytes per row of the largest era: while it leaves room for two CTAs per SM
     a.div_table = a.max_era_rows <= a.tile_rows && smem + (size_t)(a.max_era_rows + 1) * 8 <= 110 * 1024;
     if (a.div_table) smem += (size_t)(a.max_era_rows + 1) * 8;
-    dim3 grid((unsigned)((a.n_nodes + kWalkNodes - 1) / kWalkNodes), (unsigned)a.n_feat);
+    dim3 grid((unsigned)((a.n_nodes + a.cell_nodes - 1) / a.cell_nodes), (unsigned)a.n_feat);
     if (grid.y > 65535u) return fail_arg("too many features in one launch");
     prof_begin(a.prof, kProfHist, stream);
     if (a.mass) {
@@ -588,9 +616,9 @@ int launch_walk(WalkLaunch a, cudaStream_t stream) {
         mass_count_kernel<<<dim3((unsigned)a.n_feat, (unsigned)parts), 256, 0, stream>>>(a);
         count_launch(1);
     }
-    int rc = bpl == 1 ? launch_bpl<1>(a, mode, grid, smem, stream)
-             : bpl == 2 ? launch_bpl<2>(a, mode, grid, smem, stream)
-             : bpl == 4 ? launch_bpl<4>(a, mode, grid, smem, stream) : launch_bpl<8>(a, mode, grid, smem, stream);
+    int rc = bpl == 1 ? launch_bpl<1>(a, mode, copies, grid, smem, stream)
+             : bpl == 2 ? launch_bpl<2>(a, mode, copies, grid, smem, stream)
+             : bpl == 4 ? launch_bpl<4>(a, mode, copies, grid, smem, stream) : launch_bpl<8>(a, mode, copies, grid, smem, stream);
     prof_end(a.prof, kProfHist, stream);
     if (rc) return rc;
     count_launch(1);
