@@ -286,7 +286,7 @@ __host__ __device__ constexpr size_t lane_extra_bytes(int R, int fpl) {
     return lane_record_bytes(R) + (size_t)(32 / R) * fpl * (kStagePitch + sizeof(int64_t));
 }
 
-template <int A, int T, int R>
+template <int A, int T, int R, int STAGES>  // STAGES: staged blocks of codes
 __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKernelArgs a) {
     extern __shared__ __align__(16) unsigned char smb[];
     const int n_nodes = a.n_nodes_ptr ? min(*a.n_nodes_ptr, a.n_nodes) : a.n_nodes;
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
     uint32_t* cells = reinterpret_cast<uint32_t*>(smb);
     uint2* records = reinterpret_cast<uint2*>(smb + (size_t)T * slot_bytes);
     unsigned char* stage = smb + (size_t)T * slot_bytes + lane_record_bytes(R);
-    int64_t* frow_s = reinterpret_cast<int64_t*>(stage + (size_t)NF * kStagePitch);
+    int64_t* frow_s = reinterpret_cast<int64_t*>(stage + (size_t)STAGES * NF * kStagePitch);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int CB = a.count_bits, LB = a.lo_bits;
     const uint32_t lo_mask = (1u << LB) - 1u;
@@ -352,11 +352,13 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
     __syncthreads();
 
     // one block of codes: NF lines of 128 bytes, eight consecutive threads per line
-    auto fetch_block = [&](int b) {
+    auto fetch_block = [&](int b, int b_end) {   // (commits a group in any case)
+        unsigned char* to = stage + ((STAGES == 2 && (b & 1)) ? NF * kStagePitch : 0);
+        if (b < b_end)
         for (int p = threadIdx.x; p < NF * 8; p += blockDim.x) {
             const int s = p >> 3, part = p & 7;
             const unsigned char* src = a.codes + frow_s[s] + (int64_t)b * (kBlockRows / 2) + part * 16;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + s * kStagePitch + part * 16);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(to + s * kStagePitch + part * 16);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -377,17 +379,23 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
         rs = a.slot[r];
         rg = a.gq[r];
     };
+    int nraw_s = 0, nraw_g = 0;  // of the block after
     if (b0 < b1) {
-        fetch_block(b0);
+        fetch_block(b0, b1);
         load_state(b0, raw_s, raw_g);
+        if (STAGES == 2) {
+            fetch_block(b0 + 1, b1);
+            if (b0 + 1 < b1) load_state(b0 + 1, nraw_s, nraw_g);
+        }
     }
     for (int b = b0; b < b1; ++b) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 1) : "memory");
         __syncthreads();  // the block is complete
+        const unsigned char* here = stage + ((STAGES == 2 && (b & 1)) ? NF * kStagePitch : 0);
         uint32_t w[FPL][WPP];
 #pragma unroll
         for (int i = 0; i < FPL; ++i) {
-            const unsigned char* p = stage + (i * TL + col0) * kStagePitch + warp * (kLaneRows / 2) + phase * (PR / 2);
+            const unsigned char* p = here + (i * TL + col0) * kStagePitch + warp * (kLaneRows / 2) + phase * (PR / 2);
             if (R == 1) {
                 const uint4 v = *reinterpret_cast<const uint4*>(p);
                 w[i][0] = v.x; w[i][1 % WPP] = v.y; w[i][2 % WPP] = v.z; w[i][3 % WPP] = v.w;
@@ -398,8 +406,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
                 w[i][0] = *reinterpret_cast<const uint32_t*>(p);
             }
         }
-        __syncthreads();  // every warp holds its codes: the stage is free for the next block
-        if (b + 1 < b1) fetch_block(b + 1);
+        __syncthreads();  // every warp holds its codes: their stage is free
+        fetch_block(b + STAGES, b1);
 
         const int r = b * kBlockRows + warp * kLaneRows + lane;
         const bool ok = (r >= r0) & (r < r1) & (raw_s < n_nodes);
@@ -414,8 +422,14 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
             st[lane + lane / PR] = rec;
         }
         const bool chunk_on = __any_sync(0xFFFFFFFFu, ok);  // (also orders the record stores)
-        int nraw_s = 0, nraw_g = 0;
-        if (b + 1 < b1) load_state(b + 1, nraw_s, nraw_g);
+        if (STAGES == 2) {
+            raw_s = nraw_s;
+            raw_g = nraw_g;
+            if (b + 2 < b1) load_state(b + 2, nraw_s, nraw_g);
+        } else {  // (straight into the registers the records were made from: a copy would wait for the load)
+            raw_s = raw_g = 0;
+            if (b + 1 < b1) load_state(b + 1, raw_s, raw_g);
+        }
         if (n_mine > 0 && chunk_on) {
             uint32_t jw[T][2];  // joint codes of eight rows: even rows, odd rows (A == 2)
             uint2 rawn[4];
@@ -479,8 +493,6 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
             }
         }
         __syncwarp();  // the records are rewritten in the next step
-        raw_s = nraw_s;
-        raw_g = nraw_g;
     }
     __syncthreads();
 
@@ -776,13 +788,27 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
 
 template <int A, int T, int R>
 int launch_lane_r(const HistKernelArgs& a, size_t cell_bytes, cudaStream_t stream) {
-    const size_t smem = cell_bytes + lane_extra_bytes(R, A * T);
-    if (smem > 48 * 1024)
-        PB_CUDA_TRY(cudaFuncSetAttribute(hist_lane_kernel<A, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    // A second staged block while there are no more CTAs than the SMs hold at once and it costs no
+    // resident one: with nothing else to run, a block is worked through before the next one arrives
+    // (330 000 rows in 120 eras of unequal size, 102 features: 286 -> 228 us over six depths; a launch of
+    // several waves gains nothing and pays for the copies).
+    size_t smem = cell_bytes + lane_extra_bytes(R, A * T);
+    const size_t more = (size_t)(32 / R) * A * T * kStagePitch;
+    const auto resident = [](size_t bytes) { return 2 * (bytes + 1024) <= (size_t)228 * 1024 ? 2 : bytes <= (size_t)227 * 1024 ? 1 : 0; };
     const int per_cta = (32 / R) * A * T;
     dim3 grid((unsigned)(a.n_eras * a.tiles_per_era), (unsigned)((a.n_feat + per_cta - 1) / per_cta), 1);
-    hist_lane_kernel<A, T, R><<<grid, kLaneWarps * 32, smem, stream>>>(a);
+    if constexpr (A * T <= 4) {
+        if ((int64_t)grid.x * grid.y <= 148 * 2 && resident(smem + more) == resident(smem)) {
+            smem += more;
+            if (smem > 40 * 1024)   // (beside the static arrays)
+                PB_CUDA_TRY(cudaFuncSetAttribute(hist_lane_kernel<A, T, R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            hist_lane_kernel<A, T, R, 2><<<grid, kLaneWarps * 32, smem, stream>>>(a);
+            return PB_OK;
+        }
+    }
+    if (smem > 40 * 1024)
+        PB_CUDA_TRY(cudaFuncSetAttribute(hist_lane_kernel<A, T, R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    hist_lane_kernel<A, T, R, 1><<<grid, kLaneWarps * 32, smem, stream>>>(a);
     return PB_OK;
 }
 
@@ -877,7 +903,7 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
         double best = 1e30;
         int best_tile = a.tile_rows;
         {
-            constexpr double kPass = 15.0, kPassFeat = 2.2, kTuple = 33.0, kCell = 0.145, kCellAtomic = 0.45;
+            constexpr double kPass = 15.0, kPassFeat = 2.2, kTuple = 33.0, kCell = 0.145, kAtomic = 6e-5;
             const int tiles_min = a.tiles_per_era;
             int64_t c = h.max_bins;
             for (int a_try = 1; a_try <= cap; ++a_try, c *= h.max_bins) {
@@ -890,17 +916,14 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
                         const size_t smem = bytes + lane_extra_bytes(r_try, a_try * t_try) + 1024;
                         const int per_sm = (2 * smem <= (size_t)228 * 1024) ? 2 : 1;
                         const double slots = 148.0 * per_sm;
-                        // Eras that are cut into tiles anyway are cut so that the CTAs fill whole waves (1.3 M
-                        // rows without eras are 160 largest tiles, two blocks of features: 24 of 320 CTAs
-                        // ran alone: 70 us a launch, 51 with whole waves); every tile pays its flush of global atomics.
-                        for (int w = 1; w <= (a.use_atomics ? 6 : 1); ++w) {
+                        // Eras that are cut into tiles anyway may be cut so that the CTAs fill whole waves: 1.3 M
+                        // rows without eras and 57 features are 160 largest tiles, 320 CTAs, 24 of which ran
+                        // alone (one node: 63 us, 45 in whole waves).  Every tile pays a flush of global atomics.
+                        for (int w = (a.use_atomics ? 0 : 1); w <= (a.use_atomics ? 6 : 1); ++w) {  // 0: largest tiles
                             int tile = a.tile_rows, tiles = tiles_min;
                             if (a.use_atomics) {
-                                tiles = (int)(w * slots / ((double)h.n_eras * blocks));
-                                if (tiles < tiles_min) {
-                                    if (w < 6) continue;
-                                    tiles = tiles_min;
-                                }
+                                if (w > 0) tiles = (int)(w * slots / ((double)h.n_eras * blocks));
+                                if (tiles < tiles_min) continue;
                                 tile = ((h.max_era_rows + tiles - 1) / tiles + 255) / 256 * 256;
                                 if (tile > kTileRowsMax) tile = kTileRowsMax;
                                 tiles = (h.max_era_rows + tile - 1) / tile;
@@ -908,11 +931,16 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
                             const double tile_scale = (double)(a.use_atomics ? tile : max_tile) / 4700.0;
                             const double ctas = (double)h.n_eras * tiles * blocks;
                             double waves = ctas > slots ? ctas / slots : 1.0;
-                            if (a.use_atomics) waves = (double)(int64_t)(waves + 0.999);
+                            if (a.use_atomics && waves > 1.0) {  // a last wave of a few CTAs takes less than a whole one
+                                const double rest = waves - (double)(int64_t)waves;
+                                waves = (double)(int64_t)waves + (rest > 1e-9 ? 0.35 + 0.65 * rest : 0.0);
+                            }
                             // (a few per cent against more phases: equal estimates favour whole-warp tuples)
                             double cost = (r_try == 1 ? 1.0 : r_try == 2 ? 1.04 : 1.08) * waves * per_sm * (per_sm == 1 ? 1.2 : 1.0) *
                                           (tile_scale * (kPass + kPassFeat * a_try * t_try + kTuple * t_try / r_try) +
-                                           (a.use_atomics ? kCellAtomic : kCell) * (double)bytes / 1024.0);
+                                           kCell * (double)bytes / 1024.0);
+                            // the flush adds every cell of every tile to the global histogram, about 100 G atomics a second
+                            if (a.use_atomics) cost += kAtomic * (double)h.n_eras * tiles * h.n_feat * h.n_nodes * h.max_bins;
                             if (forced) cost = (a_try == forced[0] && t_try == forced[1] && r_try == forced[2]) ? cost * 1e-6 : cost + 1e9;
                             if (cost < best * (1.0 - 1e-9)) {
                                 best = cost;
