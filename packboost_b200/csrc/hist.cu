@@ -1030,11 +1030,11 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
     if (grid.y > 65535u || grid.z > 65535u) return fail_arg("histogram grid too large");
     prof_begin(h.prof, kProfHist, stream);
     if (h.code_bits == 4) {
-        if (smem > 48 * 1024)
+        if (smem > 40 * 1024)   // (48 KB without asking, and s_frow is beside the cells)
             PB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<4, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         hist_kernel<4, 256><<<grid, threads, smem, stream>>>(a);
     } else {
-        if (smem > 48 * 1024)
+        if (smem > 40 * 1024)
             PB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<8, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         hist_kernel<8, 512><<<grid, threads, smem, stream>>>(a);
     }

@@ -284,6 +284,19 @@ def test_histogram_exact_in_every_launch_shape(shape):
     assert "hist_lane_kernel<%s>" % shape.replace(" ", ",") in res.stderr, res.stderr[-2000:]
 
 
+@pytest.mark.parametrize("max_bins,n_nodes", [(96, 64), (12, 512), (191, 32), (47, 128)])
+def test_histogram_whose_cells_take_just_the_shared_memory_given_without_asking(max_bins, n_nodes):
+    """48 KB of cells or a little less beside the kernel's own arrays: such a launch has to ask for more
+    (in a child process, where no larger launch has asked before)."""
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    script = (f"import sys; sys.path.insert(0, {root!r})\nfrom tests.test_gpu_kernels import _hist_case\n"
+              f"_hist_case(3000, 5, 2, {max_bins}, {n_nodes}, seed=3)\nprint('ok')\n")
+    res = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=600)
+    assert res.returncode == 0 and res.stdout.strip().endswith("ok"), res.stdout[-2000:] + res.stderr[-4000:]
+
+
 @pytest.mark.parametrize("n,f,max_bins", [(1, 1, 5), (255, 127, 5), (256, 128, 5), (257, 129, 16), (1030, 301, 5),
                                           (513, 131, 64), (300, 33, 2), (259, 97, 128)])
 def test_pack_kernels_at_tile_edges(n, f, max_bins):
