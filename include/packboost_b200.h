@@ -234,6 +234,10 @@ int pb_round_begin(const pb_train_state* st, int64_t apply_previous, void* strea
 int pb_depth_hist_score(const pb_train_state* st, int64_t depth, const int32_t* feat_rows,
                         const int32_t* feat_pos, int64_t n_feat, int64_t n_sampled, void* stream);
 
+/* Which way pb_depth_hist_score takes a depth: *walks = 1 for the one kernel that walks the eras, 0 for
+ * the histogram, gain and chain kernels (the results are the same bit for bit).  No device work. */
+int pb_depth_walks(const pb_train_state* st, int64_t depth, int64_t n_feat, int64_t n_sampled, int64_t* walks);
+
 /* Device pointer and byte size of the candidate table of `depth` (for the cross-device
  * exchange: entries are disjoint per device, so a SUM all-reduce over int32 words merges
  * them; `pb_depth_clear_candidates` must run first when more than one device takes part). */

@@ -193,6 +193,7 @@ struct HistFuse {
 // True when launch_hist(h) would run the lane kernel with one tile per era, which is what the
 // fused flush needs (a CTA then holds the complete cells of its era).
 bool hist_can_fuse(const HistLaunch& h);
+int hist_node_chunks(int n_nodes, int max_bins);
 int launch_hist(const HistLaunch& h, cudaStream_t stream);
 int hist_max_arity();  // default tuple-size cap of the lane kernel (PACKBOOST_HIST_MAX_ARITY=1 lowers it)
 
@@ -268,6 +269,7 @@ struct WalkLaunch {
     int cell_nodes, div_table;   // set by launch_walk
 };
 int launch_walk(WalkLaunch a, cudaStream_t stream);
+double walk_estimate_us(WalkLaunch a);   // about what launch_walk(a) takes
 size_t score_scratch_bytes_per_feature(int node_stride, int n_eras, int n_thr);
 
 }  // namespace pb

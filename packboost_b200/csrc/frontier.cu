@@ -682,19 +682,9 @@ static bool use_fused_flush(const pb_train_state* st, int64_t depth) {
     return hist_can_fuse(hist_launch_of(st, depth, c));
 }
 
-// Tables of many bins are accumulated and scored by one kernel that walks the eras (walk.cu); a CTA
-// works through all rows of its feature, so few features of very many rows keep the two-step path,
-// which cuts the rows (PACKBOOST_WALK=0 keeps it everywhere, for comparisons).
-static bool use_walk(const pb_train_state* st, int64_t n_feat) {
-    static const bool enabled = [] {
-        const char* e = getenv("PACKBOOST_WALK");
-        return !(e && e[0] == '0' && e[1] == 0);
-    }();
-    return enabled && st->code_bits == 8 && n_feat <= 65535 && (n_feat >= 32 || st->n_rows <= (1 << 18));
-}
-
-static int walk_depth(const pb_train_state* st, int64_t depth, const int32_t* feat_rows, const int32_t* feat_pos, int64_t n_feat,
-                      void* mass, Cand* cand, cudaStream_t stream) {
+// The launch of walk.cu for one depth.
+static WalkLaunch walk_launch_of(const pb_train_state* st, int64_t depth, const int32_t* feat_rows, const int32_t* feat_pos,
+                                 int64_t n_feat, void* mass, Cand* cand) {
     Ctl c = ctl_view(st->ctl);
     WalkLaunch w;
     memset(&w, 0, sizeof(w));
@@ -731,7 +721,62 @@ static int walk_depth(const pb_train_state* st, int64_t depth, const int32_t* fe
     w.cand = cand;
     w.prof = st->profile;
     w.debug_flags = &c.head->debug_flags;
-    return launch_walk(w, stream);
+    return w;
+}
+
+// About what the histogram, gain and chain kernels of one depth take (fitted with walk_estimate_us, to the
+// same depths): the rows by feature, the cells of every tile, the (gain, weight) rows, the recursion, and with
+// mass cuts the CTA that sums a feature's bins over eras and nodes.
+static double two_step_estimate_us(const pb_train_state* st, int64_t depth, int64_t n_feat, const BlockPlan& plan) {
+    const double nodes = node_stride_of(depth), eras = (double)st->n_eras, bins = (double)st->max_bins;
+    const double tiles = eras * (double)(st->max_era_rows <= kTileRowsMax ? 1 : (st->max_era_rows + kTileRowsMax - 1) / kTileRowsMax);
+    const double gains = (double)n_feat * eras * nodes * (double)st->n_thresholds;
+    const double chunks = (double)hist_node_chunks((int)nodes, (int)st->max_bins);
+    const double blocks = (double)((n_feat + plan.fb - 1) / plan.fb);
+    const bool unit = st->era_alpha <= 0.0 && st->direction_weight == 0.0;
+    return blocks * (48.0 + (unit ? 0.15 : 0.4) * eras) + 1.5e-6 * (double)st->n_rows * n_feat * chunks + 9.3e-6 * gains +
+           8.8e-6 * n_feat * tiles * nodes * bins + (st->cut_mass ? 0.12 * eras * nodes + 0.02 * (double)st->n_thresholds * bins : 0.0) +
+           (st->direction_weight != 0.0 ? 1.5e-6 * gains : 0.0);
+}
+
+// Codes of 8 bits are accumulated and scored by one kernel that walks the eras (walk.cu) or by the
+// histogram, gain and chain kernels, bit for bit alike.  The walk moves no histogram and no gains, but its
+// CTAs go through all rows of a feature; the other path cuts the rows, and has the GPU full with few
+// features.  So neither is the faster one everywhere (128 bins, depth 6, a round's histogram and score;
+// walk / other path): 500 000 rows x 200 features, 100 eras 2.6 / 3.8 ms; 131 072 x 200, 574 eras 8.2 / 20.8;
+// 262 144 x 64, 20 eras 1.06 / 0.78; 1 000 000 x 64, 100 eras 3.3 / 2.4; 4 000 000 x 32, 20 eras 10.1 / 2.4.
+// The estimates decide by depth: over the 9 000 depths they were fitted to that takes 3 % more time than
+// the better path each time, where the walk everywhere takes 50 % more.  Where they come within a tenth it
+// is the walk, whose estimate is the safer one in deep frontiers of few rows.
+// PACKBOOST_WALK=0 / 1 takes one path everywhere, for comparisons.
+struct DepthPath {
+    size_t cand_bytes;   // of the candidate table, at the start of the workspace
+    bool walk;
+    WalkLaunch w;        // where it is the walk
+    BlockPlan plan;      // where it is not
+};
+
+static int depth_path(const pb_train_state* st, int64_t depth, const int32_t* feat_rows, const int32_t* feat_pos, int64_t n_feat,
+                      int64_t n_sampled, DepthPath* p) {
+    static const int forced = [] {
+        const char* e = getenv("PACKBOOST_WALK");
+        return (e && (e[0] == '0' || e[0] == '1') && e[1] == 0) ? e[0] - '0' : -1;
+    }();
+    const int stride = node_stride_of(depth);
+    p->cand_bytes = align_up(sizeof(Cand) * (size_t)n_sampled * stride, 256);
+    PB_REQUIRE((int64_t)p->cand_bytes < st->workspace_bytes, "workspace too small for the candidate table");
+    const bool planned = plan_block((size_t)st->workspace_bytes - p->cand_bytes, stride, st->n_eras, st->max_bins, st->n_thresholds,
+                                    n_feat, use_fused_flush(st, depth), st->direction_weight != 0.0, &p->plan);
+    const int64_t mass_bytes = st->cut_mass ? n_feat * 256 * (int64_t)sizeof(uint32_t) : 0;
+    p->walk = st->code_bits == 8 && n_feat <= 65535 && (int64_t)p->cand_bytes + mass_bytes <= st->workspace_bytes && forced != 0;
+    if (p->walk) {
+        char* ws = static_cast<char*>(st->workspace);
+        p->w = walk_launch_of(st, depth, feat_rows, feat_pos, n_feat, ws + p->cand_bytes, reinterpret_cast<Cand*>(ws));
+        // (a workspace may hold no feature of histogram and gains at this depth: then the walk is the only way)
+        if (forced < 0 && planned) p->walk = walk_estimate_us(p->w) <= 1.1 * two_step_estimate_us(st, depth, n_feat, p->plan);
+    }
+    PB_REQUIRE(p->walk || planned, "workspace too small for one feature of histogram at depth %lld", (long long)depth);
+    return PB_OK;
 }
 
 static int hist_score_blocks(const pb_train_state* st, int64_t depth, const int32_t* feat_rows, const int32_t* feat_pos,
@@ -913,19 +958,27 @@ extern "C" int pb_depth_hist_score(const pb_train_state* st, int64_t depth, cons
     PB_REQUIRE(n_feat >= 0 && n_feat <= n_sampled && n_sampled <= st->n_features_total, "feature counts out of range");
     if (n_feat == 0) return PB_OK;
     PB_REQUIRE(feat_rows && feat_pos, "null feature list");
-    const int stride = node_stride_of(depth);
-    const size_t cand_bytes = align_up(sizeof(Cand) * (size_t)n_sampled * stride, 256);
-    PB_REQUIRE((int64_t)cand_bytes < st->workspace_bytes, "workspace too small for the candidate table");
-    char* ws = static_cast<char*>(st->workspace);
-    const int64_t mass_bytes = st->cut_mass ? n_feat * 256 * (int64_t)sizeof(uint32_t) : 0;
-    if (use_walk(st, n_feat) && (int64_t)cand_bytes + mass_bytes <= st->workspace_bytes)
-        return walk_depth(st, depth, feat_rows, feat_pos, n_feat, ws + cand_bytes, reinterpret_cast<Cand*>(ws), (cudaStream_t)stream_);
-    BlockPlan plan;
-    PB_REQUIRE(plan_block((size_t)st->workspace_bytes - cand_bytes, stride, st->n_eras, st->max_bins, st->n_thresholds,
-                          n_feat, use_fused_flush(st, depth), st->direction_weight != 0.0, &plan),
-               "workspace too small for one feature of histogram at depth %lld", (long long)depth);
-    return hist_score_blocks(st, depth, feat_rows, feat_pos, n_feat, ws + cand_bytes, plan, reinterpret_cast<Cand*>(ws),
-                             (cudaStream_t)stream_);
+    DepthPath path;
+    rc = depth_path(st, depth, feat_rows, feat_pos, n_feat, n_sampled, &path);
+    if (rc) return rc;
+    if (path.walk) return launch_walk(path.w, (cudaStream_t)stream_);
+    return hist_score_blocks(st, depth, feat_rows, feat_pos, n_feat, static_cast<char*>(st->workspace) + path.cand_bytes, path.plan,
+                             static_cast<Cand*>(st->workspace), (cudaStream_t)stream_);
+}
+
+extern "C" int pb_depth_walks(const pb_train_state* st, int64_t depth, int64_t n_feat, int64_t n_sampled, int64_t* walks) {
+    int rc = check_state(st);
+    if (rc) return rc;
+    rc = need_workspace(st, "pb_depth_walks");
+    if (rc) return rc;
+    PB_REQUIRE(walks, "null argument");
+    PB_REQUIRE(depth >= 0 && depth < st->max_depth, "depth out of range");
+    PB_REQUIRE(n_feat >= 1 && n_feat <= n_sampled && n_sampled <= st->n_features_total, "feature counts out of range");
+    DepthPath path;
+    rc = depth_path(st, depth, nullptr, nullptr, n_feat, n_sampled, &path);
+    if (rc) return rc;
+    *walks = path.walk ? 1 : 0;
+    return PB_OK;
 }
 
 extern "C" int pb_depth_select(const pb_train_state* st, int64_t depth, const int32_t* sampled_features,

@@ -832,6 +832,15 @@ bool hist_can_fuse(const HistLaunch& h) {
            (int64_t)h.n_nodes * h.max_bins * kLaneCellBytes <= kLaneCellsMax && h.n_feat > 0 && h.n_nodes > 0;
 }
 
+// Nodes whose cells of one feature a CTA of hist_kernel holds, and the passes over the rows that makes.
+static int chunk_nodes(int n_nodes, int max_bins) {
+    return (int64_t)n_nodes * max_bins <= kSmemCellBudget ? n_nodes : kSmemCellBudget / max_bins;
+}
+int hist_node_chunks(int n_nodes, int max_bins) {
+    const int per = chunk_nodes(n_nodes, max_bins);
+    return (n_nodes + per - 1) / per;
+}
+
 int launch_hist(const HistLaunch& h, cudaStream_t stream) {
     if (h.n_feat <= 0 || h.n_nodes <= 0) return PB_OK;
     HistKernelArgs a;
@@ -996,13 +1005,9 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
 
     if (h.fuse) return fail_arg("fused flush requested for a launch that cannot fuse (check hist_can_fuse first)");
     // shared-memory plan: cells per feature, node chunks, feature group, copies
-    const int64_t per_feat_all = (int64_t)h.n_nodes * h.max_bins;
-    int nodes_per_chunk = h.n_nodes;
-    if (per_feat_all > kSmemCellBudget) {
-        nodes_per_chunk = kSmemCellBudget / h.max_bins;
-        if (nodes_per_chunk < 1) return fail_arg("max_bins=%d does not fit the histogram tile", h.max_bins);
-    }
-    const int chunks = (h.n_nodes + nodes_per_chunk - 1) / nodes_per_chunk;
+    const int nodes_per_chunk = chunk_nodes(h.n_nodes, h.max_bins);
+    if (nodes_per_chunk < 1) return fail_arg("max_bins=%d does not fit the histogram tile", h.max_bins);
+    const int chunks = hist_node_chunks(h.n_nodes, h.max_bins);
     const int64_t per_feat = (int64_t)nodes_per_chunk * h.max_bins;
     if (per_feat > 65534) return fail_arg("node chunk too large");
     int copies = 1;

@@ -580,10 +580,16 @@ int launch_bpl(const WalkLaunch& a, int mode, int copies, dim3 grid, size_t smem
 
 }  // namespace
 
-int launch_walk(WalkLaunch a, cudaStream_t stream) {
-    if (a.n_feat <= 0 || a.n_nodes <= 0) return PB_OK;
-    if (a.max_bins > 256) return fail_arg("max_bins=%d outside [2,256]", a.max_bins);
-    const int bpl = a.max_bins <= 32 ? 1 : a.max_bins <= 64 ? 2 : a.max_bins <= 128 ? 4 : 8;
+// How a launch is laid out.
+struct WalkShape {
+    int bpl, mode, copies, groups;
+    bool div_table;
+    size_t smem;
+};
+
+static WalkShape walk_shape(WalkLaunch& a) {
+    WalkShape s;
+    s.bpl = a.max_bins <= 32 ? 1 : a.max_bins <= 64 ? 2 : a.max_bins <= 128 ? 4 : 8;
     // Nodes of a CTA: sixteen, fewer while the CTAs do not fill the GPU (two per SM): the scan and the
     // recursion of an era are then spread over more SMs, each of which goes through the rows of the
     // feature.  That pays up to about 320 rows per era and node of the CTA (20 000 rows, 64 features, 20
@@ -592,19 +598,50 @@ int launch_walk(WalkLaunch a, cudaStream_t stream) {
     while (a.cell_nodes > 1 && (int64_t)a.n_feat * (a.n_nodes / a.cell_nodes) * 2 <= 148 * 2 &&
            a.n_rows <= (int64_t)320 * a.cell_nodes * a.n_eras)
         a.cell_nodes /= 2;
+    s.groups = (a.n_nodes + a.cell_nodes - 1) / a.cell_nodes;
     const bool unit = a.era_alpha <= 0.f && a.direction_weight == 0.f && a.n_eras < kWalkInv;
-    const int mode = !unit ? kGeneral : a.max_era_rows <= a.tile_rows ? kUnit : kUnitTiles;
-    const size_t plane = (size_t)kWalkNodes * 32 * bpl * 4;
+    s.mode = !unit ? kGeneral : a.max_era_rows <= a.tile_rows ? kUnit : kUnitTiles;
+    const size_t plane = (size_t)kWalkNodes * 32 * s.bpl * 4;
     // Two copies of the cells while few nodes share the rows of a warp: its lanes then meet in the bins of
     // a column of few values, which took twice as long as the others.  With many nodes they meet less and
     // the copies only lengthen the scan (500 000 rows, 256 features: 8 nodes 401 us with copies, 454
     // without, 16 nodes 594 either way, 32 nodes 1 125 and 965).
-    const int copies = (mode == kUnit && bpl <= 4 && a.n_nodes <= 8) ? 2 : 1;
-    size_t smem = (2 * copies + 2) * plane + (mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
+    s.copies = (s.mode == kUnit && s.bpl <= 4 && a.n_nodes <= 8) ? 2 : 1;
+    s.smem = (2 * s.copies + 2) * plane + (s.mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
     // the table of divisors is 8 bytes per row of the largest era: while it leaves room for two CTAs per SM
-    a.div_table = a.max_era_rows <= a.tile_rows && smem + (size_t)(a.max_era_rows + 1) * 8 <= 110 * 1024;
-    if (a.div_table) smem += (size_t)(a.max_era_rows + 1) * 8;
-    dim3 grid((unsigned)((a.n_nodes + a.cell_nodes - 1) / a.cell_nodes), (unsigned)a.n_feat);
+    s.div_table = a.max_era_rows <= a.tile_rows && s.smem + (size_t)(a.max_era_rows + 1) * 8 <= 110 * 1024;
+    if (s.div_table) s.smem += (size_t)(a.max_era_rows + 1) * 8;
+    return s;
+}
+
+// A CTA goes through all rows of its feature and all eras, whatever the other SMs do, so a launch takes
+// that chain once per wave of CTAs; two CTAs on an SM take 1.29 times as long as one.  Constants fitted
+// to 9 000 timed depths (2 000 to 4 million rows, 4 to 420 features, 1 to 600 eras, 17 to 256 bins, 1 to
+// 512 nodes, every form of the score); half of the estimates are within 13 %.
+double walk_estimate_us(WalkLaunch a) {
+    const WalkShape s = walk_shape(a);
+    const int64_t tiles = a.max_era_rows <= a.tile_rows ? 1 : (a.max_era_rows + a.tile_rows - 1) / a.tile_rows;
+    const int eras = s.mode == kUnit ? kWalkNodes / a.cell_nodes : 1;   // of a batch
+    const double batches = s.mode == kUnit ? (double)((a.n_eras + eras - 1) / eras) : (double)a.n_eras * tiles;
+    const double batch = s.mode == kUnit ? 1.2 + 0.34 * s.bpl : s.mode == kUnitTiles ? 0.63 + 0.14 * s.bpl
+                         : 1.0 + ((a.direction_weight != 0.f && tiles == 1) ? 0.33 : 0.22) * s.bpl;
+    const double chain = 2.9e-4 * a.n_rows + batches * batch;
+    const int per_sm = (s.bpl <= 4 && s.mode != kGeneral) ? 2 : 1;
+    const int64_t ctas = (int64_t)a.n_feat * s.groups, places = 148 * per_sm;
+    const double whole = per_sm == 2 ? 1.29 : 1.0;
+    const int64_t rest = ctas % places;
+    const double waves = (double)(ctas / places) * whole + (rest == 0 ? 0.0 : rest <= 148 ? 1.0 : whole);
+    return 22.0 + waves * chain + (a.mass ? 16.0 + 7.5e-7 * (double)a.n_rows * a.n_feat : 0.0);
+}
+
+int launch_walk(WalkLaunch a, cudaStream_t stream) {
+    if (a.n_feat <= 0 || a.n_nodes <= 0) return PB_OK;
+    if (a.max_bins > 256) return fail_arg("max_bins=%d outside [2,256]", a.max_bins);
+    const WalkShape s = walk_shape(a);
+    const int bpl = s.bpl, mode = s.mode, copies = s.copies;
+    const size_t smem = s.smem;
+    a.div_table = s.div_table ? 1 : 0;
+    dim3 grid((unsigned)s.groups, (unsigned)a.n_feat);
     if (grid.y > 65535u) return fail_arg("too many features in one launch");
     prof_begin(a.prof, kProfHist, stream);
     if (a.mass) {

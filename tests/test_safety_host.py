@@ -1,6 +1,7 @@
 """Host-side refusals that keep malformed input away from the GPU (no device needed)."""
 
 import ctypes as C
+import os
 
 import numpy as np
 import pytest
@@ -139,6 +140,34 @@ def test_a_state_without_workspace_is_accepted_and_workspace_entries_say_so(lib)
     st.workspace_bytes = 16            # a pointer with too few bytes still is, too
     with pytest.raises(ValueError, match="workspace too small"):
         B.check(lib.pb_train_prepare(C.byref(st), eo.ctypes.data))
+
+
+@pytest.mark.parametrize("rows,feats,eras,depth,walks", [
+    (4_000_000, 32, 20, 0, 0), (4_000_000, 32, 20, 5, 0), (1_000_000, 64, 100, 0, 0), (262_144, 16, 100, 0, 0),
+    (262_144, 64, 20, 3, 0), (500_000, 200, 100, 5, 1), (131_072, 200, 574, 0, 1), (131_072, 8, 574, 5, 1),
+    (2_000_000, 148, 574, 5, 1)])
+def test_many_bins_take_the_path_that_measured_faster(lib, rows, feats, eras, depth, walks):
+    """Sizes at which one of the two equal paths measured 1.4 to 6 times as fast as the other; and a
+    workspace too small for the stored histogram leaves the walk."""
+    from packboost_b200 import backends as B
+    if "PACKBOOST_WALK" in os.environ:
+        pytest.skip("the path is forced")
+    st = _state(B)
+    st.n_rows, st.n_eras, st.max_bins, st.code_bits, st.pitch = rows, eras, 128, 8, (rows + 255) // 256 * 256
+    st.n_features_total = st.n_features_local = feats
+    st.max_depth, st.n_thresholds, st.workspace_bytes = 6, 127, 8 << 30
+    eo = (np.arange(eras + 1, dtype=np.int64) * rows // eras).astype(np.int32)
+    B.check(lib.pb_train_prepare(C.byref(st), eo.ctypes.data))
+    got = C.c_int64(-1)
+    B.check(lib.pb_depth_walks(C.byref(st), depth, feats, feats, C.byref(got)))
+    assert got.value == walks
+    st.workspace_bytes = (24 * feats << depth) + 512
+    B.check(lib.pb_depth_walks(C.byref(st), depth, feats, feats, C.byref(got)))
+    assert got.value == 1
+    st.max_bins, st.n_thresholds, st.code_bits = 5, 4, 4
+    st.workspace_bytes = 8 << 30
+    B.check(lib.pb_depth_walks(C.byref(st), depth, feats, feats, C.byref(got)))
+    assert got.value == 0
 
 
 def test_comm_entries_validate_their_arguments_without_a_gpu(lib):
