@@ -5,9 +5,6 @@
 // a process-wide pool while the calling thread hands finished pieces to the copy engine in order.
 // The ring belongs to the caller and has to stay until the stream has passed the last copy.
 
-#include <emmintrin.h>
-#include <string.h>
-
 #include <atomic>
 #include <condition_variable>
 #include <mutex>
@@ -15,6 +12,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "stream_copy.h"
 
 namespace pb {
 
@@ -23,25 +21,6 @@ namespace {
 constexpr int kPieces = 16;                     // pieces of the ring in flight
 constexpr int64_t kPieceBytes = 1 << 20;
 constexpr int64_t kDirectBytes = 384 << 10;     // below this one thread is done before the others are awake
-
-// memcpy with stores that bypass the caches (dst 16-byte aligned).  Ordinary stores leave the ring dirty
-// in the private caches of cores that go to sleep right after, and the copy engine then reads it at
-// 8 GB/s until their lines are out (12.9 MB: 1.4 ms, 0.36 ms this way; 512 MB: 13.5 and 12.0 ms).
-void stream_copy(char* dst, const char* src, int64_t n) {
-    int64_t i = 0;
-    for (; i + 64 <= n; i += 64) {
-        const __m128i a = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i));
-        const __m128i b = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 16));
-        const __m128i c = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 32));
-        const __m128i d = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 48));
-        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i), a);
-        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 16), b);
-        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 32), c);
-        _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 48), d);
-    }
-    if (i < n) memcpy(dst + i, src + i, (size_t)(n - i));
-    _mm_sfence();
-}
 
 struct UploadJob {
     const char* src;

@@ -170,6 +170,40 @@ def test_many_bins_take_the_path_that_measured_faster(lib, rows, feats, eras, de
     assert got.value == 0
 
 
+@pytest.mark.parametrize("flags", [[], ["-U__SSE2__"]])
+def test_host_sources_need_no_x86(flags, tmp_path):
+    """The ring copy builds without x86 intrinsics (``-U__SSE2__``: as on another host) and moves every
+    byte either way; no other source includes an intrinsics header."""
+    import glob
+    import re
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "packboost_b200", "csrc")
+    for path in glob.glob(os.path.join(csrc, "*")):
+        if os.path.isfile(path) and os.path.basename(path) != "stream_copy.h":
+            assert not re.search(r"#include\s*<\w*intrin\.h>", open(path).read()), path
+    deps = subprocess.run(["g++", "-std=c++17", *flags, "-M", "-x", "c++", os.path.join(csrc, "stream_copy.h")],
+                          capture_output=True, text=True, check=True).stdout
+    assert ("intrin.h" in deps) == (not flags and "__SSE2__" in subprocess.run(
+        ["g++", "-dM", "-E", "-x", "c++", os.devnull], capture_output=True, text=True, check=True).stdout)
+    src = tmp_path / "copy.cpp"
+    src.write_text("""#include "stream_copy.h"
+#include <vector>
+int main() {
+    alignas(16) static char dst[5000];
+    std::vector<char> src(5000);
+    for (int i = 0; i < 5000; ++i) src[i] = (char)(i * 7 + 1);
+    for (int n : {0, 1, 15, 63, 64, 65, 127, 128, 1000, 4093}) {
+        memset(dst, 0, sizeof(dst));
+        pb::stream_copy(dst, src.data() + 3, n);
+        if (memcmp(dst, src.data() + 3, n) || dst[n]) return 1;
+    }
+    return 0;
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-O2", *flags, "-I", csrc, str(src), "-o", str(tmp_path / "copy")], check=True)
+    assert subprocess.run([str(tmp_path / "copy")]).returncode == 0
+
+
 def test_comm_entries_validate_their_arguments_without_a_gpu(lib):
     """The NCCL-backed exchange entries refuse bad arguments before touching NCCL or a device."""
     from packboost_b200 import backends as B
