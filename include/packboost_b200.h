@@ -46,6 +46,7 @@ extern "C" {
 #define PB_ERR_CUDA (-2)     /* a CUDA runtime call failed; message starts with "CUDA error" */
 #define PB_ERR_WORKSPACE (-3)/* workspace too small */
 #define PB_ERR_NO_DEVICE (-4)
+#define PB_ERR_HOST (-5)     /* the host ran out of memory */
 
 #define PB_SLOT_NONE 0xFFFFu
 #define PB_MAX_DEPTH 12

@@ -6,6 +6,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <exception>
+
 #include "../../include/packboost_b200.h"
 
 namespace pb {
@@ -27,6 +29,17 @@ int fail_cuda(cudaError_t e, const char* what);
         cudaError_t _e = cudaGetLastError();                \
         if (_e != cudaSuccess) return pb::fail_cuda(_e, what); \
     } while (0)
+
+// An entry point that allocates on the host: an exception must not leave it.
+template <typename F>
+int no_throw(const char* who, F f) {
+    try {
+        return f();
+    } catch (const std::exception& e) {
+        set_error("%s: %s", who, e.what());
+        return PB_ERR_HOST;
+    }
+}
 
 // ---- optional in-stream timing of the kernel families and a launch counter -----------------
 

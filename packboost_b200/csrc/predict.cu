@@ -1035,10 +1035,11 @@ static bool tree_depths(const int32_t* feature, const int32_t* threshold, const 
     return true;
 }
 
-extern "C" int pb_forest_shape(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
-                               const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
-                               int64_t* slot_nodes, int64_t* depth_out) {
+static int forest_shape(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                        const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                        int64_t* slot_nodes, int64_t* depth_out) {
     PB_REQUIRE(feature && threshold && left && right && value && is_leaf && offsets && slot_nodes && depth_out, "null buffer");
+    PB_REQUIRE(n_trees >= 0 && n_trees < (1ll << 31), "n_trees out of range");
     *slot_nodes = 0;
     int32_t deepest = 0;
     bool adjacent = true;
@@ -1063,10 +1064,11 @@ extern "C" int pb_forest_shape(const int32_t* feature, const int32_t* threshold,
     return PB_OK;
 }
 
-extern "C" int pb_forest_words(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
-                               const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
-                               int64_t slot_nodes, int64_t depth, uint32_t* out) {
+static int forest_words(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                        const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                        int64_t slot_nodes, int64_t depth, uint32_t* out) {
     PB_REQUIRE(feature && threshold && left && right && value && is_leaf && offsets && out, "null buffer");
+    PB_REQUIRE(n_trees >= 0 && n_trees < (1ll << 31) && slot_nodes >= 0, "n_trees or slot_nodes out of range");
     std::vector<int32_t> at;
     memset(out, 0, (size_t)(n_trees * slot_nodes) * 4);
     for (int64_t t = 0; t < n_trees; ++t) {
@@ -1094,4 +1096,20 @@ extern "C" int pb_forest_words(const int32_t* feature, const int32_t* threshold,
         }
     }
     return PB_OK;
+}
+
+extern "C" int pb_forest_shape(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                               const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                               int64_t* slot_nodes, int64_t* depth) {
+    return no_throw("pb_forest_shape", [&] {
+        return forest_shape(feature, threshold, left, right, value, is_leaf, offsets, n_trees, slot_nodes, depth);
+    });
+}
+
+extern "C" int pb_forest_words(const int32_t* feature, const int32_t* threshold, const int32_t* left, const int32_t* right,
+                               const float* value, const uint8_t* is_leaf, const int32_t* offsets, int64_t n_trees,
+                               int64_t slot_nodes, int64_t depth, uint32_t* out) {
+    return no_throw("pb_forest_words", [&] {
+        return forest_words(feature, threshold, left, right, value, is_leaf, offsets, n_trees, slot_nodes, depth, out);
+    });
 }

@@ -8,6 +8,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -53,13 +54,20 @@ struct UploadJob {
     }
 };
 
-// Up to seven workers that sleep between jobs.  One job at a time: a second caller copies alone.
+// Up to seven workers that sleep between jobs, fewer (or none) when the host gives no more threads.
+// One job at a time: a second caller copies alone.
 class Pool {
    public:
     Pool() {
         int n = (int)std::thread::hardware_concurrency() / 2 - 1;
         n = n < 0 ? 0 : (n > 7 ? 7 : n);
-        for (int i = 0; i < n; ++i) std::thread([this] { loop(); }).detach();
+        for (int i = 0; i < n; ++i) {
+            try {
+                std::thread([this] { loop(); }).detach();
+            } catch (const std::system_error&) {
+                break;
+            }
+        }
     }
     bool offer(UploadJob* job) {
         std::lock_guard<std::mutex> lk(mu_);
@@ -116,7 +124,7 @@ extern "C" int64_t pb_upload_ring_bytes(int64_t bytes) {
     return (all < kPieces ? all : kPieces) * kPieceBytes;
 }
 
-extern "C" int pb_upload(void* dst, const void* src, int64_t bytes, void* ring, int64_t ring_bytes, void* stream_) {
+static int upload(void* dst, const void* src, int64_t bytes, void* ring, int64_t ring_bytes, void* stream_) {
     PB_REQUIRE(bytes >= 0 && (bytes == 0 || (dst && src && ring)), "null buffer");
     PB_REQUIRE(((uintptr_t)ring % 16) == 0, "ring must be 16-byte aligned");
     PB_REQUIRE(ring_bytes >= pb_upload_ring_bytes(bytes), "ring of %lld bytes is too small", (long long)ring_bytes);
@@ -129,6 +137,7 @@ extern "C" int pb_upload(void* dst, const void* src, int64_t bytes, void* ring, 
     }
     const int n = (int)((bytes + kPieceBytes - 1) / kPieceBytes);
     UploadJob job(n);
+    Pool& helpers = pool();
     job.src = static_cast<const char*>(src);
     job.ring = static_cast<char*>(ring);
     job.bytes = bytes;
@@ -138,7 +147,7 @@ extern "C" int pb_upload(void* dst, const void* src, int64_t bytes, void* ring, 
     const bool reuse = n > kPieces;             // only then a place of the ring is written twice
     for (int i = 0; reuse && i < kPieces && err == cudaSuccess; ++i)
         err = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-    const bool shared = err == cudaSuccess && pool().offer(&job);
+    const bool shared = err == cudaSuccess && helpers.offer(&job);
     int freed = 0;
     for (int p = 0; p < n && err == cudaSuccess; ++p) {
         while (!job.done[p].load(std::memory_order_acquire)) {
@@ -163,9 +172,13 @@ extern "C" int pb_upload(void* dst, const void* src, int64_t bytes, void* ring, 
         if (err == cudaSuccess && reuse) err = cudaEventRecord(ev[p % kPieces], stream);
     }
     if (err != cudaSuccess) job.stop.store(1);
-    if (shared) pool().retract(&job);
+    if (shared) helpers.retract(&job);
     for (int i = 0; i < kPieces; ++i)
         if (ev[i]) cudaEventDestroy(ev[i]);
     if (err != cudaSuccess) return fail_cuda(err, "pb_upload");
     return PB_OK;
+}
+
+extern "C" int pb_upload(void* dst, const void* src, int64_t bytes, void* ring, int64_t ring_bytes, void* stream) {
+    return no_throw("pb_upload", [&] { return upload(dst, src, bytes, ring, ring_bytes, stream); });
 }

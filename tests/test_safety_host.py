@@ -204,6 +204,46 @@ int main() {
     assert subprocess.run([str(tmp_path / "copy")]).returncode == 0
 
 
+_NO_MEMORY = """
+import ctypes as C, resource, sys
+import numpy as np
+lib = C.CDLL({lib!r})
+n = 20_000_000
+one = np.ones(n, np.uint8)
+ints = np.zeros(n, np.int32)
+value = np.zeros(n, np.float32)
+offs = np.array([0, n], np.int32)
+src, dst, ring = np.ones(2 << 20, np.uint8), np.zeros(2 << 20, np.uint8), np.zeros((2 << 20) + 16, np.uint8)
+slot, depth, out = C.c_int64(), C.c_int64(), np.zeros(4, np.uint32)
+lib.pb_last_error.restype = C.c_char_p
+i64, p = C.c_int64, lambda a: C.c_void_p(a.ctypes.data)
+tree = [p(ints), p(ints), p(ints), p(ints), p(value), p(one), p(offs)]
+pages = int(open("/proc/self/statm").read().split()[0])
+resource.setrlimit(resource.RLIMIT_AS, (pages * 4096 + (4 << 20),) * 2)
+if {what!r} == "shape":
+    rc = lib.pb_forest_shape(*tree, i64(1), C.byref(slot), C.byref(depth))
+elif {what!r} == "words":
+    rc = lib.pb_forest_words(*tree, i64(1), i64(4), i64(0), p(out))
+elif {what!r} == "negative":
+    rc = lib.pb_forest_shape(*tree, i64(-1), C.byref(slot), C.byref(depth))
+else:   # no thread can be had (and without a device the copy itself is refused)
+    at = ring.ctypes.data + 15 & ~15
+    rc = lib.pb_upload(p(dst), p(src), i64(2 << 20), C.c_void_p(at), i64(2 << 20), None)
+print("rc", rc, lib.pb_last_error().decode())
+"""
+
+
+@pytest.mark.parametrize("what,rc", [("shape", (-5,)), ("words", (-5,)), ("negative", (-1,)), ("threads", (0, -2, -5))])
+def test_a_host_out_of_memory_or_threads_is_an_error_code(lib, what, rc):
+    """No C++ exception leaves an entry point (it would end the process): address space runs out in a child
+    process."""
+    import subprocess
+    import sys
+    from packboost_b200 import backends as B
+    res = subprocess.run([sys.executable, "-c", _NO_MEMORY.format(lib=B._LIB_PATH, what=what)], capture_output=True, text=True)
+    assert res.returncode == 0 and int(res.stdout.split()[1]) in rc, (res.returncode, res.stdout, res.stderr[-2000:])
+
+
 def test_comm_entries_validate_their_arguments_without_a_gpu(lib):
     """The NCCL-backed exchange entries refuse bad arguments before touching NCCL or a device."""
     from packboost_b200 import backends as B
