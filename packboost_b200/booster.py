@@ -63,9 +63,13 @@ class TreeNode:
     is_leaf: bool = True
 
 
+_TREE_LOCK = threading.Lock()   # held while a tree's list or arrays are made from the other form
+
+
 class Tree:
-    """A tree as node arrays, a list of ``TreeNode`` or both: a fit leaves arrays, the list is built when
-    somebody asks for it (and from then on is what counts, since nodes can be written to)."""
+    """A tree as node arrays, a list of ``TreeNode`` or both: a fit leaves arrays, the list is made when
+    somebody asks for it (and from then on is what counts, since nodes can be written to).  Any number of
+    threads may read a tree."""
 
     __slots__ = ("_nodes", "_arrays", "_values")
 
@@ -73,16 +77,6 @@ class Tree:
         self._nodes = nodes
         self._arrays = arrays
         self._values = values          # leaf values in float64 (arrays hold them as float32)
-
-    @property
-    def nodes(self) -> List[TreeNode]:
-        if self._nodes is None:
-            a = self._arrays
-            self._nodes = [TreeNode(*row) for row in
-                           zip(a["feature"].tolist(), a["threshold"].tolist(), a["left"].tolist(), a["right"].tolist(),
-                               self._values.tolist(), (a["is_leaf"] != 0).tolist())]
-            self._arrays = self._values = None
-        return self._nodes
 
     def __eq__(self, other) -> bool:
         return isinstance(other, Tree) and self.nodes == other.nodes
@@ -93,16 +87,21 @@ class Tree:
         return f"Tree(nodes={self.nodes!r})"
 
     def arrays(self) -> dict[str, np.ndarray]:
-        if self._arrays is None:
-            self._arrays = {
-                "feature": np.asarray([n.feature for n in self.nodes], dtype=np.int32),
-                "threshold": np.asarray([n.threshold for n in self.nodes], dtype=np.int32),
-                "left": np.asarray([n.left for n in self.nodes], dtype=np.int32),
-                "right": np.asarray([n.right for n in self.nodes], dtype=np.int32),
-                "value": np.asarray([n.value for n in self.nodes], dtype=np.float32),
-                "is_leaf": np.asarray([n.is_leaf for n in self.nodes], dtype=np.uint8),
-            }
-        return self._arrays
+        out = self._arrays             # (read once: making the list takes them away)
+        if out is not None:
+            return out
+        with _TREE_LOCK:
+            if self._arrays is None:
+                nodes = self._nodes
+                self._arrays = {
+                    "feature": np.asarray([n.feature for n in nodes], dtype=np.int32),
+                    "threshold": np.asarray([n.threshold for n in nodes], dtype=np.int32),
+                    "left": np.asarray([n.left for n in nodes], dtype=np.int32),
+                    "right": np.asarray([n.right for n in nodes], dtype=np.int32),
+                    "value": np.asarray([n.value for n in nodes], dtype=np.float32),
+                    "is_leaf": np.asarray([n.is_leaf for n in nodes], dtype=np.uint8),
+                }
+            return self._arrays
 
     def predict_bins(self, bins: torch.Tensor) -> torch.Tensor:
         """Leaf value per row for integer-binned features ``[N, F]``
@@ -117,6 +116,21 @@ class Tree:
         t = {k: torch.from_numpy(v).to(dev) for k, v in a.items()}
         out = B.predict_bins_cuda(fm, t["feature"], t["threshold"], t["left"], t["right"], t["value"], t["is_leaf"])
         return out.to(bins.device)
+
+
+def _tree_nodes(tree: Tree) -> List[TreeNode]:
+    if tree._nodes is None:
+        with _TREE_LOCK:
+            if tree._nodes is None:
+                a = tree._arrays
+                tree._nodes = [TreeNode(*row) for row in
+                               zip(a["feature"].tolist(), a["threshold"].tolist(), a["left"].tolist(), a["right"].tolist(),
+                                   tree._values.tolist(), (a["is_leaf"] != 0).tolist())]
+                tree._arrays = tree._values = None
+    return tree._nodes
+
+
+Tree.nodes = property(_tree_nodes)
 
 
 class TreeBuilder:

@@ -328,3 +328,67 @@ def test_row_split_upload_reassembles_the_single_gpu_layout():
             mine = torch.empty((blk, world * seg), dtype=torch.uint8)
             mine.view(blk, world, seg).copy_(recv.permute(1, 0, 2))
             assert torch.equal(mine, full[dst * blk:(dst + 1) * blk])
+
+
+def _array_tree(n=31):
+    rng = np.random.default_rng(n)
+    internal = np.arange(n) < n // 2
+    arrays = {"feature": np.where(internal, rng.integers(0, 9, n), -1).astype(np.int32),
+              "threshold": np.where(internal, rng.integers(0, 4, n), 0).astype(np.int32),
+              "left": np.where(internal, 2 * np.arange(n) + 1, -1).astype(np.int32),
+              "right": np.where(internal, 2 * np.arange(n) + 2, -1).astype(np.int32),
+              "value": rng.normal(size=n).astype(np.float32), "is_leaf": (~internal).astype(np.uint8)}
+    return arrays, arrays["value"].astype(np.float64)
+
+
+def test_a_tree_is_read_by_several_threads(monkeypatch):
+    """Whoever asks first, every thread gets the one node list and the arrays: readers that start while
+    the list is being made, and readers of the arrays at the moment they go."""
+    import sys
+    import threading
+    from packboost_b200 import booster as bm
+    arrays, values = _array_tree()
+    tree = bm.Tree(arrays=dict(arrays), values=values)
+    others, seen = [], []
+    node = bm.TreeNode
+
+    def slow_node(*row):
+        if not others:                       # the first node of the first list: others come in now
+            for _ in range(2):
+                others.append(threading.Thread(target=lambda: seen.append((tree.nodes, tree.arrays()))))
+            for t in others:
+                t.start()
+                t.join(0.05)                 # (they may have to wait for this list)
+        return node(*row)
+
+    monkeypatch.setattr(bm, "TreeNode", slow_node)
+    first = tree.nodes
+    for t in others:
+        t.join()
+    assert len(seen) == 2 and all(nodes is first for nodes, _ in seen) and tree.nodes is first
+    monkeypatch.undo()
+    errors = []
+
+    def read(t, what, start):
+        start.wait()
+        try:
+            got = t.arrays() if what == "arrays" else t.nodes
+            assert got is not None and len(got) > 0
+        except Exception as exc:             # noqa: BLE001
+            errors.append(exc)
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        for _ in range(300):
+            t = bm.Tree(arrays=dict(arrays), values=values)
+            start = threading.Barrier(4)
+            workers = [threading.Thread(target=read, args=(t, what, start)) for what in ("nodes", "arrays", "nodes", "arrays")]
+            for w in workers:
+                w.start()
+            for w in workers:
+                w.join()
+    finally:
+        sys.setswitchinterval(interval)
+    assert not errors, errors[:3]
+
