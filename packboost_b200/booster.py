@@ -66,14 +66,18 @@ class TreeNode:
 _TREE_LOCK = threading.Lock()   # held while a tree's list or arrays are made from the other form
 
 
+@dataclass(init=False, repr=False, eq=False)
 class Tree:
     """A tree as node arrays, a list of ``TreeNode`` or both: a fit leaves arrays, the list is made when
     somebody asks for it (and from then on is what counts, since nodes can be written to).  Any number of
     threads may read a tree."""
 
     __slots__ = ("_nodes", "_arrays", "_values")
+    nodes: List[TreeNode]
 
     def __init__(self, nodes: List[TreeNode] | None = None, *, arrays: dict | None = None, values: np.ndarray | None = None):
+        if nodes is None and (arrays is None or values is None):
+            raise TypeError("a tree needs its nodes, or arrays and values")
         self._nodes = nodes
         self._arrays = arrays
         self._values = values          # leaf values in float64 (arrays hold them as float32)
@@ -130,7 +134,14 @@ def _tree_nodes(tree: Tree) -> List[TreeNode]:
     return tree._nodes
 
 
-Tree.nodes = property(_tree_nodes)
+def _set_tree_nodes(tree: Tree, nodes: List[TreeNode]) -> None:
+    with _TREE_LOCK:
+        tree._nodes = nodes
+        tree._arrays = tree._values = None
+
+
+# (set after the dataclass is made, which would take a property in the class body for the field's default)
+Tree.nodes = property(_tree_nodes, _set_tree_nodes)
 
 
 class TreeBuilder:

@@ -392,3 +392,21 @@ def test_a_tree_is_read_by_several_threads(monkeypatch):
         sys.setswitchinterval(interval)
     assert not errors, errors[:3]
 
+
+def test_tree_keeps_the_dataclass_protocol_and_takes_nodes():
+    import copy
+    import dataclasses
+    import pickle
+    from packboost_b200.booster import Tree, TreeNode
+    arrays, values = _array_tree(7)
+    tree = Tree(arrays=dict(arrays), values=values)
+    assert [f.name for f in dataclasses.fields(tree)] == ["nodes"]
+    assert dataclasses.asdict(tree)["nodes"][0]["feature"] == arrays["feature"][0]
+    assert dataclasses.replace(tree, nodes=[TreeNode(value=2.0)]).nodes == [TreeNode(value=2.0)]
+    for again in (pickle.loads(pickle.dumps(tree)), copy.deepcopy(tree)):
+        assert again == tree and again.nodes is not tree.nodes
+    tree.arrays()
+    tree.nodes = [TreeNode(value=3.0)]
+    assert tree.arrays()["value"].tolist() == [3.0] and len(tree.nodes) == 1
+    with pytest.raises(TypeError):
+        Tree()
