@@ -1290,8 +1290,7 @@ class PackBoost:
         if "offsets" in forest:
             return
         cat, offs = forest["host"]
-        forest.update({k: torch.from_numpy(v).to(self._device) for k, v in cat.items()})
-        forest["offsets"] = torch.from_numpy(offs).to(self._device)
+        made = {k: torch.from_numpy(v).to(self._device) for k, v in cat.items()}
         # packed 8-byte nodes when the trees allow it (right child == left child + 1, small ids)
         internal = cat["is_leaf"] == 0
         ok = (bool(np.all(cat["right"][internal] == cat["left"][internal] + 1))
@@ -1302,14 +1301,18 @@ class PackBoost:
                           1 << 31).astype(np.uint32)
             w1 = np.where(internal, cat["left"].astype(np.int64) & 0xFFFFFFFF,
                           cat["value"].astype(np.float32).view(np.uint32).astype(np.int64)).astype(np.uint32)
-            forest["packed"] = torch.from_numpy(np.stack([w0, w1], axis=1).view(np.int32).copy()).to(self._device)
-            forest["max_tree_nodes"] = int(np.diff(offs).max()) if forest["n_trees"] else 1
+            made["max_tree_nodes"] = int(np.diff(offs).max()) if forest["n_trees"] else 1
+            made["packed"] = torch.from_numpy(np.stack([w0, w1], axis=1).view(np.int32).copy()).to(self._device)
+        made["offsets"] = torch.from_numpy(offs).to(self._device)
+        forest.update(made)   # ("offsets" last: who finds it finds the rest)
 
     def _current_forest(self) -> dict:
-        if self._forest_cache is None or self._forest_cache["n_distinct"] != len(self._distinct):
-            self._forest_cache = self._pack_forest(self._distinct)
-            self._forest_cache["n_distinct"] = len(self._distinct)
-        return self._forest_cache
+        forest, n = self._forest_cache, len(self._distinct)
+        if forest is None or forest["n_distinct"] != n:
+            forest = self._pack_forest(self._distinct)
+            forest["n_distinct"] = n
+            self._forest_cache = forest   # (complete: another thread may take it from here on)
+        return forest
 
     def _predict_table(self, X) -> np.ndarray | None:
         """The whole prediction in one library call, for small trees and a table that needs no conversion;

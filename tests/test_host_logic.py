@@ -410,3 +410,30 @@ def test_tree_keeps_the_dataclass_protocol_and_takes_nodes():
     assert tree.arrays()["value"].tolist() == [3.0] and len(tree.nodes) == 1
     with pytest.raises(TypeError):
         Tree()
+
+
+def test_a_forest_is_shared_only_when_it_is_complete(monkeypatch):
+    """A second first call of ``predict`` comes in at every step of laying the forest out."""
+    import threading
+    trainer = _ScriptedTrainer(2, 3, [])
+    b = _scripted_booster(monkeypatch, trainer, 1, 5)
+    b._distinct = [("tree", 1)]
+    errors = []
+
+    def other():
+        try:
+            assert b._current_forest()["n_distinct"] == 1
+        except Exception as exc:             # noqa: BLE001
+            errors.append(exc)
+
+    class Layout(dict):
+        def __setitem__(self, key, value):
+            if threading.current_thread() is threading.main_thread():
+                t = threading.Thread(target=other)
+                t.start()
+                t.join()
+            super().__setitem__(key, value)
+
+    monkeypatch.setattr(b, "_pack_forest", lambda distinct: Layout())
+    assert b._current_forest()["n_distinct"] == 1
+    assert not errors, errors
