@@ -1282,6 +1282,8 @@ class PackBoost:
             copies = _FOREST_COPIES if len(arrs) > 8 else 1
             out["slots"] = torch.from_numpy(slots[0].view(np.int32)).to(self._device).repeat(copies, 1)
             out["copies"], out["slot"], out["depth"] = copies, slots[0].shape[1], slots[1]
+            if copies > 1:   # (the copies are made on this stream, the next call may be on another)
+                torch.cuda.current_stream().synchronize()
         out["host"] = (cat, offs)   # for the forms below, built when a table asks for them
         return out
 

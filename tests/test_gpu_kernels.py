@@ -370,6 +370,45 @@ def test_small_tree_predictor_equals_the_general_one(rows, features, bins, depth
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
 
 
+def test_a_forest_laid_out_on_one_stream_is_there_for_another(monkeypatch):
+    """The first call's stream is busy when the copies are made; a second stream reads them right after."""
+    from packboost_b200 import PackBoost, PackBoostConfig
+    from packboost_b200.booster import TreeBuilder
+
+    def install(model, sign):
+        forest = []
+        for t in range(12):
+            tb = TreeBuilder()
+            tb.split(0, t, 1)
+            tb.nodes[1].value, tb.nodes[2].value = sign * (1.0 + t), -sign * (1.0 + t)
+            forest.append(tb.build())
+        model.set_forest(forest, 1.0)
+
+    plain = torch.Tensor.repeat
+
+    def late(self, *sizes):
+        torch.cuda._sleep(200_000_000)           # (about a tenth of a second)
+        return plain(self, *sizes)
+
+    model = PackBoost(PackBoostConfig(max_bins=5, prebinned=True))
+    install(model, 1.0)
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(first):
+        shape = model._current_forest()["slots"].shape
+    with torch.cuda.stream(second):              # (everything the second stream needs is there before)
+        got = torch.zeros(shape, dtype=torch.int32, device=_dev())
+        got.copy_(torch.ones_like(got))
+    torch.cuda.synchronize()
+    install(model, -1.0)
+    with torch.cuda.stream(first), monkeypatch.context() as m:
+        m.setattr(torch.Tensor, "repeat", late)
+        laid = model._current_forest()
+    with torch.cuda.stream(second):
+        got.copy_(laid["slots"])
+    torch.cuda.synchronize()
+    assert laid["copies"] > 1 and torch.equal(got, laid["slots"])
+
+
 @pytest.mark.parametrize("n,f,eras,bins,depth,extra", [
     (700, 32, 1, 17, 3, {}), (5_003, 33, 7, 64, 6, {}), (9_000, 40, 40, 128, 5, dict(era_alpha=4.0)),
     (20_001, 32, 2, 33, 4, {}), (6_000, 35, 9, 100, 5, dict(direction_weight=0.3)),
