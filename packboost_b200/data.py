@@ -57,6 +57,8 @@ def detect_prebinned_tensor(X: torch.Tensor, max_bins: int) -> bool:
         return False
     if X.numel() == 0:
         return max_bins > 0
+    if X.dtype in (torch.uint16, torch.uint32, torch.uint64):   # (torch has no minimum of these)
+        X = X.to(torch.int32 if X.dtype == torch.uint16 else torch.int64)
     low, top = (int(v) for v in torch.stack(torch.aminmax(X)).tolist())
     return low >= 0 and top < max_bins and top <= 127
 

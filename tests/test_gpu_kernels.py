@@ -370,6 +370,18 @@ def test_small_tree_predictor_equals_the_general_one(rows, features, bins, depth
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
 
 
+@pytest.mark.parametrize("dtype", [torch.uint16, torch.int32, torch.int64])
+def test_fit_takes_codes_of_any_integer_type_on_the_device(dtype):
+    from packboost_b200 import PackBoost, PackBoostConfig
+    rng = np.random.default_rng(3)
+    X = rng.integers(0, 5, size=(900, 12), dtype=np.uint8)
+    y = (X[:, 0] - X[:, 3] + rng.normal(size=900)).astype(np.float32)
+    cfg = PackBoostConfig(pack_size=2, max_depth=3, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=5, max_bins=5, random_state=1)
+    want = PackBoost(cfg).fit(X, y, None, num_rounds=2).train_predictions()
+    got = PackBoost(cfg).fit(torch.from_numpy(X).to(_dev()).to(dtype), y, None, num_rounds=2).train_predictions()
+    np.testing.assert_array_equal(got, want)
+
+
 def test_a_forest_laid_out_on_one_stream_is_there_for_another(monkeypatch):
     """The first call's stream is busy when the copies are made; a second stream reads them right after."""
     from packboost_b200 import PackBoost, PackBoostConfig

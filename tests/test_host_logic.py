@@ -437,3 +437,14 @@ def test_a_forest_is_shared_only_when_it_is_complete(monkeypatch):
     monkeypatch.setattr(b, "_pack_forest", lambda distinct: Layout())
     assert b._current_forest()["n_distinct"] == 1
     assert not errors, errors
+
+
+@pytest.mark.parametrize("dtype", ["uint8", "int8", "uint16", "int16", "uint32", "int32", "uint64", "int64", "float32"])
+def test_codes_are_told_from_values_in_every_type(dtype):
+    """Tensors as arrays: integers in [0, max_bins), and below 128, are codes."""
+    from packboost_b200.data import detect_prebinned, detect_prebinned_tensor
+    info = np.iinfo(dtype) if dtype != "float32" else np.iinfo(np.int8)
+    for values in ([0, 1, 4], [0, 5], [127, 3], [info.max, 0], [max(info.min, -1), 2], []):
+        a = np.asarray(values).astype(dtype)
+        for max_bins in (5, 128, 200):
+            assert detect_prebinned_tensor(torch.from_numpy(a), max_bins) == detect_prebinned(a, max_bins), (values, max_bins)
