@@ -1181,7 +1181,7 @@ class PackBoost:
                 raise ValueError(f"eval set '{name}' requires y values for correlation logging")
             Xe = np.asarray(X_eval)
             rows, top = self._pack_rows(Xe)
-            self._check_top(top)
+            self._check_top(top, Xe)
             era_e = np.zeros(Xe.shape[0], dtype=np.int16) if era_eval is None else np.asarray(era_eval, dtype=np.int16)
             if era_e.shape[0] != Xe.shape[0]:
                 raise ValueError(f"eval set '{name}' era ids must align with X rows")
@@ -1250,7 +1250,6 @@ class PackBoost:
             return pack_row_major(X, edges, max_bins, uploads=uploads), None
         top = None
         if X.dtype in (torch.uint8, torch.int8, np.dtype(np.uint8), np.dtype(np.int8)):
-            # (negative int8 values are bytes of 128 and more)
             X = X.view(torch.uint8 if isinstance(X, torch.Tensor) else np.uint8)
             top = torch.zeros(1, dtype=torch.int32, device=self._device)
         elif isinstance(X, torch.Tensor) and X.is_cuda:
@@ -1262,8 +1261,14 @@ class PackBoost:
             X = X.astype(np.uint8)
         return pack_row_major(X, None, max_bins, top=top, uploads=uploads), top
 
-    def _check_top(self, top: torch.Tensor | None) -> None:
-        if top is not None and int(top.item()) >= min(int(self.config.max_bins), 128):
+    def _code_limit(self, X) -> int:
+        """Codes of ``X`` lie below this: ``max_bins``, and 128 except for bytes that are on the device
+        (negative int8 values are bytes of 128 and more)."""
+        wide = isinstance(X, torch.Tensor) and X.is_cuda and X.dtype == torch.uint8
+        return int(self.config.max_bins) if wide else min(int(self.config.max_bins), 128)
+
+    def _check_top(self, top: torch.Tensor | None, X) -> None:
+        if top is not None and int(top.item()) >= self._code_limit(X):
             raise ValueError(_NOT_BINNED)
 
     def _pack_forest(self, distinct: Sequence[tuple[Tree, int]]) -> dict[str, torch.Tensor]:
@@ -1375,7 +1380,7 @@ class PackBoost:
         finally:
             if small:
                 self._small_lock.release()
-        if codes and top.value >= min(int(self.config.max_bins), 128):
+        if codes and top.value >= self._code_limit(X):
             raise ValueError(_NOT_BINNED)
         return out
 
@@ -1424,7 +1429,7 @@ class PackBoost:
         uploads = Uploads()
         rows, top = self._pack_rows(X, uploads)
         if not self._trees:
-            self._check_top(top)
+            self._check_top(top, X)
             torch.cuda.current_stream().synchronize()
             return np.zeros(rows.n_rows, dtype=np.float32)
         if self._tree_weight is None:
@@ -1432,7 +1437,7 @@ class PackBoost:
         if self._trained_pack_size is not None and int(self.config.pack_size) != self._trained_pack_size:
             raise RuntimeError("pack_size differs from training; keep it constant.")
         out = self._predict_packed(rows, self._current_forest()).cpu().numpy()
-        self._check_top(top)
+        self._check_top(top, X)
         return out
 
     def predict_packwise(self, X: np.ndarray, block_size_trees: int = 8) -> np.ndarray:

@@ -382,6 +382,38 @@ def test_fit_takes_codes_of_any_integer_type_on_the_device(dtype):
     np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("trees", [1, 40])
+def test_prediction_takes_device_bytes_up_to_max_bins(trees):
+    """More than 128 bins: bytes on the device count up to max_bins, host arrays and int8 up to 128."""
+    from packboost_b200 import PackBoost, PackBoostConfig
+    from packboost_b200.booster import TreeBuilder
+    rng = np.random.default_rng(trees)
+    X = rng.integers(0, 200, size=(300, 9), dtype=np.uint8)
+    X[0, 0] = 199
+    forest = []
+    for _ in range(trees):
+        tb = TreeBuilder()
+        for node in tb.split(0, int(rng.integers(9)), int(rng.integers(199))):
+            tb.split(node, int(rng.integers(9)), int(rng.integers(199)))
+        for node in tb.nodes:
+            node.value = float(np.float32(rng.normal()))
+        forest.append(tb.build())
+    model = PackBoost(PackBoostConfig(max_bins=200, prebinned=True)).set_forest(forest, 1.0)
+    on_device = torch.from_numpy(X).to(_dev())
+    got = model.predict(on_device)
+    want = torch.zeros(300, device=_dev())
+    for tree in forest:
+        want += tree.predict_bins(on_device)
+    np.testing.assert_array_equal(got, want.cpu().numpy())
+    np.testing.assert_array_equal(model.predict(on_device[:, :9].t().contiguous().t()), got)   # (the general way)
+    for refused in (X, on_device.view(torch.int8), X.view(np.int8)):
+        with pytest.raises(ValueError, match="prebinned"):
+            model.predict(refused)
+    on_device[5, 5] = 200
+    with pytest.raises(ValueError, match="prebinned"):
+        model.predict(on_device)
+
+
 def test_a_forest_laid_out_on_one_stream_is_there_for_another(monkeypatch):
     """The first call's stream is busy when the copies are made; a second stream reads them right after."""
     from packboost_b200 import PackBoost, PackBoostConfig
