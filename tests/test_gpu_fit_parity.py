@@ -479,3 +479,23 @@ def test_fit_is_bit_identical_in_forced_histogram_shapes(shape):
                          capture_output=True, text=True, timeout=1200)
     assert res.returncode == 0, res.stdout[-3000:] + res.stderr[-2000:]
     assert "hist_lane_kernel<%s>" % shape.replace(" ", ",") in res.stderr + res.stdout, "forced shape never launched"
+
+
+def test_a_fit_on_a_nearly_full_device_takes_less_workspace_and_gives_the_same(monkeypatch):
+    """8 MB free: the workspace shrinks to what that allows (features go through it in blocks) and the table is
+    streamed; trees and predictions do not change."""
+    from packboost_b200 import PackBoost, PackBoostConfig, data
+    rng = np.random.default_rng(8)
+    X = rng.normal(size=(20_000, 64)).astype(np.float32)
+    y = (X[:, 0] + X[:, 1] * X[:, 2] + rng.normal(size=20_000)).astype(np.float32)
+    era = np.sort(rng.integers(0, 20, 20_000)).astype(np.int16)
+    cfg = PackBoostConfig(pack_size=2, max_depth=6, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=5, max_bins=128, random_state=1)
+    want = PackBoost(cfg).fit(X, y, era, num_rounds=2)
+    total = torch.cuda.get_device_properties(0).total_memory
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (8 << 20, total))
+    assert not data.fits_on_device(X.nbytes)
+    got = PackBoost(cfg).fit(X, y, era, num_rounds=2)
+    assert got._trainer.workspace.numel() <= int(0.6 * (8 << 20)) < want._trainer.workspace.numel()
+    np.testing.assert_array_equal(got.train_predictions(), want.train_predictions())
+    for a, b in zip(want.split_records().values(), got.split_records().values()):
+        np.testing.assert_array_equal(a, b)

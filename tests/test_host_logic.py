@@ -448,3 +448,13 @@ def test_codes_are_told_from_values_in_every_type(dtype):
         a = np.asarray(values).astype(dtype)
         for max_bins in (5, 128, 200):
             assert detect_prebinned_tensor(torch.from_numpy(a), max_bins) == detect_prebinned(a, max_bins), (values, max_bins)
+
+
+def test_a_table_is_brought_over_whole_only_into_free_memory(monkeypatch):
+    """Small tables too: the device may be nearly full."""
+    from packboost_b200 import data
+    monkeypatch.setattr(data, "_device", lambda: torch.device("cuda", 0))
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda dev: type("P", (), {"total_memory": 180 << 30})())
+    for free, nbytes, fits in ((3 << 20, 1 << 20, True), (3 << 20, (1 << 20) + 1, False), (0, 1, False), (90 << 30, 30 << 30, True)):
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev, free=free: (free, 180 << 30))
+        assert data.fits_on_device(nbytes) is fits
