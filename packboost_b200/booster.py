@@ -736,7 +736,7 @@ class PackBoost:
         self._eval_states: list = []
         self._last_n_ctx: list[int] = []
         self._round_depths: list[int] = []   # depths with live nodes (= feature draws consumed) per round
-        self._split_log: list[tuple] = []    # (live nodes per depth, winners) per round
+        self._split_log: list[np.ndarray] = []   # the splits of each round
         self._pending_log = None
         self._predrawn = None
         self._inflight = None  # (log ticket, generator state at the round's start) of the enqueued round
@@ -987,9 +987,12 @@ class PackBoost:
         for d in range(used):
             self._depth_logs.append(self._depth_log(d, n_ctx[d], k, phase_ms[d] if d < len(phase_ms) else None))
         self._flush_pending_tree()
-        log = (head.copy(), winners[: (1 << D) - 1].copy())
-        self._pending_log = log
-        self._split_log.append((n_ctx[:used], log[1]))
+        self._pending_log = (head.copy(), winners[: (1 << D) - 1].copy())
+        # of the log only the splits stay: it has room for every node a tree might have (330 KB a round at
+        # depth 12).  Raw bytes, since structured arrays are concatenated field by field.
+        raw = winners.view(np.uint8).reshape(-1, _WINNER_DT.itemsize)
+        live = np.concatenate([raw[:0]] + [raw[(1 << d) - 1: (1 << d) - 1 + n_ctx[d]] for d in range(used)]).view(_WINNER_DT)[:, 0]
+        self._split_log.append(live[live["feature"] >= 0])
         return used == D
 
     def _drain(self) -> None:
@@ -1131,12 +1134,8 @@ class PackBoost:
         position): tree node, feature, threshold, DES score (the ``SplitDecision.score`` of
         ``packboost/booster.py:206-217``), rows sent left and rows of the node."""
         self._drain()
-        # (records as raw bytes: concatenating structured arrays promotes their types field by field)
-        size = _WINNER_DT.itemsize
-        parts = [w.view(np.uint8)[((1 << d) - 1) * size: ((1 << d) - 1 + n) * size]
-                 for n_ctx, w in self._split_log for d, n in enumerate(n_ctx)]
+        parts = [w.view(np.uint8) for w in self._split_log]
         rec = (np.concatenate(parts) if parts else np.zeros(0, dtype=np.uint8)).view(_WINNER_DT)
-        rec = rec[rec["feature"] >= 0]
         return {"node": rec["tree_node"].astype(np.int32), "feature": rec["feature"].astype(np.int32),
                 "threshold": rec["threshold"].astype(np.int32), "score": rec["score"].astype(np.float32),
                 "left_count": rec["left_count"].astype(np.int64),

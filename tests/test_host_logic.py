@@ -458,3 +458,30 @@ def test_a_table_is_brought_over_whole_only_into_free_memory(monkeypatch):
     for free, nbytes, fits in ((3 << 20, 1 << 20, True), (3 << 20, (1 << 20) + 1, False), (0, 1, False), (90 << 30, 30 << 30, True)):
         monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev, free=free: (free, 180 << 30))
         assert data.fits_on_device(nbytes) is fits
+
+
+def test_of_a_decision_log_only_the_splits_are_kept(monkeypatch):
+    """Rounds that end early or split some of their nodes: the records cost what the trees have, and
+    come in the order of the frontier."""
+
+    class Sparse(_ScriptedTrainer):
+        def read_log(self, ticket):
+            head, win = super().read_log(ticket)
+            used = self.used[self.round_of_ticket[ticket]]
+            if used > 1:                     # (at the last depth only the first node splits)
+                first = (1 << (used - 1)) - 1
+                win["feature"][first + 1: 2 * first + 1] = -1
+                head["n_tree_nodes"] = 2 * first + 3
+            win["score"] = np.arange(win.shape[0])
+            return head, win
+
+    used = [9, 1, 0, 4, 9]
+    trainer = Sparse(9, 3, used)
+    b = _scripted_booster(monkeypatch, trainer, 5, 12)
+    for r in range(len(used)):
+        b._boost_one_round(r, len(used))
+    rec = b.split_records()
+    want = [i for u in used for i in (range(1 << (u - 1)) if u else ())]   # positions in the log that split
+    assert rec["score"].tolist() == want and rec["node"].tolist() == want
+    assert sum(w.nbytes if w.base is None else w.base.nbytes for w in b._split_log) == len(want) * _WINNER_DT.itemsize
+    assert [t.arrays()["feature"].shape[0] for t in b.trees[::2]] == [2 * (1 << (u - 1)) + 1 if u else 1 for u in used]
