@@ -350,6 +350,8 @@ int pb_loop_submit(void* loop, const pb_train_state* st, int64_t slot, const int
                    int64_t k, void* log_host, int64_t apply_previous, int64_t use_graph, void* stream);
 int pb_loop_wait(void* loop, int64_t slot);
 int pb_loop_counts(void* loop, int64_t* graph_launches, int64_t* replays);
+/* Gives the captured round back; a later round is captured again. */
+int pb_loop_release_graph(void* loop);
 
 /* Node arrays (2^(max_depth + 1) - 1 entries at most) of the tree behind a decision log; an error when
  * the log's child numbering is not the order in which splits append children. */

@@ -119,6 +119,7 @@ _PROTOS: dict[str, tuple[Any, list[Any]]] = {
     "pb_round_log_buffer": (C.c_int, [C.POINTER(TrainState), C.POINTER(vp), C.POINTER(i64)]),
     "pb_loop_create": (vp, []),
     "pb_loop_destroy": (None, [vp]),
+    "pb_loop_release_graph": (C.c_int, [vp]),
     "pb_loop_submit": (C.c_int, [vp, vp, i64, vp, vp, i64, vp, i64, i64, vp]),
     "pb_loop_wait": (C.c_int, [vp, i64]),
     "pb_loop_counts": (C.c_int, [vp, vp, vp]),

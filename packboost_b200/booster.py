@@ -588,6 +588,9 @@ class _DeviceTrainer:
 
     def release_graph(self) -> None:
         """Drop the captured round graph (it is captured again if more rounds are enqueued)."""
+        if getattr(self, "loop", None):
+            torch.cuda.current_stream().synchronize()
+            B.check(self.lib.pb_loop_release_graph(self.loop))
         if self.graph is not None:
             torch.cuda.current_stream().synchronize()
             self.graph = None

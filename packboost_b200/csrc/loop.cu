@@ -118,6 +118,17 @@ extern "C" int pb_loop_wait(void* loop, int64_t slot) {
     return PB_OK;
 }
 
+extern "C" int pb_loop_release_graph(void* loop_) {
+    RoundLoop* loop = static_cast<RoundLoop*>(loop_);
+    PB_REQUIRE(loop, "null argument");
+    if (loop->exec) {
+        const cudaGraphExec_t exec = loop->exec;
+        loop->exec = nullptr;
+        PB_CUDA_TRY(cudaGraphExecDestroy(exec));
+    }
+    return PB_OK;
+}
+
 extern "C" int pb_loop_counts(void* loop, int64_t* graph_launches, int64_t* replays) {
     PB_REQUIRE(loop && graph_launches && replays, "null argument");
     *graph_launches = static_cast<RoundLoop*>(loop)->graph_launches;

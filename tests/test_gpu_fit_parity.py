@@ -499,3 +499,27 @@ def test_a_fit_on_a_nearly_full_device_takes_less_workspace_and_gives_the_same(m
     np.testing.assert_array_equal(got.train_predictions(), want.train_predictions())
     for a, b in zip(want.split_records().values(), got.split_records().values()):
         np.testing.assert_array_equal(a, b)
+
+
+def test_the_round_graph_is_given_back_at_the_end_of_a_fit():
+    """Rounds after it are captured again (a replay enqueues no kernel of its own) and go on as before."""
+    from packboost_b200 import PackBoost, PackBoostConfig
+    from packboost_b200 import backends as B
+    rng = np.random.default_rng(2)
+    X = rng.integers(0, 5, size=(3_000, 20), dtype=np.uint8)
+    y = (X[:, 0] - X[:, 7] + rng.normal(size=3_000)).astype(np.float32)
+    cfg = PackBoostConfig(pack_size=2, max_depth=4, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=5, max_bins=5,
+                          prebinned=True, random_state=1)
+    want = PackBoost(cfg).fit(X, y, None, num_rounds=8).train_predictions()
+    b = PackBoost(cfg).fit(X, y, None, num_rounds=4)
+    if not b._trainer.use_graph:
+        pytest.skip("the round graph is off")
+    assert b._trainer.graph_replays > 0
+    counts = []
+    for r in range(4, 8):
+        before = B.lib().pb_launch_count()
+        b._boost_one_round(r, 8)
+        counts.append(B.lib().pb_launch_count() - before)
+    assert counts[0] > 0 and counts[1] > 0 and counts[2] == 0     # launched, captured again, replayed
+    b._finish()
+    np.testing.assert_array_equal(b.train_predictions(), want)
