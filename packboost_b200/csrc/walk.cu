@@ -18,7 +18,7 @@
 //
 // Divisions: every divisor of the gains is count + lambda, so an era's divisors and their correctly
 // rounded reciprocals come from a table in shared memory, and a quotient takes two corrected products
-// instead of a general division (see divide_by).
+// instead of a general division (divide.cuh).
 //
 // Bound: the shared-memory atomics (two per row and feature, about four wavefronts each with 128 bins)
 // at the upper depths, the gains at the lower ones.
@@ -30,6 +30,7 @@
 
 #include "common.cuh"
 #include "des_math.cuh"
+#include "divide.cuh"
 
 namespace pb {
 
@@ -48,22 +49,7 @@ struct RowGroup {                        // four consecutive rows
 
 __device__ __forceinline__ float sign3(float v) { return v > 0.f ? 1.f : (v < 0.f ? -1.f : v); }
 
-// a / d, correctly rounded, from d and y = 1 / d correctly rounded.  Markstein (Computation of
-// elementary functions on the IBM RISC System/6000, 1990): when q is within one ulp of a / d and
-// r = a - d q is exact, q + r y rounds to the correctly rounded quotient.  The product a y is within two
-// ulps; the first correction brings it within one, the second is the theorem's.  Valid while no
-// intermediate leaves the normal range (division_in_range; zero numerators give zero).
-__device__ __forceinline__ float divide_by(float a, float2 dy) {
-    float q = f_mul(a, dy.y);
-    q = __fmaf_rn(__fmaf_rn(-dy.x, q, a), dy.y, q);
-    return __fmaf_rn(__fmaf_rn(-dy.x, q, a), dy.y, q);
-}
-
-// Gradient sums are multiples of inv_scale below 2^44 inv_scale, so the squares divided here are zero or
-// between inv_scale^2 / 2 and 2^88 inv_scale^2, the divisors between lambda and 2^13 + lambda.
-__device__ __forceinline__ bool division_in_range(float inv_scale, float lam) {
-    return inv_scale >= 3.5527137e-15f && inv_scale <= 32.f && lam >= 5.9604645e-8f && lam <= 16777216.f;  // 2^-48, 2^5; 2^-24, 2^24
-}
+__device__ __forceinline__ float divide_by(float a, float2 dy) { return pb::divide_by(a, dy.x, dy.y); }
 
 // Thresholds of one feature at the count-mass quantiles of its bins over all frontier rows, as the
 // reference's compiled split finder takes them (packboost/backends/cpu/frontier_cpu.cpp:35-109): targets

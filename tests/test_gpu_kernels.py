@@ -457,7 +457,9 @@ def test_a_forest_laid_out_on_one_stream_is_there_for_another(monkeypatch):
     (700, 32, 1, 17, 3, {}), (5_003, 33, 7, 64, 6, {}), (9_000, 40, 40, 128, 5, dict(era_alpha=4.0)),
     (20_001, 32, 2, 33, 4, {}), (6_000, 35, 9, 100, 5, dict(direction_weight=0.3)),
     (4_000, 32, 5, 64, 4, dict(k_cuts=7, cut_selection="even")), (8_000, 36, 11, 64, 6, dict(k_cuts=9, cut_selection="mass")),
-    (3_000, 32, 6, 70, 4, dict(y_scale=1e-12)), (3_000, 32, 6, 70, 4, dict(lambda_l2=1e-9))])
+    (3_000, 32, 6, 70, 4, dict(y_scale=1e-12)), (3_000, 32, 6, 70, 4, dict(lambda_l2=1e-9)),
+    (3_000, 32, 6, 70, 4, dict(y_scale=2.0 ** -20)), (3_000, 32, 6, 70, 4, dict(y_scale=2.0 ** 33)),   # (scale of the sums: its ends)
+    (3_000, 32, 6, 70, 4, dict(lambda_l2=2.0 ** -24)), (3_000, 32, 6, 70, 4, dict(lambda_l2=2.0 ** 24))])
 def test_era_walk_equals_the_stored_histogram_path(n, f, eras, bins, depth, extra, tmp_path):
     """Trees, scores and predictions bit for bit between the kernel that walks the eras and the two-step
     path (run in a child process, which the switch is read in): partly filled node groups, eras longer
@@ -511,7 +513,14 @@ def test_directional_term_streamed_with_the_gains_matches_the_oracle(form, n, er
     b = PackBoost(PackBoostConfig(device="cuda", **cfg)).fit(X, y, era, num_rounds=2)
     got = b.split_records()
     assert len(got["node"]) > 8
-    # the same splits re-scored one node at a time by the general scorer, first round's root
+    # every split of both rounds (below the root the parent's direction differs by node): float32 scores bit for bit
+    exact = po.fit(X, y, era, po.OracleParams(exact_sums=True, direction_form=form, **cfg), 2, record_depths=True)
+    for key in ("node", "feature", "threshold"):
+        np.testing.assert_array_equal(got[key], [r[key] for r in exact.depth_records], err_msg=key)
+    want = np.asarray([r["score"] for r in exact.depth_records], dtype=np.float32)
+    np.testing.assert_array_equal(got["score"].view(np.int32), want.view(np.int32))
+    np.testing.assert_array_equal(b.train_predictions().view(np.int32), exact.train_preds.view(np.int32))
+    # and the first root re-scored by the general scorer
     root = b._find_best_split(_root_shard(era, eras), torch.from_numpy(-y), torch.ones(n), torch.from_numpy(X.astype(np.int64)),
                               torch.arange(11))
     assert (got["feature"][0], got["threshold"][0]) == (root.feature, root.threshold)

@@ -244,6 +244,58 @@ def test_a_host_out_of_memory_or_threads_is_an_error_code(lib, what, rc):
     assert res.returncode == 0 and int(res.stdout.split()[1]) in rc, (res.returncode, res.stdout, res.stderr[-2000:])
 
 
+_DIVIDE = """#include "divide.cuh"
+#include <cstdio>
+#include <cstring>
+#include <random>
+int main() {
+    std::mt19937_64 rng(7);
+    long long n = 0, bad = 0;
+    auto check = [&](float a, float d) {
+        volatile float num = a, den = d;
+        const float y = 1.0f / den, want = num / den, got = pb::divide_by(a, d, y);
+        ++n;
+        if (memcmp(&want, &got, 4)) { if (bad++ < 5) std::printf("%a / %a: %a, not %a\\n", a, d, got, want); }
+    };
+    for (int es = -48; es <= 5; es += es < -40 || es >= -2 ? 1 : 7)
+        for (int el : {-24, -23, -20, -10, -3, -1, 0, 1, 5, 12, 13, 20, 23, 24}) {
+            const float inv = ldexpf(1.0f, es);
+            for (int i = 0; i < 30000; ++i) {
+                // lambda anywhere in its binade (the ends: the powers themselves), rows of an era, a sum of theirs
+                float lam = ldexpf(1.0f, el);
+                if (i % 3 && el < 24) lam += ldexpf((float)(rng() >> 40), el - 24);
+                if (!pb::division_in_range(inv, lam)) return 2;
+                const int rows = i % 5 == 0 ? (int)(rng() % 4) + 1 : (int)(rng() % 8192) + 1;
+                long long g = (long long)(rng() >> (20 + rng() % 43)) | 1;
+                if (i % 7 == 0) g = 1;
+                if (i % 11 == 0) g = (1ll << 44) - (long long)(rng() % 3);
+                const float s = (float)g * inv, d = (float)rows + lam, sq = s * s;
+                check(sq, d);
+                check(0.5f * sq, d);
+                check(0.0f, i % 2 ? d : lam);
+            }
+        }
+    const float tiny = ldexpf(1.0f, -48), lo = ldexpf(1.0f, -24), hi = ldexpf(1.0f, 24);
+    const bool ends = pb::division_in_range(tiny, lo) && pb::division_in_range(32.0f, hi) && !pb::division_in_range(0.5f * tiny, 1.0f) &&
+                      !pb::division_in_range(64.0f, 1.0f) && !pb::division_in_range(1.0f, 0.5f * lo) && !pb::division_in_range(1.0f, 2.0f * hi);
+    std::printf("%lld divisions, %lld differ\\n", n, bad);
+    return bad || !ends;
+}
+"""
+
+
+def test_division_by_a_known_reciprocal_is_the_division(tmp_path):
+    """Every quotient of the era walk's gains is the correctly rounded one (the host's division): squares of
+    gradient sums over row counts plus lambda, up to the ends of the range in which the table is used."""
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "packboost_b200", "csrc")
+    (tmp_path / "divide.cpp").write_text(_DIVIDE)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", csrc, str(tmp_path / "divide.cpp"),
+                    "-o", str(tmp_path / "divide")], check=True)
+    res = subprocess.run([str(tmp_path / "divide")], capture_output=True, text=True)
+    assert res.returncode == 0, (res.returncode, res.stdout)
+
+
 def test_comm_entries_validate_their_arguments_without_a_gpu(lib):
     """The NCCL-backed exchange entries refuse bad arguments before touching NCCL or a device."""
     from packboost_b200 import backends as B
