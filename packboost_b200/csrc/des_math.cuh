@@ -50,19 +50,23 @@ __device__ __forceinline__ float2 gain_of(uint32_t lc, long long lgq, uint32_t t
 }
 
 // Directional term of one threshold of one (node, era).  Form 0: 0, 1 or 2 children whose value points
-// where the node's does (the sign of a value -G / (H + lambda) is that of -G); form 1: 1 when the left
-// value is the larger one, else 0 (packboost/booster.py:1873-1880, 869-907).
+// where the node's does; form 1: 1 when the left value is the larger one, else 0
+// (packboost/booster.py:1873-1880, 869-907).
 __device__ __forceinline__ int parent_direction(long long gq) { return gq > 0 ? -1 : (gq < 0 ? 1 : 0); }
+
+// Sign of the value -g / d of a child: that of -g, unless the quotient rounds to zero (it is divided out
+// where it may lie below 2^-125: tiny gradients, a huge lambda).
+__device__ __forceinline__ int value_direction(float g, float d) {
+    if (fabsf(g) < f_mul(d, 2.3509887e-38f)) g = f_div(g, d);
+    return g > 0.f ? -1 : (g < 0.f ? 1 : 0);
+}
 
 __device__ __forceinline__ uint32_t agree_code(uint32_t lc, long long lgq, float tg, float th, float inv_scale, float lam,
                                                int form, int pa) {
-    const float lg = f_mul(__ll2float_rn(lgq), inv_scale), rg = f_sub(tg, lg);
-    if (form == 1) {
-        const float lh = (float)lc;
-        return f_div(-lg, f_add(lh, lam)) > f_div(-rg, f_add(f_sub(th, lh), lam)) ? 1u : 0u;
-    }
-    const int sl = lg > 0.f ? -1 : (lg < 0.f ? 1 : 0), sr = rg > 0.f ? -1 : (rg < 0.f ? 1 : 0);
-    return (sl == pa ? 1u : 0u) + (sr == pa ? 1u : 0u);
+    const float lg = f_mul(__ll2float_rn(lgq), inv_scale), rg = f_sub(tg, lg), lh = (float)lc;
+    const float dl = f_add(lh, lam), dr = f_add(f_sub(th, lh), lam);
+    if (form == 1) return f_div(-lg, dl) > f_div(-rg, dr) ? 1u : 0u;
+    return (value_direction(lg, dl) == pa ? 1u : 0u) + (value_direction(rg, dr) == pa ? 1u : 0u);
 }
 
 // Position of (feature, node, threshold) in the era-summed left-count / left-gradient tables.

@@ -527,6 +527,26 @@ def test_directional_term_streamed_with_the_gains_matches_the_oracle(form, n, er
     np.testing.assert_allclose(got["score"][0], root.score, rtol=2e-6)
 
 
+@pytest.mark.parametrize("bins,eras,n", [(5, 7, 3_000), (14, 2, 17_000), (40, 5, 3_000)])
+def test_directional_term_of_child_values_that_round_to_zero(bins, eras, n):
+    """A lambda so large that -G / (H + lambda) is no float32: such a child points nowhere.  Codes of 4 and
+    of 8 bits, bit for bit with the oracle."""
+    from packboost_b200 import PackBoost, PackBoostConfig
+    rng = np.random.default_rng(bins)
+    X = rng.integers(0, bins, size=(n, 11), dtype=np.uint8)
+    y = (5e-10 * (0.3 * X[:, 1] - 0.2 * X[:, 3] + rng.normal(size=n))).astype(np.float32)
+    era = np.sort(rng.integers(0, eras, n)).astype(np.int16)
+    cfg = dict(pack_size=2, max_depth=3, learning_rate=0.2, lambda_l2=1e37, lambda_dro=0.3, direction_weight=0.2,
+               min_samples_leaf=10, max_bins=bins, prebinned=True, random_state=5)
+    got = PackBoost(PackBoostConfig(device="cuda", **cfg)).fit(X, y, era, num_rounds=1).split_records()
+    exact = po.fit(X, y, era, po.OracleParams(exact_sums=True, **cfg), 1, record_depths=True)
+    for key in ("node", "feature", "threshold"):
+        np.testing.assert_array_equal(got[key], [r[key] for r in exact.depth_records], err_msg=key)
+    want = np.asarray([r["score"] for r in exact.depth_records], dtype=np.float32)
+    assert len(want) > 3 and len(set(want.tolist())) > 1
+    np.testing.assert_array_equal(got["score"].view(np.int32), want.view(np.int32))
+
+
 def _root_shard(era, eras):
     from packboost_b200.booster import NodeShard
     return NodeShard(tree_id=0, node_id=0, depth=0, era_rows=[torch.from_numpy(np.flatnonzero(era == e)) for e in range(eras)])
