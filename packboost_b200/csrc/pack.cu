@@ -502,7 +502,10 @@ extern "C" int pb_pack_rows_top(const void* x, int64_t x_is_f32, int64_t n_rows,
     const int64_t need = (code_bits == 4) ? (n_features + 1) / 2 : n_features;
     PB_REQUIRE(pitch_row >= need && pitch_row % 16 == 0, "pitch_row must cover a row and be a multiple of 16");
     PB_REQUIRE(pitch_row < (1ll << 31), "pitch_row out of range");
-    PB_REQUIRE(!x_is_f32 || (edges && n_edges >= 1 && n_edges <= 255), "float input needs 1 to 255 edges");
+    PB_REQUIRE(!x_is_f32 || (edges && n_edges >= 1), "float input needs edges");
+    // (edges ascend: those past max_bins - 1 only raise codes that are cut to max_bins - 1)
+    if (max_bins >= 2 && n_edges > max_bins - 1) n_edges = max_bins - 1;
+    PB_REQUIRE(!x_is_f32 || n_edges <= 255, "float input takes up to 255 edges");
     PB_REQUIRE(((uintptr_t)out % 4) == 0, "out must be 4-byte aligned");
     if (n_rows <= 0) return PB_OK;
     PackRowsArgs a{x, n_rows, n_features, edges, (int)n_edges, (int)max_bins, out, pitch_row, top, 0};

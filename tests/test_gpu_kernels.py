@@ -327,6 +327,20 @@ def test_pack_kernels_at_tile_edges(n, f, max_bins):
             np.testing.assert_array_equal(rows_of(pack_row_major(table, e, max_bins)), want)
 
 
+@pytest.mark.parametrize("n_edges,max_bins", [(15, 16), (20, 16), (127, 128), (300, 100), (300, 256), (3, 64)])
+def test_rows_are_binned_with_more_or_fewer_edges_than_bins(n_edges, max_bins):
+    """A model may bring any number of edges: codes are cut to max_bins - 1."""
+    from packboost_b200.data import pack_row_major
+    rng = np.random.default_rng(n_edges)
+    X = rng.normal(size=(333, 21)).astype(np.float32)
+    X[::9, 4], X[1, 5], X[2, 5] = np.nan, np.inf, -np.inf
+    edges = np.sort(rng.normal(size=(n_edges, 21)).astype(np.float32), axis=0)
+    raw = pack_row_major(X, edges, max_bins).codes.cpu().numpy()
+    got = (np.stack([raw & 0xF, raw >> 4], axis=2).reshape(333, -1) if max_bins <= 16 else raw)[:, :21]
+    want = np.stack([np.searchsorted(edges[:, j], X[:, j]) for j in range(21)], axis=1).clip(0, max_bins - 1)
+    np.testing.assert_array_equal(got, want)
+
+
 @pytest.mark.parametrize("nbytes", [1, (384 << 10) + 1, (1 << 20) - 3, (16 << 20) + 5, (37 << 20) + 1])
 def test_upload_moves_every_byte(nbytes):
     """The page-locked ring below, at and beyond its size."""
