@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) pack_codes_fm_kernel(PackArgs a) {
 // A lane owns a feature, a warp eight rows at a time; the edges of the 32 features sit in shared
 // memory with the feature as the bank.  Bound by the probes (steps per value, one shared load each);
 // 500 000 x 256 with 127 edges:
-// 275 us, 2.3 TB/s (334 with the probe address computed from the position)..
+// 275 us, 2.3 TB/s (334 with the probe address computed from the position).
 template <int BITS, int STEPS>
 __global__ void __launch_bounds__(256) pack_floats_fm_kernel(PackArgs a) {
     constexpr int W = kTileR * BITS / 32;
@@ -267,7 +267,7 @@ struct PackRowsArgs {
 
 // Byte input: `lanes` lanes (a power of two) share a row, a lane packs one output word (8 or 4
 // codes) per step.  Bound by HBM; 1 M x 2 376 codes: 0.73 ms, 4.9 TB/s
-// (1.34 with two loads in flight per lane)..
+// (1.34 with two loads in flight per lane).
 template <int BITS>
 __global__ void __launch_bounds__(256) pack_code_rows_kernel(PackRowsArgs a, int lanes) {
     constexpr int PER = 32 / BITS;            // codes per output word
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(256) pack_code_rows_kernel(PackRowsArgs a, int
 // Float input: a lane owns four consecutive features of a tile of 128 and takes four rows at a time
 // (sixteen independent searches); the edges of the tile sit in shared memory, a lane's features 32
 // words apart.  Bound by the probes; 300 007 x 256 with 127 edges: 120 us, 3.2 TB/s (514 with the edges
-// in global memory)..
+// in global memory).
 template <int BITS, int STEPS>
 __global__ void __launch_bounds__(256) pack_float_rows_kernel(PackRowsArgs a) {
     extern __shared__ float s_edges[];        // [2^STEPS - 1][4][32]

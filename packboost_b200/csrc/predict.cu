@@ -983,13 +983,13 @@ extern "C" int pb_predict_table(const pb_model* m, const void* x, int64_t x_on_d
         }
         if (!x_on_device) {
             rc = pb_upload(d + p.off_raw, x, p.raw, h + p.off_in, pinned_bytes - p.off_in, stream_);
-            if (rc) return rc;
             src = d + p.off_raw;
         }
     }
     uint8_t* codes = reinterpret_cast<uint8_t*>(d + p.off_codes);
-    rc = pb_pack_rows_top(src, m->edges ? 1 : 0, n_rows, n_features, m->edges, m->n_edges, m->max_bins, codes, p.pitch,
-                          m->code_bits, d_top, stream_);
+    if (rc == PB_OK)
+        rc = pb_pack_rows_top(src, m->edges ? 1 : 0, n_rows, n_features, m->edges, m->n_edges, m->max_bins, codes, p.pitch,
+                              m->code_bits, d_top, stream_);
     if (rc == PB_OK)
         rc = pb_predict_forest(codes, n_rows, p.pitch, m->code_bits, n_features, m->trees, m->copies, m->slot_nodes, m->depth,
                                m->repeat, m->total_repeat, m->n_trees, (float)m->weight, pred, nullptr, stream_);
