@@ -204,10 +204,11 @@ class Uploads:
                 dev = torch.empty(src.shape, dtype=dtype, device=_device()) if out is None else out
                 return dev.copy_(src, non_blocking=True)
             src = src.contiguous()
+            shape, at, nbytes = src.shape, src.data_ptr(), src.numel() * src.element_size()
         else:
-            src = torch.from_numpy(np.ascontiguousarray(host, dtype=_NUMPY_OF[dtype]))
-        dev = torch.empty(src.shape, dtype=dtype, device=_device()) if out is None else out
-        nbytes = src.numel() * src.element_size()
+            src = np.ascontiguousarray(host, dtype=_NUMPY_OF[dtype])
+            shape, at, nbytes = src.shape, src.ctypes.data, src.nbytes
+        dev = torch.empty(shape, dtype=dtype, device=_device()) if out is None else out
         need = int(B.lib().pb_upload_ring_bytes(nbytes))
         ring = next((r for r in self._rings if r.numel() >= need), None)
         if ring is not None:
@@ -215,7 +216,7 @@ class Uploads:
         else:
             ring = torch.empty(max(need, 1), dtype=torch.uint8, pin_memory=True)
             self._rings.append(ring)
-        B.check(B.lib().pb_upload(dev.data_ptr(), src.data_ptr(), nbytes, ring.data_ptr(), ring.numel(),
+        B.check(B.lib().pb_upload(dev.data_ptr(), at, nbytes, ring.data_ptr(), ring.numel(),
                                   torch.cuda.current_stream().cuda_stream))
         return dev
 

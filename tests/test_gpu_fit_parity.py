@@ -523,3 +523,21 @@ def test_the_round_graph_is_given_back_at_the_end_of_a_fit():
     assert counts[0] > 0 and counts[1] > 0 and counts[2] == 0     # launched, captured again, replayed
     b._finish()
     np.testing.assert_array_equal(b.train_predictions(), want)
+
+
+@pytest.mark.parametrize("codes", [True, False])
+def test_read_only_arrays_are_taken_without_a_warning(codes):
+    """Memory maps and arrow columns cannot be written to, and nobody here does."""
+    import warnings
+    from packboost_b200 import PackBoost, PackBoostConfig
+    rng = np.random.default_rng(3)
+    X = rng.integers(0, 5, size=(2_000, 12), dtype=np.uint8) if codes else rng.normal(size=(2_000, 12)).astype(np.float32)
+    y = (X[:, 0] - X[:, 7] + rng.normal(size=2_000)).astype(np.float32)
+    X.flags.writeable = False
+    cfg = PackBoostConfig(pack_size=2, max_depth=3, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=5, max_bins=5,
+                          prebinned=codes, random_state=1)
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        b = PackBoost(cfg).fit(X, y, None, num_rounds=2)
+        # (through the one library call, and the general way)
+        np.testing.assert_array_equal(b.predict(X), b.predict(X.copy(order="F")))
