@@ -343,12 +343,9 @@ class _DeviceTrainer:
         local_sampled = (k_sampled + world - 1) // world + 1
         want = 24 * self.F * stride + per_feat * min(local_sampled, max(matrix.n_features_local, 1)) + (1 << 20)
         min_bytes = int(self.lib.pb_workspace_min_bytes(C.byref(st)))
-        if workspace_bytes is None:
-            # (the query costs about 70 us of a fit)
-            cap = os.getenv("PACKBOOST_WORKSPACE_BYTES")
-            cap = min(8 << 30, int(torch.cuda.mem_get_info(self.dev)[0] * 0.6)) if cap is None else int(cap)
-            workspace_bytes = max(min_bytes, min(want, cap))
-        self.workspace = torch.empty(int(workspace_bytes), dtype=torch.uint8, device=self.dev)
+        self.workspace = (self._take_workspace(want, min_bytes) if workspace_bytes is None
+                          else torch.empty(int(workspace_bytes), dtype=torch.uint8, device=self.dev))
+        workspace_bytes = self.workspace.numel()
         st.workspace = self.workspace.data_ptr()
         st.workspace_bytes = int(workspace_bytes)
         eo = np.ascontiguousarray(era_offsets, dtype=np.int32)
@@ -401,6 +398,23 @@ class _DeviceTrainer:
             self.comm = comm
         self._prof_ms, self._prof_n = [0.0] * 5, [0] * 5
         self._prof_queue: list[tuple[int, float]] = []
+
+    def _take_workspace(self, want: int, least: int) -> torch.Tensor:
+        """``want`` bytes, or as many as leave two fifths of the free memory to the rest of the fit."""
+        def take(nbytes):
+            return torch.empty(int(nbytes), dtype=torch.uint8, device=self.dev)
+
+        cap = os.getenv("PACKBOOST_WORKSPACE_BYTES")
+        if cap is None and want <= 1 << 30:
+            # Asking for the free memory costs 0.1 ms and, now and then, tens of them (a driver lock): a small
+            # workspace is tried, with the room to be left, which goes back to the allocator at once.
+            try:
+                take(max(want, least) * 5 // 3)
+                return take(max(want, least))
+            except torch.cuda.OutOfMemoryError:
+                pass
+        cap = min(8 << 30, int(torch.cuda.mem_get_info(self.dev)[0] * 0.6)) if cap is None else int(cap)
+        return take(max(least, min(want, cap)))
 
     # -- per-phase timing (the reference fills hist_ms / score_ms / partition_ms of its depth logs
     #    with perf_counter buckets, packboost/booster.py:220-270) --------------------------------
@@ -825,10 +839,8 @@ class PackBoost:
         # ceil(F / world) features).
         c0, c1 = owned_range(F, rank, world)
         blk = block_size(F, world)
-        uploads = Uploads()
+        edges = None
         if is_binned:
-            edges = None
-            self._binner = BinningResult(bins=None, bin_edges=None, prebinned=True)
             if on_device:
                 X_src = X_np.view(torch.uint8) if X_np.dtype == torch.int8 else X_np.to(torch.uint8)
             else:
@@ -836,8 +848,6 @@ class PackBoost:
                 X_src = X_src.view(np.uint8)
         else:
             X_src = X_np.to(torch.float32) if on_device else X_np.astype(np.float32, copy=False)
-            if world == 1 and not (on_device and X_src.is_cuda) and fits_on_device(N * F * 4):
-                X_src = uploads(X_src, torch.float32)   # once: the edges and the codes are both taken from this copy
             if world > 1:
                 # each rank sorts its own columns; the edge tables are exchanged
                 own = np.zeros((cfg.max_bins - 1, blk), dtype=np.float32)
@@ -846,9 +856,6 @@ class PackBoost:
                 parts = torch.empty((world, cfg.max_bins - 1, blk), dtype=torch.float32, device=self._device)
                 torch.distributed.all_gather_into_tensor(parts, torch.from_numpy(own).to(self._device))
                 edges = np.ascontiguousarray(parts.permute(1, 0, 2).reshape(cfg.max_bins - 1, world * blk)[:, :F].cpu().numpy())
-            else:
-                edges = quantile_edges_device(X_src, cfg.max_bins)
-            self._binner = BinningResult(bins=None, bin_edges=edges, prebinned=False)
 
         # When the whole packed matrix fits comfortably in one GPU's memory it is kept on every rank
         # anyway (each rank packs its strip, an all-gather over NVLink completes the copies): each
@@ -871,8 +878,23 @@ class PackBoost:
                                                     validate_codes=validate_on_device)
         else:
             feat_local = feature_map(F, 0, 1)
-            matrix = pack_feature_major(X_src, edges, cfg.max_bins, row_order=order, validate_codes=validate_on_device,
-                                        defer_validation=True)
+
+            def bin_and_pack(src):
+                e = None if is_binned else quantile_edges_device(src, cfg.max_bins)
+                return e, pack_feature_major(src, e, cfg.max_bins, row_order=order, validate_codes=validate_on_device,
+                                             defer_validation=True)
+
+            matrix = None
+            if not is_binned and not (on_device and X_src.is_cuda) and fits_on_device(N * F * 4):
+                uploads = Uploads()
+                try:   # brought over once: the edges and the codes are both taken from this copy
+                    edges, matrix = bin_and_pack(uploads(X_src, torch.float32))
+                except torch.cuda.OutOfMemoryError:
+                    pass
+                torch.cuda.current_stream().synchronize()
+            if matrix is None:   # (the copy is gone: from the host in pieces)
+                edges, matrix = bin_and_pack(X_src)
+        self._binner = BinningResult(bins=None, bin_edges=edges, prebinned=is_binned)
         if validate_on_device and not agree_all(matrix.max_code < min(cfg.max_bins, 128), self._device):
             raise ValueError("prebinned=True requires X to contain integer bins within [0, max_bins).")
         if order is None:

@@ -225,8 +225,13 @@ _NUMPY_OF = {torch.float32: np.float32, torch.uint8: np.uint8, torch.int32: np.i
 
 
 def fits_on_device(nbytes: int) -> bool:
-    """Whether a whole table may be brought to the device for a while: up to a third of what is free."""
-    return nbytes <= torch.cuda.mem_get_info(_device())[0] // 3
+    """Whether to try bringing a whole table to the device for a while: when it is small next to the device
+    (asking for the free memory costs 0.1 ms and, now and then, tens of them), else up to a third of what is
+    free.  The caller goes on without when there is no room after all."""
+    dev = _device()
+    if nbytes <= torch.cuda.get_device_properties(dev).total_memory // 64:
+        return True
+    return nbytes <= torch.cuda.mem_get_info(dev)[0] // 3
 
 
 def pack_feature_major(

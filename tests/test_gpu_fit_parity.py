@@ -481,23 +481,35 @@ def test_fit_is_bit_identical_in_forced_histogram_shapes(shape):
     assert "hist_lane_kernel<%s>" % shape.replace(" ", ",") in res.stderr + res.stdout, "forced shape never launched"
 
 
-def test_a_fit_on_a_nearly_full_device_takes_less_workspace_and_gives_the_same(monkeypatch):
-    """8 MB free: the workspace shrinks to what that allows (features go through it in blocks) and the table is
-    streamed; trees and predictions do not change."""
-    from packboost_b200 import PackBoost, PackBoostConfig, data
+def test_a_fit_on_a_nearly_full_device_streams_the_table_and_gives_the_same(monkeypatch):
+    """An allocator of 500 MB: the table (240 MB) cannot stay while its columns are sorted and goes over in
+    pieces, the workspace shrinks and the features go through it in blocks; trees and predictions do not change."""
+    from packboost_b200 import PackBoost, PackBoostConfig
+    from packboost_b200 import booster as bm
     rng = np.random.default_rng(8)
-    X = rng.normal(size=(20_000, 64)).astype(np.float32)
-    y = (X[:, 0] + X[:, 1] * X[:, 2] + rng.normal(size=20_000)).astype(np.float32)
-    era = np.sort(rng.integers(0, 20, 20_000)).astype(np.int16)
-    cfg = PackBoostConfig(pack_size=2, max_depth=6, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=5, max_bins=128, random_state=1)
+    X = rng.standard_normal((60_000, 1_000), dtype=np.float32)
+    y = (X[:, 0] + X[:, 1] * X[:, 2] + rng.normal(size=60_000)).astype(np.float32)
+    era = np.sort(rng.integers(0, 40, 60_000)).astype(np.int16)
+    cfg = PackBoostConfig(pack_size=2, max_depth=6, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=5, max_bins=128,
+                          layer_feature_fraction=0.2, random_state=1)
     want = PackBoost(cfg).fit(X, y, era, num_rounds=2)
-    total = torch.cuda.get_device_properties(0).total_memory
-    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (8 << 20, total))
-    assert not data.fits_on_device(X.nbytes)
-    got = PackBoost(cfg).fit(X, y, era, num_rounds=2)
-    assert got._trainer.workspace.numel() <= int(0.6 * (8 << 20)) < want._trainer.workspace.numel()
-    np.testing.assert_array_equal(got.train_predictions(), want.train_predictions())
-    for a, b in zip(want.split_records().values(), got.split_records().values()):
+    wide, preds, splits = want._trainer.workspace.numel(), want.train_predictions(), want.split_records()
+    del want
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total, used, room = torch.cuda.get_device_properties(0).total_memory, torch.cuda.memory_reserved(), 500 << 20
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (used + room - torch.cuda.memory_reserved(), total))
+    sorted_from, edges_of = [], bm.quantile_edges_device
+    monkeypatch.setattr(bm, "quantile_edges_device", lambda t, n: (sorted_from.append(type(t)), edges_of(t, n))[1])
+    torch.cuda.set_per_process_memory_fraction((used + room) / total)
+    try:
+        got = PackBoost(cfg).fit(X, y, era, num_rounds=2)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert sorted_from == [torch.Tensor, np.ndarray]
+    assert got._trainer.workspace.numel() < wide
+    np.testing.assert_array_equal(got.train_predictions(), preds)
+    for a, b in zip(splits.values(), got.split_records().values()):
         np.testing.assert_array_equal(a, b)
 
 

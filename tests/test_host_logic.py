@@ -450,14 +450,27 @@ def test_codes_are_told_from_values_in_every_type(dtype):
             assert detect_prebinned_tensor(torch.from_numpy(a), max_bins) == detect_prebinned(a, max_bins), (values, max_bins)
 
 
-def test_a_table_is_brought_over_whole_only_into_free_memory(monkeypatch):
-    """Small tables too: the device may be nearly full."""
-    from packboost_b200 import data
-    monkeypatch.setattr(data, "_device", lambda: torch.device("cuda", 0))
-    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda dev: type("P", (), {"total_memory": 180 << 30})())
-    for free, nbytes, fits in ((3 << 20, 1 << 20, True), (3 << 20, (1 << 20) + 1, False), (0, 1, False), (90 << 30, 30 << 30, True)):
-        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev, free=free: (free, 180 << 30))
-        assert data.fits_on_device(nbytes) is fits
+@pytest.mark.parametrize("want,least,free,room,size", [
+    (600, 10, 5000, 1000, 600),          # with what is to be left it just fits: nobody asks
+    (600, 10, 900, 999, 540),            # it does not: as much as leaves two fifths of what is free
+    (600, 580, 900, 999, 580), (600, 10, 5000, 0, 600), (3 << 30, 10, 1 << 30, 0, int((1 << 30) * 0.6))])
+def test_a_workspace_leaves_memory_to_the_rest_of_the_fit(want, least, free, room, size, monkeypatch):
+    from packboost_b200 import booster as bm
+    monkeypatch.delenv("PACKBOOST_WORKSPACE_BYTES", raising=False)
+    trainer = bm._DeviceTrainer.__new__(bm._DeviceTrainer)
+    trainer.dev = torch.device("cpu")
+    asked = []
+
+    def empty(n, **kw):
+        if n > room and not asked:           # (the driver is asked after the first refusal; what it says can be had)
+            raise torch.cuda.OutOfMemoryError("full")
+        return n
+
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev: (asked.append(dev), (free, 180 << 30))[1])
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", empty)
+        assert trainer._take_workspace(want, least) == size
+    assert bool(asked) == (want * 5 // 3 > room)
 
 
 def test_of_a_decision_log_only_the_splits_are_kept(monkeypatch):
