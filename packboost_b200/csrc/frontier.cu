@@ -743,10 +743,10 @@ static double two_step_estimate_us(const pb_train_state* st, int64_t depth, int6
 // histogram, gain and chain kernels, bit for bit alike.  The walk moves no histogram and no gains, but its
 // CTAs go through all rows of a feature; the other path cuts the rows, and has the GPU full with few
 // features.  So neither is the faster one everywhere (128 bins, depth 6, a round's histogram and score;
-// walk / other path): 500 000 rows x 200 features, 100 eras 2.6 / 3.8 ms; 131 072 x 200, 574 eras 8.2 / 20.8;
-// 262 144 x 64, 20 eras 1.06 / 0.78; 1 000 000 x 64, 100 eras 3.3 / 2.4; 4 000 000 x 32, 20 eras 10.1 / 2.4.
-// The estimates decide by depth: over the 9 000 depths they were fitted to that takes 3 % more time than
-// the better path each time, where the walk everywhere takes 50 % more.  Where they come within a tenth it
+// walk / other path): 500 000 rows x 200 features, 100 eras 2.2 / 3.8 ms; 131 072 x 200, 574 eras 6.3 / 20.8;
+// 262 144 x 64, 20 eras 0.73 / 0.78; 1 000 000 x 64, 100 eras 2.9 / 2.4; 4 000 000 x 32, 20 eras 10.5 / 2.4.
+// The estimates decide by depth: over the 9 000 depths that they were first fitted to that took 3 % more time
+// than the better path each time, where the walk everywhere took 50 % more.  Where they come within a tenth it
 // is the walk, whose estimate is the safer one in deep frontiers of few rows.
 // PACKBOOST_WALK=0 / 1 takes one path everywhere, for comparisons.
 struct DepthPath {

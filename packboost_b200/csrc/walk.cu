@@ -4,29 +4,33 @@
 // (feature, era, node, bin) written and read back, then 8 bytes per threshold of (gain, weight) written
 // and read again - 13 GB for one round of 500 000 rows, 256 features, 100 eras, 128 bins and depth 6,
 // against 0.9 GB of codes and row state.  None of it outlives its era: the score of a threshold is a
-// Welford recursion over the eras in ascending order.  So a CTA owns one feature and up to sixteen
-// frontier nodes and walks the eras; the state of the recursion stays in registers to the end, and what
-// leaves the CTA is one candidate per node.
+// Welford recursion over the eras in ascending order.  So a CTA owns one feature and a group of frontier
+// nodes and walks the eras; the state of the recursion stays in registers to the end, and what leaves the
+// CTA is one candidate per node.  Two forms: with fewer nodes than warps the eras go by in batches
+// (walk_kernel), from sixteen nodes on a warp owns a node (walk_nodes_kernel, further down).
 //
 // Cells are the two words of the histogram kernel (sum of low gradient bits << CB | count, sum of high
-// bits).  The eras go by in batches of sixteen (era, node) pairs, sixteen eras at one node, one at
-// sixteen: (a) all warps add the rows of the batch to its cells; (b) a warp per pair scans the bins (a
+// bits).  A batch is an (era, node) pair per warp, as many eras at one node as there are warps: (a) all warps add the rows of the batch to its cells; (b) a warp per pair scans the bins (a
 // lane per BPL consecutive ones), computes the gains and leaves them in shared memory; (c) a thread per
 // threshold advances the recursion through the eras of the batch.  So the latency of the scan, its
-// shuffles and divisions, is paid once a batch by sixteen warps side by side.  An era of more rows than
+// shuffles and divisions, is paid once a batch by all warps side by side.  An era of more rows than
 // the count field holds is cut into tiles whose prefix sums are added up before (b) goes on.
 //
 // Divisions: every divisor of the gains is count + lambda, so an era's divisors and their correctly
 // rounded reciprocals come from a table in shared memory, and a quotient takes two corrected products
 // instead of a general division (divide.cuh).
 //
-// Bound: the shared-memory atomics (two per row and feature, about four wavefronts each with 128 bins)
-// at the upper depths, the gains at the lower ones.
-// 500 000 rows x 256 features, 100 eras, 128 bins, by depth: 0.24, 0.27, 0.31, 0.40, 0.59, 0.96 ms, 2.8 ms a
-// round (histogram, gain and chain kernels: 4.6 ms); 200 000 x 100, depth 10: 2.7 ms a round (6.1).
+// Bound: with few nodes the rows (two shared-memory atomics per row and feature take 3.5 wavefronts each
+// with 128 bins, 66 % of the shared-memory pipe; without them, or with rows from the L1, they still take 85 %
+// of the time: no one thing), with many the gains (issue slots).
+// 500 000 rows x 256 features, 100 eras, 128 bins, by depth: 0.22, 0.24, 0.29, 0.38, 0.41, 0.63 ms, 2.2 ms a
+// round (one form for all depths: 0.50 and 1.01 ms at the last two, 2.7 ms; histogram, gain and chain kernels:
+// 4.6); 200 000 x 100, 40 eras, depth 10: 3.0 ms a round (4.8 with the one form), of which 512 nodes 1.23 (2.07).
 //
 // Float arithmetic as in the scorer: the same separately rounded operations in the same order
 // (this file is compiled with -fmad=false), so candidates are bit-identical to the other path's.
+
+#include <stdlib.h>
 
 #include "common.cuh"
 #include "des_math.cuh"
@@ -36,9 +40,7 @@ namespace pb {
 
 namespace {
 
-constexpr int kWalkWarps = 16;
-constexpr int kWalkThreads = 32 * kWalkWarps;
-constexpr int kWalkNodes = kWalkWarps;   // (era, node) pairs of a batch, and most nodes of a CTA: one warp each
+constexpr int kWalkWarpsMax = 32;
 constexpr int kWalkInv = 4096;           // longest table of era reciprocals
 
 struct RowGroup {                        // four consecutive rows
@@ -171,16 +173,18 @@ __device__ __forceinline__ void take_words(uint32_t* at, uint32_t (&v)[W]) {  //
     }
 }
 
-// Shared memory: cells [pairs][NBP][copies] word A, then word B | gains [pairs][NBP] | agreement [pairs][NBP]
+// Shared memory: cells [pairs + 1][NBP][copies] word A, then word B | gains [pairs][NBP] | agreement [pairs][NBP]
 // (kGeneral) or 1 / n [eras + 1] | (divisor, reciprocal) [largest era + 1] when an era is one tile.
 // A pair's gains lie at i * 32 + lane for bin lane * BPL + i.  COPIES: interleaved copies of the cells.
-template <int BPL, int MODE, int COPIES>
-__global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ? 2 : 1) walk_kernel(WalkLaunch a) {
+// WARPS: of a CTA, and (era, node) pairs of a batch and most nodes of a CTA.
+template <int BPL, int MODE, int COPIES, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, (BPL <= 4 && MODE != kGeneral && WARPS == 16) ? 2 : 1) walk_kernel(WalkLaunch a) {
+    constexpr int kWalkThreads = 32 * WARPS, kWalkNodes = WARPS;
     constexpr bool UNIT = MODE != kGeneral, TILES = MODE != kUnit;
     constexpr int NBP = 32 * BPL;        // bins of a pair's cells
     constexpr int SLOTS = kWalkNodes * NBP / kWalkThreads;   // thresholds a thread may own
     constexpr int plane = kWalkNodes * NBP;
-    constexpr int words = plane * COPIES;                    // of word A; word B follows
+    constexpr int words = (plane + NBP) * COPIES;            // of word A, rows nobody counts included; word B follows
     extern __shared__ __align__(16) uint32_t s_cells[];      // [pairs][NBP][COPIES]
     float2* s_gain = reinterpret_cast<float2*>(s_cells + 2 * words);
     float* s_agree = reinterpret_cast<float*>(s_gain + plane);
@@ -224,18 +228,21 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
         __syncthreads();
     }
 
-    // ---- rows: groups of four; a row of another CTA's node is predicated off, so the usual group has
-    //      no branch per row ----
+    // ---- rows: a warp takes 128 consecutive rows, a lane four of them ----
     const uint8_t* codes = a.codes + (int64_t)a.feat_rows[f] * a.pitch;
     const bool sparse = gridDim.x > 2;   // most rows belong to other CTAs: gradients are read when a row is ours
     constexpr uint32_t PAIR = 4u * NBP * COPIES;             // bytes of a pair's cells
     const uint32_t cells_at = (uint32_t)__cvta_generic_to_shared(s_cells) + 4u * (threadIdx.x & (COPIES - 1));
-    auto load_group = [&](uint32_t g, int r1, RowGroup& x) {
-        if ((int)(4 * g) < r1) {
-            x.codes = *reinterpret_cast<const uint32_t*>(codes + 4 * g);
-            x.slots = *reinterpret_cast<const uint2*>(a.slot + 4 * g);
-            if (!sparse) x.gq = *reinterpret_cast<const int4*>(a.gq + 4 * g);
-        }
+    // Rows of other CTAs' nodes, and of none, go to cells of their own after the pairs', which nobody reads:
+    // an address is chosen, nothing is predicated (a predicate costs a branch each way around the atomics;
+    // 500 000 rows x 256 features, one node, rows alone: 204 us with predicates, 190 without)
+    const uint32_t trash = cells_at + (uint32_t)kWalkNodes * PAIR;
+    const uint32_t one_a = 1u << CB;
+    auto load_group = [&](int c, RowGroup& x) {              // chunk c, 128 rows (the row arrays are padded to 256)
+        const uint32_t g = 32u * (uint32_t)c + (uint32_t)lane;
+        x.codes = reinterpret_cast<const uint32_t*>(codes)[g];
+        x.slots = reinterpret_cast<const uint2*>(a.slot)[g];
+        if (!sparse) x.gq = reinterpret_cast<const int4*>(a.gq)[g];
     };
     auto add_row = [&](uint32_t base, uint32_t n, uint32_t code, int q) {
 #ifdef PB_DEBUG_BOUNDS
@@ -247,45 +254,43 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
         }
 #endif
         // (a byte that is no bin falls into a neighbour's cells or, after the last, into the gains)
-        asm volatile(
-            "{ .reg .pred p; setp.lt.u32 p, %0, %1;\n"
-            "@p red.shared.add.u32 [%2], %3;\n"
-            "@p red.shared.add.u32 [%2 + %5], %4; }\n" ::"r"(n), "r"(live), "r"(base + n * PAIR + code * (4u * COPIES)),
-            "r"((((uint32_t)q & lo_mask) << CB) + 1u), "r"(q >> LB), "n"(4 * words)
-            : "memory");
+        const uint32_t at = (n < (uint32_t)live ? base + n * PAIR : trash) + code * (4u * COPIES);
+        asm volatile("red.shared.add.u32 [%0], %1;\n red.shared.add.u32 [%0 + %3], %2;" ::"r"(at),
+                     "r"(((uint32_t)q & lo_mask) * one_a + 1u), "r"(q >> LB), "n"(4 * words) : "memory");
     };
-    // `e`, `lim`: era of the batch at the thread's last row and where that era ends (rows ascend)
-    auto add_group = [&](uint32_t g, int r0, int r1, RowGroup& x, int& e, int& lim) {
-        const int r = (int)(4 * g);
+    // `e`, `lim`: era of the batch at the warp's last chunk and where that era ends (rows ascend)
+    auto add_group = [&](int c, int r0, int r1, RowGroup& x, int& e, int& lim) {
+        const int first = 128 * c;       // (the warp's: all lanes decide alike)
         if (!TILES)
-            while (r >= lim) lim = s_off[++e + 1];
+            while (first >= lim) lim = s_off[++e + 1];
         const uint32_t n0 = (x.slots.x & 0xFFFFu) - (uint32_t)node0, n1 = (x.slots.x >> 16) - (uint32_t)node0;
         const uint32_t n2 = (x.slots.y & 0xFFFFu) - (uint32_t)node0, n3 = (x.slots.y >> 16) - (uint32_t)node0;
         if (sparse) {
             if (min(min(n0, n1), min(n2, n3)) >= (uint32_t)live) return;
-            x.gq = *reinterpret_cast<const int4*>(a.gq + 4 * g);
+            x.gq = reinterpret_cast<const int4*>(a.gq)[32 * c + lane];
         }
-        const uint32_t here = cells_at + (TILES ? 0u : (uint32_t)(e * CN) * PAIR);
-        if (r >= r0 && r + 4 <= (TILES ? r1 : lim)) {
+        const uint32_t step = (uint32_t)CN * PAIR;
+        uint32_t here = cells_at + (TILES ? 0u : (uint32_t)e * step);
+        if (first >= r0 && first + 128 <= (TILES ? r1 : lim)) {
             add_row(here, n0, x.codes & 0xFFu, x.gq.x);
             add_row(here, n1, __byte_perm(x.codes, 0u, 0x4441u), x.gq.y);
             add_row(here, n2, __byte_perm(x.codes, 0u, 0x4442u), x.gq.z);
             add_row(here, n3, x.codes >> 24, x.gq.w);
         } else {                         // rows of a neighbouring batch, or of several eras
-#pragma unroll 1
-            for (int j = 0; j < 4; ++j) {
-                if (r + j >= r0 && r + j < r1) {
-                    int ej = e;
-                    if (!TILES)
-                        while (r + j >= s_off[ej + 1]) ++ej;
-                    add_row(cells_at + (TILES ? 0u : (uint32_t)(ej * CN) * PAIR), (x.slots.x & 0xFFFFu) - (uint32_t)node0,
-                            x.codes & 0xFFu, x.gq.x);
+            int ej = e, end = TILES ? r1 : lim;
+            auto one = [&](int r, uint32_t n, uint32_t code, int q) {
+                if (r < r0 || r >= r1) return;
+                while (r >= end) {
+                    end = s_off[++ej + 1];
+                    here += step;
                 }
-                x.codes >>= 8;
-                x.slots.x = x.slots.x >> 16 | x.slots.y << 16;
-                x.slots.y >>= 16;
-                x.gq = make_int4(x.gq.y, x.gq.z, x.gq.w, 0);
-            }
+                add_row(here, n, code, q);
+            };
+            const int r = first + 4 * lane;
+            one(r, n0, x.codes & 0xFFu, x.gq.x);
+            one(r + 1, n1, __byte_perm(x.codes, 0u, 0x4441u), x.gq.y);
+            one(r + 2, n2, __byte_perm(x.codes, 0u, 0x4442u), x.gq.z);
+            one(r + 3, n3, x.codes >> 24, x.gq.w);
         }
     };
 
@@ -322,25 +327,24 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
         return TILES ? r1 >= end : true;                     // the batch completes its eras
     };
     bool complete = batch_end();
-    RowGroup cur;                        // the thread's next group of rows
-    load_group(r0 / 4 + threadIdx.x, r1, cur);
     if (threadIdx.x <= kWalkNodes) s_off[threadIdx.x] = a.era_offsets[min((int)threadIdx.x, E)];
     __syncthreads();                     // cells are zero; offsets and tables are there
     while (ne > 0) {
         // ---- (a) ----
         {
-            int e = 0, lim = s_off[1];
-            for (uint32_t g = r0 / 4 + threadIdx.x; (int)(4 * g) < r1; g += kWalkThreads) {
-                RowGroup x = cur;
-                load_group(g + kWalkThreads, r1, cur);
-                add_group(g, r0, r1, x, e, lim);
+            int e = 0, lim = s_off[1], chunk = r0 / 128 + warp;
+            RowGroup cur;                // the warp's next chunk of rows
+            if (128 * chunk < r1) load_group(chunk, cur);
+            for (; 128 * chunk < r1; chunk += WARPS) {
+                RowGroup x = cur;        // (two sets of registers in turn save the copy and spill elsewhere: 215 -> 228 us)
+                if (128 * (chunk + WARPS) < r1) load_group(chunk + WARPS, cur);
+                add_group(chunk, r0, r1, x, e, lim);
             }
         }
         const int n_eras_now = complete ? ne : 0;            // eras that (b) finishes
         if (complete) e0 += ne;
         r0 = r1;
         complete = batch_end();
-        load_group(r0 / 4 + threadIdx.x, r1, cur);           // (on its way during (b) and (c))
         __syncthreads();                 // the cells are complete, (c) of the batch before is done
         if (threadIdx.x <= kWalkNodes) s_off[threadIdx.x] = a.era_offsets[min(e0 + (int)threadIdx.x, E)];
 
@@ -381,55 +385,47 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
             sb -= B[BPL - 1];
             tc = (TILES ? tc : 0u) + (ta & cmask);
             tg = (TILES ? tg : 0ll) + (long long)(int32_t)tb * (1ll << LB) + (long long)(ta >> CB);
+            if (TILES) {
 #pragma unroll
-            for (int i = 0; i < BPL; ++i) {
-                const uint32_t av = A[i] + sa, bv = B[i] + sb;
-                pc[i] = (TILES ? pc[i] : 0u) + (av & cmask);
-                pg[i] = (TILES ? pg[i] : 0ll) + (long long)(int32_t)bv * (1ll << LB) + (long long)(av >> CB);
+                for (int i = 0; i < BPL; ++i) {
+                    const uint32_t av = A[i] + sa, bv = B[i] + sb;
+                    pc[i] += av & cmask;
+                    pg[i] += (long long)(int32_t)bv * (1ll << LB) + (long long)(av >> CB);
+                }
             }
             if (!TILES || n_eras_now > 0) {
                 float2* out = s_gain + warp * NBP + lane;
                 const float w_era = (tc == 0u) ? 0.f : (a.era_alpha > 0.f ? f_add((float)tc, a.era_alpha) : 1.f);
                 const float tgf = f_mul(__ll2float_rn(tg), inv_scale);
+                // (the operations of era_totals and gain_of, divisions by the table)
+                const float parent = table ? divide_by(f_mul(0.5f, f_mul(tgf, tgf)), s_div[tc])
+                                           : f_div(f_mul(0.5f, f_mul(tgf, tgf)), f_add((float)tc, lam));
 #pragma unroll
-                for (int i = 0; i < BPL; ++i) {
-                    lc_sum[i] += pc[i];
-                    lg_sum[i] += pg[i];
-                }
-                if (table) {             // the operations of era_totals and gain_of, divisions by the table
-                    const float parent = divide_by(f_mul(0.5f, f_mul(tgf, tgf)), s_div[tc]);
-#pragma unroll
-                    for (int i = 0; i < BPL; ++i) {
-                        const float lg = f_mul(__ll2float_rn(pg[i]), inv_scale), rg = f_sub(tgf, lg);
-                        const uint32_t rc = tc - pc[i];
-                        const float g2 = f_mul(0.5f, f_add(divide_by(f_mul(lg, lg), s_div[pc[i]]), divide_by(f_mul(rg, rg), s_div[rc])));
-                        out[i * 32] = make_float2(f_sub(g2, parent), (pc[i] > 0u && rc > 0u) ? w_era : 0.f);
-                    }
-                } else {
-                    const EraTotals et = era_totals(tc, tg, inv_scale, lam, a.era_alpha);
-#pragma unroll
-                    for (int i = 0; i < BPL; ++i)
-                        out[i * 32] = gain_of(pc[i], pg[i], tc, et.tg, et.th, et.parent, inv_scale, lam, et.w_era);
-                }
-                if (use_dir) {
-#pragma unroll
-                    for (int i = 0; i < BPL; ++i) {
-                        const float lg = f_mul(__ll2float_rn(pg[i]), inv_scale), lh = (float)pc[i];
-                        const float vl = f_div(-lg, f_add(lh, lam));
-                        const float vr = f_div(-f_sub(tgf, lg), f_add(f_sub((float)tc, lh), lam));
+                for (int i = 0; i < BPL; ++i) {              // (a threshold at a time: few registers)
+                    const uint32_t av = A[i] + sa, bv = B[i] + sb, lc = TILES ? pc[i] : av & cmask, rc = tc - lc;
+                    const long long lgq = TILES ? pg[i] : (long long)(int32_t)bv * (1ll << LB) + (long long)(av >> CB);
+                    lc_sum[i] += lc;
+                    lg_sum[i] += lgq;
+                    const float lg = f_mul(__ll2float_rn(lgq), inv_scale), rg = f_sub(tgf, lg);
+                    const float ll = f_mul(lg, lg), rr = f_mul(rg, rg);
+                    const float dl = f_add((float)lc, lam), dr = f_add(f_sub((float)tc, (float)lc), lam);
+                    const float ql = table ? divide_by(ll, s_div[lc]) : f_div(ll, dl);
+                    const float qr = table ? divide_by(rr, s_div[rc]) : f_div(rr, dr);
+                    out[i * 32] = make_float2(f_sub(f_mul(0.5f, f_add(ql, qr)), parent), (lc > 0u && rc > 0u) ? w_era : 0.f);
+                    if (use_dir) {
+                        const float vl = f_div(-lg, dl), vr = f_div(-rg, dr);
                         s_agree[warp * NBP + i * 32 + lane] = a.direction_form == 1
                             ? (vl > vr ? 1.f : -1.f)
                             : f_mul(0.5f, f_add(sign3(vl) == pa ? 1.f : 0.f, sign3(vr) == pa ? 1.f : 0.f));  // (an absent era has weight 0)
+                    }
+                    if (TILES) {
+                        pc[i] = 0u;
+                        pg[i] = 0ll;
                     }
                 }
                 if (TILES) {
                     tc = 0u;
                     tg = 0ll;
-#pragma unroll
-                    for (int i = 0; i < BPL; ++i) {
-                        pc[i] = 0u;
-                        pg[i] = 0ll;
-                    }
                 }
             }
         }
@@ -550,25 +546,271 @@ __global__ void __launch_bounds__(kWalkThreads, (BPL <= 4 && MODE != kGeneral) ?
     }
 }
 
-template <int BPL, int MODE, int COPIES>
+// ---- a warp per node ---------------------------------------------------------------------------------
+// Frontiers of as many nodes as a CTA has warps, or more: every warp owns a node for all eras, so the lane that
+// scans a threshold also advances its recursion and in the end scores it.  No gain passes through shared
+// memory and nothing is waited for but the cells: two eras at a time, the rows of the next two are added to one
+// set of cells while the set before is scanned, a barrier per step.  Where the batches spent more time than on
+// the gains themselves: the exchange of the gains with its second barrier, 180 of 1 016 us at 32 nodes (500 000
+// rows, 256 features), and the rows, which went by once per sixteen nodes, 544.  Now 630.
+// (Era weights 0 / 1, eras of one tile.)
+template <int BPL, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 && BPL <= 4) ? 2 : 1) walk_nodes_kernel(WalkLaunch a) {
+    constexpr int NBP = 32 * BPL, THREADS = 32 * WARPS;
+    constexpr int plane = (WARPS + 1) * NBP;                 // of word A; word B follows.  The last pair's cells: rows of no node here
+    constexpr uint32_t PAIR = 4u * NBP, ERA = 8u * plane, SET = 2u * ERA;   // bytes
+    extern __shared__ __align__(16) uint32_t s_cells[];      // [2 sets][2 eras][2 words][WARPS + 1][NBP] | 1 / n | (divisor, reciprocal)
+    float* s_inv = reinterpret_cast<float*>(s_cells + 8 * plane);
+    float2* s_div = reinterpret_cast<float2*>(s_inv + (a.n_eras + 2) / 2 * 2);
+    __shared__ uint32_t s_mass[256];
+    __shared__ uint8_t s_set[256];
+    const int n_nodes = min(*a.n_nodes_ptr, a.n_nodes);
+    const int node0 = blockIdx.x * WARPS;
+    const int live = min(WARPS, n_nodes - node0);
+    if (live <= 0) return;
+    const int f = blockIdx.y;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nb = a.max_bins, E = a.n_eras, K = a.n_thr;
+    const int CB = a.count_bits, LB = a.lo_bits;
+    const uint32_t lo_mask = (1u << LB) - 1u, cmask = (1u << CB) - 1u, one_a = 1u << CB;
+    const float inv_scale = *a.inv_scale_ptr, lam = a.lambda_l2;
+    const bool table = a.div_table && division_in_range(inv_scale, lam);
+
+    for (int i = threadIdx.x; i < 8 * plane; i += THREADS) s_cells[i] = 0u;
+    for (int n = threadIdx.x; n <= E; n += THREADS) s_inv[n] = n > 0 ? f_div(1.f, (float)n) : 0.f;
+    if (table)
+        for (int n = threadIdx.x; n <= a.max_era_rows; n += THREADS) {
+            const float d = f_add((float)n, lam);
+            s_div[n] = make_float2(d, f_div(1.f, d));
+        }
+    if (a.mass) {
+        for (int b = threadIdx.x; b < 256; b += THREADS) s_mass[b] = a.mass[(size_t)f * 256 + b];
+        __syncthreads();
+        mass_cut_set(s_mass, s_set, nb, K);
+    } else {
+        for (int b = threadIdx.x; b < 256; b += THREADS) s_set[b] = 0;
+        __syncthreads();
+        for (int k = threadIdx.x; k < K; k += THREADS) s_set[a.thr_ids[k]] = 1;
+    }
+    __syncthreads();
+
+    const uint8_t* codes = a.codes + (int64_t)a.feat_rows[f] * a.pitch;
+    const bool sparse = gridDim.x > 2;   // most rows belong to other CTAs: gradients are read when a row is ours
+    const uint32_t cells_at = (uint32_t)__cvta_generic_to_shared(s_cells);
+    auto load_group = [&](int c, RowGroup& x) {              // chunk c, 128 rows (the row arrays are padded to 256)
+        const uint32_t g = 32u * (uint32_t)c + (uint32_t)lane;
+        x.codes = reinterpret_cast<const uint32_t*>(codes)[g];
+        x.slots = reinterpret_cast<const uint2*>(a.slot)[g];
+        if (!sparse) x.gq = reinterpret_cast<const int4*>(a.gq)[g];
+    };
+    auto add_row = [&](uint32_t here, uint32_t n, uint32_t code, int q) {
+#ifdef PB_DEBUG_BOUNDS
+        const uint32_t sl = n + (uint32_t)node0;
+        if ((sl & 0xFFFFu) != kSlotNone && (int)sl >= a.n_nodes && a.debug_flags) atomicOr(a.debug_flags, kDbgSlot);
+        if (n < (uint32_t)live && code >= (uint32_t)nb) {
+            if (a.debug_flags) atomicOr(a.debug_flags, kDbgCode);
+            return;
+        }
+#endif
+        const uint32_t at = here + min(n, (uint32_t)WARPS) * PAIR + code * 4u;
+        asm volatile("red.shared.add.u32 [%0], %1;\n red.shared.add.u32 [%0 + %3], %2;" ::"r"(at),
+                     "r"(((uint32_t)q & lo_mask) * one_a + 1u), "r"(q >> LB), "n"(4 * plane) : "memory");
+    };
+    // rows [r0, r1) of two eras, the second from mid on
+    auto add_group = [&](int c, int r0, int mid, int r1, uint32_t set, RowGroup& x) {
+        const int r = 128 * c + 4 * lane;
+        const uint32_t n0 = (x.slots.x & 0xFFFFu) - (uint32_t)node0, n1 = (x.slots.x >> 16) - (uint32_t)node0;
+        const uint32_t n2 = (x.slots.y & 0xFFFFu) - (uint32_t)node0, n3 = (x.slots.y >> 16) - (uint32_t)node0;
+        if (sparse) {
+            if (min(min(n0, n1), min(n2, n3)) >= (uint32_t)live) return;
+            x.gq = reinterpret_cast<const int4*>(a.gq)[32 * c + lane];
+        }
+        if (r >= r0 && r + 4 <= r1 && (r >= mid || r + 4 <= mid)) {
+            const uint32_t here = set + (r >= mid ? ERA : 0u);
+            add_row(here, n0, x.codes & 0xFFu, x.gq.x);
+            add_row(here, n1, __byte_perm(x.codes, 0u, 0x4441u), x.gq.y);
+            add_row(here, n2, __byte_perm(x.codes, 0u, 0x4442u), x.gq.z);
+            add_row(here, n3, x.codes >> 24, x.gq.w);
+        } else {                         // rows of other steps, or of both eras
+            auto one = [&](int j, uint32_t n, uint32_t code, int q) {
+                if (r + j >= r0 && r + j < r1) add_row(set + (r + j >= mid ? ERA : 0u), n, code, q);
+            };
+            one(0, n0, x.codes & 0xFFu, x.gq.x);
+            one(1, n1, __byte_perm(x.codes, 0u, 0x4441u), x.gq.y);
+            one(2, n2, __byte_perm(x.codes, 0u, 0x4442u), x.gq.z);
+            one(3, n3, x.codes >> 24, x.gq.w);
+        }
+    };
+    auto add_rows = [&](int e, uint32_t set) {               // eras e, e + 1
+        if (e >= E) return;
+        const int r0 = a.era_offsets[e], mid = a.era_offsets[e + 1], r1 = a.era_offsets[min(e + 2, E)];
+        RowGroup cur;
+        int c = r0 / 128 + warp;
+        if (128 * c < r1) load_group(c, cur);
+        for (; 128 * c < r1; c += WARPS) {
+            RowGroup x = cur;
+            if (128 * (c + WARPS) < r1) load_group(c + WARPS, cur);
+            add_group(c, r0, mid, r1, set, x);
+        }
+    };
+
+    float mean[BPL], m2[BPL];
+    int n_valid[BPL];
+    uint32_t lc_sum[BPL];
+    long long lg_sum[BPL];
+#pragma unroll
+    for (int i = 0; i < BPL; ++i) {
+        mean[i] = m2[i] = 0.f;
+        n_valid[i] = 0;
+        lc_sum[i] = 0u;
+        lg_sum[i] = 0ll;
+    }
+    add_rows(0, cells_at);
+    __syncthreads();
+    for (int e0 = 0; e0 < E; e0 += 2) {
+        add_rows(e0 + 2, cells_at + ((e0 & 2) ? 0u : SET));
+        if (warp < live) {
+#pragma unroll 1
+            for (int e = 0; e < 2 && e0 + e < E; ++e) {
+                // prefix over the bins; the packed words are added as they are (the rows behind them are
+                // distinct rows of a tile, so no field overflows)
+                uint32_t A[BPL], B[BPL];
+                uint32_t* at = s_cells + ((e0 & 2) + e) * (2 * plane) + warp * NBP + lane * BPL;
+                take_words(at, A);
+                take_words(at + plane, B);
+#pragma unroll
+                for (int i = 1; i < BPL; ++i) {
+                    A[i] += A[i - 1];
+                    B[i] += B[i - 1];
+                }
+                uint32_t sa = A[BPL - 1], sb = B[BPL - 1];
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t ua = __shfl_up_sync(0xFFFFFFFFu, sa, d), ub = __shfl_up_sync(0xFFFFFFFFu, sb, d);
+                    if (lane >= d) {
+                        sa += ua;
+                        sb += ub;
+                    }
+                }
+                const uint32_t ta = __shfl_sync(0xFFFFFFFFu, sa, 31), tb = __shfl_sync(0xFFFFFFFFu, sb, 31);
+                sa -= A[BPL - 1];
+                sb -= B[BPL - 1];
+                const uint32_t tc = ta & cmask;
+                const long long tg = (long long)(int32_t)tb * (1ll << LB) + (long long)(ta >> CB);
+                const float tgf = f_mul(__ll2float_rn(tg), inv_scale);
+                const float parent = table ? divide_by(f_mul(0.5f, f_mul(tgf, tgf)), s_div[tc])
+                                           : f_div(f_mul(0.5f, f_mul(tgf, tgf)), f_add((float)tc, lam));
+#pragma unroll
+                for (int i = 0; i < BPL; ++i) {              // (the operations of gain_of)
+                    const uint32_t av = A[i] + sa, bv = B[i] + sb, lc = av & cmask, rc = tc - lc;
+                    const long long lgq = (long long)(int32_t)bv * (1ll << LB) + (long long)(av >> CB);
+                    lc_sum[i] += lc;
+                    lg_sum[i] += lgq;
+                    const float lg = f_mul(__ll2float_rn(lgq), inv_scale), rg = f_sub(tgf, lg);
+                    const float ll = f_mul(lg, lg), rr = f_mul(rg, rg);
+                    const float ql = table ? divide_by(ll, s_div[lc]) : f_div(ll, f_add((float)lc, lam));
+                    const float qr = table ? divide_by(rr, s_div[rc]) : f_div(rr, f_add(f_sub((float)tc, (float)lc), lam));
+                    const float gain = f_sub(f_mul(0.5f, f_add(ql, qr)), parent);
+                    const bool valid = lc > 0u && rc > 0u;
+                    n_valid[i] += valid ? 1 : 0;
+                    const float fac = valid ? s_inv[n_valid[i]] : 0.f, delta = f_sub(gain, mean[i]);
+                    mean[i] = f_add(mean[i], f_mul(fac, delta));
+                    m2[i] = f_add(m2[i], f_mul(f_mul(valid ? 1.f : 0.f, delta), f_sub(gain, mean[i])));
+                }
+            }
+        }
+        __syncthreads();                 // the next cells are complete, these are zero
+    }
+    if (warp >= live) return;
+
+    // ---- score of every threshold under the global min_samples_leaf mask; the best of the node: largest score,
+    //      then largest left count, then the last ----
+    const int64_t total = a.frontier[node0 + warp].count;
+    float bs = -INFINITY;
+    uint32_t bc = 0u, mine = 0u;         // bit i of `mine`: bin lane * BPL + i is a threshold
+    int bb = -1;                         // bin of the best threshold
+    long long bg = 0ll;
+    bool nan = false;
+#pragma unroll
+    for (int i = 0; i < BPL; ++i) {
+        const int bin = lane * BPL + i;
+        if (bin >= nb - 1 || !s_set[bin]) continue;
+        mine |= 1u << i;
+        const float ws0 = (float)n_valid[i], ws = ws0 < 1e-12f ? 1e-12f : ws0;
+        float var = f_div(m2[i], ws);
+        if (var < 0.f) var = 0.f;        // NaN stays NaN
+        float sc = f_sub(mean[i], f_mul(a.lambda_dro, __fsqrt_rn(var)));
+        const int64_t lc = lc_sum[i];
+        if (!(lc >= a.min_samples_leaf && total - lc >= a.min_samples_leaf)) sc = -INFINITY;
+        if (sc != sc) {
+            nan = true;
+        } else if (bb < 0 || sc > bs || (sc == bs && lc_sum[i] >= bc)) {
+            bs = sc;
+            bc = lc_sum[i];
+            bb = bin;
+            bg = lg_sum[i];
+        }
+    }
+    nan = __any_sync(0xFFFFFFFFu, nan);
+    for (int d = 16; d > 0; d >>= 1) {
+        const float os = __shfl_xor_sync(0xFFFFFFFFu, bs, d);
+        const uint32_t oc = __shfl_xor_sync(0xFFFFFFFFu, bc, d);
+        const int ob = __shfl_xor_sync(0xFFFFFFFFu, bb, d);
+        const long long og = __shfl_xor_sync(0xFFFFFFFFu, bg, d);
+        if (ob >= 0 && (bb < 0 || os > bs || (os == bs && (oc > bc || (oc == bc && ob > bb))))) {
+            bs = os;
+            bc = oc;
+            bb = ob;
+            bg = og;
+        }
+    }
+    const int upto = bb - lane * BPL;    // this lane's bins below the best
+    const uint32_t below = upto <= 0 ? 0u : (upto >= BPL ? mine : mine & ((1u << upto) - 1u));
+    const int k = __reduce_add_sync(0xFFFFFFFFu, __popc(below));
+    if (lane == 0) {
+        Cand out;
+        out.score = bs;
+        out.k = bb >= 0 ? k : -1;
+        out.left_count = bb >= 0 ? bc : 0u;
+        out.flags = (nan ? 1u : 0u) | ((uint32_t)(bb >= 0 ? bb : 0) << 8);
+        out.left_gq = bb >= 0 ? (int64_t)bg : 0ll;
+        a.cand[(size_t)a.feat_pos[f] * a.node_stride + node0 + warp] = out;
+    }
+}
+
+template <int BPL, int WARPS>
+int launch_nodes(const WalkLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    PB_CUDA_TRY(cudaFuncSetAttribute(walk_nodes_kernel<BPL, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    walk_nodes_kernel<BPL, WARPS><<<grid, 32 * WARPS, smem, stream>>>(a);
+    return PB_OK;
+}
+
+template <int BPL, int MODE, int COPIES, int WARPS>
 int launch_one(const WalkLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
     if (smem > 40 * 1024)   // (beside the static arrays)
-        PB_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<BPL, MODE, COPIES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    walk_kernel<BPL, MODE, COPIES><<<grid, kWalkThreads, smem, stream>>>(a);
+        PB_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<BPL, MODE, COPIES, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    walk_kernel<BPL, MODE, COPIES, WARPS><<<grid, 32 * WARPS, smem, stream>>>(a);
     return PB_OK;
 }
 
 template <int BPL>
-int launch_bpl(const WalkLaunch& a, int mode, int copies, dim3 grid, size_t smem, cudaStream_t stream) {
-    if (mode == kUnit) return copies == 2 ? launch_one<BPL, kUnit, 2>(a, grid, smem, stream) : launch_one<BPL, kUnit, 1>(a, grid, smem, stream);
-    return mode == kUnitTiles ? launch_one<BPL, kUnitTiles, 1>(a, grid, smem, stream) : launch_one<BPL, kGeneral, 1>(a, grid, smem, stream);
+int launch_bpl(const WalkLaunch& a, int mode, int copies, int warps, bool own, dim3 grid, size_t smem, cudaStream_t stream) {
+    constexpr int B = BPL <= 4 ? BPL : 4;
+    if (own)
+        return warps == 32 ? launch_nodes<B, 32>(a, grid, smem, stream) : launch_nodes<B, 16>(a, grid, smem, stream);
+    if (BPL <= 4 && mode == kUnit && warps == 32) {
+        return copies == 2 ? launch_one<B, kUnit, 2, 32>(a, grid, smem, stream) : launch_one<B, kUnit, 1, 32>(a, grid, smem, stream);
+    }
+    if (mode == kUnit) return copies == 2 ? launch_one<BPL, kUnit, 2, 16>(a, grid, smem, stream) : launch_one<BPL, kUnit, 1, 16>(a, grid, smem, stream);
+    return mode == kUnitTiles ? launch_one<BPL, kUnitTiles, 1, 16>(a, grid, smem, stream) : launch_one<BPL, kGeneral, 1, 16>(a, grid, smem, stream);
 }
 
 }  // namespace
 
 // How a launch is laid out.
 struct WalkShape {
-    int bpl, mode, copies, groups;
+    int bpl, mode, copies, warps, groups;
+    bool own;            // a warp per node (walk_nodes_kernel)
     bool div_table;
     size_t smem;
 };
@@ -576,55 +818,72 @@ struct WalkShape {
 static WalkShape walk_shape(WalkLaunch& a) {
     WalkShape s;
     s.bpl = a.max_bins <= 32 ? 1 : a.max_bins <= 64 ? 2 : a.max_bins <= 128 ? 4 : 8;
-    // Nodes of a CTA: sixteen, fewer while the CTAs do not fill the GPU (two per SM): the scan and the
-    // recursion of an era are then spread over more SMs, each of which goes through the rows of the
-    // feature.  That pays up to about 320 rows per era and node of the CTA (20 000 rows, 64 features, 20
-    // eras, 16 nodes: 57 -> 28 us; 200 000 rows, 100 features, 40 eras: 16 nodes 152 -> 135, 8 nodes 97 -> 110).
-    a.cell_nodes = a.n_nodes < kWalkNodes ? a.n_nodes : kWalkNodes;
-    while (a.cell_nodes > 1 && (int64_t)a.n_feat * (a.n_nodes / a.cell_nodes) * 2 <= 148 * 2 &&
-           a.n_rows <= (int64_t)320 * a.cell_nodes * a.n_eras)
-        a.cell_nodes /= 2;
-    s.groups = (a.n_nodes + a.cell_nodes - 1) / a.cell_nodes;
     const bool unit = a.era_alpha <= 0.f && a.direction_weight == 0.f && a.n_eras < kWalkInv;
     s.mode = !unit ? kGeneral : a.max_era_rows <= a.tile_rows ? kUnit : kUnitTiles;
-    const size_t plane = (size_t)kWalkNodes * 32 * s.bpl * 4;
+    // Thirty-two warps when the SM has one CTA at a time anyway, or when there are nodes for all of them: each
+    // warp of walk_nodes_kernel owns one, and half as many CTAs go through the rows.  (200 000 rows, 100 features,
+    // 40 eras, 1 / 8 nodes: 57 / 96 us with sixteen warps, 53 / 83 with thirty-two; 131 071 x 97, 53 eras 47 / 80
+    // and 40 / 63; 32 nodes as two CTAs of sixteen or one of thirty-two: 161 and 126, 109 and 92.)
+    // Sixteen nodes: a warp each, from about a hundred rows per era and node on (below, more and smaller CTAs).
+    const bool batched = s.mode == kUnit && s.bpl <= 4;
+    const int64_t per_node = (int64_t)a.n_nodes * a.n_eras;
+    const bool own = batched && (a.n_nodes >= 32 || (a.n_nodes == 16 && a.n_rows >= 100 * per_node));
+    s.warps = batched && (a.n_nodes >= 32 || (!own && a.n_feat <= 148 && a.n_rows >= 150 * per_node)) ? 32 : 16;
+    // Nodes of a CTA otherwise: fewer while the CTAs do not fill the GPU: the scan and the recursion of an era
+    // are then spread over more SMs, each of which goes through the rows of the feature.  That pays up to about
+    // 320 rows per era and node of the CTA (20 000 rows, 64 features, 20 eras, 16 nodes: 57 -> 28 us; 200 000
+    // rows, 100 features, 40 eras: 16 nodes 152 -> 135, 8 nodes 97 -> 110).
+    a.cell_nodes = a.n_nodes < s.warps ? a.n_nodes : s.warps;
+    const int64_t places = s.warps == 32 ? 148 : 148 * 2;
+    while (!own && a.cell_nodes > 1 && (int64_t)a.n_feat * (a.n_nodes / a.cell_nodes) * 2 <= places &&
+           a.n_rows <= (int64_t)320 * a.cell_nodes * a.n_eras)
+        a.cell_nodes /= 2;
+    s.own = own;
+    s.groups = (a.n_nodes + a.cell_nodes - 1) / a.cell_nodes;
+    const size_t plane = (size_t)s.warps * 32 * s.bpl * 4, trash = (size_t)32 * s.bpl * 4;
     // Two copies of the cells while few nodes share the rows of a warp: its lanes then meet in the bins of
     // a column of few values, which took twice as long as the others.  With many nodes they meet less and
     // the copies only lengthen the scan (500 000 rows, 256 features: 8 nodes 401 us with copies, 454
     // without, 16 nodes 594 either way, 32 nodes 1 125 and 965).
     s.copies = (s.mode == kUnit && s.bpl <= 4 && a.n_nodes <= 8) ? 2 : 1;
-    s.smem = (2 * s.copies + 2) * plane + (s.mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
-    // the table of divisors is 8 bytes per row of the largest era: while it leaves room for two CTAs per SM
-    s.div_table = a.max_era_rows <= a.tile_rows && s.smem + (size_t)(a.max_era_rows + 1) * 8 <= 110 * 1024;
+    s.smem = 2 * s.copies * (plane + trash) + 2 * plane + (s.mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
+    if (s.own)   // (walk_nodes_kernel)
+        s.smem = 8 * (plane + trash) + (size_t)(a.n_eras + 2) / 2 * 8;
+    // the table of divisors is 8 bytes per row of the largest era: while it leaves room for the SM's CTAs
+    s.div_table = a.max_era_rows <= a.tile_rows && s.smem + (size_t)(a.max_era_rows + 1) * 8 <= (s.warps == 32 ? 220 : 110) * 1024;
     if (s.div_table) s.smem += (size_t)(a.max_era_rows + 1) * 8;
     return s;
 }
 
 // A CTA goes through all rows of its feature and all eras, whatever the other SMs do, so a launch takes
-// that chain once per wave of CTAs; two CTAs on an SM take 1.29 times as long as one.  Constants fitted
-// to 9 000 timed depths (2 000 to 4 million rows, 4 to 420 features, 1 to 600 eras, 17 to 256 bins, 1 to
-// 512 nodes, every form of the score); half of the estimates are within 13 %.
+// that chain once per wave of CTAs; two CTAs on an SM take 1.29 times as long as one (1.7 where each warp owns a
+// node).  Constants of the batched form with sixteen warps fitted to 9 000 timed depths (2 000 to 4 million
+// rows, 4 to 420 features, 1 to 600 eras, 17 to 256 bins, 1 to 512 nodes, every form of the score); half of the
+// estimates were within 13 %.  Those of thirty-two warps and of walk_nodes_kernel from 131 071 to 500 000 rows,
+// 95 to 256 features, 40 to 100 eras, 63 to 128 bins and 1 to 512 nodes, all within 15 %.
 double walk_estimate_us(WalkLaunch a) {
     const WalkShape s = walk_shape(a);
     const int64_t tiles = a.max_era_rows <= a.tile_rows ? 1 : (a.max_era_rows + a.tile_rows - 1) / a.tile_rows;
-    const int eras = s.mode == kUnit ? kWalkNodes / a.cell_nodes : 1;   // of a batch
+    const int eras = s.mode == kUnit ? s.warps / a.cell_nodes : 1;   // of a batch
     const double batches = s.mode == kUnit ? (double)((a.n_eras + eras - 1) / eras) : (double)a.n_eras * tiles;
-    const double batch = s.mode == kUnit ? 1.2 + 0.34 * s.bpl : s.mode == kUnitTiles ? 0.63 + 0.14 * s.bpl
+    const double batch = s.own ? (s.warps == 32 ? 0.41 : 0.23) * s.bpl : s.mode == kUnit ? (s.warps == 32 ? 0.75 * s.bpl : 1.2 + 0.34 * s.bpl)
+                         : s.mode == kUnitTiles ? 0.63 + 0.14 * s.bpl
                          : 1.0 + ((a.direction_weight != 0.f && tiles == 1) ? 0.33 : 0.22) * s.bpl;
-    const double chain = 2.9e-4 * a.n_rows + batches * batch;
-    const int per_sm = (s.bpl <= 4 && s.mode != kGeneral) ? 2 : 1;
+    const double per_row = s.own ? 3.0e-4 : s.warps == 32 ? 2.05e-4 : 2.9e-4;
+    const double chain = per_row * a.n_rows + batches * batch;
+    const int per_sm = (s.bpl <= 4 && s.mode != kGeneral && s.warps == 16) ? 2 : 1;
     const int64_t ctas = (int64_t)a.n_feat * s.groups, places = 148 * per_sm;
-    const double whole = per_sm == 2 ? 1.29 : 1.0;
+    const double whole = per_sm == 2 ? (s.own ? 1.7 : 1.29) : 1.0;
     const int64_t rest = ctas % places;
     const double waves = (double)(ctas / places) * whole + (rest == 0 ? 0.0 : rest <= 148 ? 1.0 : whole);
-    return 22.0 + waves * chain + (a.mass ? 16.0 + 7.5e-7 * (double)a.n_rows * a.n_feat : 0.0);
+    return (s.warps == 32 || s.own ? 11.0 : 22.0) + waves * chain + (a.mass ? 16.0 + 7.5e-7 * (double)a.n_rows * a.n_feat : 0.0);
 }
 
 int launch_walk(WalkLaunch a, cudaStream_t stream) {
     if (a.n_feat <= 0 || a.n_nodes <= 0) return PB_OK;
     if (a.max_bins > 256) return fail_arg("max_bins=%d outside [2,256]", a.max_bins);
     const WalkShape s = walk_shape(a);
-    const int bpl = s.bpl, mode = s.mode, copies = s.copies;
+    const int bpl = s.bpl, mode = s.mode, copies = s.copies, warps = s.warps;
     const size_t smem = s.smem;
     a.div_table = s.div_table ? 1 : 0;
     dim3 grid((unsigned)s.groups, (unsigned)a.n_feat);
@@ -639,9 +898,9 @@ int launch_walk(WalkLaunch a, cudaStream_t stream) {
         mass_count_kernel<<<dim3((unsigned)a.n_feat, (unsigned)parts), 256, 0, stream>>>(a);
         count_launch(1);
     }
-    int rc = bpl == 1 ? launch_bpl<1>(a, mode, copies, grid, smem, stream)
-             : bpl == 2 ? launch_bpl<2>(a, mode, copies, grid, smem, stream)
-             : bpl == 4 ? launch_bpl<4>(a, mode, copies, grid, smem, stream) : launch_bpl<8>(a, mode, copies, grid, smem, stream);
+    int rc = bpl == 1 ? launch_bpl<1>(a, mode, copies, warps, s.own, grid, smem, stream)
+             : bpl == 2 ? launch_bpl<2>(a, mode, copies, warps, s.own, grid, smem, stream)
+             : bpl == 4 ? launch_bpl<4>(a, mode, copies, warps, s.own, grid, smem, stream) : launch_bpl<8>(a, mode, copies, warps, s.own, grid, smem, stream);
     prof_end(a.prof, kProfHist, stream);
     if (rc) return rc;
     count_launch(1);

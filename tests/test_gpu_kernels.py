@@ -510,6 +510,18 @@ np.savez(out, preds=b.train_predictions().view(np.int32), **{k: v.view(np.int32)
         np.testing.assert_array_equal(got[0][key], got[1][key], err_msg=key)
 
 
+@pytest.mark.parametrize("n,f,eras,bins,depth,extra", [
+    (4_801, 3, 3, 128, 6, {}),                       # a node per warp from sixteen nodes on, thirty-two warps before
+    (1_701, 150, 1, 65, 6, {}), (3_333, 4, 2, 17, 8, {}),   # one and two eras; groups of nodes, most rows another's
+    (5_003, 33, 7, 64, 8, {}), (2_600, 9, 37, 33, 6, {}),   # eras that start and end anywhere in a warp's rows
+    (2_403, 3, 3, 128, 6, dict(y_scale=1e15)),       # sums past the range of the division table
+    (2_403, 3, 3, 100, 6, dict(k_cuts=9, cut_selection="mass")), (2_403, 3, 3, 100, 6, dict(lambda_l2=1e-9))])
+def test_era_walk_with_a_warp_per_node(n, f, eras, bins, depth, extra, tmp_path):
+    """The same comparison at the sizes where the walk changes its form: the number of warps, a warp per
+    node, nodes in groups, the division table left out."""
+    test_era_walk_equals_the_stored_histogram_path(n, f, eras, bins, depth, extra, tmp_path)
+
+
 @pytest.mark.parametrize("form", ["frontier", "helper"])
 @pytest.mark.parametrize("n,eras,bins", [(3_000, 7, 5), (20_000, 1, 5), (17_000, 2, 4), (6_000, 9, 14)])
 def test_directional_term_streamed_with_the_gains_matches_the_oracle(form, n, eras, bins, monkeypatch):
