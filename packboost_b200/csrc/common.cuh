@@ -282,7 +282,7 @@ struct WalkLaunch {
     int cell_nodes, div_table;   // set by launch_walk
 };
 int launch_walk(WalkLaunch a, cudaStream_t stream);
-double walk_estimate_us(WalkLaunch a);   // about what launch_walk(a) takes
+double walk_estimate_us(const WalkLaunch& a);   // about what launch_walk(a) takes
 size_t score_scratch_bytes_per_feature(int node_stride, int n_eras, int n_thr);
 
 }  // namespace pb

@@ -746,8 +746,9 @@ static double two_step_estimate_us(const pb_train_state* st, int64_t depth, int6
 // walk / other path): 500 000 rows x 200 features, 100 eras 2.2 / 3.8 ms; 131 072 x 200, 574 eras 6.3 / 20.8;
 // 262 144 x 64, 20 eras 0.73 / 0.78; 1 000 000 x 64, 100 eras 2.9 / 2.4; 4 000 000 x 32, 20 eras 10.5 / 2.4.
 // The estimates decide by depth: over the 9 000 depths that they were first fitted to that took 3 % more time
-// than the better path each time, where the walk everywhere took 50 % more.  Where they come within a tenth it
-// is the walk, whose estimate is the safer one in deep frontiers of few rows.
+// than the better path each time, where the walk everywhere took 50 % more.  Where they come within a tenth at
+// sixteen nodes or more it is the walk, whose estimate is the safer one in deep frontiers of few rows; above,
+// the other path's is the one too high (262 144 x 16, 100 eras, one node: 73 us for 44, the walk's 77 for 68).
 // PACKBOOST_WALK=0 / 1 takes one path everywhere, for comparisons.
 struct DepthPath {
     size_t cand_bytes;   // of the candidate table, at the start of the workspace
@@ -773,7 +774,7 @@ static int depth_path(const pb_train_state* st, int64_t depth, const int32_t* fe
         char* ws = static_cast<char*>(st->workspace);
         p->w = walk_launch_of(st, depth, feat_rows, feat_pos, n_feat, ws + p->cand_bytes, reinterpret_cast<Cand*>(ws));
         // (a workspace may hold no feature of histogram and gains at this depth: then the walk is the only way)
-        if (forced < 0 && planned) p->walk = walk_estimate_us(p->w) <= 1.1 * two_step_estimate_us(st, depth, n_feat, p->plan);
+        if (forced < 0 && planned) p->walk = walk_estimate_us(p->w) <= (depth >= 4 ? 1.1 : 1.0) * two_step_estimate_us(st, depth, n_feat, p->plan);
     }
     PB_REQUIRE(p->walk || planned, "workspace too small for one feature of histogram at depth %lld", (long long)depth);
     return PB_OK;

@@ -809,46 +809,49 @@ int launch_bpl(const WalkLaunch& a, int mode, int copies, int warps, bool own, d
 
 // How a launch is laid out.
 struct WalkShape {
-    int bpl, mode, copies, warps, groups;
+    int bpl, mode, copies, warps, cell_nodes, groups;
     bool own;            // a warp per node (walk_nodes_kernel)
     bool div_table;
     size_t smem;
 };
 
-static WalkShape walk_shape(WalkLaunch& a) {
+// The forms a launch may take: batches of sixteen or thirty-two warps, a warp per node of either.
+enum WalkForm { kBatch16 = 0, kBatch32 = 1, kNodes16 = 2, kNodes32 = 3, kWalkForms = 4 };
+
+static bool walk_takes(const WalkLaunch& a, int form) {
+    if (form == kBatch16) return true;
+    const bool unit = a.era_alpha <= 0.f && a.direction_weight == 0.f && a.n_eras < kWalkInv && a.max_era_rows <= a.tile_rows;
+    if (!unit || a.max_bins > 128) return false;
+    // (a warp per node of sixteen: from about a hundred rows per era and node on; 20 000 rows, 64 features, 20
+    // eras take 40 us that way and 35 as more and smaller CTAs)
+    return form == kBatch32 || (form == kNodes16 ? a.n_nodes == 16 && a.n_rows >= (int64_t)1600 * a.n_eras : a.n_nodes >= 32);
+}
+
+static WalkShape walk_shape(const WalkLaunch& a, int form) {
     WalkShape s;
     s.bpl = a.max_bins <= 32 ? 1 : a.max_bins <= 64 ? 2 : a.max_bins <= 128 ? 4 : 8;
     const bool unit = a.era_alpha <= 0.f && a.direction_weight == 0.f && a.n_eras < kWalkInv;
     s.mode = !unit ? kGeneral : a.max_era_rows <= a.tile_rows ? kUnit : kUnitTiles;
-    // Thirty-two warps when the SM has one CTA at a time anyway, or when there are nodes for all of them: each
-    // warp of walk_nodes_kernel owns one, and half as many CTAs go through the rows.  (200 000 rows, 100 features,
-    // 40 eras, 1 / 8 nodes: 57 / 96 us with sixteen warps, 53 / 83 with thirty-two; 131 071 x 97, 53 eras 47 / 80
-    // and 40 / 63; 32 nodes as two CTAs of sixteen or one of thirty-two: 161 and 126, 109 and 92.)
-    // Sixteen nodes: a warp each, from about a hundred rows per era and node on (below, more and smaller CTAs).
-    const bool batched = s.mode == kUnit && s.bpl <= 4;
-    const int64_t per_node = (int64_t)a.n_nodes * a.n_eras;
-    const bool own = batched && (a.n_nodes >= 32 || (a.n_nodes == 16 && a.n_rows >= 100 * per_node));
-    s.warps = batched && (a.n_nodes >= 32 || (!own && a.n_feat <= 148 && a.n_rows >= 150 * per_node)) ? 32 : 16;
-    // Nodes of a CTA otherwise: fewer while the CTAs do not fill the GPU: the scan and the recursion of an era
-    // are then spread over more SMs, each of which goes through the rows of the feature.  That pays up to about
+    s.warps = form == kBatch32 || form == kNodes32 ? 32 : 16;
+    s.own = form == kNodes16 || form == kNodes32;
+    // Nodes of a batched CTA: fewer while the CTAs do not fill the GPU: the scan and the recursion of an era are
+    // then spread over more SMs, each of which goes through the rows of the feature.  That pays up to about
     // 320 rows per era and node of the CTA (20 000 rows, 64 features, 20 eras, 16 nodes: 57 -> 28 us; 200 000
     // rows, 100 features, 40 eras: 16 nodes 152 -> 135, 8 nodes 97 -> 110).
-    a.cell_nodes = a.n_nodes < s.warps ? a.n_nodes : s.warps;
+    s.cell_nodes = a.n_nodes < s.warps ? a.n_nodes : s.warps;
     const int64_t places = s.warps == 32 ? 148 : 148 * 2;
-    while (!own && a.cell_nodes > 1 && (int64_t)a.n_feat * (a.n_nodes / a.cell_nodes) * 2 <= places &&
-           a.n_rows <= (int64_t)320 * a.cell_nodes * a.n_eras)
-        a.cell_nodes /= 2;
-    s.own = own;
-    s.groups = (a.n_nodes + a.cell_nodes - 1) / a.cell_nodes;
+    while (!s.own && s.cell_nodes > 1 && (int64_t)a.n_feat * (a.n_nodes / s.cell_nodes) * 2 <= places &&
+           a.n_rows <= (int64_t)320 * s.cell_nodes * a.n_eras)
+        s.cell_nodes /= 2;
+    s.groups = (a.n_nodes + s.cell_nodes - 1) / s.cell_nodes;
     const size_t plane = (size_t)s.warps * 32 * s.bpl * 4, trash = (size_t)32 * s.bpl * 4;
     // Two copies of the cells while few nodes share the rows of a warp: its lanes then meet in the bins of
     // a column of few values, which took twice as long as the others.  With many nodes they meet less and
     // the copies only lengthen the scan (500 000 rows, 256 features: 8 nodes 401 us with copies, 454
     // without, 16 nodes 594 either way, 32 nodes 1 125 and 965).
     s.copies = (s.mode == kUnit && s.bpl <= 4 && a.n_nodes <= 8) ? 2 : 1;
-    s.smem = 2 * s.copies * (plane + trash) + 2 * plane + (s.mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
-    if (s.own)   // (walk_nodes_kernel)
-        s.smem = 8 * (plane + trash) + (size_t)(a.n_eras + 2) / 2 * 8;
+    s.smem = s.own ? 8 * (plane + trash) + (size_t)(a.n_eras + 2) / 2 * 8
+                   : 2 * s.copies * (plane + trash) + 2 * plane + (s.mode == kGeneral ? plane : (size_t)(a.n_eras + 2) / 2 * 8);
     // the table of divisors is 8 bytes per row of the largest era: while it leaves room for the SM's CTAs
     s.div_table = a.max_era_rows <= a.tile_rows && s.smem + (size_t)(a.max_era_rows + 1) * 8 <= (s.warps == 32 ? 220 : 110) * 1024;
     if (s.div_table) s.smem += (size_t)(a.max_era_rows + 1) * 8;
@@ -859,14 +862,13 @@ static WalkShape walk_shape(WalkLaunch& a) {
 // that chain once per wave of CTAs; two CTAs on an SM take 1.29 times as long as one (1.7 where each warp owns a
 // node).  Constants of the batched form with sixteen warps fitted to 9 000 timed depths (2 000 to 4 million
 // rows, 4 to 420 features, 1 to 600 eras, 17 to 256 bins, 1 to 512 nodes, every form of the score); half of the
-// estimates were within 13 %.  Those of thirty-two warps and of walk_nodes_kernel from 131 071 to 500 000 rows,
-// 95 to 256 features, 40 to 100 eras, 63 to 128 bins and 1 to 512 nodes, all within 15 %.
-double walk_estimate_us(WalkLaunch a) {
-    const WalkShape s = walk_shape(a);
+// estimates were within 13 %.  Those of the other forms from 60 000 to 1 million rows, 8 to 256 features, 20 to
+// 574 eras, 63 to 128 bins and 1 to 512 nodes: within 15 %, but for one node over many short eras (121 us, not 92).
+static double walk_estimate_us(const WalkLaunch& a, const WalkShape& s) {
     const int64_t tiles = a.max_era_rows <= a.tile_rows ? 1 : (a.max_era_rows + a.tile_rows - 1) / a.tile_rows;
-    const int eras = s.mode == kUnit ? s.warps / a.cell_nodes : 1;   // of a batch
+    const int eras = s.mode == kUnit ? s.warps / s.cell_nodes : 1;   // of a batch
     const double batches = s.mode == kUnit ? (double)((a.n_eras + eras - 1) / eras) : (double)a.n_eras * tiles;
-    const double batch = s.own ? (s.warps == 32 ? 0.41 : 0.23) * s.bpl : s.mode == kUnit ? (s.warps == 32 ? 0.75 * s.bpl : 1.2 + 0.34 * s.bpl)
+    const double batch = s.own ? (s.warps == 32 ? 0.41 : 0.23) * s.bpl : s.mode == kUnit ? (s.warps == 32 ? 1.0 + 0.65 * s.bpl : 1.2 + 0.34 * s.bpl)
                          : s.mode == kUnitTiles ? 0.63 + 0.14 * s.bpl
                          : 1.0 + ((a.direction_weight != 0.f && tiles == 1) ? 0.33 : 0.22) * s.bpl;
     const double per_row = s.own ? 3.0e-4 : s.warps == 32 ? 2.05e-4 : 2.9e-4;
@@ -879,10 +881,35 @@ double walk_estimate_us(WalkLaunch a) {
     return (s.warps == 32 || s.own ? 11.0 : 22.0) + waves * chain + (a.mass ? 16.0 + 7.5e-7 * (double)a.n_rows * a.n_feat : 0.0);
 }
 
+// The form with the least estimate.  (Measured, batches of sixteen / of thirty-two / a warp per node: 200 000
+// rows, 100 features, 40 eras, 128 bins 57 / 53 us at one node, 96 / 83 at eight, 135 / 142 / 107 at sixteen,
+// - / 207 / 126 at thirty-two; 500 000 x 256, 100 eras 215 / 236 at one, - / 552 / 414 at sixteen; 131 072 x 8,
+// 574 eras, 32 nodes 1 120 with a warp per node, where more and smaller CTAs take a fifth of that.)
+static double best_walk(const WalkLaunch& a, WalkShape* best) {
+    double us = 1e300;
+    for (int form = 0; form < kWalkForms; ++form) {
+        if (!walk_takes(a, form)) continue;
+        const WalkShape s = walk_shape(a, form);
+        const double e = walk_estimate_us(a, s);
+        if (e < us) {
+            us = e;
+            *best = s;
+        }
+    }
+    return us;
+}
+
+double walk_estimate_us(const WalkLaunch& a) {
+    WalkShape s;
+    return best_walk(a, &s);
+}
+
 int launch_walk(WalkLaunch a, cudaStream_t stream) {
     if (a.n_feat <= 0 || a.n_nodes <= 0) return PB_OK;
     if (a.max_bins > 256) return fail_arg("max_bins=%d outside [2,256]", a.max_bins);
-    const WalkShape s = walk_shape(a);
+    WalkShape s;
+    best_walk(a, &s);
+    a.cell_nodes = s.cell_nodes;
     const int bpl = s.bpl, mode = s.mode, copies = s.copies, warps = s.warps;
     const size_t smem = s.smem;
     a.div_table = s.div_table ? 1 : 0;
