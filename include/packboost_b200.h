@@ -193,8 +193,8 @@ typedef struct pb_train_state {
  * a violation is recorded in a sticky word of the control block and the offending index is skipped
  * - nothing traps.  pb_debug_flags copies that word to the host (it synchronises the device):
  * bit 0 slot out of range, bit 1 bin code >= max_bins, bit 2 feature id out of range.  In a regular
- * build the checks are compiled out and the word stays 0; pb_debug_bounds_enabled says which build
- * this is. */
+ * build the checks are compiled out; pb_debug_bounds_enabled says which build this is.  Bit 3 may be
+ * set by any build: a wait inside a kernel ran into its limit.  pb_tree_from_log refuses such a round. */
 int pb_debug_bounds_enabled(void);
 int pb_debug_flags(const pb_train_state* st, uint32_t* flags_out);
 
@@ -382,7 +382,8 @@ typedef struct pb_round_log_header {
     int64_t root_gq;
     int32_t n_ctx[PB_MAX_DEPTH + 1]; /* frontier nodes per depth; winners of depth d start at (1<<d)-1 */
     int32_t n_tree_nodes;
-    int32_t reserved[2];
+    int32_t faults;       /* not 0: a bounded wait of a kernel ran out, the round is not to be used */
+    int32_t reserved;
 } pb_round_log_header;
 /* The log is a pb_round_log_header followed by (1 << max_depth) - 1 pb_winner records. */
 

@@ -213,9 +213,9 @@ _WINNER_DT = np.dtype({
     "itemsize": 80,
 })
 _HEADER_DT = np.dtype({
-    "names": ["root_value", "scale", "max_abs_grad", "root_gq", "n_ctx", "n_tree_nodes"],
-    "formats": ["<f8", "<f4", "<f4", "<i8", ("<i4", (B.PB_MAX_DEPTH + 1,)), "<i4"],
-    "offsets": [0, 8, 12, 16, 24, 24 + 4 * (B.PB_MAX_DEPTH + 1)],
+    "names": ["root_value", "scale", "max_abs_grad", "root_gq", "n_ctx", "n_tree_nodes", "faults"],
+    "formats": ["<f8", "<f4", "<f4", "<i8", ("<i4", (B.PB_MAX_DEPTH + 1,)), "<i4", "<i4"],
+    "offsets": [0, 8, 12, 16, 24, 24 + 4 * (B.PB_MAX_DEPTH + 1), 28 + 4 * (B.PB_MAX_DEPTH + 1)],
     "itemsize": 88,
 })
 

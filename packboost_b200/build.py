@@ -17,11 +17,11 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_NAME = "libpackboost_b200.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
 
-SOURCES = ["api.cu", "hist.cu", "score.cu", "walk.cu", "frontier.cu", "pack.cu", "predict.cu", "metrics.cu", "upload.cu", "loop.cu", "comm.cu"]
+SOURCES = ["api.cu", "hist.cu", "hist_mma.cu", "score.cu", "walk.cu", "frontier.cu", "pack.cu", "predict.cu", "metrics.cu", "upload.cu", "loop.cu", "comm.cu"]
 # The scorer, and the histogram kernel whose flush computes the per-era gains, must round every
 # product and sum separately (no fused multiply-add) to keep the float32 operation order of the
 # algorithm they implement.
-EXTRA = {"score.cu": ["-fmad=false"], "hist.cu": ["-fmad=false"], "walk.cu": ["-fmad=false"]}
+EXTRA = {"score.cu": ["-fmad=false"], "hist.cu": ["-fmad=false"], "hist_mma.cu": ["-fmad=false"], "walk.cu": ["-fmad=false"]}
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]

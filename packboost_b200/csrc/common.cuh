@@ -114,6 +114,8 @@ struct CtlHead {
 constexpr uint32_t kDbgSlot = 1u;     // a row's frontier slot is neither "none" nor below the frontier's capacity
 constexpr uint32_t kDbgCode = 2u;     // a bin code is >= max_bins
 constexpr uint32_t kDbgFeature = 4u;  // a winner's feature id is outside the data set or not held by this device
+// (every build) a wait inside a kernel ran into its limit: the histograms of the round are not to be used
+constexpr uint32_t kFaultWait = 8u;
 
 // Addresses of the sub-tables inside the caller's control block.
 struct Ctl {
@@ -167,6 +169,7 @@ struct HistLaunch {
     int n_feat;
     const int32_t* gq;
     const uint16_t* slot;
+    int64_t rows_pad;            // entries of gq and slot
     const int32_t* era_offsets;
     int n_eras;
     int max_bins;
@@ -208,6 +211,9 @@ struct HistFuse {
 bool hist_can_fuse(const HistLaunch& h);
 int hist_node_chunks(int n_nodes, int max_bins);
 int launch_hist(const HistLaunch& h, cudaStream_t stream);
+// Few-bin codes on the tensor cores (hist_mma.cu): whether a launch is one of those, and the launch.
+bool hist_mma_takes(const HistLaunch& h);
+int launch_hist_mma(const HistLaunch& h, cudaStream_t stream);
 int hist_max_arity();  // default tuple-size cap of the lane kernel (PACKBOOST_HIST_MAX_ARITY=1 lowers it)
 
 // ---- scorer launch (score.cu) -------------------------------------------------------------

@@ -528,6 +528,7 @@ __global__ void __launch_bounds__(kRowThreads) partition_kernel(PartArgs a) {
 
 __global__ void delta_kernel(Ctl c, int pack_size, float lr) {
     const int n = c.head->n_tree_nodes;
+    if (blockIdx.x == 0 && threadIdx.x == 0) c.log_head->faults = (int32_t)(c.head->debug_flags & kFaultWait);
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const float v = (float)c.node_value[t];
         float acc = 0.f;
@@ -650,6 +651,7 @@ static HistLaunch hist_launch_of(const pb_train_state* st, int64_t depth, const 
     h.n_feat = 1;
     h.gq = st->gq;
     h.slot = st->slot;
+    h.rows_pad = rows_padded(st->n_rows);
     h.era_offsets = st->era_offsets;
     h.n_eras = (int)st->n_eras;
     h.max_bins = (int)st->max_bins;
@@ -1128,6 +1130,7 @@ extern "C" int pb_hist_build(const pb_train_state* st, const int32_t* feat_rows,
     h.n_feat = (int)n_feat;
     h.gq = st->gq;
     h.slot = st->slot;
+    h.rows_pad = rows_padded(st->n_rows);
     h.era_offsets = st->era_offsets;
     h.n_eras = (int)st->n_eras;
     h.max_bins = (int)st->max_bins;

@@ -843,6 +843,7 @@ int hist_node_chunks(int n_nodes, int max_bins) {
 
 int launch_hist(const HistLaunch& h, cudaStream_t stream) {
     if (h.n_feat <= 0 || h.n_nodes <= 0) return PB_OK;
+    if (hist_mma_takes(h)) return launch_hist_mma(h, stream);
     HistKernelArgs a;
     a.codes = h.codes;
     a.pitch = h.pitch;

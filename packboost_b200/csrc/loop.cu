@@ -145,6 +145,7 @@ extern "C" int pb_tree_from_log(const void* log_head, const void* log_winners, i
     PB_REQUIRE(max_depth >= 1 && max_depth <= PB_MAX_DEPTH, "max_depth out of range");
     const pb_round_log_header* h = static_cast<const pb_round_log_header*>(log_head);
     const pb_winner* winners = static_cast<const pb_winner*>(log_winners);
+    if (h->faults != 0) return fail_arg("a wait inside a histogram kernel ran into its limit: the round's sums are not complete");
     const int64_t cap = (2ll << max_depth) - 1;
     auto leaf = [&](int64_t n, double v) {
         feature[n] = -1;

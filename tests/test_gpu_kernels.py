@@ -284,6 +284,71 @@ def test_histogram_exact_in_every_launch_shape(shape):
     assert "hist_lane_kernel<%s>" % shape.replace(" ", ",") in res.stderr, res.stderr[-2000:]
 
 
+_MMA_SCRIPT = """
+import sys
+sys.path.insert(0, {root!r})
+from tests.test_gpu_kernels import _hist_case
+for n, f, e, nb, nodes, big in {cases!r}:
+    _hist_case(n, f, e, nb, nodes, seed=n + nodes, big_era=big)
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("cases", [
+    [(8_161, 2, 1, 5, 1, False), (20_001, 270, 1, 5, 1, False), (33_000, 258, 2, 4, 2, True)],    # four thresholds a lane
+    [(17_000, 262, 1, 5, 4, False), (16_500, 20, 1, 2, 3, False), (40_000, 70, 3, 8, 4, True)],
+    [(20_001, 130, 1, 5, 5, False), (17_000, 24, 1, 6, 16, False), (26_000, 9, 2, 3, 9, True)],   # two
+    [(20_001, 65, 1, 5, 17, False), (17_000, 24, 1, 8, 32, False), (30_000, 8, 2, 5, 33, True), (17_000, 70, 1, 7, 64, False)]])  # one
+def test_histogram_exact_on_the_tensor_cores(cases):
+    """Exact sums of the contraction for eras of several tiles: every number of thresholds a lane holds, either
+    layout of the nodes' columns, more than 256 columns, features past a whole block of lanes, tiles that start
+    and end anywhere.  (The switch that takes it at every size is read once per process.)"""
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", _MMA_SCRIPT.format(root=root, cases=cases)], env=dict(os.environ, PACKBOOST_HIST_MMA="1"),
+                         capture_output=True, text=True, timeout=600)
+    assert res.returncode == 0 and res.stdout.strip().endswith("ok"), res.stdout[-2000:] + res.stderr[-4000:]
+
+
+@pytest.mark.parametrize("n,f,eras,bins,depth,extra", [
+    (6_001, 300, 7, 5, 4, {}), (5_003, 40, 40, 5, 6, {}), (700, 33, 1, 2, 3, {}), (9_000, 70, 200, 8, 6, {}),
+    (6_000, 150, 9, 4, 6, dict(direction_weight=0.3)), (6_000, 35, 11, 5, 5, dict(era_alpha=4.0)),
+    (6_000, 35, 5, 7, 5, dict(k_cuts=3, cut_selection="even")), (20_001, 45, 2, 5, 7, {}), (17_000, 200, 1, 6, 7, {})])
+def test_fit_on_the_tensor_cores_equals_the_one_by_atomics(n, f, eras, bins, depth, extra, tmp_path):
+    """Trees, scores and predictions bit for bit: gains made in the flush, every form of the score, eras shorter
+    than a step of the rows and longer than a tile."""
+    import json
+    import subprocess
+    import sys
+    script = r"""
+import json, sys
+import numpy as np
+from packboost_b200 import PackBoost, PackBoostConfig
+n, f, eras, bins, depth, extra, out = json.loads(sys.argv[1])
+rng = np.random.default_rng(n + f)
+X = rng.integers(0, bins, size=(n, f)).astype(np.uint8)
+y = (X[:, 0] + X[:, 1] * (X[:, 2] > 1) + rng.normal(size=n)).astype(np.float32)
+era = np.sort((rng.random(n) ** 2 * eras).astype(np.int16))
+cfg = dict(pack_size=2, max_depth=depth, learning_rate=0.2, lambda_l2=1.0, lambda_dro=0.4, min_samples_leaf=5, max_bins=bins,
+           random_state=1, prebinned=True)
+cfg.update(extra)
+b = PackBoost(PackBoostConfig(**cfg)).fit(X, y, era, num_rounds=3)
+np.savez(out, preds=b.train_predictions().view(np.int32), **{k: v.view(np.int32) if v.dtype == np.float32 else v for k, v in b.split_records().items()})
+"""
+    got = []
+    for mma in ("1", "0"):
+        path = str(tmp_path / f"{mma}.npz")
+        res = subprocess.run([sys.executable, "-c", script, json.dumps([n, f, eras, bins, depth, extra, path])],
+                             env=dict(os.environ, PACKBOOST_HIST_MMA=mma), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                             capture_output=True, text=True)
+        assert res.returncode == 0, res.stderr[-2000:]
+        got.append(np.load(path))
+    assert len(got[0]["node"]) > 3
+    for key in got[0].files:
+        np.testing.assert_array_equal(got[0][key], got[1][key], err_msg=key)
+
+
 @pytest.mark.parametrize("max_bins,n_nodes", [(96, 64), (12, 512), (191, 32), (47, 128)])
 def test_histogram_whose_cells_take_just_the_shared_memory_given_without_asking(max_bins, n_nodes):
     """48 KB of cells or a little less beside the kernel's own arrays: such a launch has to ask for more

@@ -54,6 +54,15 @@ def test_tree_replay_numbers_children_like_the_reference():
     assert [n.value for n in tree.nodes][2:] == [0.25, -0.3, 0.4]
 
 
+def test_tree_replay_refuses_a_round_whose_kernels_gave_up_waiting():
+    rows = {(0, 0): dict(feature=3, threshold=1, tree_node=0, left_id=1, right_id=2, left_value=0.0, right_value=0.0)}
+    head, win = _log(rows, [1, 0, 0], n_nodes=3)
+    assert len(_tree_from_log(head, win, 3)[0].nodes) == 3
+    head["faults"] = 8
+    with pytest.raises(RuntimeError, match="ran into its limit"):
+        _tree_from_log(head, win, 3)
+
+
 def test_tree_replay_detects_numbering_mismatch():
     rows = {(0, 0): dict(feature=3, threshold=1, tree_node=0, left_id=2, right_id=3, left_value=0.0, right_value=0.0)}
     head, win = _log(rows, [1, 0, 0], n_nodes=3)
