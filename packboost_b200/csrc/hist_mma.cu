@@ -19,8 +19,8 @@
 //            and left sums (summed over the CTA's eras before they go out), or a tile's share of the histogram.
 // Operands pass in batches of 64 or 128 rows through three places, each with code and row warps of its own.
 //
-// Bound: the instructions of all roles together (367 per 32 rows and 128 features, 164 of them permutes and the
-// like; ALU pipe 58 %, issue slots 61 % of the time, tensor pipe 11 % at four nodes).  What it took:
+// Bound: the instructions of all roles together (485 per 32 rows and 128 features at one node, 164 of them for A;
+// ALU pipe 62 %, issue slots 60 %, tensor pipe 16 % of the time).  What it took:
 // the warps of a place wait at one barrier behind one poller (two dozen polling warps made a wait that is over
 // cost 350 cycles), the issuers wait at a barrier too (a ready mbarrier costs a thread that issues tcgen05.mma
 // 200 cycles, a barrier a few), codes come by cp.async from four warps (bulk copies of a line each: 35 cycles
@@ -590,17 +590,17 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         // ---- codes, frontier slots and gradients of a block; eight consecutive threads per line ----
         const int cw = warp - kCopyWarp0;
         constexpr int kMine = (128 / 2 + kCopyWarps - 1) / kCopyWarps;   // features of a half warp at most
-        const uint32_t pitch16 = (uint32_t)(a.pitch / 16);
+        const uint32_t pitch = (uint32_t)a.pitch;    // (of fewer than 2^31 rows)
         const int part = lane & 15;
         int stage = 0;
         uint32_t phase = 1u;
         for (int t = t0; t < t1 && good; ++t) {
             if (!task_at(t, x)) continue;
-            uint32_t from[kMine];                    // in units of 16 bytes
+            uint32_t rows[kMine];
 #pragma unroll
             for (int i = 0; i < kMine; ++i) {
                 const int fl = (i * kCopyWarps + cw) * 2 + (lane >> 4);
-                from[i] = fl < FC ? (uint32_t)a.feat_rows[min(x.fb * FC + fl, a.n_feat - 1)] * pitch16 : 0u;
+                rows[i] = fl < FC ? (uint32_t)a.feat_rows[min(x.fb * FC + fl, a.n_feat - 1)] : 0u;
             }
             for (int b = x.b0; b < x.b1; ++b) {
                 good = warp_wait(empty_c + stage, phase, &s_fail);
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                     const uint32_t mine = to + (uint32_t)((2 * cw + (lane >> 4)) * kPitch + part * 16);
 #pragma unroll
                     for (int i = 0; i < kMine; ++i)
-                        if ((i * kCopyWarps + cw) * 2 < FC) copy16(mine + (uint32_t)(2 * kCopyWarps * i * kPitch), base + (uint64_t)from[i] * 16u);
+                        if ((i * kCopyWarps + cw) * 2 < FC) copy16(mine + (uint32_t)(2 * kCopyWarps * i * kPitch), base + (uint64_t)rows[i] * pitch);
                 }
                 const uint32_t state = to + (uint32_t)(FC * kPitch);
                 const int64_t row0 = (int64_t)b * kBlock;
