@@ -459,7 +459,7 @@ def main():
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "strong",
             "vs_baseline": None, "dtype": "int64", "data": "synthetic", "config": config,
-            "roofline": {"bound": "hbm", "kernel": "hist_lane_kernel (fused flush)", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": "hist_mma_kernel and hist_lane_kernel (fused flush)", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_src,
                          "peak_source": peak_src,
                          "bytes": "input bytes only (packed codes of the sampled columns, row state, era offsets): the "
@@ -502,21 +502,21 @@ def hist_traffic(n_rows, world):
     figure is withheld and the reason is given instead."""
     import hashlib
     import re
-    path = os.path.join(ROOT, "profiles", "hist_lane_kernel_fused_config3_small.md")
-    src = os.path.join(ROOT, "packboost_b200", "csrc", "hist.cu")
+    path = os.path.join(ROOT, "profiles", "hist_kernels_fused_config3.md")
     if not os.path.exists(path):
-        return None, "no ncu summary of the fused kernel is committed"
+        return None, "no ncu summary of the fused kernels is committed"
     text = open(path).read()
     m_bytes = re.search(r"dram_bytes_per_launch:\s*([0-9.eE+]+)", text)
     m_rows = re.search(r"captured_rows:\s*([0-9]+)", text)
-    m_sha = re.search(r"hist_cu_sha256:\s*([0-9a-f]+)", text)
-    if not (m_bytes and m_rows and m_sha):
+    if not (m_bytes and m_rows):
         return None, "the committed ncu summary lacks the traffic fields"
-    now = source_digest(src)
-    if not now.startswith(m_sha.group(1)):
-        return None, "hist.cu has changed since the committed ncu capture: traffic withheld until it is re-captured"
+    for name in ("hist.cu", "hist_mma.cu"):
+        m_sha = re.search(name.replace(".", "_") + r"_sha256:\s*([0-9a-f]+)", text)
+        now = source_digest(os.path.join(ROOT, "packboost_b200", "csrc", name))
+        if not (m_sha and now.startswith(m_sha.group(1))):
+            return None, name + " has changed since the committed ncu capture: traffic withheld until it is re-captured"
     return float(m_bytes.group(1)) * n_rows / float(m_rows.group(1)) / world, \
-        "ncu dram__bytes_read+write of the committed small-case capture of this kernel source, scaled by rows"
+        "ncu dram__bytes_read+write of the committed reduced capture of these kernel sources, scaled by rows"
 
 
 if __name__ == "__main__":
