@@ -36,6 +36,7 @@
 
 #include "common.cuh"
 #include "des_math.cuh"
+#include "rows.cuh"
 
 namespace pb {
 
@@ -85,10 +86,8 @@ __global__ void __launch_bounds__(THREADS) hist_kernel(HistKernelArgs a) {
     const int node_hi = min(n_nodes, node_lo + a.nodes_per_chunk);
     const int era = blockIdx.x / a.tiles_per_era;
     const int tile = blockIdx.x - era * a.tiles_per_era;
-    const int era_begin = a.era_offsets[era];
-    const int era_end = a.era_offsets[era + 1];
-    const int r0 = era_begin + tile * a.tile_rows;
-    const int r1 = min(era_end, r0 + a.tile_rows);
+    int r0, r1;
+    tile_range(a.era_offsets[era], a.era_offsets[era + 1], tile, a.tile_rows, r0, r1);
     if (r0 >= r1 && a.use_atomics) return;  // (without atomics an empty tile still writes its zeros)
 
     const int fa = blockIdx.y * a.feats_per_cta;
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(THREADS) hist_kernel(HistKernelArgs a) {
 
     // ---- row state of this thread's chunk, kept in registers for the whole CTA ----
     const int c = r0 / RPI + threadIdx.x;
-    const bool has = (r0 < r1) && (c * RPI < r1);
+    const bool has = (r0 < r1) && (c < (r1 + RPI - 1) / RPI);
     int32_t g[RPI];
     uint32_t cb2[RPI / 2];  // two 16-bit cell bases per word; 0xFFFF: row not accumulated here
     if (has) {
@@ -293,10 +292,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) hist_lane_kernel(HistKerne
     if (n_nodes <= 0) return;
     const int era = blockIdx.x / a.tiles_per_era;
     const int tile = blockIdx.x - era * a.tiles_per_era;
-    const int era_begin = a.era_offsets[era];
-    const int era_end = a.era_offsets[era + 1];
-    const int r0 = era_begin + tile * a.tile_rows;
-    const int r1 = min(era_end, r0 + a.tile_rows);
+    int r0, r1;
+    tile_range(a.era_offsets[era], a.era_offsets[era + 1], tile, a.tile_rows, r0, r1);
     if (r0 >= r1 && a.use_atomics) return;
 
     const int nb = a.max_bins;
@@ -871,7 +868,7 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
         a.tiles_per_era = 1;
         a.use_atomics = 0;
     } else {
-        a.tiles_per_era = (h.max_era_rows + a.tile_rows - 1) / a.tile_rows;
+        a.tiles_per_era = tiles_of(h.max_era_rows, a.tile_rows);
         a.use_atomics = 1;
     }
     const int max_tile = (h.max_era_rows < a.tile_rows) ? h.max_era_rows : a.tile_rows;
@@ -880,6 +877,7 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
     const int thread_cap = (h.code_bits == 4) ? 256 : 512;
     if (threads > thread_cap) return fail_arg("histogram tile of %d rows exceeds the thread block", max_tile);
 
+    if ((int64_t)a.n_eras * a.tiles_per_era > 0x7FFFFFFF) return fail_arg("histogram of too many tiles");   // (of a grid)
     const size_t out_cells = (size_t)h.n_feat * h.node_stride * h.n_eras * h.max_bins;
     if (a.use_atomics && !h.zeroed) {
         PB_CUDA_TRY(cudaMemsetAsync(h.cnt, 0, out_cells * sizeof(uint32_t), stream));
@@ -934,9 +932,9 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
                             if (a.use_atomics) {
                                 if (w > 0) tiles = (int)(w * slots / ((double)h.n_eras * blocks));
                                 if (tiles < tiles_min) continue;
-                                tile = ((h.max_era_rows + tiles - 1) / tiles + 255) / 256 * 256;
+                                tile = (tiles_of(h.max_era_rows, tiles) + 255) / 256 * 256;
                                 if (tile > kTileRowsMax) tile = kTileRowsMax;
-                                tiles = (h.max_era_rows + tile - 1) / tile;
+                                tiles = tiles_of(h.max_era_rows, tile);
                             }
                             const double tile_scale = (double)(a.use_atomics ? tile : max_tile) / 4700.0;
                             const double ctas = (double)h.n_eras * tiles * blocks;
@@ -966,7 +964,7 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
             }
             if (a.use_atomics) {
                 a.tile_rows = best_tile;
-                a.tiles_per_era = (h.max_era_rows + best_tile - 1) / best_tile;
+                a.tiles_per_era = tiles_of(h.max_era_rows, best_tile);
             }
         }
         if (forced)

@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "des_math.cuh"
+#include "rows.cuh"
 
 namespace pb {
 
@@ -251,9 +252,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         x.fb = t / a.tiles;
         const int et = t - x.fb * a.tiles;
         x.era = et / a.tiles_per_era;
-        const int era_end = a.era_offsets[x.era + 1];
-        x.r0 = a.era_offsets[x.era] + (et - x.era * a.tiles_per_era) * a.tile_rows;
-        x.r1 = min(era_end, x.r0 + a.tile_rows);
+        tile_range(a.era_offsets[x.era], a.era_offsets[x.era + 1], et - x.era * a.tiles_per_era, a.tile_rows, x.r0, x.r1);
         x.b0 = x.r0 / kBlock;
         x.b1 = x.r0 < x.r1 ? (x.r1 + kBlock - 1) / kBlock : x.b0;
         return x.r0 < x.r1 || a.fuse;
@@ -747,12 +746,12 @@ int launch_hist_mma(const HistLaunch& h, cudaStream_t stream) {
     a.tiles_per_era = 1;
     if (h.max_era_rows > kTileRowsMax) {
         // as many tiles as fill whole waves of CTAs
-        const int64_t least = (h.max_era_rows + kMmaTileRows - 1) / kMmaTileRows, per_tile = (int64_t)h.n_eras * blocks;
+        const int64_t least = tiles_of(h.max_era_rows, kMmaTileRows), per_tile = (int64_t)h.n_eras * blocks;
         const int64_t waves = (least * per_tile + 147) / 148;
         int64_t tiles = waves * 148 / per_tile;
         if (tiles < least) tiles = least;
-        a.tile_rows = (int)(((h.max_era_rows + tiles - 1) / tiles + kBlock - 1) / kBlock * kBlock);
-        a.tiles_per_era = (h.max_era_rows + a.tile_rows - 1) / a.tile_rows;
+        a.tile_rows = tiles_of(tiles_of(h.max_era_rows, tiles), kBlock) * kBlock;
+        a.tiles_per_era = tiles_of(h.max_era_rows, a.tile_rows);
         if (!h.zeroed) {
             const size_t cells = (size_t)h.n_feat * h.node_stride * h.n_eras * h.max_bins;
             PB_CUDA_TRY(cudaMemsetAsync(h.cnt, 0, cells * sizeof(uint32_t), stream));

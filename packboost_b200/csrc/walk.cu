@@ -35,6 +35,7 @@
 #include "common.cuh"
 #include "des_math.cuh"
 #include "divide.cuh"
+#include "rows.cuh"
 
 namespace pb {
 
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(32 * WARPS, (BPL <= 4 && MODE != kGeneral && W
     auto batch_end = [&]() {
         ne = min(EB, E - e0);
         const int end = ne > 0 ? a.era_offsets[e0 + ne] : r0;
-        r1 = TILES ? min(end, r0 + a.tile_rows) : end;
+        r1 = TILES && end - r0 > a.tile_rows ? r0 + a.tile_rows : end;
         return TILES ? r1 >= end : true;                     // the batch completes its eras
     };
     bool complete = batch_end();
@@ -333,11 +334,12 @@ __global__ void __launch_bounds__(32 * WARPS, (BPL <= 4 && MODE != kGeneral && W
         // ---- (a) ----
         {
             int e = 0, lim = s_off[1], chunk = r0 / 128 + warp;
+            const int chunks = (r1 + 127) / 128;             // (128 times a chunk past the last may leave 32 bits)
             RowGroup cur;                // the warp's next chunk of rows
-            if (128 * chunk < r1) load_group(chunk, cur);
-            for (; 128 * chunk < r1; chunk += WARPS) {
+            if (chunk < chunks) load_group(chunk, cur);
+            for (; chunk < chunks; chunk += WARPS) {
                 RowGroup x = cur;        // (two sets of registers in turn save the copy and spill elsewhere: 215 -> 228 us)
-                if (128 * (chunk + WARPS) < r1) load_group(chunk + WARPS, cur);
+                if (chunk + WARPS < chunks) load_group(chunk + WARPS, cur);
                 add_group(chunk, r0, r1, x, e, lim);
             }
         }
@@ -646,10 +648,11 @@ __global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 && BPL <= 4) ? 2 : 1)
         const int r0 = a.era_offsets[e], mid = a.era_offsets[e + 1], r1 = a.era_offsets[min(e + 2, E)];
         RowGroup cur;
         int c = r0 / 128 + warp;
-        if (128 * c < r1) load_group(c, cur);
-        for (; 128 * c < r1; c += WARPS) {
+        const int chunks = (r1 + 127) / 128;
+        if (c < chunks) load_group(c, cur);
+        for (; c < chunks; c += WARPS) {
             RowGroup x = cur;
-            if (128 * (c + WARPS) < r1) load_group(c + WARPS, cur);
+            if (c + WARPS < chunks) load_group(c + WARPS, cur);
             add_group(c, r0, mid, r1, set, x);
         }
     };
@@ -865,7 +868,7 @@ static WalkShape walk_shape(const WalkLaunch& a, int form) {
 // estimates were within 13 %.  Those of the other forms from 60 000 to 1 million rows, 8 to 256 features, 20 to
 // 574 eras, 63 to 128 bins and 1 to 512 nodes: within 15 %, but for one node over many short eras (121 us, not 92).
 static double walk_estimate_us(const WalkLaunch& a, const WalkShape& s) {
-    const int64_t tiles = a.max_era_rows <= a.tile_rows ? 1 : (a.max_era_rows + a.tile_rows - 1) / a.tile_rows;
+    const int64_t tiles = a.max_era_rows <= a.tile_rows ? 1 : tiles_of(a.max_era_rows, a.tile_rows);
     const int eras = s.mode == kUnit ? s.warps / s.cell_nodes : 1;   // of a batch
     const double batches = s.mode == kUnit ? (double)((a.n_eras + eras - 1) / eras) : (double)a.n_eras * tiles;
     const double batch = s.own ? (s.warps == 32 ? 0.41 : 0.23) * s.bpl : s.mode == kUnit ? (s.warps == 32 ? 1.0 + 0.65 * s.bpl : 1.2 + 0.34 * s.bpl)
@@ -919,7 +922,7 @@ int launch_walk(WalkLaunch a, cudaStream_t stream) {
     if (a.mass) {
         PB_CUDA_TRY(cudaMemsetAsync(a.mass, 0, (size_t)a.n_feat * 256 * sizeof(uint32_t), stream));
         int parts = (148 * 8 + a.n_feat - 1) / a.n_feat;   // about eight CTAs per SM
-        const int most = (a.n_rows + 4095) / 4096;
+        const int most = tiles_of(a.n_rows, 4096);
         if (parts > most) parts = most;
         if (parts < 1) parts = 1;
         mass_count_kernel<<<dim3((unsigned)a.n_feat, (unsigned)parts), 256, 0, stream>>>(a);

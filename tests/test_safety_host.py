@@ -170,6 +170,38 @@ def test_many_bins_take_the_path_that_measured_faster(lib, rows, feats, eras, de
     assert got.value == 0
 
 
+_ROWS = """#include "rows.cuh"
+#include <cstdio>
+int main() {
+    long long b, e, i, t, n;
+    while (std::scanf("%lld %lld %lld %lld %lld", &b, &e, &i, &t, &n) == 5) {
+        int r0, r1;
+        pb::tile_range((int)b, (int)e, (int)i, (int)t, r0, r1);
+        std::printf("%d %d %d\\n", r0, r1, pb::tiles_of(n, t));
+    }
+    return 0;
+}
+"""
+
+
+def test_row_ranges_of_tiles_up_to_the_largest_table(tmp_path):
+    """Tiles of an era that ends at the last row of the largest table (2^31 - 513 rows), and the tiles past the
+    end of a short era behind a very long one, where 32-bit sums would come out negative."""
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "packboost_b200", "csrc")
+    (tmp_path / "rows.cpp").write_text(_ROWS)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fsanitize=undefined", "-fno-sanitize-recover", "-I", csrc,
+                    str(tmp_path / "rows.cpp"), "-o", str(tmp_path / "rows")], check=True)
+    last = 2 ** 31 - 513
+    asked = [(b, e, i, t, n) for t in (512, 8160, 32256) for b, e in ((0, 0), (0, 10), (0, last), (last - 7, last), (2 ** 30 + 9, last), (last, last))
+             for i in (0, 1, -(-(last) // t) - 1, -(-(e - b) // t)) for n in (0, 1, t, t + 1, last)]
+    out = subprocess.run([str(tmp_path / "rows")], input="\n".join(" ".join(map(str, a)) for a in asked), capture_output=True,
+                         text=True, check=True).stdout.split()
+    for k, (b, e, i, t, n) in enumerate(asked):
+        r0 = min(b + i * t, e)
+        assert [int(v) for v in out[3 * k: 3 * k + 3]] == [r0, min(r0 + t, e), -(-n // t)], (b, e, i, t, n)
+
+
 @pytest.mark.parametrize("flags", [[], ["-U__SSE2__"]])
 def test_host_sources_need_no_x86(flags, tmp_path):
     """The ring copy builds without x86 intrinsics (``-U__SSE2__``: as on another host) and moves every
