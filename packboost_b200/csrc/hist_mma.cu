@@ -52,7 +52,7 @@ constexpr int kPitch = 272;             // bytes per feature of a staged block: 
                                         // consecutive features touch every bank
 constexpr int kColumns = 512;           // all of the tensor memory: a CTA per SM
 constexpr int kMmaTileRows = 32256;     // rows of a tile: sums of its digits stay below 2^22, two of them make 32 bits
-constexpr int kSpin = 1 << 15;          // eights of tries of a wait, up to 2 us a try
+constexpr int kTries = 1 << 15;         // eights of tries of a wait, up to 2 us a try
 
 struct MmaArgs {
     const uint8_t* codes;
@@ -77,6 +77,7 @@ struct MmaArgs {
     uint32_t* flags;
     int groups;                         // lanes of a feature: TP / L
     int stages, buffers;                // blocks of codes; accumulators: 2 where they fit
+    int failed;                         // 1: as after a wait that ran out
 };
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -87,12 +88,17 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("{ .reg .b64 s; mbarrier.arrive.shared::cta.b64 s, [%0]; }" ::"r"(smem_at(bar)) : "memory");
 }
-// False when the phase does not end within the limit, or another warp has given up.  IDLE: nothing hangs on a
-// microsecond here, and a warp that keeps asking takes issue slots from the others.
+// Waits for the end of a phase; IDLE: nothing hangs on a microsecond here, and a warp that keeps asking takes issue
+// slots from the others.  A wait that runs out marks the launch as failed, after which every wait ends within
+// eight tries and no product is issued any more, but each role still goes through all of its steps: no warp decides
+// alone to leave.  So the named barriers, which have no limit, are met by all of their warps as often as ever; and
+// since nothing else then keeps a place from being handed over twice, its warps wait until the issuing warps, which
+// take the places in turn whatever happens, have taken it (s_taken).  The launch ends, its sums are not to be used,
+// and the control block says so.
 template <bool IDLE = false>
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile int* fail) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
     const uint32_t at = smem_at(bar);
-    for (int i = 0; i < kSpin; ++i) {
+    for (int i = 0; i < kTries; ++i) {
 #pragma unroll 1
         for (int j = 0; j < 8; ++j) {
             uint32_t ok;
@@ -103,11 +109,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
         }
         if (*fail) return false;
     }
+    *fail = 1;
     return false;
 }
 // The same for a whole warp, which goes on together.
 template <bool IDLE = false>
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const volatile int* fail) {
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
     return __all_sync(0xFFFFFFFFu, mbar_wait<IDLE>(bar, parity, fail));
 }
 __device__ __forceinline__ bool elect_one() {
@@ -125,12 +132,9 @@ __device__ __forceinline__ void mma_i8(uint32_t d, uint32_t a_at, uint64_t b_des
     asm volatile("{ .reg .pred p; setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p; }"
                  ::"r"(d), "r"(a_at), "l"(b_desc), "r"(idesc), "r"(add) : "memory");
 }
-// `threads` threads meet at a barrier of the CTA; true when all bring true.
-__device__ __forceinline__ bool meet(int barrier, int threads, bool v) {
-    uint32_t r;
-    asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; barrier.cta.red.and.pred q, %2, %3, p; selp.u32 %0, 1, 0, q; }"
-                 : "=r"(r) : "r"(v ? 1u : 0u), "r"(barrier), "r"(threads) : "memory");
-    return r != 0u;
+// `threads` threads meet at a barrier of the CTA.
+__device__ __forceinline__ void meet(int barrier, int threads) {
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(barrier), "r"(threads) : "memory");
 }
 constexpr int kFlushBarrier = 1, kSlotBarrier = 2, kFullBarrier = kSlotBarrier + kSlots;   // (the latter two: one per slot)
 constexpr int kSlotThreads = 32 * 6;
@@ -185,6 +189,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
     __shared__ __align__(8) uint64_t full_c[kStagesMax], empty_c[kStagesMax], empty[kSlots], acc_full[2], acc_empty[2], tot_full[2], last;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_fail;
+    __shared__ uint32_t s_taken[kSlots];   // times the issuing warps have taken over a place, all together
     __shared__ float4 s_era[64];         // {gradient total, hessian total, parent term, era weight} of a node
     __shared__ long long s_tgq[64];
     __shared__ uint32_t s_tc[64];
@@ -216,6 +221,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         }
         for (int i = 0; i < kSlots; ++i) {
             mbar_init(empty + i, kIssueWarps);
+            s_taken[i] = 0u;
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(acc_full + i, kIssueWarps);
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
             mbar_init(tot_full + i, kRowWarps);
         }
         mbar_init(&last, kIssueWarps);
-        s_fail = 0;
+        s_fail = a.failed;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     {
@@ -260,7 +266,6 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
     // (a CTA's tasks are neighbours, the feature block the slowest: totals over the eras gather here)
     const int t0 = (int)((int64_t)a.tasks * blockIdx.x / gridDim.x), t1 = (int)((int64_t)a.tasks * (blockIdx.x + 1) / gridDim.x);
     Task x;
-    bool good = true;
 
     if (warp < kCodeWarps) {
         // ---- A: this lane's feature and its L thresholds ----
@@ -281,17 +286,16 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const uint32_t to = a_col + ((uint32_t)quarter << 21);
         const uint32_t at = to + (uint32_t)(wg * (kBatch * L * 8));
         int stage = 0;
-        for (int t = t0; t < t1 && good; ++t) {
+        for (int t = t0; t < t1; ++t) {
             if (!task_at(t, x)) continue;
-            for (int b = x.b0; b < x.b1 && good; ++b) {
+            for (int b = x.b0; b < x.b1; ++b) {
                 bool met = false;
 #pragma unroll 1
                 for (int u = first_unit(b); u < kUnits; u += kSlots) {
                     const int i = u * kBatchRows, r = b * kBlock + i;
                     if (r + kBatchRows <= x.r0 || r >= x.r1) continue;
                     met = true;
-                    good = meet(kSlotBarrier + wg, kSlotThreads, true);
-                    if (!good) break;
+                    meet(kSlotBarrier + wg, kSlotThreads);
                     const uint32_t from = smem_at(s_codes + stage * stage_bytes + fl * kPitch + i / 2);
                     tc_fence_after();
 #pragma unroll
@@ -316,14 +320,12 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                     __syncwarp();
                     hand_over(wg, kIssueWarps);
                 }
-                if (good && !met) good = meet(kSlotBarrier + wg, kSlotThreads, true);   // (a stage is given back only after it came)
-                if (!good) break;
+                if (!met) meet(kSlotBarrier + wg, kSlotThreads);   // (a stage is given back only after it came)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty_c + stage);
                 if (++stage == a.stages) stage = 0;
             }
         }
-        if (!good) hand_over(wg, kIssueWarps);        // (nobody is to wait for what will not come)
     } else if (warp < kRowWarp0) {
         // ---- flush ----
         constexpr int U = L == 4 ? 1 : 2;            // nodes at a time
@@ -334,15 +336,16 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const int K = z.n_thr, lanes_total = a.blocks * FC;
         int buf = 0;
         uint32_t phase = 0u;
-        for (int t = t0; t < t1 && good; ++t) {
+        for (int t = t0; t < t1; ++t) {
             if (!task_at(t, x)) continue;
             const int era = x.era, f = x.fb * FC + fl;
             const bool mine = f < a.n_feat, empty_tile = x.b0 == x.b1;
             const bool fresh = t == t0 || t % a.tiles == 0, last = t + 1 == t1 || (t + 1) % a.tiles == 0;   // of a feature block here
-            // (a wait that ran out is answered by all warps of the role together: they meet at barriers)
-            good = warp_wait<true>(acc_full + buf, phase, &s_fail) && warp_wait<true>(tot_full + buf, phase, &s_fail);
+            warp_wait<true>(acc_full + buf, phase, &s_fail);
+            warp_wait<true>(tot_full + buf, phase, &s_fail);
             uint32_t* tot = s_tot + buf * 3 * tot_plane;
-            for (int n = warp - kFlushWarp0; good && n < n_nodes; n += kFlushWarps) {
+#pragma unroll 1                                 // (unrolled by four: 2 us a launch for the fetch of its instructions)
+            for (int n = warp - kFlushWarp0; n < n_nodes; n += kFlushWarps) {
                 uint32_t* at = tot + n * 32 + lane;
                 uint32_t tc = at[0];
                 long long tg = (long long)(int32_t)at[2 * tot_plane] * 65536ll + (long long)at[tot_plane];
@@ -360,8 +363,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                     }
                 }
             }
-            good = meet(kFlushBarrier, 32 * kFlushWarps, good);
-            if (!good) break;
+            meet(kFlushBarrier, 32 * kFlushWarps);
             tc_fence_after();
             const uint32_t from = tmem + ((uint32_t)quarter << 21) + (uint32_t)(buf * L * N_max);
             for (int n0 = U * fg; n0 < n_nodes; n0 += U * kFlushWarps / 4) {
@@ -454,7 +456,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + buf);
             if (++buf == a.buffers) { buf = 0; phase ^= 1u; }
-            meet(kFlushBarrier, 32 * kFlushWarps, true);             // the nodes' totals are read
+            meet(kFlushBarrier, 32 * kFlushWarps);             // the nodes' totals are read
         }
     } else if (warp < kIssueWarp) {
         // ---- B: a row of two K-steps of each batch ----
@@ -467,28 +469,32 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
 #pragma unroll
         for (int k = 0; k < kMine; ++k) held[k] = 0u;
         int stage = 0, buf = 0;
-        uint32_t phase = 1u, c_phase = 0u, acc_phase = 1u;
-        bool stop = false;
-        for (int t = t0; t < t1 && !stop; ++t) {
+        uint32_t turn = 0u, c_phase = 0u, acc_phase = 1u;   // (turn: how often this place was handed over)
+        for (int t = t0; t < t1; ++t) {
             if (!task_at(t, x)) continue;
-            // the totals of this buffer are zero (a wait that runs out is brought to the meeting)
-            good = warp_wait(acc_empty + buf, acc_phase, &s_fail) && good;
+            warp_wait(acc_empty + buf, acc_phase, &s_fail);   // the totals of this buffer are zero
             uint32_t* tot = s_tot + buf * 3 * tot_plane + lane;
-            for (int b = x.b0; b < x.b1 && !stop; ++b) {
+            for (int b = x.b0; b < x.b1; ++b) {
                 bool met = false;
 #pragma unroll 1
                 for (int u = first_unit(b); u < kUnits; u += kSlots) {
                     const int i = u * kBatchRows, r = b * kBlock + i;
                     if (r + kBatchRows <= x.r0 || r >= x.r1) continue;
                     // the two warps wait for the six of a slot, one for the codes, one for the operands' place
-                    if (half != 0) good = warp_wait(empty + wg, phase, &s_fail) && good;
-                    else if (!met) good = warp_wait(full_c + stage, c_phase, &s_fail) && good;
+                    if (half != 0) {
+                        warp_wait(empty + wg, ~turn & 1u, &s_fail);
+                        if (s_fail) {        // a place is not handed over again before all took it
+                            const volatile uint32_t* taken = s_taken + wg;
+#pragma unroll 1
+                            for (int i = 0; i < kTries && *taken != turn * kIssueWarps; ++i) __nanosleep(1000);
+                            __syncwarp();
+                        }
+                    } else if (!met) {
+                        warp_wait(full_c + stage, c_phase, &s_fail);
+                    }
                     met = true;
-                    if (!good) s_fail = 1;
-                    good = meet(kSlotBarrier + wg, kSlotThreads, good);
-                    stop = !good;
-                    if (stop) break;
-                    phase ^= 1u;
+                    meet(kSlotBarrier + wg, kSlotThreads);
+                    ++turn;
                     const unsigned char* rows = s_codes + stage * stage_bytes + FC * kPitch;
                     const int mine = i + half * kMine * 32 + lane;
                     uint32_t s[kMine], q[kMine];
@@ -525,21 +531,17 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                     hand_over(wg, kIssueWarps);
                 }
                 if (!met) {
-                    if (half == 0) good = warp_wait(full_c + stage, c_phase, &s_fail) && good;
-                    if (!good) s_fail = 1;
-                    good = meet(kSlotBarrier + wg, kSlotThreads, good);
-                    stop = !good;
+                    if (half == 0) warp_wait(full_c + stage, c_phase, &s_fail);
+                    meet(kSlotBarrier + wg, kSlotThreads);
                 }
-                if (stop) break;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty_c + stage);
                 if (++stage == a.stages) { stage = 0; c_phase ^= 1u; }
             }
             __syncwarp();
-            if (good && lane == 0) mbar_arrive(tot_full + buf);
+            if (lane == 0) mbar_arrive(tot_full + buf);
             if (++buf == a.buffers) { buf = 0; acc_phase ^= 1u; }
         }
-        if (stop) hand_over(wg, kIssueWarps);
     } else if (warp < kCopyWarp0) {
         // ---- products ----
         const int n1 = WIDE ? min(N, 256) : N, n2 = max(N - n1, 16);   // (of a narrower frontier: columns nobody reads)
@@ -551,17 +553,18 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const int first = (warp - kIssueWarp) * kTilesOf;    // of this warp's accumulators
         int buf = 0;
         uint32_t acc_phase = 1u;
-        for (int t = t0; t < t1 && good; ++t) {
+        for (int t = t0; t < t1; ++t) {
             if (!task_at(t, x)) continue;
-            good = warp_wait(acc_empty + buf, acc_phase, &s_fail);
-            if (!good) break;
+            warp_wait(acc_empty + buf, acc_phase, &s_fail);
             uint32_t add = 0u;
             const int u0 = x.r0 / kBatchRows, u1 = x.r0 < x.r1 ? (x.r1 + kBatchRows - 1) / kBatchRows : u0;
             int slot = u0 % kSlots;
-            for (int u = u0; u < u1 && good; ++u) {
+            bool lives = s_fail == 0;
+            for (int u = u0; u < u1; ++u) {
                 asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(kFullBarrier + slot), "r"(kSlotThreads + 32 * kIssueWarps) : "memory");
                 tc_fence_after();
-                if (elect_one()) {
+                if (lane == 0) atomicAdd(s_taken + slot, 1u);
+                if (elect_one() && lives) {
                     const uint32_t lo = desc_lo + (uint32_t)(slot * kBatch) * k16, at0 = a_col + (uint32_t)((slot * kBatch * L + first) * 8);
                     const uint32_t d0 = tmem + (uint32_t)((buf * L + first) * N_max);
 #pragma unroll
@@ -579,9 +582,9 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                 __syncwarp();
                 add = 1u;
                 if (++slot == kSlots) slot = 0;
-                good = s_fail == 0;
+                lives = s_fail == 0;
             }
-            if (elect_one()) tc_commit(acc_full + buf);
+            if (elect_one() && lives) tc_commit(acc_full + buf);
             __syncwarp();
             if (++buf == a.buffers) { buf = 0; acc_phase ^= 1u; }
         }
@@ -593,7 +596,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const int part = lane & 15;
         int stage = 0;
         uint32_t phase = 1u;
-        for (int t = t0; t < t1 && good; ++t) {
+        for (int t = t0; t < t1; ++t) {
             if (!task_at(t, x)) continue;
             uint32_t rows[kMine];
 #pragma unroll
@@ -602,8 +605,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                 rows[i] = fl < FC ? (uint32_t)a.feat_rows[min(x.fb * FC + fl, a.n_feat - 1)] : 0u;
             }
             for (int b = x.b0; b < x.b1; ++b) {
-                good = warp_wait(empty_c + stage, phase, &s_fail);
-                if (!good) break;
+                warp_wait(empty_c + stage, phase, &s_fail);
                 const uint32_t to = smem_at(s_codes + stage * stage_bytes);
                 const int64_t column = (int64_t)b * (kBlock / 2) + part * 16;
                 if (column < a.pitch) {              // (a row is padded to whole lines, not to whole blocks)
@@ -626,13 +628,10 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    if (!good) {
-        s_fail = 1;
-        if (a.flags && lane == 0) atomicOr(a.flags, kFaultWait);
-    }
     __syncwarp();
     __syncthreads();
     if (s_fail) {                            // what has been issued ends before the tensor memory goes
+        if (a.flags && threadIdx.x == 0) atomicOr(a.flags, kFaultWait);
         if (warp >= kIssueWarp && warp < kCopyWarp0) {
             if (elect_one()) tc_commit(&last);
             __syncwarp();
@@ -741,6 +740,11 @@ int launch_hist_mma(const HistLaunch& h, cudaStream_t stream) {
     a.groups = s.groups;
     a.buffers = s.buffers;
     a.stages = s.stages;
+    static const int failed = [] {   // PACKBOOST_WAIT_FAILS=1: launches go the way of a wait that ran out, for the test of it
+        const char* e = getenv("PACKBOOST_WAIT_FAILS");
+        return (e && e[0] == '1' && e[1] == 0) ? 1 : 0;
+    }();
+    a.failed = failed;
     const int blocks = (h.n_feat + s.features - 1) / s.features;
     a.tile_rows = kMmaTileRows;
     a.tiles_per_era = 1;

@@ -349,6 +349,44 @@ np.savez(out, preds=b.train_predictions().view(np.int32), **{k: v.view(np.int32)
         np.testing.assert_array_equal(got[0][key], got[1][key], err_msg=key)
 
 
+_LIMIT_SCRIPT = r"""
+import json, sys
+import numpy as np, torch
+from packboost_b200 import PackBoost, PackBoostConfig
+for n, f, eras, bins, depth in json.loads(sys.argv[1]):
+    rng = np.random.default_rng(n + f)
+    X = rng.integers(0, bins, size=(n, f)).astype(np.uint8)
+    y = (X[:, 0] + rng.normal(size=n)).astype(np.float32)
+    era = np.sort(rng.integers(0, eras, n)).astype(np.int16)
+    cfg = PackBoostConfig(pack_size=2, max_depth=depth, lambda_l2=1.0, min_samples_leaf=5, max_bins=bins, prebinned=True)
+    try:
+        PackBoost(cfg).fit(X, y, era, num_rounds=3)
+        print("no error")
+    except RuntimeError as e:
+        print("error" if "ran into its limit" in str(e) else e)
+    torch.cuda.synchronize()
+    assert int(torch.arange(1000, device="cuda").sum().item()) == 499500
+"""
+
+
+@pytest.mark.parametrize("fails,says", [(True, "error"), (False, "no error")])
+def test_waits_that_run_out_end_the_launch_and_are_reported(fails, says):
+    """Launches of the contraction that are marked as failed from the start, so that no product is issued and whatever
+    waits for one gives up: they end, the fit says why, and the device goes on working.  One and two issuing warps, batches of 64 and 128 rows, gains made
+    in the flush and a stored histogram, eras shorter than a batch."""
+    import json
+    import subprocess
+    import sys
+    shapes = [(6_001, 300, 7, 5, 4), (5_003, 40, 40, 5, 6), (700, 33, 1, 2, 3), (20_001, 45, 2, 5, 7), (17_000, 200, 1, 6, 7), (3_000, 70, 900, 8, 5)]
+    env = dict(os.environ, PACKBOOST_HIST_MMA="1")
+    if fails:
+        env["PACKBOOST_WAIT_FAILS"] = "1"
+    res = subprocess.run([sys.executable, "-c", _LIMIT_SCRIPT, json.dumps(shapes)], env=env, capture_output=True, text=True, timeout=300,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert res.returncode == 0, res.stderr[-2000:]
+    assert res.stdout.split("\n")[:-1] == [says] * len(shapes), res.stdout
+
+
 @pytest.mark.parametrize("max_bins,n_nodes", [(96, 64), (12, 512), (191, 32), (47, 128)])
 def test_histogram_whose_cells_take_just_the_shared_memory_given_without_asking(max_bins, n_nodes):
     """48 KB of cells or a little less beside the kernel's own arrays: such a launch has to ask for more
