@@ -194,7 +194,8 @@ typedef struct pb_train_state {
  * - nothing traps.  pb_debug_flags copies that word to the host (it synchronises the device):
  * bit 0 slot out of range, bit 1 bin code >= max_bins, bit 2 feature id out of range.  In a regular
  * build the checks are compiled out; pb_debug_bounds_enabled says which build this is.  Bit 3 may be
- * set by any build: a wait inside a kernel ran into its limit.  pb_tree_from_log refuses such a round. */
+ * set by any build: a wait inside a kernel ran into its limit.  pb_tree_from_log refuses such a round;
+ * a caller of pb_hist_build looks at the bit itself. */
 int pb_debug_bounds_enabled(void);
 int pb_debug_flags(const pb_train_state* st, uint32_t* flags_out);
 
@@ -391,7 +392,8 @@ typedef struct pb_round_log_header {
 
 /* Histogram pass alone (packboost/booster.py:933-977, counts and gradient sums; the
  * hessian of the squared loss is 1, so its histogram is the count).  Output layout
- * `[n_feat][n_eras][node_stride][max_bins]`. `n_nodes` frontier slots are accumulated. */
+ * `[n_feat][n_eras][node_stride][max_bins]`. `n_nodes` frontier slots are accumulated.  No log goes with
+ * it: after the stream was waited for, bit 3 of pb_debug_flags says that the sums are not complete. */
 int pb_hist_build(const pb_train_state* st, const int32_t* feat_rows, int64_t n_feat,
                   int64_t n_nodes, int64_t node_stride, uint32_t* cnt, int64_t* gsum, void* stream);
 

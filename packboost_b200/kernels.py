@@ -28,6 +28,18 @@ def _fixed_point(values: torch.Tensor, bits: int) -> tuple[torch.Tensor, float]:
     return q, 2.0 ** (-sh)
 
 
+_FAULT_WAIT = 8   # pb_debug_flags: a wait inside a kernel ran into its limit
+
+
+def _refuse_incomplete(lib, st: B.TrainState) -> None:
+    """Raises when a kernel gave up a wait since the control block was zeroed: its sums are not complete, and
+    ``pb_hist_build``, which only enqueues, has no log to say so."""
+    flags = C.c_uint32(0)
+    B.check(lib.pb_debug_flags(C.byref(st), C.byref(flags)))
+    if flags.value & _FAULT_WAIT:
+        raise RuntimeError("a wait inside a histogram kernel ran into its limit: the sums are not complete")
+
+
 def histograms_nodes(bins_matrix: torch.Tensor, grad_rows: torch.Tensor, hess_rows: torch.Tensor,
                      era_ids: torch.Tensor, node_ids: torch.Tensor, num_nodes: int, num_eras: int,
                      num_bins: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
@@ -97,6 +109,7 @@ def histograms_raw(bins_matrix: torch.Tensor, addends: list[torch.Tensor], era_i
                                   gsum.data_ptr(), stream))
         out.append((gsum, inv))
     torch.cuda.current_stream().synchronize()   # (the temporaries above are released after the kernels ran)
+    _refuse_incomplete(lib, st)
     return cnt, out
 
 

@@ -387,6 +387,34 @@ def test_waits_that_run_out_end_the_launch_and_are_reported(fails, says):
     assert res.stdout.split("\n")[:-1] == [says] * len(shapes), res.stdout
 
 
+_RAW_SCRIPT = r"""
+import torch
+from packboost_b200 import kernels
+n, f = 20_001, 45
+X = torch.randint(0, 5, (n, f), dtype=torch.uint8)
+node = torch.randint(0, 3, (n,))
+try:
+    cnt, sums, _ = kernels.histograms_nodes(X, torch.randn(n), torch.ones(n), torch.zeros(n, dtype=torch.int64), node, 3, 1, 5)
+    assert torch.equal(cnt.sum((2, 3)).cpu(), torch.bincount(node).expand(f, 3))
+    print("no error")
+except RuntimeError as e:
+    print("error" if "ran into its limit" in str(e) else e)
+"""
+
+
+@pytest.mark.parametrize("fails,says", [(True, "error"), (False, "no error")])
+def test_histograms_whose_waits_ran_out_are_refused(fails, says):
+    """The histogram entry only enqueues and has no log: its caller looks at the control block."""
+    import subprocess
+    import sys
+    env = dict(os.environ, PACKBOOST_HIST_MMA="1")
+    if fails:
+        env["PACKBOOST_WAIT_FAILS"] = "1"
+    res = subprocess.run([sys.executable, "-c", _RAW_SCRIPT], env=env, capture_output=True, text=True, timeout=300,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert res.returncode == 0 and res.stdout.strip() == says, res.stdout + res.stderr[-2000:]
+
+
 @pytest.mark.parametrize("max_bins,n_nodes", [(96, 64), (12, 512), (191, 32), (47, 128)])
 def test_histogram_whose_cells_take_just_the_shared_memory_given_without_asking(max_bins, n_nodes):
     """48 KB of cells or a little less beside the kernel's own arrays: such a launch has to ask for more
