@@ -71,6 +71,25 @@ constexpr uint16_t kSlotNone = 0xFFFFu;
 constexpr int kTileRowsMax = 8160;      // rows one histogram CTA accumulates (255 chunks of 32 rows)
 constexpr int kGqBitsMax = 30;          // |gq| <= 2^30 at most; fewer bits when tiles are large
 
+// ---- shared memory of a launch ----------------------------------------------------------------
+
+// More shared memory than a launch gets without asking (48 KB, its static arrays included) is allowed per kernel, not
+// per launch.  The limit set is the same for all launches of a kernel, the most that any asks for: with the size
+// of the launch, a thread that launches it small would take the limit away between the two calls of another.
+constexpr size_t kSharedMost = 224 * 1024;   // beside static arrays of up to 3 KB
+template <typename K>
+int allow_shared(K* kernel, size_t smem, size_t most = kSharedMost) {
+    if (smem <= 40 * 1024) return PB_OK;
+    if (smem > most) return fail_arg("%zu bytes of shared memory asked for, %zu at most", smem, most);
+    PB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return PB_OK;
+}
+#define PB_TRY(expr)                \
+    do {                            \
+        const int _rc = (expr);     \
+        if (_rc) return _rc;        \
+    } while (0)
+
 // ---- device-side tables -----------------------------------------------------------------
 
 // Best threshold of one (sampled feature, frontier node) pair.

@@ -797,14 +797,12 @@ int launch_lane_r(const HistKernelArgs& a, size_t cell_bytes, cudaStream_t strea
     if constexpr (A * T <= 4) {
         if ((int64_t)grid.x * grid.y <= 148 * 2 && resident(smem + more) == resident(smem)) {
             smem += more;
-            if (smem > 40 * 1024)   // (beside the static arrays)
-                PB_CUDA_TRY(cudaFuncSetAttribute(hist_lane_kernel<A, T, R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PB_TRY(allow_shared(hist_lane_kernel<A, T, R, 2>, smem));
             hist_lane_kernel<A, T, R, 2><<<grid, kLaneWarps * 32, smem, stream>>>(a);
             return PB_OK;
         }
     }
-    if (smem > 40 * 1024)
-        PB_CUDA_TRY(cudaFuncSetAttribute(hist_lane_kernel<A, T, R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_TRY(allow_shared(hist_lane_kernel<A, T, R, 1>, smem));
     hist_lane_kernel<A, T, R, 1><<<grid, kLaneWarps * 32, smem, stream>>>(a);
     return PB_OK;
 }
@@ -1034,12 +1032,10 @@ int launch_hist(const HistLaunch& h, cudaStream_t stream) {
     if (grid.y > 65535u || grid.z > 65535u) return fail_arg("histogram grid too large");
     prof_begin(h.prof, kProfHist, stream);
     if (h.code_bits == 4) {
-        if (smem > 40 * 1024)   // (48 KB without asking, and s_frow is beside the cells)
-            PB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<4, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(hist_kernel<4, 256>, smem));
         hist_kernel<4, 256><<<grid, threads, smem, stream>>>(a);
     } else {
-        if (smem > 40 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<8, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(hist_kernel<8, 512>, smem));
         hist_kernel<8, 512><<<grid, threads, smem, stream>>>(a);
     }
     prof_end(h.prof, kProfHist, stream);

@@ -662,14 +662,14 @@ MmaShape mma_shape(int n_nodes, int n_feat, int max_bins, bool fused) {
     const size_t sums = fused ? (size_t)n_nodes * L * 128 * 12 : 0;
     const size_t fixed = (size_t)kSlots * s.batch * N * 32 + sums + (size_t)s.buffers * n_nodes * 32 * 12;
     s.stages = kStagesMax;
-    while (s.stages > 2 && fixed + (size_t)s.stages * mma_stage_bytes(s.features) > 224 * 1024) --s.stages;
+    while (s.stages > 2 && fixed + (size_t)s.stages * mma_stage_bytes(s.features) > kSharedMost) --s.stages;
     s.smem = fixed + (size_t)s.stages * mma_stage_bytes(s.features);
     return s;
 }
 
 template <int L, int KB, bool GROUPS, bool WIDE>
 int launch_l(const MmaArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    PB_CUDA_TRY(cudaFuncSetAttribute(hist_mma_kernel<L, KB, GROUPS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_TRY(allow_shared(hist_mma_kernel<L, KB, GROUPS, WIDE>, smem));
     hist_mma_kernel<L, KB, GROUPS, WIDE><<<grid, mma_threads(GROUPS, L), smem, stream>>>(a);
     return PB_OK;
 }

@@ -408,8 +408,7 @@ int pack_fm(const PackArgs& a, bool f32, cudaStream_t stream) {
         });
     } else {
         const size_t smem = sizeof(uint32_t) * kCodeTileF * (kTileR * BITS / 32 + 1) + (size_t)kTileR * kRowBytes + 16;
-        if (smem > 48 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(pack_codes_fm_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(pack_codes_fm_kernel<BITS>, smem));
         pack_codes_fm_kernel<BITS><<<(unsigned)blocks, 256, smem, stream>>>(a);
     }
     if (rc) return rc;
@@ -432,8 +431,7 @@ int pack_rows(PackRowsArgs a, bool f32, cudaStream_t stream) {
         rc = with_steps(a.n_edges, [&](auto steps) {
             constexpr int S = decltype(steps)::value;
             const size_t smem = sizeof(float) * (size_t)((1 << S) - 1) * 128;
-            if (smem > 48 * 1024)
-                PB_CUDA_TRY(cudaFuncSetAttribute(pack_float_rows_kernel<BITS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PB_TRY(allow_shared(pack_float_rows_kernel<BITS, S>, smem));
             pack_float_rows_kernel<BITS, S><<<grid, 256, smem, stream>>>(a);
             return PB_OK;
         });

@@ -429,6 +429,7 @@ constexpr int kTreesPerWalker = 4;  // walked at a time by a lane: independent c
 constexpr int kAddGroup = 8;        // trees whose terms an adder holds; a batch is a multiple of it
 // Batches of trees in shared memory: the one being walked and those on their way.
 constexpr int kTreeBuffers = 2;
+constexpr int kForestShared = 227 * 1024;   // (no static arrays beside it)
 
 // Words per feature.  The words of 32 rows are `bits` neighbouring banks; an odd number of groups puts
 // those of different features at every multiple of that, an even one needs a word of padding.
@@ -698,12 +699,10 @@ extern "C" int pb_predict_rows(const uint8_t* codes, int64_t n_rows, int64_t pit
     }
     const unsigned grid = (unsigned)((n_rows + a.rows_per_cta - 1) / a.rows_per_cta);
     if (code_bits == 4) {
-        if (smem > 48 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(predict_rows_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(predict_rows_kernel<4>, smem));
         predict_rows_kernel<4><<<grid, 128, smem, stream>>>(a);
     } else {
-        if (smem > 48 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(predict_rows_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(predict_rows_kernel<8>, smem));
         predict_rows_kernel<8><<<grid, 128, smem, stream>>>(a);
     }
     count_launch(1);
@@ -791,23 +790,17 @@ extern "C" int pb_predict_rows_packed(const uint8_t* codes, int64_t n_rows, int6
     const int threads = (a.rows_per_cta * kTpr + 31) / 32 * 32;
     if (a.stage && tb > 0) {  // rows and trees both staged: the all-shared-memory form
         if (code_bits == 4) {
-            if (smem > 48 * 1024)
-                PB_CUDA_TRY(cudaFuncSetAttribute(predict_rows_packed_smem_kernel<4>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PB_TRY(allow_shared(predict_rows_packed_smem_kernel<4>, smem));
             predict_rows_packed_smem_kernel<4><<<grid, threads, smem, stream>>>(a);
         } else {
-            if (smem > 48 * 1024)
-                PB_CUDA_TRY(cudaFuncSetAttribute(predict_rows_packed_smem_kernel<8>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PB_TRY(allow_shared(predict_rows_packed_smem_kernel<8>, smem));
             predict_rows_packed_smem_kernel<8><<<grid, threads, smem, stream>>>(a);
         }
     } else if (code_bits == 4) {
-        if (smem > 48 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(predict_rows_packed_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(predict_rows_packed_kernel<4>, smem));
         predict_rows_packed_kernel<4><<<grid, threads, smem, stream>>>(a);
     } else {
-        if (smem > 48 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(predict_rows_packed_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(predict_rows_packed_kernel<8>, smem));
         predict_rows_packed_kernel<8><<<grid, threads, smem, stream>>>(a);
     }
     count_launch(1);
@@ -855,7 +848,7 @@ extern "C" int pb_predict_forest(const uint8_t* codes, int64_t n_rows, int64_t p
             if (threads > 1024) continue;
             const double tb = kTreesPerWalker * ww;
             const int64_t smem = forest_smem(n_features, (int)code_bits, g, ww, slot_nodes);
-            if (smem > 227 * 1024) continue;
+            if (smem > kForestShared) continue;
             int per_sm = (int)(228 * 1024 / (smem + 1024));
             if (per_sm > 2048 / threads) per_sm = 2048 / threads;
             const double ctas = (double)((n_rows + 32 * g - 1) / (32 * g));
@@ -883,7 +876,7 @@ extern "C" int pb_predict_forest(const uint8_t* codes, int64_t n_rows, int64_t p
         return (e && sscanf(e, "%d %d", &v[0], &v[1]) == 2) ? v : (const int*)nullptr;
     }();
     if (forced && forced[0] >= 1 && forced[1] >= 1 && forced[1] * kTreesPerWalker % kAddGroup == 0 && forest_threads(forced[0], forced[1]) <= 1024 &&
-        forest_smem(n_features, (int)code_bits, forced[0], forced[1], slot_nodes) <= 227 * 1024) {
+        forest_smem(n_features, (int)code_bits, forced[0], forced[1], slot_nodes) <= kForestShared) {
         a.groups = forced[0];
         a.walk_warps = forced[1];
         best_smem = (size_t)forest_smem(n_features, (int)code_bits, forced[0], forced[1], slot_nodes);
@@ -892,10 +885,10 @@ extern "C" int pb_predict_forest(const uint8_t* codes, int64_t n_rows, int64_t p
     const unsigned grid = (unsigned)((n_rows + R - 1) / R);
     const int threads = forest_threads(a.groups, a.walk_warps);
     if (code_bits == 4) {
-        PB_CUDA_TRY(cudaFuncSetAttribute(predict_forest_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best_smem));
+        PB_TRY(allow_shared(predict_forest_kernel<4>, best_smem, kForestShared));
         predict_forest_kernel<4><<<grid, threads, best_smem, stream>>>(a);
     } else {
-        PB_CUDA_TRY(cudaFuncSetAttribute(predict_forest_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best_smem));
+        PB_TRY(allow_shared(predict_forest_kernel<8>, best_smem, kForestShared));
         predict_forest_kernel<8><<<grid, threads, best_smem, stream>>>(a);
     }
     count_launch(1);
@@ -904,7 +897,7 @@ extern "C" int pb_predict_forest(const uint8_t* codes, int64_t n_rows, int64_t p
 }
 
 extern "C" int64_t pb_predict_forest_fits(int64_t n_features, int64_t code_bits, int64_t slot_nodes) {
-    return forest_smem(n_features, (int)code_bits, 1, kAddGroup / kTreesPerWalker, slot_nodes) <= 227 * 1024 ? 1 : 0;
+    return forest_smem(n_features, (int)code_bits, 1, kAddGroup / kTreesPerWalker, slot_nodes) <= kForestShared ? 1 : 0;
 }
 
 // ---- a whole prediction in one call ----------------------------------------------------------------------

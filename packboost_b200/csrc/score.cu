@@ -975,8 +975,7 @@ int launch_score(const ScoreLaunch& s, cudaStream_t stream) {
         const int npck2 = (npc * K + 1) & ~1;
         const size_t smem = (size_t)npck2 * 8 + (size_t)npc * K * 12 + (size_t)3 * ec * npc * K * sizeof(float2) +
                             (size_t)(s.n_eras + 1) * 4;
-        if (smem > 48 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(chain_unit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(chain_unit_kernel, smem));
         dim3 grid((unsigned)s.n_feat, (unsigned)((s.n_nodes_max + npc - 1) / npc));
         if (grid.y > 65535u) return fail_arg("scorer grid too large");
         const int half = ((npc * K + 31) / 32) * 32;
@@ -992,8 +991,7 @@ int launch_score(const ScoreLaunch& s, cudaStream_t stream) {
         if (ec > s.n_eras) ec = s.n_eras;
         c.era_chunk = ec;
         const size_t smem = (size_t)npc * K * 16 + (size_t)2 * ec * npc * K * sizeof(float2);
-        if (smem > 48 * 1024)
-            PB_CUDA_TRY(cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_TRY(allow_shared(chain_kernel, smem));
         dim3 grid((unsigned)s.n_feat, (unsigned)((s.n_nodes_max + npc - 1) / npc));
         if (grid.y > 65535u) return fail_arg("scorer grid too large");
         const int threads = ((npc * K + 31) / 32) * 32;

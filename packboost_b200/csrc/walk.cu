@@ -783,15 +783,14 @@ __global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 && BPL <= 4) ? 2 : 1)
 
 template <int BPL, int WARPS>
 int launch_nodes(const WalkLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    PB_CUDA_TRY(cudaFuncSetAttribute(walk_nodes_kernel<BPL, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_TRY(allow_shared(walk_nodes_kernel<BPL, WARPS>, smem));
     walk_nodes_kernel<BPL, WARPS><<<grid, 32 * WARPS, smem, stream>>>(a);
     return PB_OK;
 }
 
 template <int BPL, int MODE, int COPIES, int WARPS>
 int launch_one(const WalkLaunch& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    if (smem > 40 * 1024)   // (beside the static arrays)
-        PB_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<BPL, MODE, COPIES, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_TRY(allow_shared(walk_kernel<BPL, MODE, COPIES, WARPS>, smem));
     walk_kernel<BPL, MODE, COPIES, WARPS><<<grid, 32 * WARPS, smem, stream>>>(a);
     return PB_OK;
 }

@@ -415,6 +415,54 @@ def test_histograms_whose_waits_ran_out_are_refused(fails, says):
     assert res.returncode == 0 and res.stdout.strip() == says, res.stdout + res.stderr[-2000:]
 
 
+def test_threads_that_launch_a_kernel_at_different_sizes_do_not_disturb_each_other():
+    """Two threads, each with a state of its own, launch the same instantiations at sizes that need different
+    amounts of shared memory: neither lowers the limit between the other's asking and its launch."""
+    import threading
+    from packboost_b200 import backends as B
+    lib, dev = B.lib(), _dev()
+    errors, keep = [], []
+
+    def state(n_bins):
+        n, f, nb = 4_096, 8, n_bins
+        codes = torch.zeros((f, n), dtype=torch.uint8, device=dev)
+        row = torch.zeros(4 * n, dtype=torch.float32, device=dev)
+        eo = torch.tensor([0, n], dtype=torch.int32, device=dev)
+        ids = torch.arange(256, dtype=torch.int32, device=dev)
+        ctl = torch.zeros(int(lib.pb_ctl_bytes()), dtype=torch.uint8, device=dev)
+        out = (torch.empty(f * 512 * nb, dtype=torch.int32, device=dev), torch.empty(f * 512 * nb, dtype=torch.int64, device=dev))
+        st = B.TrainState()
+        st.n_rows, st.n_features_total, st.n_features_local, st.n_eras = n, f, f, 1
+        st.max_bins, st.code_bits, st.pitch = nb, 8, n
+        st.max_depth, st.pack_size, st.min_samples_leaf, st.n_thresholds, st.feature_block_size = 6, 1, 1, nb - 1, 32
+        st.lambda_l2 = 1.0
+        st.codes, st.era_offsets, st.thr_ids, st.feat_local = codes.data_ptr(), eo.data_ptr(), ids.data_ptr(), ids.data_ptr()
+        st.y = st.preds = st.gq = st.slot = st.leaf = row.data_ptr()
+        st.ctl = ctl.data_ptr()
+        eo_host = np.array([0, n], np.int32)
+        B.check(lib.pb_train_prepare(C.byref(st), eo_host.ctypes.data))
+        keep.append((codes, row, eo, ids, ctl, out))
+        return st, ids, out
+
+    def launch(st, ids, out, nodes, stream):
+        try:
+            for _ in range(4_000):
+                B.check(lib.pb_hist_build(C.byref(st), ids.data_ptr(), 8, nodes, nodes, out[0].data_ptr(), out[1].data_ptr(), stream))
+        except Exception as e:   # noqa: BLE001
+            errors.append(str(e))
+
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    jobs = [(*state(128), nodes, s.cuda_stream) for nodes, s in zip((60, 180), streams)]
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=launch, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors[0]
+
+
 @pytest.mark.parametrize("max_bins,n_nodes", [(96, 64), (12, 512), (191, 32), (47, 128)])
 def test_histogram_whose_cells_take_just_the_shared_memory_given_without_asking(max_bins, n_nodes):
     """48 KB of cells or a little less beside the kernel's own arrays: such a launch has to ask for more
