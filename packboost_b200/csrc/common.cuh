@@ -97,7 +97,8 @@ struct Cand {
     float score;
     int32_t k;            // index into thr_ids, -1: empty entry
     uint32_t left_count;
-    uint32_t flags;       // bit 0: a globally valid threshold of this feature scored NaN; bits 8-15: bin id of threshold k
+    uint32_t flags;       // bit 0: a globally valid threshold of this feature scored NaN; bits 8-15: bin id of threshold k;
+                          // bit 1 (kCandFault): on the device that made it a wait had run into its limit
     int64_t left_gq;
 };
 static_assert(sizeof(Cand) == 24, "Cand layout");
@@ -125,16 +126,19 @@ struct CtlHead {
     int32_t n_ctx[kMaxDepth + 2];
     int32_t any_dir[kMaxDepth + 2];
     uint32_t select_ticket;  // CTAs of the running select launch that have written their node (reset by the last)
-    uint32_t debug_flags;    // PB_DEBUG_BOUNDS builds: sticky bits of index violations seen by the kernels
+    uint32_t debug_flags;    // sticky bits, below
 };
 
-// Bits of CtlHead::debug_flags (builds with -DPB_DEBUG_BOUNDS check the indices they are handed and
-// record a violation here instead of using the index; other builds never set them).
+// Bits of CtlHead::debug_flags.  The first three are index violations: builds with -DPB_DEBUG_BOUNDS check the
+// indices they are handed and record a violation here instead of using the index; other builds never set those.
 constexpr uint32_t kDbgSlot = 1u;     // a row's frontier slot is neither "none" nor below the frontier's capacity
 constexpr uint32_t kDbgCode = 2u;     // a bin code is >= max_bins
 constexpr uint32_t kDbgFeature = 4u;  // a winner's feature id is outside the data set or not held by this device
 // (every build) a wait inside a kernel ran into its limit: the histograms of the round are not to be used
 constexpr uint32_t kFaultWait = 8u;
+// The same in a candidate, which goes to every device: all of them find it in the round's log, none is left
+// waiting for one that stopped.
+constexpr uint32_t kCandFault = 2u;
 
 // Addresses of the sub-tables inside the caller's control block.
 struct Ctl {
@@ -257,6 +261,7 @@ struct ScoreLaunch {
     int direction_form;          // 0: agreement with the parent's direction, 1: +1 / -1 by comparing the child values
     int min_samples_leaf;
     Cand* cand;                  // [n_sampled][node_stride]
+    const uint32_t* debug_flags; // &CtlHead::debug_flags
     // scratch of the two-kernel scorer, for the n_feat features of this block
     float2* gw;                  // [n_feat][n_eras][node_stride][n_thr] (gain, validity weight)
     uint8_t* agree;              // directional term like HistFuse::agree, or null; a fused flush has filled it

@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(SelectArgs a) {
             for (int p = b0 + lane; p < b1; p += 32) {
                 const Cand cd = a.cand[(size_t)p * a.node_stride + n];
                 if (cd.flags & 1u) has_nan = true;
+                if (cd.flags & kCandFault) atomicOr(&c.head->debug_flags, kFaultWait);
                 if (cd.k < 0) continue;
                 // (the k field of a block winner carries the candidate's threshold bin id from here on)
                 const BlockBest x{cd.score, (long long)cd.left_count, cd.left_gq, p, (int)((cd.flags >> 8) & 0xFFu), a.sampled[p]};
@@ -855,6 +856,7 @@ static int hist_score_blocks(const pb_train_state* st, int64_t depth, const int3
         s.era_alpha = (float)(st->era_alpha > 0.0 ? st->era_alpha : 0.0);
         s.min_samples_leaf = (int)st->min_samples_leaf;
         s.cand = cand;
+        s.debug_flags = &c.head->debug_flags;
         s.gw = reinterpret_cast<float2*>(scratch + plan.off_gw);
         s.lg_tot = reinterpret_cast<int64_t*>(scratch + plan.off_lg);
         s.lc_tot = reinterpret_cast<uint32_t*>(scratch + plan.off_lc);

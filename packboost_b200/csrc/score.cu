@@ -351,6 +351,7 @@ __device__ __forceinline__ void finish_pairs(const ScoreLaunch& s, int f, int no
                                              float a_den, float* res_score, uint32_t* res_cnt, long long* res_lg) {
     const int K = s.n_thr;
     const int node = node0 + (scorer ? my_i : 0);
+    const uint32_t faults = s.debug_flags ? *s.debug_flags & kFaultWait : 0u;
     if (scorer) {
         const float ws = (wsum < 1e-12f) ? 1e-12f : wsum;
         float var = f_div(m2, ws);
@@ -375,7 +376,7 @@ __device__ __forceinline__ void finish_pairs(const ScoreLaunch& s, int f, int no
         float bs = -INFINITY;
         int64_t bc = -1;
         int bk = -1;
-        uint32_t flags = 0;
+        uint32_t flags = faults ? kCandFault : 0u;
         for (int k = 0; k < K; ++k) {
             const float sc = res_score[i * K + k];
             if (sc != sc) {

@@ -755,3 +755,69 @@ def test_directional_term_of_child_values_that_round_to_zero(bins, eras, n):
 def _root_shard(era, eras):
     from packboost_b200.booster import NodeShard
     return NodeShard(tree_id=0, node_id=0, depth=0, era_rows=[torch.from_numpy(np.flatnonzero(era == e)) for e in range(eras)])
+
+
+@pytest.mark.parametrize("alpha", [0.0, 3.0])
+def test_a_wait_that_ran_out_reaches_every_device(alpha):
+    """A device's fault goes out with its candidates, and a candidate that brings one marks the round's log: the
+    bit is set by the host, once where a kernel leaves it and once as the exchange brings it from elsewhere."""
+    import ctypes as C
+    from packboost_b200 import backends as B
+    from packboost_b200.booster import _HEADER_DT, _DeviceTrainer
+    from packboost_b200.config import PackBoostConfig
+    from packboost_b200.data import pack_feature_major
+    from packboost_b200.sharding import feature_map
+    rng = np.random.default_rng(11)
+    n, f, eras, depth = 3_000, 40, 7, 2
+    X = rng.integers(0, 5, size=(n, f), dtype=np.uint8)
+    y = (X[:, 0] - X[:, 3] + rng.normal(size=n)).astype(np.float32)
+    offsets = np.linspace(0, n, eras + 1).astype(np.int32)
+    cfg = PackBoostConfig(device="cuda", pack_size=1, max_depth=depth, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=5,
+                          max_bins=5, prebinned=True, era_alpha=alpha)
+    lib = B.lib()
+    tr = _DeviceTrainer(cfg, pack_feature_major(X, None, 5), y, offsets, f, feature_map(f, 0, 1), 0, 1)
+    st, stream = C.byref(tr.st), torch.cuda.current_stream().cuda_stream
+    feats = torch.arange(f, dtype=torch.int32, device=_dev())
+    ctl = next(t for t in vars(tr).values() if isinstance(t, torch.Tensor) and t.data_ptr() == tr.st.ctl)
+    ptr, nbytes, flags = C.c_void_p(), C.c_int64(), C.c_uint32()
+
+    def word_of_flags():         # (the only word of the control block that the getter follows)
+        head = ctl.view(torch.int32)
+        for i in range(64):
+            old = head[i].item()
+            head[i] = old ^ 8
+            B.check(lib.pb_debug_flags(st, C.byref(flags)))
+            head[i] = old
+            if flags.value & 8:
+                return i
+        raise AssertionError("no such word")
+
+    def round_(own: bool, other: bool):
+        head = ctl.view(torch.int32)
+        head[at] = 0
+        B.check(lib.pb_round_begin(st, 0, stream))
+        carried = []
+        for d in range(depth):
+            if own and d == 1:
+                head[at] = 8
+            B.check(lib.pb_depth_hist_score(st, d, feats.data_ptr(), feats.data_ptr(), f, f, stream))
+            B.check(lib.pb_candidates_buffer(st, d, f, C.byref(ptr), C.byref(nbytes)))
+            off = ptr.value - tr.workspace.data_ptr()
+            cand = tr.workspace[off: off + nbytes.value].view(torch.int32).view(f, 1 << d, 6)
+            carried.append((cand[:, :, 3] & 2).ne(0).cpu().numpy())
+            if other and d == 0:
+                cand[7, 0, 3] |= 2
+            B.check(lib.pb_depth_select(st, d, feats.data_ptr(), f, stream))
+            B.check(lib.pb_depth_partition(st, d, stream))
+        B.check(lib.pb_round_end(st, stream))
+        log = tr.log_dev[: _HEADER_DT.itemsize].cpu().numpy().view(_HEADER_DT)[0]
+        assert log["n_ctx"][1] == 2                  # (both nodes of the second depth are there)
+        return carried, int(log["faults"])
+
+    at = word_of_flags()
+    carried, faults = round_(False, False)
+    assert not any(c.any() for c in carried) and faults == 0
+    carried, faults = round_(True, False)
+    assert not carried[0].any() and carried[1].all() and faults == 8
+    carried, faults = round_(False, True)
+    assert faults == 8
