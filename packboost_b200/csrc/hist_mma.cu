@@ -47,7 +47,7 @@ __host__ __device__ constexpr int mma_flush_warps(bool groups) { return groups ?
 __host__ __device__ constexpr int mma_issue_warps(int L) { return L > 1 ? 2 : 1; }
 __host__ __device__ constexpr int mma_threads(bool groups, int L) { return 32 * (kCodeWarps + mma_flush_warps(groups) + kRowWarps + mma_issue_warps(L) + kCopyWarps); }
 constexpr int kStagesMax = 3;           // blocks of codes on their way
-constexpr int kBlock = 512;             // rows of a block: 256 bytes of a feature
+constexpr int kBlock = kCutRows;           // rows of a block: 256 bytes of a feature
 constexpr int kPitch = 272;             // bytes per feature of a staged block: lanes that read 16 bytes of
                                         // consecutive features touch every bank
 constexpr int kColumns = 512;           // all of the tensor memory: a CTA per SM
@@ -65,8 +65,7 @@ struct MmaArgs {
     const int32_t* era_offsets;
     int n_eras;
     int max_bins;
-    int tiles_per_era, tile_rows;
-    int blocks, tiles, tasks;           // feature blocks, tiles of all eras, pairs of the two
+    int blocks;                         // feature blocks
     const int32_t* n_nodes_ptr;
     int n_nodes;                        // upper bound
     int node_stride;
@@ -194,6 +193,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
     __shared__ long long s_tgq[64];
     __shared__ uint32_t s_tc[64];
     __shared__ int s_kof[8];             // position of a bin among the thresholds, -1: none
+    __shared__ int s_cut[2][3];          // where this CTA's rows begin and end: feature block, era, row
 
     const int n_nodes = a.n_nodes_ptr ? min(*a.n_nodes_ptr, a.n_nodes) : a.n_nodes;
     if (n_nodes <= 0) return;
@@ -243,6 +243,29 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
             if (a.fz.thr_ids[i] == (int)threadIdx.x) k = i;
         s_kof[threadIdx.x] = k;
     }
+    // The CTAs' shares are ranges of (feature block, row), the block the slowest (totals over the eras gather in a
+    // CTA), cut at equal rows, since eras differ in length; with gains in the flush an era is not divided.  (Shares of
+    // as many tasks, and tiles counted by the longest era, where this takes, us at one and eight nodes, five bins:
+    // 2 700 000 rows x 238 features, 574 eras that grow to 2.8 times the first 163 and 313, now 131 and 264; 2 600 000
+    // x 238, 200 eras of gamma(4) lengths 170 and 295, now 109 and 213; 1 100 000 x 57, two eras, one a tenth of the
+    // other 41 and 47, now 31 and 38; equal eras 123 and 233, now 123 and 248.)
+    const int E = a.n_eras;
+    const int64_t block_work = (int64_t)a.era_offsets[E] + (a.fuse ? (int64_t)kEraRows * E : 0);
+#pragma unroll 1
+    for (int end = 0; end < 2; ++end) {
+        const int64_t work = block_work * a.blocks * (blockIdx.x + end) / gridDim.x;
+        const int fb = (int)(work / block_work);
+        const int64_t at = work - fb * block_work;
+#pragma unroll 1
+        for (int e = threadIdx.x; e <= E; e += kMmaThreads) {
+            int row = 0;
+            if (fb == a.blocks ? e == 0 : a.fuse ? cut_in_era<true>(a.era_offsets, E, at, e, row) : cut_in_era<false>(a.era_offsets, E, at, e, row)) {
+                s_cut[end][0] = e == E ? fb + 1 : fb;
+                s_cut[end][1] = e == E ? 0 : e;
+                s_cut[end][2] = e == E ? 0 : row;
+            }
+        }
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
@@ -250,22 +273,12 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
     constexpr uint32_t tmem = 0u;        // (all columns are this CTA's)
     const uint32_t a_col = tmem + (uint32_t)(a.buffers * L * N_max);
 
-    // Every role goes through the same tasks; a task's rows are [r0, r1), its blocks [b0, b1).
-    struct Task {
-        int era, fb, r0, r1, b0, b1;
-    };
-    auto task_at = [&](int t, Task& x) {     // false: nothing to do (an empty tile that would add nothing)
-        x.fb = t / a.tiles;
-        const int et = t - x.fb * a.tiles;
-        x.era = et / a.tiles_per_era;
-        tile_range(a.era_offsets[x.era], a.era_offsets[x.era + 1], et - x.era * a.tiles_per_era, a.tile_rows, x.r0, x.r1);
-        x.b0 = x.r0 / kBlock;
-        x.b1 = x.r0 < x.r1 ? (x.r1 + kBlock - 1) / kBlock : x.b0;
-        return x.r0 < x.r1 || a.fuse;
-    };
-    // (a CTA's tasks are neighbours, the feature block the slowest: totals over the eras gather here)
-    const int t0 = (int)((int64_t)a.tasks * blockIdx.x / gridDim.x), t1 = (int)((int64_t)a.tasks * (blockIdx.x + 1) / gridDim.x);
-    Task x;
+    // Every role goes through the same tasks.
+    auto next_task = [&](RowTask& x) { return next_row_task(a.era_offsets, E, a.fuse != 0, s_cut[1], kMmaTileRows, x); };
+    RowTask x;
+    x.fb = s_cut[0][0];
+    x.next = s_cut[0][1];
+    x.r1 = s_cut[0][2];
 
     if (warp < kCodeWarps) {
         // ---- A: this lane's feature and its L thresholds ----
@@ -286,8 +299,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const uint32_t to = a_col + ((uint32_t)quarter << 21);
         const uint32_t at = to + (uint32_t)(wg * (kBatch * L * 8));
         int stage = 0;
-        for (int t = t0; t < t1; ++t) {
-            if (!task_at(t, x)) continue;
+        while (next_task(x)) {
             for (int b = x.b0; b < x.b1; ++b) {
                 bool met = false;
 #pragma unroll 1
@@ -336,11 +348,10 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const int K = z.n_thr, lanes_total = a.blocks * FC;
         int buf = 0;
         uint32_t phase = 0u;
-        for (int t = t0; t < t1; ++t) {
-            if (!task_at(t, x)) continue;
+        for (bool first = true; next_task(x); first = false) {
             const int era = x.era, f = x.fb * FC + fl;
             const bool mine = f < a.n_feat, empty_tile = x.b0 == x.b1;
-            const bool fresh = t == t0 || t % a.tiles == 0, last = t + 1 == t1 || (t + 1) % a.tiles == 0;   // of a feature block here
+            const bool fresh = first || era == 0, last = x.next == E || (x.fb == s_cut[1][0] && x.next == s_cut[1][1]);   // of a feature block here
             warp_wait<true>(acc_full + buf, phase, &s_fail);
             warp_wait<true>(tot_full + buf, phase, &s_fail);
             uint32_t* tot = s_tot + buf * 3 * tot_plane;
@@ -470,8 +481,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         for (int k = 0; k < kMine; ++k) held[k] = 0u;
         int stage = 0, buf = 0;
         uint32_t turn = 0u, c_phase = 0u, acc_phase = 1u;   // (turn: how often this place was handed over)
-        for (int t = t0; t < t1; ++t) {
-            if (!task_at(t, x)) continue;
+        while (next_task(x)) {
             warp_wait(acc_empty + buf, acc_phase, &s_fail);   // the totals of this buffer are zero
             uint32_t* tot = s_tot + buf * 3 * tot_plane + lane;
             for (int b = x.b0; b < x.b1; ++b) {
@@ -553,8 +563,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const int first = (warp - kIssueWarp) * kTilesOf;    // of this warp's accumulators
         int buf = 0;
         uint32_t acc_phase = 1u;
-        for (int t = t0; t < t1; ++t) {
-            if (!task_at(t, x)) continue;
+        while (next_task(x)) {
             warp_wait(acc_empty + buf, acc_phase, &s_fail);
             uint32_t add = 0u;
             const int u0 = x.r0 / kBatchRows, u1 = x.r0 < x.r1 ? (x.r1 + kBatchRows - 1) / kBatchRows : u0;
@@ -596,8 +605,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         const int part = lane & 15;
         int stage = 0;
         uint32_t phase = 1u;
-        for (int t = t0; t < t1; ++t) {
-            if (!task_at(t, x)) continue;
+        while (next_task(x)) {
             uint32_t rows[kMine];
 #pragma unroll
             for (int i = 0; i < kMine; ++i) {
@@ -746,21 +754,10 @@ int launch_hist_mma(const HistLaunch& h, cudaStream_t stream) {
     }();
     a.failed = failed;
     const int blocks = (h.n_feat + s.features - 1) / s.features;
-    a.tile_rows = kMmaTileRows;
-    a.tiles_per_era = 1;
-    if (h.max_era_rows > kTileRowsMax) {
-        // as many tiles as fill whole waves of CTAs
-        const int64_t least = tiles_of(h.max_era_rows, kMmaTileRows), per_tile = (int64_t)h.n_eras * blocks;
-        const int64_t waves = (least * per_tile + 147) / 148;
-        int64_t tiles = waves * 148 / per_tile;
-        if (tiles < least) tiles = least;
-        a.tile_rows = tiles_of(tiles_of(h.max_era_rows, tiles), kBlock) * kBlock;
-        a.tiles_per_era = tiles_of(h.max_era_rows, a.tile_rows);
-        if (!h.zeroed) {
-            const size_t cells = (size_t)h.n_feat * h.node_stride * h.n_eras * h.max_bins;
-            PB_CUDA_TRY(cudaMemsetAsync(h.cnt, 0, cells * sizeof(uint32_t), stream));
-            PB_CUDA_TRY(cudaMemsetAsync(h.gsum, 0, cells * sizeof(int64_t), stream));
-        }
+    if (!h.fuse && !h.zeroed) {
+        const size_t cells = (size_t)h.n_feat * h.node_stride * h.n_eras * h.max_bins;
+        PB_CUDA_TRY(cudaMemsetAsync(h.cnt, 0, cells * sizeof(uint32_t), stream));
+        PB_CUDA_TRY(cudaMemsetAsync(h.gsum, 0, cells * sizeof(int64_t), stream));
     }
     if (h.fuse) {
         a.fuse = 1;
@@ -773,12 +770,9 @@ int launch_hist_mma(const HistLaunch& h, cudaStream_t stream) {
             PB_CUDA_TRY(cudaMemsetAsync(a.fz.lg_tot, 0, tot * sizeof(int64_t), stream));
         }
     }
-    const int64_t tasks = (int64_t)h.n_eras * a.tiles_per_era * blocks;
-    if (tasks > (1 << 30)) return fail_arg("histogram of too many tiles");
     a.blocks = blocks;
-    a.tiles = h.n_eras * a.tiles_per_era;
-    a.tasks = (int)tasks;
-    const dim3 grid((unsigned)(tasks < 148 ? tasks : 148));
+    const int64_t shares = (int64_t)blocks * (h.fuse ? h.n_eras : tiles_of(h.rows_pad, kCutRows));
+    const dim3 grid((unsigned)(shares < 148 ? shares : 148));
     prof_begin(h.prof, kProfHist, stream);
     const int rc = s.thresholds_per_lane == 4 ? (s.batch == 4 ? launch_l<4, 4, false, false>(a, grid, s.smem, stream) : launch_l<4, 2, false, false>(a, grid, s.smem, stream))
                    : s.thresholds_per_lane == 2 ? (mma_groups(h.n_nodes) ? launch_l<2, 4, true, false>(a, grid, s.smem, stream) : launch_l<2, 4, false, false>(a, grid, s.smem, stream))

@@ -22,4 +22,49 @@ PB_ROWS_FN void tile_range(int era_begin, int era_end, int index, int tile, int&
     r1 = era_end - r0 > tile ? r0 + tile : era_end;
 }
 
+// Where a share of the work of a feature block ends.  `at` counts rows (WHOLE: and kEraRows more for each era, which
+// stand for its flush).  WHOLE: between two eras, at the nearest place, so that a share differs from its part of the
+// work by half an era at each end at most; otherwise at any multiple of kCutRows.  True for exactly one e of
+// [0, n_eras], the era in which the rows after the cut begin, at `row`; n_eras: none is left (WHOLE alone).
+constexpr int kEraRows = 512, kCutRows = 512;
+template <bool WHOLE>
+PB_ROWS_FN bool cut_in_era(const int* offsets, int n_eras, int64_t at, int e, int& row) {
+    row = WHOLE ? offsets[e] : (int)(at / kCutRows * kCutRows);
+    if (!WHOLE) return e < n_eras && offsets[e] <= row && row < offsets[e + 1];
+    // twice the work before the middle of an era
+    auto middle = [&](int i) { return (int64_t)offsets[i] + offsets[i + 1] + (int64_t)kEraRows * (2 * i + 1); };
+    return (e == 0 || middle(e - 1) < 2 * at) && (e == n_eras || middle(e) >= 2 * at);
+}
+
+// A step through the rows of a share: rows [r0, r1), blocks [b0, b1) of kCutRows rows, of an era, or (not `whole`) of
+// as much of it as a tile may have.  Eras without rows are steps where they are whole: their gains have to be written.
+struct RowTask {
+    int fb, era, r0, r1, b0, b1;
+    int next;                            // era of the rows from r1 on
+};
+
+// The step after x up to the cut at `end` = {feature block, era, row}; false: none.  x starts as {fb, next, r1} of a cut.
+PB_ROWS_FN bool next_row_task(const int* offsets, int n_eras, bool whole, const int* end, int tile, RowTask& x) {
+    for (;;) {
+        if (x.next == n_eras) {
+            ++x.fb;
+            x.next = x.r1 = 0;
+        }
+        const bool last_block = x.fb == end[0];
+        if (x.fb > end[0] || (last_block && (x.next > end[1] || (x.next == end[1] && x.r1 >= end[2])))) return false;
+        const int era_end = offsets[x.next + 1];
+        x.era = x.next;
+        x.r0 = x.r1;
+        x.r1 = era_end;
+        if (!whole) {
+            if (era_end - x.r0 > tile) x.r1 = (x.r0 + tile) / kCutRows * kCutRows;
+            if (last_block && x.era == end[1] && end[2] < x.r1) x.r1 = end[2];
+        }
+        if (x.r1 == era_end) ++x.next;
+        x.b0 = x.r0 / kCutRows;
+        x.b1 = x.r0 < x.r1 ? (x.r1 + kCutRows - 1) / kCutRows : x.b0;
+        if (x.r0 < x.r1 || whole) return true;
+    }
+}
+
 }  // namespace pb

@@ -202,6 +202,78 @@ def test_row_ranges_of_tiles_up_to_the_largest_table(tmp_path):
         assert [int(v) for v in out[3 * k: 3 * k + 3]] == [r0, min(r0 + t, e), -(-n // t)], (b, e, i, t, n)
 
 
+_SHARES = """#include "rows.cuh"
+#include <cstdio>
+#include <vector>
+using namespace pb;
+int main() {                             // eras, feature blocks, shares, whole, tile, offsets -> share, block, era, r0, r1, b0, b1
+    int E, blocks, grid, whole, tile;
+    while (std::scanf("%d %d %d %d %d", &E, &blocks, &grid, &whole, &tile) == 5) {
+        std::vector<int> off(E + 1);
+        for (int& o : off) std::scanf("%d", &o);
+        const int64_t work = off[E] + (whole ? (int64_t)kEraRows * E : 0);
+        auto cut = [&](int64_t share, int* c) {
+            const int64_t at = work * blocks * share / grid;
+            const int fb = (int)(at / work);
+            int hits = 0, row = 0;
+            for (int e = 0; e <= E; ++e)
+                if (fb == blocks ? e == 0 : whole ? cut_in_era<true>(off.data(), E, at - fb * work, e, row) : cut_in_era<false>(off.data(), E, at - fb * work, e, row)) {
+                    ++hits;
+                    c[0] = e == E ? fb + 1 : fb;
+                    c[1] = e == E ? 0 : e;
+                    c[2] = e == E || fb == blocks ? 0 : row;
+                }
+            return hits == 1;
+        };
+        for (int i = 0; i < grid; ++i) {
+            int from[3], to[3];
+            if (!cut(i, from) || !cut(i + 1, to)) return 1;
+            RowTask x{from[0], 0, 0, from[2], 0, 0, from[1]};
+            while (next_row_task(off.data(), E, whole != 0, to, tile, x))
+                std::printf("%d %d %d %d %d %d %d\\n", i, x.fb, x.era, x.r0, x.r1, x.b0, x.b1);
+        }
+        std::printf("-1\\n");
+    }
+    return 0;
+}
+"""
+
+
+def test_shares_of_rows_are_even_and_complete(tmp_path):
+    """Shares of a histogram launch: every row of every feature block in one of them, and none longer than its part by
+    more than an era (eras kept whole; half a one at each end) or a block of rows (eras divided), whatever the lengths."""
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "packboost_b200", "csrc")
+    (tmp_path / "shares.cpp").write_text(_SHARES)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fsanitize=undefined", "-fno-sanitize-recover", "-I", csrc,
+                    str(tmp_path / "shares.cpp"), "-o", str(tmp_path / "shares")], check=True)
+    rng = np.random.default_rng(5)
+    last = 2 ** 31 - 513
+    lengths = [[1], [700], [9_000], [0, 5, 0, 0, 9_000, 0], [1_000_000, 100_000], [10] * 300 + [40_000] + [0] * 7, [last - 70_000, 0, 70_000],
+               [4_700] * 574, rng.gamma(4.0, 1_175.0, 574).astype(int).tolist(), np.linspace(2_500, 6_900, 574).astype(int).tolist(),
+               rng.gamma(4.0, 700.0, 120).astype(int).tolist(), [0] * 40 + [3] * 40]
+    asked = [(n, blocks, grid, whole) for n in lengths for blocks in (1, 2, 7) for whole in (0, 1) for grid in (1, 3, 148)
+             if grid <= blocks * (len(n) if whole else -(-sum(n) // 512)) and (not whole or sum(n) < 1 << 30)]
+    text = "\n".join(" ".join(map(str, [len(n), blocks, grid, whole, 32_256] + np.concatenate([[0], np.cumsum(n)]).tolist())) for n, blocks, grid, whole in asked)
+    out = subprocess.run([str(tmp_path / "shares")], input=text, capture_output=True, text=True, check=True).stdout
+    for (n, blocks, grid, whole), part in zip(asked, out.split("-1\n")):
+        off = np.concatenate([[0], np.cumsum(n)]).astype(np.int64)
+        t = np.array([line.split() for line in part.splitlines()], dtype=np.int64).reshape(-1, 7)
+        share, fb, era, r0, r1, b0, b1 = t.T
+        assert ((off[era] <= r0) & (r0 <= r1) & (r1 <= off[era + 1]) & (b0 == r0 // 512) & (b1 == np.where(r0 < r1, -(-r1 // 512), b0))).all()
+        assert (np.diff(share) >= 0).all()
+        if whole:                                   # every era of every block once, in order
+            assert (fb * len(n) + era).tolist() == list(range(blocks * len(n))) and (r0 == off[era]).all() and (r1 == off[era + 1]).all()
+            most = max(n) + 512
+        else:                                       # the rows follow on one another
+            assert (r0 < r1).all() and (r1 - r0 <= 32_256).all()
+            place = fb * off[-1] + r0
+            assert (place[1:] == (fb * off[-1] + r1)[:-1]).all() and place[0] == 0 and fb[-1] * off[-1] + r1[-1] == blocks * off[-1]
+            most = 512
+        loads = np.bincount(share, weights=(r1 - r0) + 512 * whole, minlength=grid)
+        assert loads.max() <= blocks * (off[-1] + 512 * whole * len(n)) / grid + most, (n[:5], blocks, grid, whole)
+
+
 @pytest.mark.parametrize("flags", [[], ["-U__SSE2__"]])
 def test_host_sources_need_no_x86(flags, tmp_path):
     """The ring copy builds without x86 intrinsics (``-U__SSE2__``: as on another host) and moves every
