@@ -53,7 +53,7 @@ def build(force: bool = False, verbose: bool = False, debug_bounds: bool = False
     lib_path = DEBUG_LIB_PATH if debug_bounds else LIB_PATH
     os.makedirs(objdir, exist_ok=True)
     headers = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "des_math.cuh"), os.path.join(CSRC, "stream_copy.h"),
-               os.path.join(CSRC, "divide.cuh"), os.path.join(CSRC, "rows.cuh"),
+               os.path.join(CSRC, "divide.cuh"), os.path.join(CSRC, "rows.cuh"), os.path.join(CSRC, "hist_rule.h"),
                os.path.join(HERE, "..", "include", "packboost_b200.h")]
     objs = []
     log_lines = []

@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "des_math.cuh"
+#include "hist_rule.h"
 #include "rows.cuh"
 
 namespace pb {
@@ -659,12 +660,11 @@ struct MmaShape {
 
 MmaShape mma_shape(int n_nodes, int n_feat, int max_bins, bool fused) {
     MmaShape s;
-    const int N = mma_columns(n_nodes, mma_groups(n_nodes)), tp = max_bins <= 5 ? 4 : 8;
-    const int L = n_nodes <= 4 && n_feat > 128 * 2 / tp ? 4 : n_nodes <= 16 ? 2 : 1;
+    const int N = mma_columns(n_nodes, mma_groups(n_nodes)), L = mma_per_lane(n_nodes, n_feat, max_bins);
     s.thresholds_per_lane = L;
     s.batch = n_nodes > 2 && L == 4 ? 2 : 4;
-    s.groups = tp / L;
-    s.features = 128 / s.groups;
+    s.groups = mma_thresholds(max_bins) / L;
+    s.features = mma_features(n_nodes, n_feat, max_bins);
     const int operands = kSlots * s.batch * L * 8;
     s.buffers = 2 * L * N + operands <= kColumns ? 2 : 1;
     const size_t sums = fused ? (size_t)n_nodes * L * 128 * 12 : 0;
@@ -684,22 +684,6 @@ int launch_l(const MmaArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
 
 }  // namespace
 
-// Where the contraction is the faster one (us, this kernel / hist_lane_kernel, five bins, at 1, 2, 4, 8, 16, 32
-// nodes unless said).  Eras of several tiles, whose sums both add to a stored histogram:
-//   1 300 000 rows x 57 features, one era     33/56 36/54 42/63 39/61 47/78 59/87, 64 nodes 83/129
-//   2 600 000 x 238, 200 eras                 118/181 120/191 158/197 181/229 203/269 333/407, 64 nodes 596/619
-//   1 000 000 x 100, 20 eras                  33/46 34/46 43/49 52/51 57/58 92/81, 64 nodes 142/125
-//   300 000 x 40, one era                     20/39 23/37 28/33 30/34 32/32 32/37;   100 000 x 30  16/22 ... 21/25 22/21
-//   1 300 000 x 57, six bins                  43/54 47/55 55/59 53/61 59/96 94/98, 64 nodes 148/120
-//   10 000 x 20, one era                      14/12 14/12 14/12 16/13 18/13 20/13
-// Eras of one tile, whose flush makes the gains:
-//   2 700 000 x 238, 574 eras                 126/172 128/172 165/188 202/229 227/255 486/385
-//   1 500 000 x 200, 300 eras                 88/138 90/138 116/127 127/141 143/152 243/212
-//   700 000 x 100, 300 eras                   38/48 40/46 48/47 51/51 69/57 131/83
-//   300 000 x 60, 60 eras                     24/20 26/20 30/22 30/28 32/28 36/29
-//   1 500 000 x 200, 300 eras, six bins       144/153 147/156 188/155 203/196 257/274 495/297
-// So: it takes features for most of a CTA's lanes and rows for many tiles, and with many nodes the flush and
-// the columns of the nodes weigh more than the row steps saved.
 bool hist_mma_takes(const HistLaunch& h) {
 #ifdef PB_DEBUG_BOUNDS
     return false;   // codes are no index here: the build that checks them keeps to the kernel where they are
@@ -712,16 +696,7 @@ bool hist_mma_takes(const HistLaunch& h) {
     const bool fused = h.fuse != nullptr, tiled = h.max_era_rows > kTileRowsMax;
     if (forced == 0 || h.code_bits != 4 || h.max_bins > 8 || h.n_nodes > (fused ? 32 : 64) || fused == tiled) return false;
     if (forced == 1) return true;
-    const MmaShape s = mma_shape(h.n_nodes, h.n_feat, h.max_bins, fused);
-    const int64_t lanes = (int64_t)(h.n_feat + s.features - 1) / s.features * s.features;   // features there would be room for
-    if (fused) {
-        if (h.max_bins > 5 || (int64_t)h.n_eras * (lanes / s.features) < 100) return false;
-        return h.n_feat > 128 ? h.n_nodes <= 16 && (int64_t)h.n_eras * (lanes / s.features) >= 444 : h.n_feat > 64 && h.n_nodes <= 2;
-    }
-    const int64_t work = h.rows_pad * h.n_feat;
-    if (h.n_nodes <= 8) return work >= 3000000;
-    if (h.n_nodes <= 16) return work >= 10000000;
-    return work >= 10000000 && h.n_feat * 100 >= lanes * 85 && (h.n_nodes <= 32 || h.max_bins <= 5);
+    return mma_pays(fused, h.n_nodes, h.n_feat, h.max_bins, h.rows_pad, h.n_eras);
 #endif
 }
 

@@ -274,6 +274,60 @@ def test_shares_of_rows_are_even_and_complete(tmp_path):
         assert loads.max() <= blocks * (off[-1] + 512 * whole * len(n)) / grid + most, (n[:5], blocks, grid, whole)
 
 
+_RULE = """#include "hist_rule.h"
+#include <cstdio>
+int main() {
+    long long fused, nodes, feats, bins, rows, eras;
+    while (std::scanf("%lld %lld %lld %lld %lld %lld", &fused, &nodes, &feats, &bins, &rows, &eras) == 6)
+        std::printf("%d\\n", (int)pb::mma_pays(fused != 0, (int)nodes, (int)feats, (int)bins, rows, eras));
+    return 0;
+}
+"""
+
+
+def test_few_bins_take_the_kernel_that_measured_faster(tmp_path):
+    """us of the contraction and of the atomics, measured side by side, by number of bins and nodes: where they are
+    a tenth apart or more in favour of the atomics, the rule is with them, and with the contraction where it saves a quarter
+    of a launch of up to four nodes and five bins."""
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "packboost_b200", "csrc")
+    (tmp_path / "rule.cpp").write_text(_RULE)
+    subprocess.run(["g++", "-std=c++17", "-I", csrc, str(tmp_path / "rule.cpp"), "-o", str(tmp_path / "rule")], check=True)
+    measured = [      # gains in the flush, rows, features, eras, bins, (nodes, contraction, atomics) ...
+        (1, 2_700_000, 238, 574, 2, [(1, 122, 179), (2, 125, 182), (4, 156, 198), (8, 248, 227), (32, 589, 379)]),
+        (1, 2_700_000, 238, 574, 5, [(1, 123, 170), (2, 129, 171), (4, 160, 187), (8, 248, 229), (16, 289, 256), (32, 572, 393)]),
+        (1, 2_700_000, 238, 574, 6, [(1, 226, 192), (2, 232, 199), (4, 291, 240)]),
+        (1, 1_000_000, 238, 574, 3, [(1, 69, 129), (2, 86, 133), (16, 278, 223), (32, 567, 371)]),
+        (1, 1_000_000, 238, 574, 5, [(1, 68, 119), (2, 88, 121), (8, 180, 131), (16, 269, 159), (32, 537, 242)]),
+        (1, 1_500_000, 200, 300, 5, [(1, 86, 136), (2, 90, 137), (8, 156, 138), (16, 176, 154), (32, 296, 211)]),
+        (1, 700_000, 100, 300, 5, [(1, 37, 57), (2, 39, 57), (8, 66, 53), (16, 94, 61), (32, 167, 96)]),
+        (1, 150_000, 70, 150, 5, [(1, 24, 21), (4, 31, 22), (8, 35, 22), (16, 49, 28), (32, 72, 36)]),
+        (1, 300_000, 60, 60, 5, [(1, 25, 20), (2, 27, 18), (4, 31, 20), (8, 31, 27), (16, 37, 27), (32, 39, 29)]),
+        (0, 1_300_000, 57, 1, 2, [(1, 33, 48), (32, 64, 53)]),
+        (0, 1_300_000, 57, 1, 5, [(1, 35, 47), (32, 66, 74)]),
+        (0, 2_600_000, 238, 200, 2, [(1, 109, 203), (2, 111, 207), (4, 137, 216), (32, 401, 312), (64, 646, 418)]),
+        (0, 2_600_000, 238, 200, 3, [(1, 109, 203), (2, 113, 207), (4, 139, 221), (32, 401, 362)]),
+        (0, 2_600_000, 238, 200, 5, [(1, 111, 200), (2, 115, 206), (4, 145, 210)]),
+        (0, 2_600_000, 238, 200, 6, [(8, 397, 307), (32, 724, 480), (64, 1190, 678)]),
+        (0, 1_000_000, 128, 20, 2, [(32, 92, 62), (64, 127, 78)]),
+        (0, 1_000_000, 128, 20, 6, [(4, 61, 53), (8, 88, 59), (32, 164, 100), (64, 242, 141)]),
+        (0, 1_000_000, 100, 20, 5, [(1, 33, 56), (2, 35, 55), (4, 41, 57), (32, 93, 78)]),
+        (0, 300_000, 40, 1, 5, [(1, 19, 35), (2, 23, 35), (16, 34, 29), (64, 39, 29)]),
+        (0, 300_000, 40, 1, 8, [(64, 61, 43)]),
+        (0, 100_000, 30, 1, 3, [(1, 15, 25), (8, 25, 16), (16, 27, 16), (32, 25, 14), (64, 35, 16)]),
+        (0, 100_000, 30, 1, 5, [(4, 22, 20), (8, 20, 18), (32, 25, 18), (64, 31, 20)]),
+        (0, 30_000, 100, 3, 5, [(1, 16, 11), (2, 16, 10), (4, 18, 12), (8, 18, 12), (16, 23, 12), (32, 28, 14)]),
+        (0, 150_000, 16, 2, 5, [(2, 16, 14), (4, 20, 16), (8, 18, 14), (16, 23, 16), (32, 29, 16), (64, 43, 20)])]
+    flat = [(fused, n, feats, bins, rows, eras, a, b) for fused, rows, feats, eras, bins, at in measured for n, a, b in at]
+    out = subprocess.run([str(tmp_path / "rule")], input="\n".join(" ".join(map(str, c[:6])) for c in flat), capture_output=True, text=True,
+                         check=True).stdout.split()
+    for c, takes in zip(flat, out):
+        if c[6] >= 1.1 * c[7]:
+            assert takes == "0", c
+        if c[6] <= 0.75 * c[7] and c[1] <= 4 and c[3] <= 5:
+            assert takes == "1", c
+
+
 @pytest.mark.parametrize("flags", [[], ["-U__SSE2__"]])
 def test_host_sources_need_no_x86(flags, tmp_path):
     """The ring copy builds without x86 intrinsics (``-U__SSE2__``: as on another host) and moves every
