@@ -30,6 +30,7 @@
 // Float arithmetic as in the scorer: the same separately rounded operations in the same order
 // (this file is compiled with -fmad=false), so candidates are bit-identical to the other path's.
 
+#include <stdio.h>
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -43,6 +44,17 @@ namespace {
 
 constexpr int kWalkWarpsMax = 32;
 constexpr int kWalkInv = 4096;           // longest table of era reciprocals
+
+// Four codes, each within the cells of its node (32 BPL of them) whatever the byte: one that is no bin would else be
+// counted in another node's cells, or add a sum to counts, which index the table of divisors.
+template <int BPL>
+__device__ __forceinline__ uint32_t cells_of(uint32_t codes) {
+#ifdef PB_DEBUG_BOUNDS
+    return codes;                        // (each is looked at where it is used)
+#else
+    return BPL < 8 ? codes & (uint32_t)(32 * BPL - 1) * 0x01010101u : codes;
+#endif
+}
 
 struct RowGroup {                        // four consecutive rows
     uint32_t codes;
@@ -254,13 +266,13 @@ __global__ void __launch_bounds__(32 * WARPS, (BPL <= 4 && MODE != kGeneral && W
             return;
         }
 #endif
-        // (a byte that is no bin falls into a neighbour's cells or, after the last, into the gains)
         const uint32_t at = (n < (uint32_t)live ? base + n * PAIR : trash) + code * (4u * COPIES);
         asm volatile("red.shared.add.u32 [%0], %1;\n red.shared.add.u32 [%0 + %3], %2;" ::"r"(at),
                      "r"(((uint32_t)q & lo_mask) * one_a + 1u), "r"(q >> LB), "n"(4 * words) : "memory");
     };
     // `e`, `lim`: era of the batch at the warp's last chunk and where that era ends (rows ascend)
     auto add_group = [&](int c, int r0, int r1, RowGroup& x, int& e, int& lim) {
+        x.codes = cells_of<BPL>(x.codes);
         const int first = 128 * c;       // (the warp's: all lanes decide alike)
         if (!TILES)
             while (first >= lim) lim = s_off[++e + 1];
@@ -620,6 +632,7 @@ __global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 && BPL <= 4) ? 2 : 1)
     };
     // rows [r0, r1) of two eras, the second from mid on
     auto add_group = [&](int c, int r0, int mid, int r1, uint32_t set, RowGroup& x) {
+        x.codes = cells_of<BPL>(x.codes);
         const int r = 128 * c + 4 * lane;
         const uint32_t n0 = (x.slots.x & 0xFFFFu) - (uint32_t)node0, n1 = (x.slots.x >> 16) - (uint32_t)node0;
         const uint32_t n2 = (x.slots.y & 0xFFFFu) - (uint32_t)node0, n3 = (x.slots.y >> 16) - (uint32_t)node0;
@@ -820,10 +833,24 @@ struct WalkShape {
 // The forms a launch may take: batches of sixteen or thirty-two warps, a warp per node of either.
 enum WalkForm { kBatch16 = 0, kBatch32 = 1, kNodes16 = 2, kNodes32 = 3, kWalkForms = 4 };
 
-static bool walk_takes(const WalkLaunch& a, int form) {
-    if (form == kBatch16) return true;
+static bool walk_can(const WalkLaunch& a, int form) {
     const bool unit = a.era_alpha <= 0.f && a.direction_weight == 0.f && a.n_eras < kWalkInv && a.max_era_rows <= a.tile_rows;
-    if (!unit || a.max_bins > 128) return false;
+    return form == kBatch16 || (unit && a.max_bins <= 128);
+}
+
+// PACKBOOST_WALK_FORM=0 .. 3: that form wherever it can be had, and a line for each launch, for comparisons.
+static int forced_walk() {
+    static const int form = [] {
+        const char* e = getenv("PACKBOOST_WALK_FORM");
+        return e && e[0] >= '0' && e[0] < '0' + kWalkForms && e[1] == 0 ? e[0] - '0' : -1;
+    }();
+    return form;
+}
+
+static bool walk_takes(const WalkLaunch& a, int form) {
+    if (!walk_can(a, form)) return false;
+    if (forced_walk() >= 0 && walk_can(a, forced_walk())) return form == forced_walk();
+    if (form == kBatch16) return true;
     // (a warp per node of sixteen: from about a hundred rows per era and node on; 20 000 rows, 64 features, 20
     // eras take 40 us that way and 35 as more and smaller CTAs)
     return form == kBatch32 || (form == kNodes16 ? a.n_nodes == 16 && a.n_rows >= (int64_t)1600 * a.n_eras : a.n_nodes >= 32);
@@ -911,6 +938,9 @@ int launch_walk(WalkLaunch a, cudaStream_t stream) {
     if (a.max_bins > 256) return fail_arg("max_bins=%d outside [2,256]", a.max_bins);
     WalkShape s;
     best_walk(a, &s);
+    if (forced_walk() >= 0)
+        fprintf(stderr, "%s<%d> warps=%d mode=%d copies=%d nodes=%d groups=%d table=%d mass=%d\n", s.own ? "walk_nodes_kernel" : "walk_kernel",
+                s.bpl, s.warps, s.mode, s.copies, a.n_nodes, s.groups, (int)s.div_table, a.mass ? 1 : 0);
     a.cell_nodes = s.cell_nodes;
     const int bpl = s.bpl, mode = s.mode, copies = s.copies, warps = s.warps;
     const size_t smem = s.smem;

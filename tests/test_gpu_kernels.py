@@ -701,6 +701,48 @@ def test_era_walk_with_a_warp_per_node(n, f, eras, bins, depth, extra, tmp_path)
     test_era_walk_equals_the_stored_histogram_path(n, f, eras, bins, depth, extra, tmp_path)
 
 
+@pytest.mark.parametrize("form", range(4))
+def test_era_walk_with_a_byte_that_is_no_bin(form):
+    """Bytes of 255 in a column that packing did not check stay within the cells of their node: to the right of every
+    threshold, so nothing changes.  (Four rows are fewer than min_samples_leaf: the column, constant but for
+    them, is never split.)"""
+    import subprocess
+    import sys
+    script = r"""
+import sys
+import numpy as np, torch
+from packboost_b200.booster import _DeviceTrainer
+from packboost_b200.config import PackBoostConfig
+from packboost_b200.data import pack_feature_major
+from packboost_b200.sharding import feature_map
+rng = np.random.default_rng(2)
+n, f, eras, depth = 6_000, 6, 8, 6
+X = rng.integers(0, 17, size=(n, f), dtype=np.uint8)
+y = (X[:, 1] + X[:, 2] * (X[:, 3] > 4) + rng.normal(size=n)).astype(np.float32)
+X[:, 0] = 16
+logs = []
+for bad in (False, True):
+    if bad:
+        X[[5, 2_500, 4_900, 5_999], 0] = 255         # (the last: in the eighth era, whose cells are the last)
+    cfg = PackBoostConfig(device="cuda", pack_size=1, max_depth=depth, learning_rate=0.2, lambda_l2=1.0, min_samples_leaf=30,
+                          max_bins=17, prebinned=True)
+    tr = _DeviceTrainer(cfg, pack_feature_major(X, None, 17), y, np.linspace(0, n, eras + 1).astype(np.int32), f, feature_map(f, 0, 1), 0, 1)
+    ticket = tr.run_round([np.arange(f, dtype=np.int32)] * depth)
+    head, winners = tr.read_log(ticket)
+    logs.append((head.copy(), winners.copy()))
+(h0, w0), (h1, w1) = logs
+assert np.array_equal(h0["n_ctx"], h1["n_ctx"]) and h0["n_ctx"].reshape(-1)[4] == 16 and h0["n_ctx"].reshape(-1)[5] > 16
+for d in range(depth):
+    a, b = (1 << d) - 1, (1 << d) - 1 + int(h0["n_ctx"].reshape(-1)[d])
+    assert np.array_equal(w0[a:b], w1[a:b]) and (w1["feature"][a:b] != 0).all(), d
+print("ok")
+"""
+    res = subprocess.run([sys.executable, "-c", script], env=dict(os.environ, PACKBOOST_WALK="1", PACKBOOST_WALK_FORM=str(form)),
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True)
+    assert res.returncode == 0 and res.stdout.strip().endswith("ok"), res.stderr[-2000:]
+    assert ("walk_nodes_kernel<1>" if form >= 2 else "walk_kernel<1>") in res.stderr
+
+
 @pytest.mark.parametrize("form", ["frontier", "helper"])
 @pytest.mark.parametrize("n,eras,bins", [(3_000, 7, 5), (20_000, 1, 5), (17_000, 2, 4), (6_000, 9, 14)])
 def test_directional_term_streamed_with_the_gains_matches_the_oracle(form, n, eras, bins, monkeypatch):
