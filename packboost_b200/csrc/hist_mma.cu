@@ -19,15 +19,17 @@
 //            and left sums (summed over the CTA's eras before they go out), or a tile's share of the histogram.
 // Operands pass in batches of 64 or 128 rows through three places, each with code and row warps of its own.
 //
-// Bound: the instructions of all roles together (485 per 32 rows and 128 features at one node, 164 of them for A;
-// ALU pipe 62 %, issue slots 60 %, tensor pipe 16 % of the time).  What it took:
+// Bound: no unit of the SM (ALU pipe 62 % of the time, issue slots 60 %, tensor pipe 16 %; 485 instructions per 32 rows and
+// 128 features at one node, 164 of them for A) but the hand-overs between the roles: a batch waits for its stores into
+// tensor memory and at two barriers, in one of three places.  What it took:
 // the warps of a place wait at one barrier behind one poller (two dozen polling warps made a wait that is over
 // cost 350 cycles), the issuers wait at a barrier too (a ready mbarrier costs a thread that issues tcgen05.mma
 // 200 cycles, a barrier a few), codes come by cp.async from four warps (bulk copies of a line each: 35 cycles
 // each, 416 us where this takes 126), and three places (two: 141 us).
 // 2 700 000 rows x 238 features, 574 eras: 172 us by atomics, 126 so, at one node (2.7 TB/s of codes and row
-// state, 41 % of measured copy bandwidth); figures by size at the rule below.
+// state, 41 % of measured copy bandwidth); figures by size in hist_rule.h.
 
+#include <stdio.h>
 #include <stdlib.h>
 
 #include <type_traits>
@@ -47,7 +49,7 @@ constexpr int kCodeWarps = 4 * kSlots, kRowWarps = 2 * kSlots, kCopyWarps = 4;  
 __host__ __device__ constexpr int mma_flush_warps(bool groups) { return groups ? 8 : 4; }
 __host__ __device__ constexpr int mma_issue_warps(int L) { return L > 1 ? 2 : 1; }
 __host__ __device__ constexpr int mma_threads(bool groups, int L) { return 32 * (kCodeWarps + mma_flush_warps(groups) + kRowWarps + mma_issue_warps(L) + kCopyWarps); }
-constexpr int kStagesMax = 3;           // blocks of codes on their way
+constexpr int kStages = 3;           // blocks of codes on their way
 constexpr int kBlock = kCutRows;           // rows of a block: 256 bytes of a feature
 constexpr int kPitch = 272;             // bytes per feature of a staged block: lanes that read 16 bytes of
                                         // consecutive features touch every bank
@@ -76,7 +78,7 @@ struct MmaArgs {
     HistFuse fz;
     uint32_t* flags;
     int groups;                         // lanes of a feature: TP / L
-    int stages, buffers;                // blocks of codes; accumulators: 2 where they fit
+    int buffers;                        // accumulators: 2 where they fit
     int failed;                         // 1: as after a wait that ran out
 };
 
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
     constexpr int kFlushWarp0 = kCodeWarps, kRowWarp0 = kFlushWarp0 + kFlushWarps, kIssueWarp = kRowWarp0 + kRowWarps, kCopyWarp0 = kIssueWarp + mma_issue_warps(L);
     constexpr int kIssueWarps = mma_issue_warps(L), kTilesOf = L / kIssueWarps;   // (accumulators of one issuing warp)
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t full_c[kStagesMax], empty_c[kStagesMax], empty[kSlots], acc_full[2], acc_empty[2], tot_full[2], last;
+    __shared__ __align__(8) uint64_t full_c[kStages], empty_c[kStages], empty[kSlots], acc_full[2], acc_empty[2], tot_full[2], last;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_fail;
     __shared__ uint32_t s_taken[kSlots];   // times the issuing warps have taken over a place, all together
@@ -204,7 +206,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
     const int k_bytes = N_max * 32, batch_bytes = kBatch * k_bytes;   // of B
     const int stage_bytes = mma_stage_bytes(FC);
     unsigned char* s_codes = smem;                            // [stages]{[FC][kPitch], slots, gradients}
-    unsigned char* s_b = smem + a.stages * stage_bytes;        // [kSlots][kBatch][N / 8][2][8][16]
+    unsigned char* s_b = smem + kStages * stage_bytes;        // [kSlots][kBatch][N / 8][2][8][16]
     uint32_t* s_tot = reinterpret_cast<uint32_t*>(s_b + kSlots * batch_bytes);   // [buffers][count, low, high][n_nodes][32]: a lane's own cells
     const int tot_plane = a.n_nodes * 32;
     // (fused) left sums over the CTA's eras of a feature block: a flush thread's own, [n_nodes][L][128]
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 32) {
-        for (int i = 0; i < kStagesMax; ++i) {
+        for (int i = 0; i < kStages; ++i) {
             mbar_init(full_c + i, 32 * kCopyWarps);
             mbar_init(empty_c + i, kCodeWarps + kRowWarps);
         }
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                 if (!met) meet(kSlotBarrier + wg, kSlotThreads);   // (a stage is given back only after it came)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty_c + stage);
-                if (++stage == a.stages) stage = 0;
+                if (++stage == kStages) stage = 0;
             }
         }
     } else if (warp < kRowWarp0) {
@@ -547,7 +549,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty_c + stage);
-                if (++stage == a.stages) { stage = 0; c_phase ^= 1u; }
+                if (++stage == kStages) { stage = 0; c_phase ^= 1u; }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(tot_full + buf);
@@ -632,7 +634,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                     if (row < a.rows_pad) copy16(state + (uint32_t)(i * 16), g ? (const void*)(a.gq + row) : (const void*)(a.slot + row));
                 }
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_at(full_c + stage)) : "memory");
-                if (++stage == a.stages) { stage = 0; phase ^= 1u; }
+                if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -654,7 +656,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
 }
 
 struct MmaShape {
-    int thresholds_per_lane, batch, groups, features, stages, buffers;
+    int thresholds_per_lane, batch, groups, features, buffers;
     size_t smem;
 };
 
@@ -669,9 +671,7 @@ MmaShape mma_shape(int n_nodes, int n_feat, int max_bins, bool fused) {
     s.buffers = 2 * L * N + operands <= kColumns ? 2 : 1;
     const size_t sums = fused ? (size_t)n_nodes * L * 128 * 12 : 0;
     const size_t fixed = (size_t)kSlots * s.batch * N * 32 + sums + (size_t)s.buffers * n_nodes * 32 * 12;
-    s.stages = kStagesMax;
-    while (s.stages > 2 && fixed + (size_t)s.stages * mma_stage_bytes(s.features) > kSharedMost) --s.stages;
-    s.smem = fixed + (size_t)s.stages * mma_stage_bytes(s.features);
+    s.smem = fixed + (size_t)kStages * mma_stage_bytes(s.features);   // (183 KB at most: 64 nodes)
     return s;
 }
 
@@ -684,18 +684,23 @@ int launch_l(const MmaArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
 
 }  // namespace
 
-bool hist_mma_takes(const HistLaunch& h) {
-#ifdef PB_DEBUG_BOUNDS
-    return false;   // codes are no index here: the build that checks them keeps to the kernel where they are
-#else
-    static const int forced = [] {   // PACKBOOST_HIST_MMA=0 / 1: nowhere / wherever it can, for comparisons
+// PACKBOOST_HIST_MMA=0 / 1: nowhere / wherever it can (and a line for each launch), for comparisons.
+static int forced_mma() {
+    static const int forced = [] {
         const char* e = getenv("PACKBOOST_HIST_MMA");
         if (getenv("PACKBOOST_HIST_SHAPE")) return 0;   // (a shape of the other kernel is asked for)
         return (e && (e[0] == '0' || e[0] == '1') && e[1] == 0) ? e[0] - '0' : -1;
     }();
+    return forced;
+}
+
+bool hist_mma_takes(const HistLaunch& h) {
+#ifdef PB_DEBUG_BOUNDS
+    return false;   // codes are no index here: the build that checks them keeps to the kernel where they are
+#else
     const bool fused = h.fuse != nullptr, tiled = h.max_era_rows > kTileRowsMax;
-    if (forced == 0 || h.code_bits != 4 || h.max_bins > 8 || h.n_nodes > (fused ? 32 : 64) || fused == tiled) return false;
-    if (forced == 1) return true;
+    if (forced_mma() == 0 || h.code_bits != 4 || h.max_bins > 8 || h.n_nodes > (fused ? 32 : 64) || fused == tiled) return false;
+    if (forced_mma() == 1) return true;
     return mma_pays(fused, h.n_nodes, h.n_feat, h.max_bins, h.rows_pad, h.n_eras);
 #endif
 }
@@ -722,7 +727,6 @@ int launch_hist_mma(const HistLaunch& h, cudaStream_t stream) {
     a.flags = h.debug_flags;
     a.groups = s.groups;
     a.buffers = s.buffers;
-    a.stages = s.stages;
     static const int failed = [] {   // PACKBOOST_WAIT_FAILS=1: launches go the way of a wait that ran out, for the test of it
         const char* e = getenv("PACKBOOST_WAIT_FAILS");
         return (e && e[0] == '1' && e[1] == 0) ? 1 : 0;
@@ -748,6 +752,11 @@ int launch_hist_mma(const HistLaunch& h, cudaStream_t stream) {
     a.blocks = blocks;
     const int64_t shares = (int64_t)blocks * (h.fuse ? h.n_eras : tiles_of(h.rows_pad, kCutRows));
     const dim3 grid((unsigned)(shares < 148 ? shares : 148));
+    if (s.smem > kSharedMost) return fail_arg("histogram of %d nodes does not fit shared memory", h.n_nodes);
+    if (forced_mma() == 1)
+        fprintf(stderr, "hist_mma_kernel<%d,%d,%d,%d> fused=%d nodes=%d features=%d blocks=%d buffers=%d\n", s.thresholds_per_lane, s.batch,
+                (int)mma_groups(h.n_nodes), (int)(s.thresholds_per_lane == 1 && mma_columns(h.n_nodes, true) > 256), a.fuse, h.n_nodes, h.n_feat,
+                blocks, s.buffers);
     prof_begin(h.prof, kProfHist, stream);
     const int rc = s.thresholds_per_lane == 4 ? (s.batch == 4 ? launch_l<4, 4, false, false>(a, grid, s.smem, stream) : launch_l<4, 2, false, false>(a, grid, s.smem, stream))
                    : s.thresholds_per_lane == 2 ? (mma_groups(h.n_nodes) ? launch_l<2, 4, true, false>(a, grid, s.smem, stream) : launch_l<2, 4, false, false>(a, grid, s.smem, stream))
