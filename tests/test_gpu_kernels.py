@@ -294,12 +294,13 @@ print("ok")
 """
 
 
-@pytest.mark.parametrize("cases", [
-    [(8_161, 2, 1, 5, 1, False), (20_001, 270, 1, 5, 1, False), (33_000, 258, 2, 4, 2, True)],    # four thresholds a lane
-    [(17_000, 262, 1, 5, 4, False), (16_500, 20, 1, 2, 3, False), (40_000, 70, 3, 8, 4, True)],
-    [(20_001, 130, 1, 5, 5, False), (17_000, 24, 1, 6, 16, False), (26_000, 9, 2, 3, 9, True)],   # two
-    [(20_001, 65, 1, 5, 17, False), (17_000, 24, 1, 8, 32, False), (30_000, 8, 2, 5, 33, True), (17_000, 70, 1, 7, 64, False)]])  # one
-def test_histogram_exact_on_the_tensor_cores(cases):
+@pytest.mark.parametrize("cases,kernels", [
+    ([(8_161, 2, 1, 5, 1, False), (20_001, 270, 1, 5, 1, False), (33_000, 258, 2, 4, 2, True)], {"2,4,0,0", "4,4,0,0"}),   # two and four thresholds a lane
+    ([(17_000, 262, 1, 5, 4, False), (16_500, 20, 1, 2, 3, False), (40_000, 70, 3, 8, 4, True)], {"4,2,0,0", "2,4,0,0"}),
+    ([(20_001, 130, 1, 5, 5, False), (17_000, 24, 1, 6, 16, False), (26_000, 9, 2, 3, 9, True)], {"2,4,1,0"}),   # two
+    ([(20_001, 65, 1, 5, 17, False), (17_000, 24, 1, 8, 32, False), (30_000, 8, 2, 5, 33, True), (17_000, 70, 1, 7, 64, False)],
+     {"1,4,1,0", "1,4,1,1"})])  # one
+def test_histogram_exact_on_the_tensor_cores(cases, kernels):
     """Exact sums of the contraction for eras of several tiles: every number of thresholds a lane holds, either
     layout of the nodes' columns, more than 256 columns, features past a whole block of lanes, tiles that start
     and end anywhere.  (The switch that takes it at every size is read once per process.)"""
@@ -309,12 +310,15 @@ def test_histogram_exact_on_the_tensor_cores(cases):
     res = subprocess.run([sys.executable, "-c", _MMA_SCRIPT.format(root=root, cases=cases)], env=dict(os.environ, PACKBOOST_HIST_MMA="1"),
                          capture_output=True, text=True, timeout=600)
     assert res.returncode == 0 and res.stdout.strip().endswith("ok"), res.stdout[-2000:] + res.stderr[-4000:]
+    ran = [line for line in res.stderr.splitlines() if line.startswith("hist_mma_kernel<")]
+    assert len(ran) >= len(cases) and {line.split("<")[1].split(">")[0] for line in ran} == kernels, ran
 
 
 @pytest.mark.parametrize("n,f,eras,bins,depth,extra", [
     (6_001, 300, 7, 5, 4, {}), (5_003, 40, 40, 5, 6, {}), (700, 33, 1, 2, 3, {}), (9_000, 70, 200, 8, 6, {}),
     (6_000, 150, 9, 4, 6, dict(direction_weight=0.3)), (6_000, 35, 11, 5, 5, dict(era_alpha=4.0)),
-    (6_000, 35, 5, 7, 5, dict(k_cuts=3, cut_selection="even")), (20_001, 45, 2, 5, 7, {}), (17_000, 200, 1, 6, 7, {})])
+    (6_000, 35, 5, 7, 5, dict(k_cuts=3, cut_selection="even")), (20_001, 45, 2, 5, 7, {}), (17_000, 200, 1, 6, 7, {}),
+    (6_001, 300, 7, 5, 4, dict(workspace=460_000))])
 def test_fit_on_the_tensor_cores_equals_the_one_by_atomics(n, f, eras, bins, depth, extra, tmp_path):
     """Trees, scores and predictions bit for bit: gains made in the flush, every form of the score, eras shorter
     than a step of the rows and longer than a tile."""
@@ -336,14 +340,23 @@ cfg.update(extra)
 b = PackBoost(PackBoostConfig(**cfg)).fit(X, y, era, num_rounds=3)
 np.savez(out, preds=b.train_predictions().view(np.int32), **{k: v.view(np.int32) if v.dtype == np.float32 else v for k, v in b.split_records().items()})
 """
-    got = []
+    got, ran = [], []
+    extra = dict(extra)
+    env = {"PACKBOOST_WORKSPACE_BYTES": str(extra.pop("workspace"))} if "workspace" in extra else {}
     for mma in ("1", "0"):
         path = str(tmp_path / f"{mma}.npz")
         res = subprocess.run([sys.executable, "-c", script, json.dumps([n, f, eras, bins, depth, extra, path])],
-                             env=dict(os.environ, PACKBOOST_HIST_MMA=mma), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                             env=dict(os.environ, PACKBOOST_HIST_MMA=mma, **env), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
                              capture_output=True, text=True)
         assert res.returncode == 0, res.stderr[-2000:]
+        ran.append([dict(kv.split("=") for kv in line.split()[1:]) for line in res.stderr.splitlines() if line.startswith("hist_mma_kernel<")])
         got.append(np.load(path))
+    # the kernel ran at every depth it takes, made the gains where an era is one tile, and never with the switch off
+    one_tile = np.max(np.diff(np.sqrt(np.arange(eras + 1) / eras))) * n < 8_000
+    nodes = {int(r["nodes"]) for r in ran[0]}
+    assert nodes >= {1 << d for d in range(min(depth, 6))} and not ran[1], ran
+    assert {r["fused"] for r in ran[0]} == {"1" if one_tile else "0"}
+    assert (min(int(r["features"]) for r in ran[0]) < f) == bool(env)
     assert len(got[0]["node"]) > 3
     for key in got[0].files:
         np.testing.assert_array_equal(got[0][key], got[1][key], err_msg=key)
@@ -699,6 +712,62 @@ def test_era_walk_with_a_warp_per_node(n, f, eras, bins, depth, extra, tmp_path)
     """The same comparison at the sizes where the walk changes its form: the number of warps, a warp per
     node, nodes in groups, the division table left out."""
     test_era_walk_equals_the_stored_histogram_path(n, f, eras, bins, depth, extra, tmp_path)
+
+
+_WALK_FORMS = [                                          # eras, groups of nodes that are partly filled
+    (4_801, 5, 7, 128, 7, {}), (5_003, 9, 9, 64, 6, {}), (1_900, 4, 37, 17, 6, {}),
+    (2_600, 6, 11, 33, 6, dict(y_scale=1e15)), (3_000, 6, 6, 100, 6, dict(lambda_l2=1e-9)),     # divisions without the table
+    (3_403, 5, 5, 100, 6, dict(k_cuts=9, cut_selection="mass")), (3_403, 5, 5, 64, 6, dict(k_cuts=7, cut_selection="even"))]
+_WALK_FORMS_SCRIPT = r"""
+import json, sys
+import numpy as np
+from packboost_b200 import PackBoost, PackBoostConfig
+out = {}
+for i, (n, f, eras, bins, depth, extra) in enumerate(json.loads(sys.argv[1])):
+    rng = np.random.default_rng(n + f)
+    X = rng.normal(size=(n, f)).astype(np.float32)
+    X[:, ::5] = rng.integers(0, 6, size=X[:, ::5].shape)
+    y = ((X[:, 0] + X[:, 1] * X[:, 2] + 0.3 * rng.normal(size=n)) * extra.pop("y_scale", 1.0)).astype(np.float32)
+    era = np.sort(rng.integers(0, eras, n)).astype(np.int16)
+    cfg = dict(pack_size=2, max_depth=depth, learning_rate=0.2, lambda_l2=1.0, lambda_dro=0.4, min_samples_leaf=5, max_bins=bins, random_state=1)
+    cfg.update(extra)
+    b = PackBoost(PackBoostConfig(**cfg)).fit(X, y, era, num_rounds=2)
+    out[f"preds{i}"] = b.train_predictions().view(np.int32)
+    for k, v in b.split_records().items():
+        out[f"{k}{i}"] = v.view(np.int32) if v.dtype == np.float32 else v
+np.savez(sys.argv[2], **out)
+"""
+
+
+def _walk_forms(path, **env):
+    import json
+    import subprocess
+    import sys
+    res = subprocess.run([sys.executable, "-c", _WALK_FORMS_SCRIPT, json.dumps(_WALK_FORMS), str(path)], env=dict(os.environ, **env),
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr[-2000:]
+    return np.load(path), [line for line in res.stderr.splitlines() if line.startswith("walk_")]
+
+
+@pytest.fixture(scope="module")
+def stored_histogram_fits(tmp_path_factory):
+    return _walk_forms(tmp_path_factory.mktemp("walk") / "stored.npz", PACKBOOST_WALK="0", PACKBOOST_WALK_FORM="0")
+
+
+@pytest.mark.parametrize("form,kernel", list(enumerate(["walk_kernel<{}> warps=16", "walk_kernel<{}> warps=32", "walk_nodes_kernel<{}> warps=16",
+                                                   "walk_nodes_kernel<{}> warps=32"])))
+def test_every_form_of_the_era_walk_equals_the_stored_histogram_path(form, kernel, stored_histogram_fits, tmp_path):
+    """Trees, scores and predictions bit for bit, each form taken at every depth of every fit."""
+    want, none = stored_histogram_fits
+    got, ran = _walk_forms(tmp_path / "walk.npz", PACKBOOST_WALK="1", PACKBOOST_WALK_FORM=str(form))
+    assert not none
+    assert {" ".join(line.split()[:2]) for line in ran} == {kernel.format(bpl) for bpl in (1, 2, 4)}, ran
+    shapes = [dict(kv.split("=") for kv in line.split()[1:]) for line in ran]
+    assert {int(r["nodes"]) for r in shapes} == {1 << d for d in range(7)} and {r["mass"] for r in shapes} == {"0", "1"}
+    assert max(int(r["groups"]) for r in shapes) > 1
+    assert sum(len(want[f"node{i}"]) for i in range(len(_WALK_FORMS))) > 200
+    for key in want.files:
+        np.testing.assert_array_equal(got[key], want[key], err_msg=key)
 
 
 @pytest.mark.parametrize("form", range(4))
