@@ -192,7 +192,7 @@ struct HistLaunch {
     int n_feat;
     const int32_t* gq;
     const uint16_t* slot;
-    int64_t rows_pad;            // entries of gq and slot
+    int64_t n_rows, rows_pad;    // rows; entries of gq and slot
     const int32_t* era_offsets;
     int n_eras;
     int max_bins;

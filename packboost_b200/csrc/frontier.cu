@@ -652,6 +652,7 @@ static HistLaunch hist_launch_of(const pb_train_state* st, int64_t depth, const 
     h.n_feat = 1;
     h.gq = st->gq;
     h.slot = st->slot;
+    h.n_rows = st->n_rows;
     h.rows_pad = rows_padded(st->n_rows);
     h.era_offsets = st->era_offsets;
     h.n_eras = (int)st->n_eras;
@@ -1132,6 +1133,7 @@ extern "C" int pb_hist_build(const pb_train_state* st, const int32_t* feat_rows,
     h.n_feat = (int)n_feat;
     h.gq = st->gq;
     h.slot = st->slot;
+    h.n_rows = st->n_rows;
     h.rows_pad = rows_padded(st->n_rows);
     h.era_offsets = st->era_offsets;
     h.n_eras = (int)st->n_eras;

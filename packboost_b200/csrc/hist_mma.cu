@@ -69,6 +69,8 @@ struct MmaArgs {
     int n_eras;
     int max_bins;
     int blocks;                         // feature blocks
+    Shares shares;                      // of the CTAs
+    int era_rows;                       // work of an era beside its rows
     const int32_t* n_nodes_ptr;
     int n_nodes;                        // upper bound
     int node_stride;
@@ -180,8 +182,9 @@ __host__ __device__ constexpr int mma_columns(int n_nodes, bool groups) {
 }
 __host__ __device__ constexpr int mma_stage_bytes(int features) { return features * kPitch + kBlock * 6; }
 
-// L: thresholds of a lane; KB: K-steps of a batch; GROUPS: layout of the columns; WIDE: more than 256, two products
-template <int L, int KB, bool GROUPS, bool WIDE>
+// L: thresholds of a lane; KB: K-steps of a batch; GROUPS: layout of the columns; WIDE: more than 256, two products;
+// FUSE: the flush makes the gains
+template <int L, int KB, bool GROUPS, bool WIDE, bool FUSE>
 __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(MmaArgs a) {
     constexpr int kMmaThreads = mma_threads(GROUPS, L), kFlushWarps = mma_flush_warps(GROUPS), kBatch = KB, kBatchRows = 32 * KB;
     constexpr int kUnits = kBlock / kBatchRows;              // batches of a block
@@ -235,39 +238,37 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         s_fail = a.failed;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    {
-        uint4* z = reinterpret_cast<uint4*>(s_b);
-        const int n16 = (kSlots * batch_bytes + a.buffers * 3 * tot_plane * 4) / 16;
-        for (int i = threadIdx.x; i < n16; i += kMmaThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    if (a.fuse && threadIdx.x < 8) {
-        int k = -1;
-        for (int i = 0; i < a.fz.n_thr; ++i)
-            if (a.fz.thr_ids[i] == (int)threadIdx.x) k = i;
-        s_kof[threadIdx.x] = k;
-    }
     // The CTAs' shares are ranges of (feature block, row), the block the slowest (totals over the eras gather in a
     // CTA), cut at equal rows, since eras differ in length; with gains in the flush an era is not divided.  (Shares of
     // as many tasks, and tiles counted by the longest era, where this takes, us at one and eight nodes, five bins:
-    // 2 700 000 rows x 238 features, 574 eras that grow to 2.8 times the first 163 and 313, now 131 and 264; 2 600 000
-    // x 238, 200 eras of gamma(4) lengths 170 and 295, now 109 and 213; 1 100 000 x 57, two eras, one a tenth of the
-    // other 41 and 47, now 31 and 38; equal eras 123 and 233, now 123 and 248.)
+    // 2 700 000 rows x 238 features, 574 eras that grow to 2.8 times the first 163 and 313, now 133 and 264; 2 600 000
+    // x 238, 200 eras of gamma(4) lengths 170 and 295, now 109 and 207; 1 100 000 x 57, two eras, one a tenth of the
+    // other 41 and 47, now 31 and 38; equal eras 123 and 238, now 123 and 249.)
     const int E = a.n_eras;
-    const int64_t block_work = (int64_t)a.era_offsets[E] + (a.fuse ? (int64_t)kEraRows * E : 0);
 #pragma unroll 1
     for (int end = 0; end < 2; ++end) {
-        const int64_t work = block_work * a.blocks * (blockIdx.x + end) / gridDim.x;
-        const int fb = (int)(work / block_work);
-        const int64_t at = work - fb * block_work;
+        int fb;
+        const int64_t at = share_begin(a.shares, (int)blockIdx.x + end, fb);
 #pragma unroll 1
-        for (int e = threadIdx.x; e <= E; e += kMmaThreads) {
+        for (int e = kMmaThreads - 1 - threadIdx.x; e <= E; e += kMmaThreads) {   // (the first warp has other things to do)
             int row = 0;
-            if (fb == a.blocks ? e == 0 : a.fuse ? cut_in_era<true>(a.era_offsets, E, at, e, row) : cut_in_era<false>(a.era_offsets, E, at, e, row)) {
+            if (fb == a.blocks ? e == 0 : FUSE ? cut_in_era<true>(a.era_offsets, E, at, a.era_rows, e, row) : cut_in_era<false>(a.era_offsets, E, at, 0, e, row)) {
                 s_cut[end][0] = e == E ? fb + 1 : fb;
                 s_cut[end][1] = e == E ? 0 : e;
                 s_cut[end][2] = e == E ? 0 : row;
             }
         }
+    }
+    {
+        uint4* z = reinterpret_cast<uint4*>(s_b);
+        const int n16 = (kSlots * batch_bytes + a.buffers * 3 * tot_plane * 4) / 16;
+        for (int i = threadIdx.x; i < n16; i += kMmaThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (FUSE && threadIdx.x < 8) {
+        int k = -1;
+        for (int i = 0; i < a.fz.n_thr; ++i)
+            if (a.fz.thr_ids[i] == (int)threadIdx.x) k = i;
+        s_kof[threadIdx.x] = k;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
     const uint32_t a_col = tmem + (uint32_t)(a.buffers * L * N_max);
 
     // Every role goes through the same tasks.
-    auto next_task = [&](RowTask& x) { return next_row_task(a.era_offsets, E, a.fuse != 0, s_cut[1], kMmaTileRows, x); };
+    auto next_task = [&](RowTask& x) { return next_row_task(a.era_offsets, E, FUSE, s_cut[1], kMmaTileRows, x); };
     RowTask x;
     x.fb = s_cut[0][0];
     x.next = s_cut[0][1];
@@ -347,14 +348,15 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
         constexpr int J = GROUPS ? 8 : 1;            // columns between the digits of a node
         const int quarter = warp & 3, fg = (warp - kFlushWarp0) >> 2, row = quarter * 32 + lane, fl = row / G, g = row - fl * G;
         const HistFuse& z = a.fz;
-        const float inv_scale = a.fuse ? *z.inv_scale_ptr : 0.f;
+        const float inv_scale = FUSE ? *z.inv_scale_ptr : 0.f;
         const int K = z.n_thr, lanes_total = a.blocks * FC;
         int buf = 0;
         uint32_t phase = 0u;
-        for (bool first = true; next_task(x); first = false) {
+        while (next_task(x)) {
             const int era = x.era, f = x.fb * FC + fl;
             const bool mine = f < a.n_feat, empty_tile = x.b0 == x.b1;
-            const bool fresh = first || era == 0, last = x.next == E || (x.fb == s_cut[1][0] && x.next == s_cut[1][1]);   // of a feature block here
+            // the first and the last of a feature block in this CTA (where the flush makes the gains)
+            const bool fresh = era == 0 || (era == s_cut[0][1] && x.fb == s_cut[0][0]), last = x.next == E || (x.next == s_cut[1][1] && x.fb == s_cut[1][0]);
             warp_wait<true>(acc_full + buf, phase, &s_fail);
             warp_wait<true>(tot_full + buf, phase, &s_fail);
             uint32_t* tot = s_tot + buf * 3 * tot_plane;
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                 if (lane == 0) {
                     s_tc[n] = tc;
                     s_tgq[n] = tg;
-                    if (a.fuse) {
+                    if (FUSE) {
                         const EraTotals e = era_totals(tc, tg, inv_scale, z.lambda_l2, z.era_alpha);
                         s_era[n] = make_float4(e.tg, e.th, e.parent, e.w_era);
                     }
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(mma_threads(GROUPS, L), 1) hist_mma_kernel(Mma
                     }
                     const uint32_t tc = s_tc[n];
                     const long long tgq = s_tgq[n];
-                    if (a.fuse) {
+                    if (FUSE) {
                         if (!mine) continue;
                         const float4 e = s_era[n];
                         const size_t at = (((size_t)f * a.n_eras + era) * a.node_stride + n) * K;
@@ -677,8 +679,13 @@ MmaShape mma_shape(int n_nodes, int n_feat, int max_bins, bool fused) {
 
 template <int L, int KB, bool GROUPS, bool WIDE>
 int launch_l(const MmaArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    PB_TRY(allow_shared(hist_mma_kernel<L, KB, GROUPS, WIDE>, smem));
-    hist_mma_kernel<L, KB, GROUPS, WIDE><<<grid, mma_threads(GROUPS, L), smem, stream>>>(a);
+    if (a.fuse && !WIDE) {
+        PB_TRY(allow_shared(hist_mma_kernel<L, KB, GROUPS, false, true>, smem));
+        hist_mma_kernel<L, KB, GROUPS, false, true><<<grid, mma_threads(GROUPS, L), smem, stream>>>(a);
+    } else {
+        PB_TRY(allow_shared(hist_mma_kernel<L, KB, GROUPS, WIDE, false>, smem));
+        hist_mma_kernel<L, KB, GROUPS, WIDE, false><<<grid, mma_threads(GROUPS, L), smem, stream>>>(a);
+    }
     return PB_OK;
 }
 
@@ -701,7 +708,7 @@ bool hist_mma_takes(const HistLaunch& h) {
     const bool fused = h.fuse != nullptr, tiled = h.max_era_rows > kTileRowsMax;
     if (forced_mma() == 0 || h.code_bits != 4 || h.max_bins > 8 || h.n_nodes > (fused ? 32 : 64) || fused == tiled) return false;
     if (forced_mma() == 1) return true;
-    return mma_pays(fused, h.n_nodes, h.n_feat, h.max_bins, h.rows_pad, h.n_eras);
+    return mma_pays(fused, h.n_nodes, h.n_feat, h.max_bins, h.n_rows, h.n_eras);
 #endif
 }
 
@@ -750,8 +757,14 @@ int launch_hist_mma(const HistLaunch& h, cudaStream_t stream) {
         }
     }
     a.blocks = blocks;
-    const int64_t shares = (int64_t)blocks * (h.fuse ? h.n_eras : tiles_of(h.rows_pad, kCutRows));
-    const dim3 grid((unsigned)(shares < 148 ? shares : 148));
+    // An era costs its flush too, more than its rows where it is short: about 1 200 to 3 300 rows' time by the number of
+    // nodes, most of it beside the rows of the next one.
+    a.era_rows = !h.fuse ? 0 : h.n_nodes > 8 || h.n_rows < (int64_t)1500 * h.n_eras ? 2048 : 512;
+    const int64_t most = (int64_t)blocks * (h.fuse ? h.n_eras : tiles_of(h.n_rows, kCutRows));
+    // (A CTA with rows of two feature blocks adds two tiles to a stored histogram: 160 000 rows x 78 features, 64 nodes:
+    // 51 us, 36 with blocks of their own.)
+    a.shares = shares_of(blocks, h.n_rows + (int64_t)a.era_rows * h.n_eras, (int)(most < 148 ? most : 148), !h.fuse);
+    const dim3 grid((unsigned)a.shares.count);
     if (s.smem > kSharedMost) return fail_arg("histogram of %d nodes does not fit shared memory", h.n_nodes);
     if (forced_mma() == 1)
         fprintf(stderr, "hist_mma_kernel<%d,%d,%d,%d> fused=%d nodes=%d features=%d blocks=%d buffers=%d\n", s.thresholds_per_lane, s.batch,

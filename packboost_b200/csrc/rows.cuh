@@ -22,17 +22,50 @@ PB_ROWS_FN void tile_range(int era_begin, int era_end, int index, int tile, int&
     r1 = era_end - r0 > tile ? r0 + tile : era_end;
 }
 
-// Where a share of the work of a feature block ends.  `at` counts rows (WHOLE: and kEraRows more for each era, which
+// Shares of the rows of all feature blocks, the block the slowest.
+struct Shares {
+    int64_t block_work, share;           // work of a block, of a share (rounded down)
+    int blocks, more;                    // (blocks;) shares with one more, of a block's where it has its own
+    int per_block;                       // shares of a block, 0: a share may begin in one block and end in another
+    int count;
+};
+
+// At most `count` shares.  `own`: none of two blocks, where that leaves four of `count` out at most.
+inline Shares shares_of(int blocks, int64_t block_work, int count, bool own) {
+    Shares s;
+    s.block_work = block_work;
+    s.blocks = blocks;
+    s.per_block = own && count / blocks * blocks + 4 >= count ? count / blocks : 0;
+    s.count = s.per_block ? s.per_block * blocks : count;
+    const int64_t work = block_work * (s.per_block ? 1 : blocks);
+    const int parts = s.per_block ? s.per_block : count;
+    s.share = work / parts;
+    s.more = (int)(work % parts);
+    return s;
+}
+
+// Where share i begins: the feature block, and the work of it that lies before.  (A few subtractions: a 64-bit
+// division by every warp is 2 us a launch.)
+PB_ROWS_FN int64_t share_begin(const Shares& s, int i, int& fb) {
+    fb = s.per_block ? i / s.per_block : 0;
+    i -= fb * s.per_block;
+    int64_t at = s.share * i + (i < s.more ? i : s.more);
+    if (!s.per_block)
+        for (; at >= s.block_work; at -= s.block_work) ++fb;
+    return at;
+}
+
+// Where a share of the work of a feature block ends.  `at` counts rows (WHOLE: and era_rows more for each era, which
 // stand for its flush).  WHOLE: between two eras, at the nearest place, so that a share differs from its part of the
 // work by half an era at each end at most; otherwise at any multiple of kCutRows.  True for exactly one e of
 // [0, n_eras], the era in which the rows after the cut begin, at `row`; n_eras: none is left (WHOLE alone).
-constexpr int kEraRows = 512, kCutRows = 512;
+constexpr int kCutRows = 512;
 template <bool WHOLE>
-PB_ROWS_FN bool cut_in_era(const int* offsets, int n_eras, int64_t at, int e, int& row) {
+PB_ROWS_FN bool cut_in_era(const int* offsets, int n_eras, int64_t at, int era_rows, int e, int& row) {
     row = WHOLE ? offsets[e] : (int)(at / kCutRows * kCutRows);
     if (!WHOLE) return e < n_eras && offsets[e] <= row && row < offsets[e + 1];
     // twice the work before the middle of an era
-    auto middle = [&](int i) { return (int64_t)offsets[i] + offsets[i + 1] + (int64_t)kEraRows * (2 * i + 1); };
+    auto middle = [&](int i) { return (int64_t)offsets[i] + offsets[i + 1] + (int64_t)era_rows * (2 * i + 1); };
     return (e == 0 || middle(e - 1) < 2 * at) && (e == n_eras || middle(e) >= 2 * at);
 }
 

@@ -206,18 +206,19 @@ _SHARES = """#include "rows.cuh"
 #include <cstdio>
 #include <vector>
 using namespace pb;
-int main() {                             // eras, feature blocks, shares, whole, tile, offsets -> share, block, era, r0, r1, b0, b1
+int main() {                             // eras, feature blocks, shares, whole, tile, offsets -> shares; share, block, era, r0, r1, b0, b1
     int E, blocks, grid, whole, tile;
     while (std::scanf("%d %d %d %d %d", &E, &blocks, &grid, &whole, &tile) == 5) {
         std::vector<int> off(E + 1);
         for (int& o : off) std::scanf("%d", &o);
-        const int64_t work = off[E] + (whole ? (int64_t)kEraRows * E : 0);
-        auto cut = [&](int64_t share, int* c) {
-            const int64_t at = work * blocks * share / grid;
-            const int fb = (int)(at / work);
-            int hits = 0, row = 0;
+        const int64_t work = off[E] + (whole ? (int64_t)512 * E : 0);
+        const Shares s = shares_of(blocks, work, grid, !whole);
+        std::printf("%d\\n", s.count);
+        auto cut = [&](int share, int* c) {
+            int fb, hits = 0, row = 0;
+            const int64_t at = share_begin(s, share, fb);
             for (int e = 0; e <= E; ++e)
-                if (fb == blocks ? e == 0 : whole ? cut_in_era<true>(off.data(), E, at - fb * work, e, row) : cut_in_era<false>(off.data(), E, at - fb * work, e, row)) {
+                if (fb == blocks ? e == 0 : whole ? cut_in_era<true>(off.data(), E, at, 512, e, row) : cut_in_era<false>(off.data(), E, at, 0, e, row)) {
                     ++hits;
                     c[0] = e == E ? fb + 1 : fb;
                     c[1] = e == E ? 0 : e;
@@ -225,7 +226,7 @@ int main() {                             // eras, feature blocks, shares, whole,
                 }
             return hits == 1;
         };
-        for (int i = 0; i < grid; ++i) {
+        for (int i = 0; i < s.count; ++i) {
             int from[3], to[3];
             if (!cut(i, from) || !cut(i + 1, to)) return 1;
             RowTask x{from[0], 0, 0, from[2], 0, 0, from[1]};
@@ -258,7 +259,10 @@ def test_shares_of_rows_are_even_and_complete(tmp_path):
     out = subprocess.run([str(tmp_path / "shares")], input=text, capture_output=True, text=True, check=True).stdout
     for (n, blocks, grid, whole), part in zip(asked, out.split("-1\n")):
         off = np.concatenate([[0], np.cumsum(n)]).astype(np.int64)
-        t = np.array([line.split() for line in part.splitlines()], dtype=np.int64).reshape(-1, 7)
+        head, *lines = part.splitlines()
+        shares = int(head)
+        assert grid - 4 * (not whole) <= shares <= grid
+        t = np.array([line.split() for line in lines], dtype=np.int64).reshape(-1, 7)
         share, fb, era, r0, r1, b0, b1 = t.T
         assert ((off[era] <= r0) & (r0 <= r1) & (r1 <= off[era + 1]) & (b0 == r0 // 512) & (b1 == np.where(r0 < r1, -(-r1 // 512), b0))).all()
         assert (np.diff(share) >= 0).all()
@@ -270,8 +274,10 @@ def test_shares_of_rows_are_even_and_complete(tmp_path):
             place = fb * off[-1] + r0
             assert (place[1:] == (fb * off[-1] + r1)[:-1]).all() and place[0] == 0 and fb[-1] * off[-1] + r1[-1] == blocks * off[-1]
             most = 512
+            if shares % blocks == 0:                # a share has rows of one block
+                assert all(len(set(fb[share == i])) == 1 for i in set(share.tolist()))
         loads = np.bincount(share, weights=(r1 - r0) + 512 * whole, minlength=grid)
-        assert loads.max() <= blocks * (off[-1] + 512 * whole * len(n)) / grid + most, (n[:5], blocks, grid, whole)
+        assert loads.max() <= blocks * (off[-1] + 512 * whole * len(n)) / shares + most, (n[:5], blocks, grid, whole)
 
 
 _RULE = """#include "hist_rule.h"
