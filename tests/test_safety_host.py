@@ -300,14 +300,20 @@ def test_few_bins_take_the_kernel_that_measured_faster(tmp_path):
     (tmp_path / "rule.cpp").write_text(_RULE)
     subprocess.run(["g++", "-std=c++17", "-I", csrc, str(tmp_path / "rule.cpp"), "-o", str(tmp_path / "rule")], check=True)
     measured = [      # gains in the flush, rows, features, eras, bins, (nodes, contraction, atomics) ...
-        (1, 2_700_000, 238, 574, 2, [(1, 122, 179), (2, 125, 182), (4, 156, 198), (8, 248, 227), (32, 589, 379)]),
-        (1, 2_700_000, 238, 574, 5, [(1, 123, 170), (2, 129, 171), (4, 160, 187), (8, 248, 229), (16, 289, 256), (32, 572, 393)]),
+        (1, 2_700_000, 238, 574, 2, [(1, 122, 180), (2, 129, 182), (4, 154, 199), (8, 244, 227), (32, 577, 381)]),
+        (1, 2_700_000, 238, 574, 4, [(1, 123, 187), (2, 129, 190), (4, 158, 211)]),
+        (1, 2_700_000, 238, 574, 5, [(1, 123, 171), (2, 129, 172), (4, 158, 188), (8, 248, 231), (16, 323, 256), (32, 553, 393)]),
         (1, 2_700_000, 238, 574, 6, [(1, 226, 192), (2, 232, 199), (4, 291, 240)]),
-        (1, 1_000_000, 238, 574, 3, [(1, 69, 129), (2, 86, 133), (16, 278, 223), (32, 567, 371)]),
-        (1, 1_000_000, 238, 574, 5, [(1, 68, 119), (2, 88, 121), (8, 180, 131), (16, 269, 159), (32, 537, 242)]),
-        (1, 1_500_000, 200, 300, 5, [(1, 86, 136), (2, 90, 137), (8, 156, 138), (16, 176, 154), (32, 296, 211)]),
-        (1, 700_000, 100, 300, 5, [(1, 37, 57), (2, 39, 57), (8, 66, 53), (16, 94, 61), (32, 167, 96)]),
-        (1, 150_000, 70, 150, 5, [(1, 24, 21), (4, 31, 22), (8, 35, 22), (16, 49, 28), (32, 72, 36)]),
+        (1, 1_000_000, 238, 574, 3, [(1, 68, 140), (2, 83, 132), (4, 109, 149), (16, 251, 225), (32, 517, 372)]),
+        (1, 1_000_000, 238, 574, 5, [(1, 67, 118), (2, 89, 122), (8, 183, 130), (16, 250, 159), (32, 494, 243)]),
+        (1, 1_500_000, 200, 300, 5, [(1, 85, 136), (2, 90, 137), (8, 154, 139), (16, 187, 154), (32, 286, 211)]),
+        (1, 253_890, 218, 308, 4, [(1, 33, 66), (2, 39, 58), (4, 54, 72), (16, 122, 92), (32, 230, 125)]),
+        (1, 253_890, 218, 308, 5, [(4, 55, 39), (8, 75, 49), (16, 116, 75)]),
+        (1, 250_000, 218, 1000, 2, [(2, 74, 66), (4, 111, 88), (8, 176, 138), (16, 292, 234)]),
+        (1, 250_000, 218, 1000, 5, [(1, 54, 49), (2, 76, 51), (4, 117, 64)]),
+        (1, 600_000, 300, 2000, 4, [(1, 142, 420), (8, 457, 343), (16, 806, 512)]),
+        (1, 700_000, 100, 300, 5, [(1, 37, 59), (2, 39, 57), (8, 68, 53), (16, 89, 62), (32, 160, 94)]),
+        (1, 150_000, 70, 150, 5, [(2, 25, 22), (4, 31, 22), (8, 35, 24), (16, 50, 29), (32, 71, 36)]),
         (1, 300_000, 60, 60, 5, [(1, 25, 20), (2, 27, 18), (4, 31, 20), (8, 31, 27), (16, 37, 27), (32, 39, 29)]),
         (0, 1_300_000, 57, 1, 2, [(1, 33, 48), (32, 64, 53)]),
         (0, 1_300_000, 57, 1, 5, [(1, 35, 47), (32, 66, 74)]),
@@ -320,6 +326,10 @@ def test_few_bins_take_the_kernel_that_measured_faster(tmp_path):
         (0, 1_000_000, 100, 20, 5, [(1, 33, 56), (2, 35, 55), (4, 41, 57), (32, 93, 78)]),
         (0, 300_000, 40, 1, 5, [(1, 19, 35), (2, 23, 35), (16, 34, 29), (64, 39, 29)]),
         (0, 300_000, 40, 1, 8, [(64, 61, 43)]),
+        (0, 248_795, 33, 1, 5, [(1, 18, 27), (2, 21, 30), (4, 23, 21), (8, 24, 21)]),
+        (0, 461_197, 55, 1, 5, [(1, 20, 33), (2, 26, 35)]),
+        (0, 160_630, 42, 1, 5, [(1, 17, 27), (2, 20, 18), (4, 21, 18), (8, 23, 20), (16, 27, 23), (64, 33, 24)]),
+        (0, 1_000_000, 60, 1, 6, [(1, 33, 46), (32, 86, 78), (64, 111, 92)]),
         (0, 100_000, 30, 1, 3, [(1, 15, 25), (8, 25, 16), (16, 27, 16), (32, 25, 14), (64, 35, 16)]),
         (0, 100_000, 30, 1, 5, [(4, 22, 20), (8, 20, 18), (32, 25, 18), (64, 31, 20)]),
         (0, 30_000, 100, 3, 5, [(1, 16, 11), (2, 16, 10), (4, 18, 12), (8, 18, 12), (16, 23, 12), (32, 28, 14)]),
