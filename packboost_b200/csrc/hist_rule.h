@@ -57,7 +57,8 @@ inline bool mma_pays(bool fused, int n_nodes, int n_feat, int max_bins, int64_t 
     if (n_nodes <= 2) return work >= (max_bins > 5 ? 10000000 : n_nodes == 1 ? 3000000 : 8000000);
     const bool one_block = n_feat <= 64 && work >= 13000000;   // (at two thresholds a lane, up to five bins)
     const bool many = work >= 200000000;
-    if (n_nodes <= 4) return one_block || (max_bins <= 5 ? work >= 13000000 : max_bins >= 7 && many);
+    // (more than five bins: but where the atomics have a feature on every lane)
+    if (n_nodes <= 4) return work >= 13000000 && (max_bins <= 5 || n_feat * 100 < (n_feat + 31) / 32 * 32 * 95);
     if (n_nodes <= 16) return one_block || (max_bins <= 5 && many);
     if (max_bins < 3 || max_bins > 5) return false;
     return one_block || (n_nodes <= 32 && max_bins > 3 && work >= 50000000 && n_feat * 100 >= blocks * features * 85);
