@@ -749,10 +749,11 @@ static double two_step_estimate_us(const pb_train_state* st, int64_t depth, int6
 // features.  So neither is the faster one everywhere (128 bins, depth 6, a round's histogram and score;
 // walk / other path): 500 000 rows x 200 features, 100 eras 2.2 / 3.8 ms; 131 072 x 200, 574 eras 6.3 / 20.8;
 // 262 144 x 64, 20 eras 0.73 / 0.78; 1 000 000 x 64, 100 eras 2.9 / 2.4; 4 000 000 x 32, 20 eras 10.5 / 2.4.
-// The estimates decide by depth: over the 9 000 depths that they were first fitted to that took 3 % more time
-// than the better path each time, where the walk everywhere took 50 % more.  Where they come within a tenth at
-// sixteen nodes or more it is the walk, whose estimate is the safer one in deep frontiers of few rows; above,
-// the other path's is the one too high (262 144 x 16, 100 eras, one node: 73 us for 44, the walk's 77 for 68).
+// The estimates decide by depth.  (With their first constants, since replaced, that took 3 % more time than the
+// better path each time over the 9 000 depths they were fitted to, the walk everywhere 50 % more; the present ones
+// were compared at the sizes above.)  Where they come within a tenth at sixteen nodes or more it is the walk,
+// whose estimate is the safer one in deep frontiers of few rows; above, the other path's is too high where it was
+// looked at (one shape: 262 144 x 16, 100 eras, one node 73 us for 44, the walk's 77 for 68).
 // PACKBOOST_WALK=0 / 1 takes one path everywhere, for comparisons.
 struct DepthPath {
     size_t cand_bytes;   // of the candidate table, at the start of the workspace

@@ -22,8 +22,8 @@
 //
 // Bound: with few nodes the rows (two shared-memory atomics per row and feature take 3.5 wavefronts each
 // with 128 bins, 66 % of the shared-memory pipe; without them, or with rows from the L1, they still take 85 %
-// of the time: no one thing), with many the gains (issue slots).
-// 500 000 rows x 256 features, 100 eras, 128 bins, by depth: 0.22, 0.24, 0.29, 0.38, 0.41, 0.63 ms, 2.2 ms a
+// of the time: no one thing), with many the gains (issue slots 60 to 64 %).
+// 500 000 rows x 256 features, 100 eras, 128 bins, by depth: 0.22, 0.24, 0.29, 0.39, 0.41, 0.62 ms, 2.2 ms a
 // round (one form for all depths: 0.50 and 1.01 ms at the last two, 2.7 ms; histogram, gain and chain kernels:
 // 4.6); 200 000 x 100, 40 eras, depth 10: 3.0 ms a round (4.8 with the one form), of which 512 nodes 1.23 (2.07).
 //
