@@ -42,7 +42,6 @@ namespace pb {
 
 namespace {
 
-constexpr int kWalkWarpsMax = 32;
 constexpr int kWalkInv = 4096;           // longest table of era reciprocals
 
 // Four codes, each within the cells of its node (32 BPL of them) whatever the byte: one that is no bin would else be
